@@ -1687,42 +1687,47 @@ extern "C" int sfd_get_gradient(sfd_plan *p, int transform, float *g0, float *g1
 {
     if (!p) return SFD_ERR_ARG;
     if (!p->a.grad[0]) return fail(p, SFD_ERR_STATE, "no gradient has been accumulated");
-    int64_t n = (int64_t)p->g.nz * p->g.ny * p->g.nx;
-    std::vector<double> gr(n), gM(n), gmu(n);
-    if (int rc_ = fetch_sum(p, p->a.grad[GRHO], gr.data(), n)) return rc_;
-    if (int rc_ = fetch_sum(p, p->a.grad[GM], gM.data(), n)) return rc_;
-    if (int rc_ = fetch_sum(p, p->a.grad[GMU], gmu.data(), n)) return rc_;
-    // the DFT gradient is already in the param_type's basis (no transf_grad)
-    if (!transform || p->cfg.back_prop_type == 2) {
-        for (int64_t i = 0; i < n; i++) {
-            if (g0) g0[i] = (float)gM[i];
-            if (g1) g1[i] = (float)gmu[i];
-            if (g2) g2[i] = (float)gr[i];
-        }
-        return SFD_OK;
+    const bool chain = transform && p->cfg.back_prop_type != 2;
+    if (chain && !p->model_set) return fail(p, SFD_ERR_STATE, "no model");
+    GradOut o;
+    memset(&o, 0, sizeof o);
+    o.sum[0] = p->a.grad[GM];
+    o.sum[1] = p->a.grad[GMU];
+    o.sum[2] = p->a.grad[GRHO];
+    o.ncopy = p->batch;
+    o.n = (int64_t)p->g.nz * p->g.ny * p->g.nx;
+    o.dt = p->cfg.dt;
+    o.dh = p->cfg.dh;
+    // src/calc_grad.c:975-1107; the DFT gradient is already in the
+    // param_type's basis (no transf_grad)
+    o.par_type = -1;
+    if (chain) {
+        if (int rc_ = prepare_adjoint_params(p)) return rc_;
+        o.par_type = p->cfg.param_type;
+        o.rho = p->padj[PRHO];
+        o.M = p->padj[PM];
+        o.mu = p->padj[PMU];
     }
-    // src/calc_grad.c:975-1107
-    const double dt = p->cfg.dt, dh = p->cfg.dh;
-    const int pt = p->cfg.param_type;
-    for (int64_t i = 0; i < n; i++) {
-        double rho = 1.0 / p->hp[PRHO][i] * dt / dh;
-        double M = p->hp[PM][i] * dh / dt, mu = p->hp[PMU][i] * dh / dt;
-        double grho = gr[i] / dt, gm = gM[i] / dt, gs = gmu[i] / dt;
-        if (pt == 0 || pt == 2) {
-            grho += M / rho * gm;
-            if (mu > 0) grho += mu / rho * gs;
-        }
-        if (pt == 0) {
-            gm = 2.0 * std::sqrt(rho * M) * gm;
-            gs = 2.0 * std::sqrt(rho * mu) * gs;
-        } else if (pt == 2) {
-            gm = 2.0 * std::sqrt(M / rho) * gm;
-            gs = 2.0 * std::sqrt(mu / rho) * gs;
-        }
-        if (g0) g0[i] = (float)gm;
-        if (g1) g1[i] = (float)gs;
-        if (g2) g2[i] = (float)grho;
+    // the result passes through a bounded staging area: a plan whose stores
+    // fill the device still returns its gradient
+    const int64_t chunk = std::min<int64_t>(o.n, 8 << 20);
+    cudaError_t e;
+    float *stage = (float *)dalloc_raw(p, sizeof(float) * 3 * chunk, &e);
+    if (!stage) return fail(p, SFD_ERR_MEMORY, "gradient staging does not fit in device memory");
+    float *const host[3] = {g0, g1, g2};
+    for (o.first = 0; o.first < o.n && e == cudaSuccess; o.first += chunk) {
+        o.count = std::min(chunk, o.n - o.first);
+        for (int k = 0; k < 3; k++) o.out[k] = stage + k * chunk;
+        launch_gradient_out(o, p->stream);
+        e = cudaGetLastError();
+        for (int k = 0; k < 3 && e == cudaSuccess; k++)
+            if (host[k])
+                e = cudaMemcpyAsync(host[k] + o.first, o.out[k], sizeof(float) * o.count, cudaMemcpyDeviceToHost,
+                                    p->stream);
     }
+    dfree(p, stage, sizeof(float) * 3 * chunk);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
+    if (e != cudaSuccess) return fail(p, SFD_ERR_CUDA, std::string("gradient: ") + cudaGetErrorString(e));
     return SFD_OK;
 }
 

@@ -78,6 +78,18 @@ struct PackSet {
 };
 void launch_pack(const PackSet &ps, int prec, bool unpack, cudaStream_t st, bool half_src = false);
 
+// gradient sums -> gradient of the parameters (sfd_gradient.cu)
+struct GradOut {
+    const double *sum[3];   // M, mu, rho: [ncopy][n]
+    int ncopy;
+    int64_t n, first, count;   // cells of a copy; the range of this launch
+    int par_type;           // param_type of the chain rule, -1: the sums as they are
+    const float *rho, *M, *mu;
+    double dt, dh;
+    float *out[3];          // [count] each: M, mu, rho or their param_type counterparts
+};
+void launch_gradient_out(const GradOut &o, cudaStream_t st);
+
 // DFT gradient (sfd_dft.cu)
 struct DftSet {             // variables transformed by one accumulation launch
     const float *v[NW + NR];

@@ -151,9 +151,12 @@ oom:
 }
 
 // host-side mapping of a shot's sources and receivers, uploaded to the device
+// (inside: whether every point that is not dropped lies on a physical cell
+// along z, none in the padding above or below)
 int upload_shots(sfd_plan *p, int nshot, const sfd_shot *shots, int mask, PointSet &S, PointSet &R,
-                 cudaStream_t st)
+                 cudaStream_t st, bool *inside = nullptr)
 {
+    bool in = true;
     const Grid &g = p->g;
     const int F = g.F, NT = p->cfg.nt;
     int nsrc = 0, nrec = 0;
@@ -176,6 +179,7 @@ int upload_shots(sfd_plan *p, int nshot, const sfd_shot *shots, int mask, PointS
             if (j < 0 || j >= g.NY || k < 0 || k >= g.NZ)
                 return fail(p, SFD_ERR_ARG, "source position outside the padded grid");
             scell[s] = base + ((int64_t)i * g.NY + j) * g.NZ + k;
+            in = in && k >= F && k < g.NZ - F;
             skz[s] = k;
             int type = (int)shot->src_pos[5 * q + 4];
             snt[s] = source_targets(g.nd, mask, type, &sfield[3 * s], &sdiv[3 * s]);
@@ -188,8 +192,10 @@ int upload_shots(sfd_plan *p, int nshot, const sfd_shot *shots, int mask, PointS
             if (j < 0 || j >= g.NY || k < 0 || k >= g.NZ)
                 return fail(p, SFD_ERR_ARG, "receiver position outside the padded grid");
             rcell[r] = base + ((int64_t)i * g.NY + j) * g.NZ + k;
+            in = in && k >= F && k < g.NZ - F;
         }
     }
+    if (inside) *inside = in;
     {
         if (nsrc) {
             CKC(cudaMemcpyAsync(p->d_src_cell, scell.data(), sizeof(int64_t) * nsrc, cudaMemcpyHostToDevice, st));
@@ -277,9 +283,14 @@ int alloc_model(sfd_plan *p)
     }
     p->f.taper = cst + 3 * NC * nc;
     // block counter of the fused steps, instability flag
-    p->d_ticket = (int *)dalloc(p, 2 * sizeof(int), &e);
+    p->d_ticket = (int *)dalloc(p, 3 * sizeof(int), &e);
     if (e) return fail(p, SFD_ERR_MEMORY, "step counter allocation failed");
     p->d_unstable = p->d_ticket + 1;
+    p->d_words = nullptr;
+    if (const int64_t wb = resident2d_bytes(g, p->batch)) {
+        p->d_words = (unsigned long long *)dalloc(p, (size_t)wb, &e);
+        if (e) return fail(p, SFD_ERR_MEMORY, "step exchange allocation failed");
+    }
     // fused 3D step: ticket counter and per-unit flags (single-shot plans)
     const FusedShape fsh = fused_shape(g);
     p->d_fsync = nullptr;
@@ -449,18 +460,20 @@ const float *check_field(float *const *w)
 int arm_unstable(sfd_plan *p, cudaStream_t st)
 {
     CKC(cudaMemsetAsync(p->d_unstable, 0x7f, sizeof(int), st));
+    CKC(cudaMemsetAsync(p->d_unstable + 1, 0, sizeof(int), st));
     return SFD_OK;
 }
 
 // call after the loop's stream has been synchronised
 int take_unstable(sfd_plan *p, cudaStream_t st, const char *what)
 {
-    int v = 0;
-    CKC(cudaMemcpyAsync(&v, p->d_unstable, sizeof(int), cudaMemcpyDeviceToHost, st));
+    int v[2] = {0, 0};
+    CKC(cudaMemcpyAsync(v, p->d_unstable, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
     CKC(cudaStreamSynchronize(st));
-    if (v == 0x7f7f7f7f) return SFD_OK;
+    if (v[1]) return fail(p, SFD_ERR_CUDA, "a resident 2D step did not see its neighbours' edges within its time bound");
+    if (v[0] == 0x7f7f7f7f) return SFD_OK;
     char buf[200];
-    snprintf(buf, sizeof buf, "Simulation has become unstable: non-finite %s wave field at step %d", what, v);
+    snprintf(buf, sizeof buf, "Simulation has become unstable: non-finite %s wave field at step %d", what, v[0]);
     return fail(p, SFD_ERR_UNSTABLE, buf);
 }
 
@@ -1047,6 +1060,7 @@ extern "C" int sfd_plan_create(const sfd_config *cfg, sfd_plan **out)
     p->d_surf_q = nullptr;
     p->d_ticket = nullptr;
     p->d_unstable = nullptr;
+    p->d_words = nullptr;
     p->d_fsync = nullptr;
     p->dev_bytes = 0;
     p->batch = std::max(1, c.batch);
@@ -1101,7 +1115,8 @@ extern "C" int sfd_footprint(const sfd_config *cfg, int gradient, int nsrc, int6
     // ensure_shot_buffers: source maps and signatures, receiver maps, seismograms and residuals
     const int64_t cs = std::max<int64_t>(nsrc, 16), cr = std::max<int64_t>(nrec_sel, 16);
     b += cs * (8 + 4 + 12 + 4 + 12 + 4 * nt) + cr * (8 + 8 * nt);
-    b += 2 * sizeof(int);   // fused-step block counter, instability flag
+    b += 3 * sizeof(int);   // fused-step block counter, instability flag, resident-step status
+    b += resident2d_bytes(g, (int)B);
     {
         const FusedShape fsh = fused_shape(g);
         if (B == 1 && fsh.units) b += 4 * (1 + fsh.units);   // fused 3D step tickets and flags
@@ -1283,7 +1298,8 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
     unsigned omask = outmask_of(outsel, g.nd, &nsel);
     if ((rc = ensure_shot_buffers(p, sb.nsrc, sb.nrec, nsel))) return rc;
     PointSet S, R;
-    if ((rc = upload_shots(p, nshot, shots, mask, S, R, st))) return rc;
+    bool points_inside;
+    if ((rc = upload_shots(p, nshot, shots, mask, S, R, st, &points_inside))) return rc;
     if ((rc = zero_forward_state(p, st))) return rc;
     // a batch without receivers has no seismogram buffer (none is allocated
     // for zero traces): no copy of zero bytes goes to a null pointer
@@ -1384,6 +1400,11 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
     const FusedShape fsh = fused_shape(g);
     const bool fuse3d = g.nd == 3 && nshot == 1 && p->d_fsync && fsh.units && !save_boundaries && !dft && !mv.n;
     const bool bnd_shells = save_boundaries && !dft && !ckpt;
+    // 2D P-SV runs whose wave fields fit on chip: the time loop in segments,
+    // one cooperative launch each (sfd_resident2d.cu)
+    const Res2d rs = resident2d_shape(g, nshot, S.n + R.n);
+    const bool resident = rs.ctas > 0 && p->d_words && points_inside && !dft && !ckpt && !mv.n;
+    if (resident) CKC(cudaMemsetAsync(p->d_words, 0, sizeof(*p->d_words) * (size_t)resident2d_words(rs), st));
     LoopKey key;
     key.add(mv.n); key.add(p->movout); key.add(p->d_mov); key.add(fuse2d); key.add(p->d_ticket); key.add(fuse3d);
     key.add(1); key.add(p->g); key.add(p->f); key.add_points(S); key.add_points(R); key.add(p->d_src);
@@ -1400,7 +1421,17 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
     };
     if ((rc = arm_unstable(p, st))) return rc;
     CKC(cudaEventRecord(p->ev0, st));
-    int rcl = run_loop(p, p->gfwd, key.s, st, [&](cudaStream_t s) {
+    int rcl = SFD_OK;
+    if (resident) {
+        if (tmax > 0) launch_sources(g, p->f, S, p->d_src, NT, 0, 1, st);
+        Res2dRun a{R, S, p->d_src, p->d_seis, omask, NT, 0, 0, tmax, bs, p->cfg.precision, p->d_words, p->d_unstable,
+                   p->d_unstable + 1};
+        for (a.t0 = 0; a.t0 < tmax; a.t0 = a.t1) {
+            a.t1 = std::min(a.t0 + RES2D_SEGMENT, tmax);
+            CKC(launch_resident2d(g, p->f, rs, a, p->device, st));
+        }
+    } else
+    rcl = run_loop(p, p->gfwd, key.s, st, [&](cudaStream_t s) {
         if (fuse2d) {
             if (tmax > 0) launch_sources(g, p->f, S, p->d_src, NT, 0, 1, s);
             for (int t = 0; t < tmax; t++) {

@@ -161,7 +161,9 @@ struct sfd_plan {
     float *d_src_div, *d_src, *d_seis, *d_res;
     float *d_surf_q;        // surface-adjoint scratch [nx][ny]
     int *d_ticket;          // fused 2D steps: block counter of the stress launch
-    int *d_unstable;        // first checked step with a non-finite wave field (INT_MAX: none)
+    int *d_unstable;        // first checked step with a non-finite wave field (0x7f7f7f7f: none), then
+                            // the status of the resident 2D steps (0, or 1: a wait ran out)
+    unsigned long long *d_words;   // exchange words of the resident 2D steps
     int *d_fsync;           // fused 3D step: ticket counter + one flag per work unit
     // checkpointed gradients (cfg.checkpoint = K > 0)
     char *d_snap;           // [nseg] snapshots: wave fields, memory variables (store type; FP16 wave-field

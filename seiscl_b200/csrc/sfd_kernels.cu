@@ -23,338 +23,11 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "sfd_device.cuh"
 #include "sfd_internal.h"
 #include "sfd_kernels.h"
 
 namespace sfd {
-
-typedef int64_t i64;
-
-// ---------------------------------------------------------------- helpers
-// forward difference c1 (v[i+1]-v[i]) + c2 (v[i+2]-v[i-1]) + ...  (Dxp)
-template <int F>
-__device__ __forceinline__ float dfw(const float *__restrict__ v, i64 i, i64 st, const float *hc)
-{
-    float acc = hc[0] * (__ldg(v + i + st) - __ldg(v + i));
-#pragma unroll
-    for (int m = 2; m <= F; m++) acc = fmaf(hc[m - 1], __ldg(v + i + m * st) - __ldg(v + i - (m - 1) * st), acc);
-    return acc;
-}
-// backward difference c1 (v[i]-v[i-1]) + c2 (v[i+1]-v[i-2]) + ...  (Dxm)
-template <int F>
-__device__ __forceinline__ float dbw(const float *__restrict__ v, i64 i, i64 st, const float *hc)
-{
-    float acc = hc[0] * (__ldg(v + i) - __ldg(v + i - st));
-#pragma unroll
-    for (int m = 2; m <= F; m++) acc = fmaf(hc[m - 1], __ldg(v + i + (m - 1) * st) - __ldg(v + i - m * st), acc);
-    return acc;
-}
-// non-cached variants for arrays written by the same kernel
-template <int F>
-__device__ __forceinline__ float dfw_rw(const float *v, i64 i, i64 st, const float *hc)
-{
-    float acc = hc[0] * (v[i + st] - v[i]);
-#pragma unroll
-    for (int m = 2; m <= F; m++) acc = fmaf(hc[m - 1], v[i + m * st] - v[i - (m - 1) * st], acc);
-    return acc;
-}
-template <int F>
-__device__ __forceinline__ float dbw_rw(const float *v, i64 i, i64 st, const float *hc)
-{
-    float acc = hc[0] * (v[i] - v[i - st]);
-#pragma unroll
-    for (int m = 2; m <= F; m++) acc = fmaf(hc[m - 1], v[i + (m - 1) * st] - v[i - m * st], acc);
-    return acc;
-}
-
-// Wave-field storage access: FP32, or FP16 holding the field times a power
-// of two (the kernels compute in FP32 either way).
-template <class T> __device__ __forceinline__ float ldv(const T *p);
-template <> __device__ __forceinline__ float ldv<float>(const float *p) { return *p; }
-template <> __device__ __forceinline__ float ldv<__half>(const __half *p) { return __half2float(*p); }
-template <class T> __device__ __forceinline__ float ldgv(const T *p);
-template <> __device__ __forceinline__ float ldgv<float>(const float *p) { return __ldg(p); }
-template <> __device__ __forceinline__ float ldgv<__half>(const __half *p) { return __half2float(__ldg(p)); }
-template <class T> __device__ __forceinline__ void stv(T *p, float v);
-template <> __device__ __forceinline__ void stv<float>(float *p, float v) { *p = v; }
-template <> __device__ __forceinline__ void stv<__half>(__half *p, float v) { *p = __float2half_rn(v); }
-template <class T> __device__ __forceinline__ T *fld(float *p) { return reinterpret_cast<T *>(p); }
-
-template <int F, class T>
-__device__ __forceinline__ float dfwT(const T *__restrict__ v, i64 i, i64 st, const float *hc)
-{
-    float acc = hc[0] * (ldgv(v + i + st) - ldgv(v + i));
-#pragma unroll
-    for (int m = 2; m <= F; m++) acc = fmaf(hc[m - 1], ldgv(v + i + m * st) - ldgv(v + i - (m - 1) * st), acc);
-    return acc;
-}
-template <int F, class T>
-__device__ __forceinline__ float dbwT(const T *__restrict__ v, i64 i, i64 st, const float *hc)
-{
-    float acc = hc[0] * (ldgv(v + i) - ldgv(v + i - st));
-#pragma unroll
-    for (int m = 2; m <= F; m++) acc = fmaf(hc[m - 1], ldgv(v + i + (m - 1) * st) - ldgv(v + i - m * st), acc);
-    return acc;
-}
-template <int F, class T>
-__device__ __forceinline__ float dbw_rwT(const T *v, i64 i, i64 st, const float *hc)
-{
-    float acc = hc[0] * (ldv(v + i) - ldv(v + i - st));
-#pragma unroll
-    for (int m = 2; m <= F; m++) acc = fmaf(hc[m - 1], ldv(v + i + (m - 1) * st) - ldv(v + i - m * st), acc);
-    return acc;
-}
-
-// psi = b psi + a d ; d = d/K + psi    (the CPML recursion of every kernel)
-__device__ __forceinline__ void cpml(float *psi, i64 q, const float *K, const float *a, const float *b, int ci,
-                                     float &d)
-{
-    float ps = __ldg(b + ci) * psi[q] + __ldg(a + ci) * d;
-    psi[q] = ps;
-    d = d / __ldg(K + ci) + ps;
-}
-
-template <typename T> __device__ __forceinline__ float to_f(T v);
-template <> __device__ __forceinline__ float to_f<float>(float v) { return v; }
-template <> __device__ __forceinline__ float to_f<__half>(__half v) { return __half2float(v); }
-template <> __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
-
-// Programmatic dependent launch (the 3D modelling loop's kernels, see
-// pdl_enabled): a kernel launched with programmatic stream serialization may
-// be resident before the previous kernel of the stream has finished.
-// pdl_wait returns once that kernel has completed and its stores are
-// visible (at once for an ordinary launch); nothing it writes may be read,
-// and nothing at all written, before it.  pdl_trigger lets the next
-// kernel's CTAs launch once every CTA of this grid has passed it.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-template <typename T> __device__ __forceinline__ T from_f(float v);
-template <> __device__ __forceinline__ float from_f<float>(float v) { return v; }
-template <> __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half_rn(v); }
-template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
-
-// batched shots: shot b of a launch (blockIdx.z) works on copy b of every
-// per-shot array
-__device__ __forceinline__ void shot_fields(const Grid &g, Fields &f, int b)
-{
-#pragma unroll
-    for (int w = 0; w < NW; w++)
-        if (f.w[w]) f.w[w] += b * g.sb_w;
-#pragma unroll
-    for (int r = 0; r < NR; r++)
-        if (f.r[r]) f.r[r] += b * g.sb_r;
-#pragma unroll
-    for (int i = 0; i < NPSI; i++)
-        if (f.psi[i]) f.psi[i] += b * g.sb_psi;
-}
-__device__ __forceinline__ void shot_adj(const Grid &g, AdjFields &a, int b)
-{
-#pragma unroll
-    for (int w = 0; w < NW; w++) {
-        if (a.wr[w]) a.wr[w] += b * g.sb_w;
-        if (a.bnd[w]) a.bnd[w] = (const char *)a.bnd[w] + b * g.sb_bnd;
-    }
-#pragma unroll
-    for (int r = 0; r < NR; r++)
-        if (a.rr[r]) a.rr[r] += b * g.sb_r;
-#pragma unroll
-    for (int k = 0; k < NG; k++) {
-        if (a.grad[k]) a.grad[k] += b * g.sb_g;
-        if (a.hess[k]) a.hess[k] += b * g.sb_g;
-    }
-}
-#define SHOT_F  if (g.nb > 1) shot_fields(g, f, blockIdx.z);
-#define SHOT_FA if (g.nb > 1) { shot_fields(g, f, blockIdx.z); shot_adj(g, a, blockIdx.z); }
-
-// a saved boundary value (slice t-1) back in field units: FP16 stores carry
-// a power-of-two scale (exact; 1 for FP32 and BF16 stores)
-template <class T>
-__device__ __forceinline__ float bnd_at(const Grid &g, const AdjFields &a, int w, i64 m)
-{
-    return to_f<T>(((const T *)a.bnd[w])[m]) * g.bsci[w];
-}
-
-// checkpointed gradients (g.ckpt): the forward wave field of the adjoint
-// step, stored when the forward run was recomputed from a snapshot (same
-// storage type and scales as the saved boundaries)
-template <class T>
-__device__ __forceinline__ float fwd_at(const Grid &g, const AdjFields &a, int w, i64 iv)
-{
-    return to_f<T>(((const T *)a.fwd[w])[iv]) * g.bsci[w];
-}
-
-// ------------------------------------------------------- boundary shells
-struct BndDims {
-    int NXbnd, NYbnd, NZbnd, lbnd, lbnds;
-};
-__device__ __host__ inline BndDims bnd_dims(const Grid &g)
-{
-    BndDims b;
-    b.NXbnd = g.NX - 2 * g.F - 2 * g.nab;
-    b.NYbnd = g.nd == 3 ? g.NY - 2 * g.F - 2 * g.nab : 1;
-    if (!g.freesurf) {
-        b.NZbnd = g.NZ - 2 * g.F - 2 * g.nab;
-        b.lbnd = g.F + g.nab;
-        b.lbnds = g.F + g.nab;
-    } else {
-        b.NZbnd = g.NZ - 2 * g.F - g.nab;
-        b.lbnd = g.F + g.nab;
-        b.lbnds = g.F;
-    }
-    return b;
-}
-
-// index of cell (k, i) in the saved shell, -1 if not a shell cell
-// (src/header_injectbnd.cl:238-283)
-__device__ __forceinline__ int inject_ind2d(const Grid &g, int k, int i)
-{
-    BndDims b = bnd_dims(g);
-    int F = g.F, m = -1;
-    i -= b.lbnd;
-    k -= b.lbnds;
-    if ((k > F - 1 && k < b.NZbnd - F) && (i > F - 1 && i < b.NXbnd - F)) m = -1;
-    else if (k < 0 || k > b.NZbnd - 1 || i < 0 || i > b.NXbnd - 1) m = -1;
-    else if (i < F) m = i * b.NZbnd + k;
-    else if (i > b.NXbnd - 1 - F) { i = i - b.NXbnd + F; m = b.NZbnd * F + i * b.NZbnd + k; }
-    else if (k < F) { i = i - F; m = b.NZbnd * F * 2 + (b.NXbnd - 2 * F) * F + i + k * (b.NXbnd - 2 * F); }
-    else { i = i - F; k = k - b.NZbnd + F; m = b.NZbnd * F * 2 + i + k * (b.NXbnd - 2 * F); }
-    return m;
-}
-// (src/header_injectbnd.cl:25-84)
-__device__ __forceinline__ int inject_ind3d(const Grid &g, int k, int j, int i)
-{
-    BndDims b = bnd_dims(g);
-    int F = g.F, m = -1;
-    i -= b.lbnd; j -= b.lbnd; k -= b.lbnds;
-    int NX = b.NXbnd, NY = b.NYbnd, NZ = b.NZbnd;
-    if ((k > F - 1 && k < NZ - F) && (j > F - 1 && j < NY - F) && (i > F - 1 && i < NX - F)) m = -1;
-    else if (k < 0 || k > NZ - 1 || j < 0 || j > NY - 1 || i < 0 || i > NX - 1) m = -1;
-    else if (i < F) m = i * NY * NZ + j * NZ + k;
-    else if (i > NX - 1 - F) { i = i - NX + F; m = NY * NZ * F + i * NY * NZ + j * NZ + k; }
-    else if (j < F) { i = i - F; m = NY * NZ * F * 2 + i * F * NZ + j * NZ + k; }
-    else if (j > NY - 1 - F) { i = i - F; j = j - NY + F; m = NY * NZ * F * 2 + (NX - 2 * F) * NZ * F + i * F * NZ + j * NZ + k; }
-    else if (k < F) {
-        i = i - F; j = j - F;
-        m = NY * NZ * F * 2 + (NX - 2 * F) * NZ * F * 2 + (NX - 2 * F) * (NY - 2 * F) * F + i * (NY - 2 * F) * F + j * F + k;
-    } else {
-        i = i - F; j = j - F; k = k - NZ + F;
-        m = NY * NZ * F * 2 + (NX - 2 * F) * NZ * F * 2 + i * (NY - 2 * F) * F + j * F + k;
-    }
-    return m;
-}
-
-// shell cell of saved index gid (src/savebnd2D.cl:52-93, savebnd3D.cl:46-103)
-__device__ __forceinline__ bool shell_cell(const Grid &g, int gid, int &i, int &j, int &k)
-{
-    BndDims b = bnd_dims(g);
-    int F = g.F, NAB = g.nab, gidf;
-    if (g.nd != 3) {
-        j = 0;
-        int NZ = b.NZbnd, NX = b.NXbnd;
-        if (gid < NZ * F) { gidf = gid; i = gidf / NZ + b.lbnd; k = gidf % NZ + b.lbnds; }
-        else if (gid < NZ * F * 2) { gidf = gid - NZ * F; i = gidf / NZ + NX + NAB; k = gidf % NZ + b.lbnds; }
-        else if (gid < NZ * F * 2 + (NX - 2 * F) * F) {
-            gidf = gid - NZ * F * 2; i = gidf % (NX - 2 * F) + b.lbnd + F; k = gidf / (NX - 2 * F) + NZ + b.lbnds - F;
-        } else if (gid < NZ * F * 2 + (NX - 2 * F) * 2 * F) {
-            gidf = gid - NZ * F * 2 - (NX - 2 * F) * F; i = gidf % (NX - 2 * F) + b.lbnd + F; k = gidf / (NX - 2 * F) + b.lbnds;
-        } else return false;
-        return true;
-    }
-    int NX = b.NXbnd, NY = b.NYbnd, NZ = b.NZbnd;
-    int a0 = NY * NZ * F, a1 = NZ * (NX - 2 * F) * F, a2 = (NY - 2 * F) * (NX - 2 * F) * F;
-    if (gid < a0) { gidf = gid; i = gidf / (NY * NZ) + b.lbnd; j = (gidf / NZ) % NY + b.lbnd; k = gidf % NZ + b.lbnds; }
-    else if (gid < 2 * a0) { gidf = gid - a0; i = gidf / (NY * NZ) + NX + NAB; j = (gidf / NZ) % NY + b.lbnd; k = gidf % NZ + b.lbnds; }
-    else if (gid < 2 * a0 + a1) { gidf = gid - 2 * a0; i = gidf / (NZ * F) + b.lbnd + F; j = (gidf / NZ) % F + b.lbnd; k = gidf % NZ + b.lbnds; }
-    else if (gid < 2 * a0 + 2 * a1) { gidf = gid - 2 * a0 - a1; i = gidf / (NZ * F) + b.lbnd + F; j = (gidf / NZ) % F + NY + NAB; k = gidf % NZ + b.lbnds; }
-    else if (gid < 2 * a0 + 2 * a1 + a2) {
-        gidf = gid - 2 * a0 - 2 * a1;
-        i = gidf / (F * (NY - 2 * F)) + b.lbnd + F; j = (gidf / F) % (NY - 2 * F) + b.lbnd + F; k = gidf % F + NZ + b.lbnds - F;
-    } else if (gid < 2 * a0 + 2 * a1 + 2 * a2) {
-        gidf = gid - 2 * a0 - 2 * a1 - a2;
-        i = gidf / (F * (NY - 2 * F)) + b.lbnd + F; j = (gidf / F) % (NY - 2 * F) + b.lbnd + F; k = gidf % F + b.lbnds;
-    } else return false;
-    return true;
-}
-
-// ------------------------------------------------------------------ taper
-template <int NF, class T = float>
-__device__ __forceinline__ void apply_taper(const Grid &g, const float *taper, int gz, int gy, int gx,
-                                            T *const *fs, i64 iv)
-{
-    int F = g.F, NAB = g.nab;
-    auto mul = [&](float t) {
-        for (int q = 0; q < NF; q++) stv(fs[q] + iv, ldv(fs[q] + iv) * t);
-    };
-    if (!g.freesurf && gz - F < NAB) mul(__ldg(taper + gz - F));
-    if (gz > g.NZ - NAB - F - 1) mul(__ldg(taper + g.NZ - F - gz - 1));
-    if (g.nd == 3) {
-        if (gy - F < NAB) mul(__ldg(taper + gy - F));
-        if (gy > g.NY - NAB - F - 1) mul(__ldg(taper + g.NY - F - gy - 1));
-    }
-    if (gx - F < NAB) mul(__ldg(taper + gx - F));
-    if (gx > g.NX - NAB - F - 1) mul(__ldg(taper + g.NX - F - gx - 1));
-}
-
-// ===================================================================== 2D
-// CPML on the stress derivatives (update_v2D.cl:146-207)
-__device__ __forceinline__ void cpml_v2d(const Grid &g, const Fields &f, int gz, int gx, float &sxx_x,
-                                         float &szz_z, float &sxz_x, float &sxz_z)
-{
-    int F = g.F, NAB = g.nab, NZ = g.NZ, NX = g.NX;
-    if (gz > NZ - NAB - F - 1) {
-        int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
-        i64 q = (i64)i * (2 * NAB) + k;
-        cpml(f.psi[PSXZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], ind + 1, sxz_z);
-        cpml(f.psi[PSZZ_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], ind, szz_z);
-    } else if (!g.freesurf && gz - F < NAB) {
-        int i = gx - F, k = gz - F;
-        i64 q = (i64)i * (2 * NAB) + k;
-        cpml(f.psi[PSXZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], k, sxz_z);
-        cpml(f.psi[PSZZ_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], k, szz_z);
-    }
-    if (gx - F < NAB) {
-        int i = gx - F, k = gz - F;
-        i64 q = (i64)i * g.nz + k;
-        cpml(f.psi[PSXX_X], q, f.cx[CKH], f.cx[CAH], f.cx[CBH], i, sxx_x);
-        cpml(f.psi[PSXZ_X], q, f.cx[CK], f.cx[CA], f.cx[CB], i, sxz_x);
-    }
-    if (gx > NX - NAB - F - 1) {
-        int i = gx - NX + NAB + F + NAB, k = gz - F, ind = 2 * NAB - 1 - i;
-        i64 q = (i64)i * g.nz + k;
-        cpml(f.psi[PSXX_X], q, f.cx[CKH], f.cx[CAH], f.cx[CBH], ind, sxx_x);
-        cpml(f.psi[PSXZ_X], q, f.cx[CK], f.cx[CA], f.cx[CB], ind + 1, sxz_x);
-    }
-}
-
-// CPML on the velocity derivatives (update_s2D.cl:145-208)
-__device__ __forceinline__ void cpml_s2d(const Grid &g, const Fields &f, int gz, int gx, float &vxx, float &vxz,
-                                         float &vzx, float &vzz)
-{
-    int F = g.F, NAB = g.nab, NZ = g.NZ, NX = g.NX;
-    if (gz > NZ - NAB - F - 1) {
-        int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
-        i64 q = (i64)i * (2 * NAB) + k;
-        cpml(f.psi[PVX_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], ind, vxz);
-        cpml(f.psi[PVZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], ind + 1, vzz);
-    } else if (!g.freesurf && gz - F < NAB) {
-        int i = gx - F, k = gz - F;
-        i64 q = (i64)i * (2 * NAB) + k;
-        cpml(f.psi[PVX_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], k, vxz);
-        cpml(f.psi[PVZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], k, vzz);
-    }
-    if (gx - F < NAB) {
-        int i = gx - F, k = gz - F;
-        i64 q = (i64)i * g.nz + k;
-        cpml(f.psi[PVX_X], q, f.cx[CK], f.cx[CA], f.cx[CB], i, vxx);
-        cpml(f.psi[PVZ_X], q, f.cx[CKH], f.cx[CAH], f.cx[CBH], i, vzx);
-    }
-    if (gx > NX - NAB - F - 1) {
-        int i = gx - NX + NAB + F + NAB, k = gz - F, ind = 2 * NAB - 1 - i;
-        i64 q = (i64)i * g.nz + k;
-        cpml(f.psi[PVX_X], q, f.cx[CK], f.cx[CA], f.cx[CB], ind + 1, vxx);
-        cpml(f.psi[PVZ_X], q, f.cx[CKH], f.cx[CAH], f.cx[CBH], ind, vzx);
-    }
-}
 
 // T: storage of the wave fields and memory variables (float, or __half
 // holding them times power-of-two scales; the arithmetic is FP32)
@@ -373,8 +46,8 @@ __global__ void __launch_bounds__(256) k_v2d(Grid g, Fields f)
     float sxz_z = dbwT<F>(fld<T>(f.w[SXZ]), iv, 1, hc);
     float sxz_x = dbwT<F>(fld<T>(f.w[SXZ]), iv, g.NZ, hc);
     if (g.abs_type == 1) cpml_v2d(g, f, gz, gx, sxx_x, szz_z, sxz_x, sxz_z);
-    stv(vx + iv, ldv(vx + iv) + (sxx_x + sxz_z) * __ldg(f.p[PRIP] + ip));
-    stv(vz + iv, ldv(vz + iv) + (szz_z + sxz_x) * __ldg(f.p[PRKP] + ip));
+    stv(vx + iv, v2d_math(ldv(vx + iv), sxx_x, sxz_z, __ldg(f.p[PRIP] + ip)));
+    stv(vz + iv, v2d_math(ldv(vz + iv), szz_z, sxz_x, __ldg(f.p[PRKP] + ip)));
     if (g.abs_type == 2) {
         T *fs[2] = {vx, vz};
         apply_taper<2>(g, f.taper, gz, 0, gx, fs, iv);
@@ -394,47 +67,39 @@ __device__ __forceinline__ void s2d_cell(const Grid &g, const Fields &f, int gz,
     float vzx = dfwT<F>(fld<T>(f.w[VZ]), iv, g.NZ, hc);
     if (g.abs_type == 1) cpml_s2d(g, f, gz, gx, vxx, vxz, vzx, vzz);
     const int L = g.L;
+    const float tr = __fadd_rn(vxx, vzz), sh = __fadd_rn(vxz, vzx);
     if (L == 0) {
-        float fipkp = __ldg(f.p[PMUIPKP] + ip);
-        float fm = 2.0f * __ldg(f.p[PMU] + ip);
-        float gm = __ldg(f.p[PM] + ip);
-        stv(wsxz + iv, ldv(wsxz + iv) + fipkp * (vxz + vzx));
-        stv(wsxx + iv, ldv(wsxx + iv) + (gm * (vxx + vzz) - fm * vzz));
-        stv(wszz + iv, ldv(wszz + iv) + (gm * (vxx + vzz) - fm * vxx));
+        const S2dMat m = s2d_elastic(__ldg(f.p[PM] + ip), __ldg(f.p[PMU] + ip), __ldg(f.p[PMUIPKP] + ip));
+        stv(wsxz + iv, __fmaf_rn(m.fipkp, sh, ldv(wsxz + iv)));
+        stv(wsxx + iv, __fadd_rn(ldv(wsxx + iv), s2d_normal(m.gm, tr, m.fm, vzz)));
+        stv(wszz + iv, __fadd_rn(ldv(wszz + iv), s2d_normal(m.gm, tr, m.fm, vxx)));
     } else {
-        float lM = __ldg(f.p[PM] + ip), lmu = __ldg(f.p[PMU] + ip), lmuipkp = __ldg(f.p[PMUIPKP] + ip);
-        float ltaup = __ldg(f.p[PTAUP] + ip), ltaus = __ldg(f.p[PTAUS] + ip), ltausipkp = __ldg(f.p[PTAUSIPKP] + ip);
-        float fipkp = lmuipkp * (1.0f + (float)L * ltausipkp);
-        float gm = lM * (1.0f + (float)L * ltaup);
-        float fm = 2.0f * lmu * (1.0f + (float)L * ltaus);
-        float dipkp = lmuipkp * ltausipkp / g.dt;
-        float d = 2.0f * lmu * ltaus / g.dt;
-        float e = lM * ltaup / g.dt;
+        const S2dMat m = s2d_visco(L, g.dt, __ldg(f.p[PM] + ip), __ldg(f.p[PMU] + ip), __ldg(f.p[PMUIPKP] + ip),
+                                   __ldg(f.p[PTAUP] + ip), __ldg(f.p[PTAUS] + ip), __ldg(f.p[PTAUSIPKP] + ip));
         T *rxx = fld<T>(f.r[RXX]), *rzz = fld<T>(f.r[RZZ]), *rxz = fld<T>(f.r[RXZ]);
         float sxz_ = 0, sxx_ = 0, szz_ = 0;
         for (int l = 0; l < L; l++) {
             i64 ir = l * g.nvol + iv;
             sxz_ += ldv(rxz + ir); sxx_ += ldv(rxx + ir); szz_ += ldv(rzz + ir);
         }
-        float lsxz = fipkp * (vxz + vzx) + g.dt2 * sxz_;
-        float lsxx = (gm * (vxx + vzz) - fm * vzz) + g.dt2 * sxx_;
-        float lszz = (gm * (vxx + vzz) - fm * vxx) + g.dt2 * szz_;
+        const float lsxz = __fmaf_rn(m.fipkp, sh, __fmul_rn(g.dt2, sxz_));
+        const float lsxx = __fmaf_rn(g.dt2, sxx_, s2d_normal(m.gm, tr, m.fm, vzz));
+        const float lszz = __fmaf_rn(g.dt2, szz_, s2d_normal(m.gm, tr, m.fm, vxx));
         sxz_ = sxx_ = szz_ = 0;
         for (int l = 0; l < L; l++) {
-            float el = g.eta[l];
-            float b = 1.0f / (1.0f + el * 0.5f), c = 1.0f - el * 0.5f;
+            const float el = g.eta[l];
             i64 ir = l * g.nvol + iv;
-            float a1 = b * (ldv(rxz + ir) * c - el * (dipkp * (vxz + vzx)));
-            float a2 = b * (ldv(rxx + ir) * c - el * (e * (vxx + vzz) - d * vzz));
-            float a3 = b * (ldv(rzz + ir) * c - el * (e * (vxx + vzz) - d * vxx));
+            float a1 = s2d_memory(ldv(rxz + ir), el, g.eta_b[l], g.eta_c[l], __fmul_rn(m.dipkp, sh));
+            float a2 = s2d_memory(ldv(rxx + ir), el, g.eta_b[l], g.eta_c[l], s2d_normal(m.e, tr, m.d, vzz));
+            float a3 = s2d_memory(ldv(rzz + ir), el, g.eta_b[l], g.eta_c[l], s2d_normal(m.e, tr, m.d, vxx));
             stv(rxz + ir, a1); stv(rxx + ir, a2); stv(rzz + ir, a3);
             // the stored values (rounded to T) are what the next step reads;
             // the sums use the FP32 ones, as the FP32 build does
             sxz_ += a1; sxx_ += a2; szz_ += a3;
         }
-        stv(wsxz + iv, ldv(wsxz + iv) + (lsxz + g.dt2 * sxz_));
-        stv(wsxx + iv, ldv(wsxx + iv) + (lsxx + g.dt2 * sxx_));
-        stv(wszz + iv, ldv(wszz + iv) + (lszz + g.dt2 * szz_));
+        stv(wsxz + iv, s2d_add(ldv(wsxz + iv), lsxz, g.dt2, sxz_));
+        stv(wsxx + iv, s2d_add(ldv(wsxx + iv), lsxx, g.dt2, sxx_));
+        stv(wszz + iv, s2d_add(ldv(wszz + iv), lszz, g.dt2, szz_));
     }
     if (g.abs_type == 2) {
         T *fs[3] = {wsxx, wszz, wsxz};
@@ -463,36 +128,32 @@ __device__ __forceinline__ void surf2d_column(const Grid &g, const Fields &f, in
     if (g.abs_type == 1) {
         if (gx - F < NAB) {
             int i = gx - F;
-            vxx = vxx / f.cx[CK][i] + f.psi[PVX_X][(i64)i * g.nz + (gz - F)];
+            vxx = __fmaf_rn(vxx, f.kinv[0][0][i], f.psi[PVX_X][(i64)i * g.nz + (gz - F)]);
         }
         if (gx > g.NX - NAB - F - 1) {
             int i = gx - g.NX + NAB + F + NAB, ind = 2 * NAB - 1 - i;
-            vxx = vxx / f.cx[CK][ind + 1] + f.psi[PVX_X][(i64)i * g.nz + (gz - F)];
+            vxx = __fmaf_rn(vxx, f.kinv[0][0][ind + 1], f.psi[PVX_X][(i64)i * g.nz + (gz - F)]);
         }
     }
+    const float sg = (float)pdir;
     if (L == 0) {
-        float fm = f.p[PMU][ip] * 2.0f, gm = f.p[PM][ip];
-        float h = -((gm - fm) * (gm - fm) * vxx / gm) - ((gm - fm) * vzz);
-        stv(sxx + iv, ldv(sxx + iv) + pdir * h);
+        const S2dMat m = s2d_elastic(f.p[PM][ip], f.p[PMU][ip], 0.0f);
+        stv(sxx + iv, __fmaf_rn(sg, surf2d_h(surf2d_of(m), vxx, vzz), ldv(sxx + iv)));
     } else {
-        float taus = f.p[PTAUS][ip], taup = f.p[PTAUP][ip], mu = f.p[PMU][ip], M = f.p[PM][ip];
-        float fm = mu * 2.0f * (1.0f + L * taus);
-        float gm = M * (1.0f + L * taup);
-        float h = -((gm - fm) * (gm - fm) * vxx / gm) - ((gm - fm) * vzz);
+        const S2dMat m = s2d_visco(L, g.dt, f.p[PM][ip], f.p[PMU][ip], 0.0f, f.p[PTAUP][ip], f.p[PTAUS][ip], 0.0f);
         float sump = 0;
         for (int l = 0; l < L; l++) sump += ldv(rxx + l * g.nvol + iv);
-        h += -g.dt2 * sump;
-        stv(sxx + iv, ldv(sxx + iv) + pdir * h);
-        float d = 2.0f * mu * taus / g.dt, e = M * taup / g.dt;
+        const Surf2d su = surf2d_of(m);
+        const float h = __fmaf_rn(-g.dt2, sump, surf2d_h(su, vxx, vzz));
+        stv(sxx + iv, __fmaf_rn(sg, h, ldv(sxx + iv)));
         sump = 0;
         for (int l = 0; l < L; l++) {
-            float b = g.eta[l] / (1.0f + g.eta[l] * 0.5f);
-            float hh = b * (((d - e) * ((fm / gm) - 1.0f) * vxx) - ((d - e) * vzz));
-            float r = ldv(rxx + l * g.nvol + iv) + pdir * hh;
+            const float hh = surf2d_hr(su, surf2d_b(g.eta[l]), vxx, vzz);
+            float r = __fmaf_rn(sg, hh, ldv(rxx + l * g.nvol + iv));
             stv(rxx + l * g.nvol + iv, r);
             sump += r;
         }
-        stv(sxx + iv, ldv(sxx + iv) + pdir * (g.dt2 * sump));
+        stv(sxx + iv, __fmaf_rn(sg, __fmul_rn(g.dt2, sump), ldv(sxx + iv)));
     }
 }
 
@@ -525,44 +186,44 @@ __device__ __forceinline__ void cpml_v3d(const Grid &g, const Fields &f, int gz,
         i64 i = gx - F, j = gy - F, k = gz - NZ + NAB + F + NAB;
         int ind = 2 * NAB - 1 - (int)k;
         i64 q = (i * ny + j) * (2 * NAB) + k;
-        cpml(f.psi[PSXZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], ind + 1, sxz_z);
-        cpml(f.psi[PSYZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], ind + 1, syz_z);
-        cpml(f.psi[PSZZ_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], ind, szz_z);
+        cpml(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, sxz_z);
+        cpml(f.psi[PSYZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, syz_z);
+        cpml(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, szz_z);
     } else if (!g.freesurf && gz - F < NAB) {
         i64 i = gx - F, j = gy - F, k = gz - F;
         i64 q = (i * ny + j) * (2 * NAB) + k;
-        cpml(f.psi[PSXZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], (int)k, sxz_z);
-        cpml(f.psi[PSYZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], (int)k, syz_z);
-        cpml(f.psi[PSZZ_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], (int)k, szz_z);
+        cpml(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, sxz_z);
+        cpml(f.psi[PSYZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, syz_z);
+        cpml(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, szz_z);
     }
     if (gy - F < NAB) {
         i64 i = gx - F, j = gy - F, k = gz - F;
         i64 q = (i * (2 * NAB) + j) * nz + k;
-        cpml(f.psi[PSXY_Y], q, f.cy[CK], f.cy[CA], f.cy[CB], (int)j, sxy_y);
-        cpml(f.psi[PSYY_Y], q, f.cy[CKH], f.cy[CAH], f.cy[CBH], (int)j, syy_y);
-        cpml(f.psi[PSYZ_Y], q, f.cy[CK], f.cy[CA], f.cy[CB], (int)j, syz_y);
+        cpml(f.psi[PSXY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], (int)j, sxy_y);
+        cpml(f.psi[PSYY_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], (int)j, syy_y);
+        cpml(f.psi[PSYZ_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], (int)j, syz_y);
     } else if (gy > NY - NAB - F - 1) {
         i64 i = gx - F, j = gy - NY + NAB + F + NAB, k = gz - F;
         int ind = 2 * NAB - 1 - (int)j;
         i64 q = (i * (2 * NAB) + j) * nz + k;
-        cpml(f.psi[PSXY_Y], q, f.cy[CK], f.cy[CA], f.cy[CB], ind + 1, sxy_y);
-        cpml(f.psi[PSYY_Y], q, f.cy[CKH], f.cy[CAH], f.cy[CBH], ind, syy_y);
-        cpml(f.psi[PSYZ_Y], q, f.cy[CK], f.cy[CA], f.cy[CB], ind + 1, syz_y);
+        cpml(f.psi[PSXY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], ind + 1, sxy_y);
+        cpml(f.psi[PSYY_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ind, syy_y);
+        cpml(f.psi[PSYZ_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], ind + 1, syz_y);
     }
     if (gx - F < NAB) {
         i64 i = gx - F, j = gy - F, k = gz - F;
         i64 q = (i * ny + j) * nz + k;
-        cpml(f.psi[PSXX_X], q, f.cx[CKH], f.cx[CAH], f.cx[CBH], (int)i, sxx_x);
-        cpml(f.psi[PSXY_X], q, f.cx[CK], f.cx[CA], f.cx[CB], (int)i, sxy_x);
-        cpml(f.psi[PSXZ_X], q, f.cx[CK], f.cx[CA], f.cx[CB], (int)i, sxz_x);
+        cpml(f.psi[PSXX_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], (int)i, sxx_x);
+        cpml(f.psi[PSXY_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], (int)i, sxy_x);
+        cpml(f.psi[PSXZ_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], (int)i, sxz_x);
     }
     if (gx > NX - NAB - F - 1) {
         i64 i = gx - NX + NAB + F + NAB, j = gy - F, k = gz - F;
         int ind = 2 * NAB - 1 - (int)i;
         i64 q = (i * ny + j) * nz + k;
-        cpml(f.psi[PSXX_X], q, f.cx[CKH], f.cx[CAH], f.cx[CBH], ind, sxx_x);
-        cpml(f.psi[PSXY_X], q, f.cx[CK], f.cx[CA], f.cx[CB], ind + 1, sxy_x);
-        cpml(f.psi[PSXZ_X], q, f.cx[CK], f.cx[CA], f.cx[CB], ind + 1, sxz_x);
+        cpml(f.psi[PSXX_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, sxx_x);
+        cpml(f.psi[PSXY_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, sxy_x);
+        cpml(f.psi[PSXZ_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, sxz_x);
     }
 }
 
@@ -579,47 +240,47 @@ __device__ __forceinline__ void cpml_s3d(const Grid &g, const Fields &f, int gz,
         i64 i = gx - F, j = gy - F, k = gz - NZ + NAB + F + NAB;
         int ind = 2 * NAB - 1 - (int)k;
         i64 q = (i * ny + j) * (2 * NAB) + k;
-        cpml(f.psi[PVX_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], ind, vxz);
-        cpml(f.psi[PVY_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], ind, vyz);
-        cpml(f.psi[PVZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], ind + 1, vzz);
+        cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vxz);
+        cpml(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vyz);
+        cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, vzz);
     }
     if (!g.freesurf && gz - F < NAB && !(adjoint_form && zb)) {
         i64 i = gx - F, j = gy - F, k = gz - F;
         i64 q = (i * ny + j) * (2 * NAB) + k;
-        cpml(f.psi[PVX_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], (int)k, vxz);
-        cpml(f.psi[PVY_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], (int)k, vyz);
-        cpml(f.psi[PVZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], (int)k, vzz);
+        cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, vxz);
+        cpml(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, vyz);
+        cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, vzz);
     }
     bool yb = gy - F < NAB;
     if (yb) {
         i64 i = gx - F, j = gy - F, k = gz - F;
         i64 q = (i * (2 * NAB) + j) * nz + k;
-        cpml(f.psi[PVX_Y], q, f.cy[CKH], f.cy[CAH], f.cy[CBH], (int)j, vxy);
-        cpml(f.psi[PVY_Y], q, f.cy[CK], f.cy[CA], f.cy[CB], (int)j, vyy);
-        cpml(f.psi[PVZ_Y], q, f.cy[CKH], f.cy[CAH], f.cy[CBH], (int)j, vzy);
+        cpml(f.psi[PVX_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], (int)j, vxy);
+        cpml(f.psi[PVY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], (int)j, vyy);
+        cpml(f.psi[PVZ_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], (int)j, vzy);
     }
     if (gy > NY - NAB - F - 1 && !(adjoint_form && yb)) {
         i64 i = gx - F, j = gy - NY + NAB + F + NAB, k = gz - F;
         int ind = 2 * NAB - 1 - (int)j;
         i64 q = (i * (2 * NAB) + j) * nz + k;
-        cpml(f.psi[PVX_Y], q, f.cy[CKH], f.cy[CAH], f.cy[CBH], ind, vxy);
-        cpml(f.psi[PVY_Y], q, f.cy[CK], f.cy[CA], f.cy[CB], ind + 1, vyy);
-        cpml(f.psi[PVZ_Y], q, f.cy[CKH], f.cy[CAH], f.cy[CBH], ind, vzy);
+        cpml(f.psi[PVX_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ind, vxy);
+        cpml(f.psi[PVY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], ind + 1, vyy);
+        cpml(f.psi[PVZ_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ind, vzy);
     }
     if (gx - F < NAB) {
         i64 i = gx - F, j = gy - F, k = gz - F;
         i64 q = (i * ny + j) * nz + k;
-        cpml(f.psi[PVX_X], q, f.cx[CK], f.cx[CA], f.cx[CB], (int)i, vxx);
-        cpml(f.psi[PVY_X], q, f.cx[CKH], f.cx[CAH], f.cx[CBH], (int)i, vyx);
-        cpml(f.psi[PVZ_X], q, f.cx[CKH], f.cx[CAH], f.cx[CBH], (int)i, vzx);
+        cpml(f.psi[PVX_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], (int)i, vxx);
+        cpml(f.psi[PVY_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], (int)i, vyx);
+        cpml(f.psi[PVZ_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], (int)i, vzx);
     }
     if (gx > NX - NAB - F - 1) {
         i64 i = gx - NX + NAB + F + NAB, j = gy - F, k = gz - F;
         int ind = 2 * NAB - 1 - (int)i;
         i64 q = (i * ny + j) * nz + k;
-        cpml(f.psi[PVX_X], q, f.cx[CK], f.cx[CA], f.cx[CB], ind + 1, vxx);
-        cpml(f.psi[PVY_X], q, f.cx[CKH], f.cx[CAH], f.cx[CBH], ind, vyx);
-        cpml(f.psi[PVZ_X], q, f.cx[CKH], f.cx[CAH], f.cx[CBH], ind, vzx);
+        cpml(f.psi[PVX_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, vxx);
+        cpml(f.psi[PVY_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, vyx);
+        cpml(f.psi[PVZ_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, vzx);
     }
 }
 
@@ -1066,15 +727,15 @@ __device__ __forceinline__ void cpml_v3d_q4(const Grid &g, const Fields &f, int 
                 i64 i = gx - F, jj = gy - F, k = gz - NZ + NAB + F + NAB;
                 int ind = 2 * NAB - 1 - (int)k;
                 i64 q = (i * ny + jj) * (2 * NAB) + k;
-                cpml(f.psi[PSXZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], ind + 1, sxz_z.v[j]);
-                cpml(f.psi[PSYZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], ind + 1, syz_z.v[j]);
-                cpml(f.psi[PSZZ_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], ind, szz_z.v[j]);
+                cpml(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, sxz_z.v[j]);
+                cpml(f.psi[PSYZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, syz_z.v[j]);
+                cpml(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, szz_z.v[j]);
             } else if (!g.freesurf && gz - F < NAB) {
                 i64 i = gx - F, jj = gy - F, k = gz - F;
                 i64 q = (i * ny + jj) * (2 * NAB) + k;
-                cpml(f.psi[PSXZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], (int)k, sxz_z.v[j]);
-                cpml(f.psi[PSYZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], (int)k, syz_z.v[j]);
-                cpml(f.psi[PSZZ_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], (int)k, szz_z.v[j]);
+                cpml(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, sxz_z.v[j]);
+                cpml(f.psi[PSYZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, syz_z.v[j]);
+                cpml(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, szz_z.v[j]);
             }
         }
     }
@@ -1481,16 +1142,16 @@ __device__ __forceinline__ void cpml_s3d_q4(const Grid &g, const Fields &f, int 
                 i64 i = gx - F, jj = gy - F, k = gz - NZ + NAB + F + NAB;
                 int ind = 2 * NAB - 1 - (int)k;
                 i64 q = (i * ny + jj) * (2 * NAB) + k;
-                cpml(f.psi[PVX_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], ind, vxz.v[j]);
-                cpml(f.psi[PVY_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], ind, vyz.v[j]);
-                cpml(f.psi[PVZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], ind + 1, vzz.v[j]);
+                cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vxz.v[j]);
+                cpml(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vyz.v[j]);
+                cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, vzz.v[j]);
             }
             if (!g.freesurf && gz - F < NAB) {
                 i64 i = gx - F, jj = gy - F, k = gz - F;
                 i64 q = (i * ny + jj) * (2 * NAB) + k;
-                cpml(f.psi[PVX_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], (int)k, vxz.v[j]);
-                cpml(f.psi[PVY_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], (int)k, vyz.v[j]);
-                cpml(f.psi[PVZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], (int)k, vzz.v[j]);
+                cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, vxz.v[j]);
+                cpml(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, vyz.v[j]);
+                cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, vzz.v[j]);
             }
         }
     }
@@ -2116,15 +1777,15 @@ __device__ __forceinline__ void cpml_s3d_adj_q4(const Grid &g, const Fields &f, 
                 i64 i = gx - F, jj = gy - F, k = gz - NZ + NAB + F + NAB;
                 int ind = 2 * NAB - 1 - (int)k;
                 i64 q = (i * ny + jj) * (2 * NAB) + k;
-                cpml(f.psi[PVX_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], ind, vxz.v[j]);
-                cpml(f.psi[PVY_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], ind, vyz.v[j]);
-                cpml(f.psi[PVZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], ind + 1, vzz.v[j]);
+                cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vxz.v[j]);
+                cpml(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vyz.v[j]);
+                cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, vzz.v[j]);
             } else if (!g.freesurf && gz - F < NAB) {
                 i64 i = gx - F, jj = gy - F, k = gz - F;
                 i64 q = (i * ny + jj) * (2 * NAB) + k;
-                cpml(f.psi[PVX_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], (int)k, vxz.v[j]);
-                cpml(f.psi[PVY_Z], q, f.cz[CKH], f.cz[CAH], f.cz[CBH], (int)k, vyz.v[j]);
-                cpml(f.psi[PVZ_Z], q, f.cz[CK], f.cz[CA], f.cz[CB], (int)k, vzz.v[j]);
+                cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, vxz.v[j]);
+                cpml(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, vyz.v[j]);
+                cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, vzz.v[j]);
             }
         }
     }
@@ -2718,18 +2379,18 @@ __global__ void __launch_bounds__(256) k_v2d_acc(Grid g, Fields f)
     if (g.abs_type == 1) {
         if (gz > NZ - NAB - F - 1) {
             int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
-            cpml(f.psi[PSZZ_Z], (i64)i * (2 * NAB) + k, f.cz[CKH], f.cz[CAH], f.cz[CBH], ind, p_z);
+            cpml(f.psi[PSZZ_Z], (i64)i * (2 * NAB) + k, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, p_z);
         } else if (!g.freesurf && gz - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PSZZ_Z], (i64)i * (2 * NAB) + k, f.cz[CKH], f.cz[CAH], f.cz[CBH], k, p_z);
+            cpml(f.psi[PSZZ_Z], (i64)i * (2 * NAB) + k, f.kinv[2][1], f.cz[CAH], f.cz[CBH], k, p_z);
         }
         if (gx - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PSXX_X], (i64)i * g.nz + k, f.cx[CKH], f.cx[CAH], f.cx[CBH], i, p_x);
+            cpml(f.psi[PSXX_X], (i64)i * g.nz + k, f.kinv[0][1], f.cx[CAH], f.cx[CBH], i, p_x);
         }
         if (gx > NX - NAB - F - 1) {
             int i = gx - NX + NAB + F + NAB, k = gz - F, ind = 2 * NAB - 1 - i;
-            cpml(f.psi[PSXX_X], (i64)i * g.nz + k, f.cx[CKH], f.cx[CAH], f.cx[CBH], ind, p_x);
+            cpml(f.psi[PSXX_X], (i64)i * g.nz + k, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, p_x);
         }
     }
     float vx = f.w[VX][iv] + p_x * __ldg(f.p[PRIP] + ip);
@@ -2757,18 +2418,18 @@ __device__ __forceinline__ void s2d_acc_cell(const Grid &g, const Fields &f, int
     if (g.abs_type == 1) {
         if (gz > NZ - NAB - F - 1) {
             int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
-            cpml(f.psi[PVZ_Z], (i64)i * (2 * NAB) + k, f.cz[CK], f.cz[CA], f.cz[CB], ind + 1, vzz);
+            cpml(f.psi[PVZ_Z], (i64)i * (2 * NAB) + k, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, vzz);
         } else if (!g.freesurf && gz - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PVZ_Z], (i64)i * (2 * NAB) + k, f.cz[CK], f.cz[CA], f.cz[CB], k, vzz);
+            cpml(f.psi[PVZ_Z], (i64)i * (2 * NAB) + k, f.kinv[2][0], f.cz[CA], f.cz[CB], k, vzz);
         }
         if (gx - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PVX_X], (i64)i * g.nz + k, f.cx[CK], f.cx[CA], f.cx[CB], i, vxx);
+            cpml(f.psi[PVX_X], (i64)i * g.nz + k, f.kinv[0][0], f.cx[CA], f.cx[CB], i, vxx);
         }
         if (gx > NX - NAB - F - 1) {
             int i = gx - NX + NAB + F + NAB, k = gz - F, ind = 2 * NAB - 1 - i;
-            cpml(f.psi[PVX_X], (i64)i * g.nz + k, f.cx[CK], f.cx[CA], f.cx[CB], ind + 1, vxx);
+            cpml(f.psi[PVX_X], (i64)i * g.nz + k, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, vxx);
         }
     }
     float p = f.w[SXX][iv];
@@ -2829,18 +2490,18 @@ __global__ void __launch_bounds__(256) k_v2d_sh(Grid g, Fields f)
     if (g.abs_type == 1) {
         if (gz > NZ - NAB - F - 1) {
             int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
-            cpml(f.psi[PSYZ_Z], (i64)i * (2 * NAB) + k, f.cz[CK], f.cz[CA], f.cz[CB], ind + 1, syz_z);
+            cpml(f.psi[PSYZ_Z], (i64)i * (2 * NAB) + k, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, syz_z);
         } else if (!g.freesurf && gz - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PSYZ_Z], (i64)i * (2 * NAB) + k, f.cz[CK], f.cz[CA], f.cz[CB], k, syz_z);
+            cpml(f.psi[PSYZ_Z], (i64)i * (2 * NAB) + k, f.kinv[2][0], f.cz[CA], f.cz[CB], k, syz_z);
         }
         if (gx - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PSXY_X], (i64)i * g.nz + k, f.cx[CK], f.cx[CA], f.cx[CB], i, sxy_x);
+            cpml(f.psi[PSXY_X], (i64)i * g.nz + k, f.kinv[0][0], f.cx[CA], f.cx[CB], i, sxy_x);
         }
         if (gx > NX - NAB - F - 1) {
             int i = gx - NX + NAB + F + NAB, k = gz - F, ind = 2 * NAB - 1 - i;
-            cpml(f.psi[PSXY_X], (i64)i * g.nz + k, f.cx[CK], f.cx[CA], f.cx[CB], ind, sxy_x);
+            cpml(f.psi[PSXY_X], (i64)i * g.nz + k, f.kinv[0][0], f.cx[CA], f.cx[CB], ind, sxy_x);
         }
     }
     float vy = f.w[VY][iv] + (sxy_x + syz_z) * __ldg(f.p[PRHO] + ip);
@@ -2869,18 +2530,18 @@ __global__ void __launch_bounds__(256) k_s2d_sh(Grid g, Fields f)
     if (g.abs_type == 1) {
         if (gz > NZ - NAB - F - 1) {
             int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
-            cpml(f.psi[PVY_Z], (i64)i * (2 * NAB) + k, f.cz[CKH], f.cz[CAH], f.cz[CBH], ind, vyz);
+            cpml(f.psi[PVY_Z], (i64)i * (2 * NAB) + k, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vyz);
         } else if (!g.freesurf && gz - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PVY_Z], (i64)i * (2 * NAB) + k, f.cz[CKH], f.cz[CAH], f.cz[CBH], k, vyz);
+            cpml(f.psi[PVY_Z], (i64)i * (2 * NAB) + k, f.kinv[2][1], f.cz[CAH], f.cz[CBH], k, vyz);
         }
         if (gx - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PVY_X], (i64)i * g.nz + k, f.cx[CKH], f.cx[CAH], f.cx[CBH], i, vyx);
+            cpml(f.psi[PVY_X], (i64)i * g.nz + k, f.kinv[0][1], f.cx[CAH], f.cx[CBH], i, vyx);
         }
         if (gx > NX - NAB - F - 1) {
             int i = gx - NX + NAB + F + NAB, k = gz - F, ind = 2 * NAB - 1 - i;
-            cpml(f.psi[PVY_X], (i64)i * g.nz + k, f.cx[CKH], f.cx[CAH], f.cx[CBH], ind, vyx);
+            cpml(f.psi[PVY_X], (i64)i * g.nz + k, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, vyx);
         }
     }
     float mu = __ldg(f.p[PMU] + ip);

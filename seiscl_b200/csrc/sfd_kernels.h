@@ -46,6 +46,29 @@ void launch_surface(const Grid &g, const Fields &f, int pdir, cudaStream_t st);
 // 2D P-SV and acoustic forward: stress update, free surface, receivers of
 // step tl.t and sources of step tl.tsrc in one launch (false: not 2D)
 bool launch_update_s_step(const Grid &g, const Fields &f, const StepTail &tl, cudaStream_t st);
+// 2D P-SV modelling with the wave fields resident on chip (sfd_resident2d.cu)
+struct Res2d {              // tiles of a launch: ctas = ntz x ntx x shots, 0 where it does not apply
+    int ntz, ntx, tz, tx;   // tiles along z and x, the largest tile
+    int side, ctas, F, nc;  // longer side of a tile, CTAs, half width, cells per thread
+    size_t smem;
+};
+struct Res2dRun {           // a segment of the time loop: steps t0 .. t1-1 of tmax
+    PointSet rec, src;
+    const float *stf;       // [nsrc][nt_total]
+    float *out;             // [nsel][nrec][nt_total]
+    unsigned outmask;
+    int nt_total, t0, t1, tmax;
+    BndSlot bnd;            // boundary shells to save (nfield = 0: none), in storage type prec
+    int prec;
+    unsigned long long *words;   // exchange words, zeroed before the run's first segment
+    int *first_bad, *status;
+};
+constexpr int RES2D_SEGMENT = 256;   // steps of one launch: bounds how long it holds the SMs
+Res2d resident2d_shape(const Grid &g, int nb, int npoints);
+int64_t resident2d_words(const Res2d &r);
+int64_t resident2d_bytes(const Grid &g, int batch);   // exchange words of launches of up to `batch` shots
+cudaError_t launch_resident2d(const Grid &g, const Fields &f, const Res2d &r, const Res2dRun &a, int device,
+                              cudaStream_t st);
 void launch_savebnd(const Grid &g, const Fields &f, const BndSlot &b, int prec, int64_t tofs, cudaStream_t st);
 void launch_update_adj(const Grid &g, const Fields &f, const AdjFields &a, bool stress, int prec, cudaStream_t st);
 void launch_surface_adj(const Grid &g, const Fields &f, const AdjFields &a, float *q, cudaStream_t st);

@@ -188,11 +188,11 @@ __device__ __host__ inline BndDims bnd_dims(const Grid &g)
     b.NXbnd = g.NX - 2 * g.F - 2 * g.nab;
     b.NYbnd = g.nd == 3 ? g.NY - 2 * g.F - 2 * g.nab : 1;
     if (!g.freesurf) {
-        b.NZbnd = g.NZ - 2 * g.F - 2 * g.nab;
+        b.NZbnd = g.NZl - 2 * g.F - 2 * g.nab;
         b.lbnd = g.F + g.nab;
         b.lbnds = g.F + g.nab;
     } else {
-        b.NZbnd = g.NZ - 2 * g.F - g.nab;
+        b.NZbnd = g.NZl - 2 * g.F - g.nab;
         b.lbnd = g.F + g.nab;
         b.lbnds = g.F;
     }
@@ -281,11 +281,27 @@ __device__ __forceinline__ void apply_taper(const Grid &g, const float *taper, i
         for (int q = 0; q < NF; q++) stv(fs[q] + iv, ldv(fs[q] + iv) * t);
     };
     if (!g.freesurf && gz - F < NAB) mul(__ldg(taper + gz - F));
-    if (gz > g.NZ - NAB - F - 1) mul(__ldg(taper + g.NZ - F - gz - 1));
+    if (gz > g.NZl - NAB - F - 1 && gz < g.NZl - F) mul(__ldg(taper + g.NZl - F - gz - 1));
     if (g.nd == 3) {
         if (gy - F < NAB) mul(__ldg(taper + gy - F));
         if (gy > g.NY - NAB - F - 1) mul(__ldg(taper + g.NY - F - gy - 1));
     }
+    if (gx - F < NAB) mul(__ldg(taper + gx - F));
+    if (gx > g.NX - NAB - F - 1) mul(__ldg(taper + g.NX - F - gx - 1));
+}
+
+template <int NF>
+__device__ __forceinline__ void taper_regs(const Grid &g, const float *taper, int gz, int gy, int gx, float (&v)[NF])
+{
+    const int F = g.F, NAB = g.nab;
+    auto mul = [&](float t) {
+#pragma unroll
+        for (int q = 0; q < NF; q++) v[q] *= t;
+    };
+    if (!g.freesurf && gz - F < NAB) mul(__ldg(taper + gz - F));
+    if (gz > g.NZl - NAB - F - 1 && gz < g.NZl - F) mul(__ldg(taper + g.NZl - F - gz - 1));
+    if (gy - F < NAB) mul(__ldg(taper + gy - F));
+    if (gy > g.NY - NAB - F - 1) mul(__ldg(taper + g.NY - F - gy - 1));
     if (gx - F < NAB) mul(__ldg(taper + gx - F));
     if (gx > g.NX - NAB - F - 1) mul(__ldg(taper + g.NX - F - gx - 1));
 }

@@ -22,12 +22,12 @@ typedef int64_t i64;
 __global__ void __launch_bounds__(256) k_gradient_out(GradOut o)
 {
     for (i64 q = (i64)blockIdx.x * blockDim.x + threadIdx.x; q < o.count; q += (i64)gridDim.x * blockDim.x) {
-        const i64 i = o.first + q;
+        const i64 u = o.first + q, i = u / o.nz * o.pitch + u % o.nz;
         double s[3];   // M, mu, rho
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             s[k] = o.sum[k][i];
-            for (int b = 1; b < o.ncopy; b++) s[k] += o.sum[k][(i64)b * o.n + i];
+            for (int b = 1; b < o.ncopy; b++) s[k] += o.sum[k][b * o.copy + i];
         }
         if (o.par_type >= 0) {
             const double rho = 1.0 / o.rho[i] * o.dt / o.dh;

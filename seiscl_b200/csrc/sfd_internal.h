@@ -49,6 +49,10 @@ struct Grid {
     int F;                  // stencil half width
     int nz, ny, nx;         // physical sizes (ny = 1 in 2D)
     int NZ, NY, NX;         // padded sizes
+    int zpad, zshift;       // 3D, 4-cell kernels: dummy z rows at the bottom that fill nz up to whole quads (nz and NZ
+                            // count them; parameters are zero there), and the elements by which the fields'
+                            // base is moved so that every row's first physical cell is 16-byte aligned
+    int NZl;                // NZ without the dummy rows
     int nab, L, freesurf, abs_type;
     int64_t nvol;           // padded cell count
     float hc[6];            // FD coefficients

@@ -24,6 +24,12 @@ bool tma_ready(const Grid &g, const Fields &f);  // the TMA kernels will run for
 int tma_take_status();      // 1 if a TMA stage of the last launches never arrived (and clears it)
 // 3D stress-update family of a plan: 0 not 3D, 1 general, 2 register-blocked,
 // 3 TMA-pipelined, 4 streaming, 5 4-cell vectorised
+// 4-cell vectorised 3D kernels (sfd_quad3d.cuh), half width 2 or 4;
+// quad_update_s returns whether the launch applied the free surface
+template <int F> void quad_update_v(const Grid &g, const Fields &f, cudaStream_t st);
+template <int F> bool quad_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool surf);
+template <int F>
+void quad_update_adj(const Grid &g, const Fields &f, const AdjFields &a, bool stress, int prec, cudaStream_t st);
 int stress_family(const Grid &g, const Fields &f);
 // fold_surface: single-shot FP32 4-cell kernels may apply the free surface in
 // the same launch (true returned: the caller skips launch_surface)
@@ -103,8 +109,9 @@ void launch_pack(const PackSet &ps, int prec, bool unpack, cudaStream_t st, bool
 
 // gradient sums -> gradient of the parameters (sfd_gradient.cu)
 struct GradOut {
-    const double *sum[3];   // M, mu, rho: [ncopy][n]
-    int ncopy;
+    const double *sum[3];   // M, mu, rho: ncopy copies, `copy` apart, of rows of `pitch` with nz cells each
+    int ncopy, nz, pitch;
+    int64_t copy;
     int64_t n, first, count;   // cells of a copy; the range of this launch
     int par_type;           // param_type of the chain rule, -1: the sums as they are
     const float *rho, *M, *mu;

@@ -70,7 +70,7 @@ __global__ void k_noalloc_map(Grid g, double DH, const float *src_pos, int nsrc,
     int k = (int)((double)pos[2] / DH) + g.F;
     int64_t cell = -1;
     if (i >= g.F && i <= g.NX - g.F - 1) {
-        if (j < 0 || j >= g.NY || k < 0 || k >= g.NZ) atomicExch(bad, 1);
+        if (j < 0 || j >= g.NY || k < 0 || k >= g.NZl) atomicExch(bad, 1);
         else cell = ((int64_t)i * g.NY + j) * g.NZ + k;
     }
     if (gid < nsrc) {
@@ -108,6 +108,7 @@ extern "C" int sfd_forward_noalloc(sfd_plan *p, const float *src_pos, const floa
     // one shot, whatever the plan's batch; a local copy leaves the plan's
     // state as it was
     Grid g = p->g;
+    g.zshift = 0;   // fields in the scratch array start unshifted
     g.nb = 1;
     unsigned omask = 0;
     int nsel = 0;

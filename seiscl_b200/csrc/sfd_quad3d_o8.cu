@@ -1,0 +1,9 @@
+// sfd_quad3d_o8.cu -- the 4-cell 3D forward kernels of order 8.
+#include "sfd_quad3d.cuh"
+
+namespace sfd {
+
+template void quad_update_v<4>(const Grid &, const Fields &, cudaStream_t);
+template bool quad_update_s<4>(const Grid &, const Fields &, cudaStream_t, bool);
+
+}  // namespace sfd

@@ -1,0 +1,128 @@
+"""3D grids whose rows are not whole aligned quads (nz = 4 n + 2, or order 4)
+on the 4-cell kernels, which the default selection gives them through dummy
+rows and a shifted field base, against the one-cell general kernels: forward
+runs, batches, gradients from saved boundaries and from checkpoints, the DFT
+gradient, movies, final fields.
+
+Tolerance: both sides are FP32 with the same operation order up to the
+contraction of products; 5e-6 relative L2 over some tens of steps, as for the
+other kernel families (tests/test_gpu_parity.py), 2e-5 for gradients, whose
+products of two fields double it and whose boundary shells amplify it."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from tests._cases import engine_config, make_case, rel_l2
+
+CASES = [
+    dict(nz=38, ny=30, nx=34, nt=60, nab=8, fdorder=8, freesurf=1, L=0),
+    dict(nz=38, ny=30, nx=34, nt=60, nab=8, fdorder=4, freesurf=1, L=1),
+    dict(nz=40, ny=26, nx=30, nt=60, nab=8, fdorder=4, freesurf=0, L=2),
+    dict(nz=42, ny=27, nx=31, nt=60, nab=6, fdorder=8, freesurf=0, L=3),       # slab edges inside quads
+    dict(nz=26, ny=24, nx=25, nt=50, nab=12, fdorder=4, freesurf=0, L=0),      # slabs nearly touching
+    dict(nz=22, ny=21, nx=20, nt=40, nab=12, fdorder=8, freesurf=0, L=1),      # overlapping
+    dict(nz=34, ny=25, nx=29, nt=60, nab=7, fdorder=4, freesurf=1, L=1, abs_type=2, src_type=2),
+    dict(nz=18, ny=140, nx=20, nt=40, nab=4, fdorder=8, freesurf=1, L=0, src_type=1),
+]
+IDS = ["%dx%dx%d-o%d-L%d" % (k["nz"], k["ny"], k["nx"], k["fdorder"], k["L"]) for k in CASES]
+OUTS = ["vx", "vy", "vz", "p"]
+
+
+def _case(kw):
+    """make_case with the source at the centre and receivers across the grid,
+    whatever the absorbing layers leave."""
+    cfg, model, acq = make_case(nd=3, **kw)
+    nz, ny, nx = kw["nz"], kw["ny"], kw["nx"]
+    acq["src_pos"][0, :3] = [nx // 2 * 10.0, ny // 2 * 10.0, nz // 2 * 10.0]
+    x = np.arange(2, nx - 2, 3)
+    rec = np.zeros((2 * len(x), 8), np.float32)
+    rec[:, 0], rec[:, 1] = np.tile(x, 2) * 10.0, ny // 2 * 10.0
+    rec[:, 2] = np.repeat([2, nz - 3], len(x)) * 10.0
+    rec[:, 4] = np.arange(1, len(rec) + 1)
+    acq["rec_pos"] = rec
+    return cfg, model, acq
+
+
+def _plans(cfg, model, **kw):
+    from seiscl_b200.engine import Plan
+
+    out = []
+    for kernels in ("fast", "general"):
+        p = Plan(dataclasses.replace(engine_config(cfg), kernels=kernels, **kw))
+        p.set_model(model["vp"], model["vs"], model["rho"], model["taup"], model["taus"])
+        out.append(p)
+    return out
+
+
+def _close(a, b, tol):
+    for k in b:
+        assert a[k].shape == b[k].shape and rel_l2(a[k], b[k]) < tol, (k, rel_l2(a[k], b[k]))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kw", CASES, ids=IDS)
+def test_forward(kw, cuda_device):
+    cfg, model, acq = _case(kw)
+    got = []
+    for p in _plans(cfg, model):
+        mov = p.set_movie(20, ["vz"])
+        d = p.forward(acq["src_pos"], acq["src"], acq["rec_pos"], OUTS)
+        d.update({"f%d" % i: p.debug_array(0, i, p.nvol) for i in range(9)}, movie=mov["vz"])
+        if cfg["L"]:
+            d["rxx"] = p.debug_array(2, 0, p.nvol * cfg["L"])
+        if cfg["abs_type"] == 1:
+            d["psi"] = p.debug_array(5, 12, 2 * cfg["nab"] * cfg["nx"] * cfg["nz"])
+        d["M"] = p.debug_array(3, 0, cfg["nz"] * cfg["ny"] * cfg["nx"])
+        got.append(d)
+    assert np.abs(got[1]["vz"]).max() > 0 and (p.NZp, p.nvol) == (kw["nz"] + kw["fdorder"], got[1]["f0"].size)
+    _close(*got, 5e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kw", CASES[:4], ids=IDS[:4])
+@pytest.mark.parametrize("how", [dict(), dict(precision="bf16"), dict(checkpoint=17), dict(batch=2),
+                                 dict(back_prop_type=2, gradfreqs=(40.0, 60.0))],
+                         ids=["bnd", "bnd-bf16", "ckpt", "batch", "dft"])
+def test_gradient(kw, how, cuda_device):
+    cfg, model, acq = _case(kw)
+    shots = [(acq["src_pos"], acq["src"] * (1 + b), acq["rec_pos"]) for b in range(how.get("batch", 1))]
+    outs = OUTS[:3]
+    got = []
+    for p in _plans(cfg, model, **how):
+        d = p.forward_batch(shots, outs, save_boundaries=True)
+        p.zero_gradient()
+        if not got:
+            res = d   # the same adjoint sources for both
+        p.adjoint_batch(shots, res)
+        got.append(p.gradient())
+    # BF16 shells round a value either way when it lies near a tie: 2^-9 of
+    # a few values in a thousand
+    _close(*got, 1e-3 if how.get("precision") else 2e-5)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kw", [CASES[0], CASES[2], CASES[3]], ids=[IDS[0], IDS[2], IDS[3]])
+def test_fp16_fields(kw, cuda_device):
+    """The same FP16 storage in both layouts: one rounding of 2^-11 a step on
+    fields that differ in the last FP32 bit, far below the storage's own error."""
+    from seiscl_b200.engine import Plan
+
+    cfg, model, acq = _case(dict(kw, nt=150))
+    got = []
+    for field in ("fp16", "fp32"):
+        p = Plan(dataclasses.replace(engine_config(cfg), field_precision=field))
+        p.set_model(model["vp"], model["vs"], model["rho"], model["taup"], model["taus"])
+        got.append(p.forward(acq["src_pos"], acq["src"], acq["rec_pos"], OUTS))
+    num = sum(float(((got[0][n].astype(np.float64) - got[1][n]) ** 2).sum()) for n in OUTS)
+    den = sum(float((got[1][n].astype(np.float64) ** 2).sum()) for n in OUTS)
+    assert 0 < den and num / den < 1e-3   # the criterion of tests/test_gpu_parity.py
+
+
+def test_footprint_counts_dummy_rows():
+    from seiscl_b200.engine import Config, footprint
+
+    def b(nz, **kw):
+        return footprint(Config(N=[nz, 30, 31], ND=3, NT=10, FDORDER=8, nab=8, **kw))
+
+    assert b(42) == b(44) and b(42, kernels="general") < b(42)

@@ -163,11 +163,14 @@ oom:
     return fail(p, SFD_ERR_MEMORY, std::string("device allocation failed: ") + cudaGetErrorString(e));
 }
 
+struct PointLayout {
+    bool inside;   // every point that is not dropped lies on a physical cell along z, none in the padding
+    bool apart;    // no receiver on a source's cell
+};
 // host-side mapping of a shot's sources and receivers, uploaded to the device
-// (inside: whether every point that is not dropped lies on a physical cell
-// along z, none in the padding above or below)
+// (how: see PointLayout)
 int upload_shots(sfd_plan *p, int nshot, const sfd_shot *shots, int mask, PointSet &S, PointSet &R,
-                 cudaStream_t st, bool *inside = nullptr)
+                 cudaStream_t st, PointLayout *how = nullptr)
 {
     bool in = true;
     const Grid &g = p->g;
@@ -208,7 +211,14 @@ int upload_shots(sfd_plan *p, int nshot, const sfd_shot *shots, int mask, PointS
             in = in && k >= F && k < g.NZ - F;
         }
     }
-    if (inside) *inside = in;
+    if (how) {
+        how->inside = in;
+        std::vector<int64_t> sorted(scell);
+        std::sort(sorted.begin(), sorted.end());
+        how->apart = true;
+        for (int64_t c : rcell)
+            if (c >= 0 && std::binary_search(sorted.begin(), sorted.end(), c)) { how->apart = false; break; }
+    }
     {
         if (nsrc) {
             CKC(cudaMemcpyAsync(p->d_src_cell, scell.data(), sizeof(int64_t) * nsrc, cudaMemcpyHostToDevice, st));
@@ -794,7 +804,7 @@ int adjoint_ckpt(sfd_plan *p, const PointSet &S, const PointSet &R, unsigned oma
             for (int t = thi; t >= tlo; t--) {
                 ckpt_slot(p, t - t0, a);
                 if (g.freesurf) launch_surface_adj(ga, fa, a, p->d_surf_q, s);
-                launch_residuals(ga, a, R, p->d_res, NT, t, omask, s);
+                launch_residuals(ga, fa, a, R, p->d_res, NT, t, omask, S, p->d_src, -1, s);
                 launch_update_adj(ga, fa, a, true, p->cfg.precision, s);
                 launch_update_adj(ga, fa, a, false, p->cfg.precision, s);
                 if (t % FINITE_CHECK_EVERY == 0 || t == tmin + 1)
@@ -923,7 +933,7 @@ int adjoint_dft(sfd_plan *p, const PointSet &R, unsigned omask, cudaStream_t st)
     int rc2 = run_loop(p, p->gadj, key.s, st, [&](cudaStream_t s) {
         for (int t = p->cfg.tmax - 1; t > tmin; t--) {
             if (g.freesurf) launch_surface_adj(ga, p->f, a, p->d_surf_q, s);
-            launch_residuals(ga, a, R, p->d_res, NT, t, omask, s);
+            launch_residuals(ga, p->f, a, R, p->d_res, NT, t, omask, R, nullptr, -1, s);
             launch_update_adj(ga, p->f, a, true, SFD_PREC_FP32, s);
             launch_update_adj(ga, p->f, a, false, SFD_PREC_FP32, s);
             if ((t - tmin) % p->dtnyq == 0) dft_sample(p, 1, (t - tmin) / p->dtnyq, s);
@@ -1018,12 +1028,12 @@ void init_grid(const sfd_config &c, Grid &g)
     g.nz = c.n[0];
     if (c.nd == 3) { g.ny = c.n[1]; g.nx = c.n[2]; }
     else { g.ny = 1; g.nx = c.n[1]; }
-    // 3D grids of the default selection take the 4-cell kernels at orders 4
+    // grids of the default selection take the 4-cell kernels at orders 4
     // and 8 whatever nz: rows of 4 n + 2 cells get two dummy rows, and at
     // order 4 the fields' base moves by two elements.  One-cell streaming
     // kernels on the same grids were 1.7-2.4 times slower.
     g.zpad = g.zshift = 0;
-    if (c.nd == 3 && c.kernels == 0 && (g.F == 2 || g.F == 4) && c.L <= 3) {
+    if ((c.nd == 3 || (c.nd == 2 && c.field_precision == 0)) && c.kernels == 0 && (g.F == 2 || g.F == 4) && c.L <= 3) {
         g.zpad = (4 - g.nz % 4) % 4;
         g.zshift = (4 - g.F) % 4;
     }
@@ -1336,8 +1346,8 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
     unsigned omask = outmask_of(outsel, g.nd, &nsel);
     if ((rc = ensure_shot_buffers(p, sb.nsrc, sb.nrec, nsel))) return rc;
     PointSet S, R;
-    bool points_inside;
-    if ((rc = upload_shots(p, nshot, shots, mask, S, R, st, &points_inside))) return rc;
+    PointLayout points;
+    if ((rc = upload_shots(p, nshot, shots, mask, S, R, st, &points))) return rc;
     if ((rc = zero_forward_state(p, st))) return rc;
     // a batch without receivers has no seismogram buffer (none is allocated
     // for zero traces): no copy of zero bytes goes to a null pointer
@@ -1431,7 +1441,8 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
     // blocks of a launch a fence and an atomic round trip, and a surface
     // done by the top blocks of the stress kernel holds them on the SMs;
     // both made a 256^3 step slower (1.31 and 1.19 ms against 1.13).
-    const bool fuse2d = (g.nd == 2 || g.nd == 22) && g.kernels != 1 && !save_boundaries && !dft && !mv.n;
+    const bool quads2d = quad2d_ok(g);   // their step: velocity, stress with the surface, points
+    const bool fuse2d = (g.nd == 22 || (g.nd == 2 && !quads2d)) && g.kernels != 1 && !save_boundaries && !dft && !mv.n;
     if (fuse2d) CKC(cudaMemsetAsync(p->d_ticket, 0, sizeof(int), st));
     // 3D modelling runs: one launch per step for the velocity, stress and
     // free-surface updates (sfd_kernels.cu, fused 3D forward step)
@@ -1441,10 +1452,10 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
     // 2D P-SV runs whose wave fields fit on chip: the time loop in segments,
     // one cooperative launch each (sfd_resident2d.cu)
     const Res2d rs = resident2d_shape(g, nshot, S.n + R.n);
-    const bool resident = rs.ctas > 0 && p->d_words && points_inside && !dft && !ckpt && !mv.n;
+    const bool resident = rs.ctas > 0 && p->d_words && points.inside && !dft && !ckpt && !mv.n;
     if (resident) CKC(cudaMemsetAsync(p->d_words, 0, sizeof(*p->d_words) * (size_t)resident2d_words(rs), st));
     LoopKey key;
-    key.add(mv.n); key.add(p->movout); key.add(p->d_mov); key.add(fuse2d); key.add(p->d_ticket); key.add(fuse3d);
+    key.add(points.apart); key.add(mv.n); key.add(p->movout); key.add(p->d_mov); key.add(fuse2d); key.add(p->d_ticket); key.add(fuse3d);
     key.add(1); key.add(p->g); key.add(p->f); key.add_points(S); key.add_points(R); key.add(p->d_src);
     key.add(p->d_seis); key.add(omask); key.add(dft); key.add(save_boundaries != 0); key.add(bs);
     key.add(p->cfg.precision); key.add(tmax); key.add(tmin); key.add(ckpt); key.add(p->d_snap);
@@ -1490,18 +1501,29 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
             }
             return;
         }
+        // receivers of a step and sources of the next in one launch, unless
+        // something must see the fields between the two
+        const bool merged = points.apart && !dft && !ckpt && !mv.n && (g.nd == 3 || quads2d);
+        if (merged && tmax > 0) launch_sources(g, p->f, S, p->d_src, NT, 0, 1, s);
         for (int t = 0; t < tmax; t++) {
             // the state after t steps, before the sources of step t (time_stepping.c:766-781)
             if (dft && t >= tmin && (t - tmin) % p->dtnyq == 0) dft_sample(p, 0, (t - tmin) / p->dtnyq, s);
             if (ckpt && t % p->cfg.checkpoint == 0) ckpt_snapshot(p, t / p->cfg.checkpoint, false, s);
-            launch_sources(g, p->f, S, p->d_src, NT, t, 1, s);
+            if (!merged) launch_sources(g, p->f, S, p->d_src, NT, t, 1, s);
             launch_update_v(g, p->f, s);
             // the stress kernel may apply the free surface itself, unless the
             // saved boundaries must see the stresses before it
-            const bool folded = launch_update_s(g, p->f, s, !bnd_shells);
-            if (bnd_shells) launch_savebnd(g, p->f, bs, p->cfg.precision, (int64_t)t * g.nbnd, s);
-            if (g.freesurf && !folded) launch_surface(g, p->f, 1, s);
-            launch_record(g, p->f, R, p->d_seis, NT, t, omask, s);
+            if (quads2d) {
+                launch_quad2d_s(g, p->f, bs, p->cfg.precision, (int64_t)t * g.nbnd, g.freesurf != 0, s);
+            } else {
+                const bool folded = launch_update_s(g, p->f, s, !bnd_shells);
+                if (bnd_shells) launch_savebnd(g, p->f, bs, p->cfg.precision, (int64_t)t * g.nbnd, s);
+                if (g.freesurf && !folded) launch_surface(g, p->f, 1, s);
+            }
+            if (merged)
+                launch_record_sources(g, p->f, R, p->d_seis, NT, t, omask, S, p->d_src, t + 1 < tmax ? t + 1 : -1, s);
+            else
+                launch_record(g, p->f, R, p->d_seis, NT, t, omask, s);
             if (mv.n && (t + 1) % p->movout == 0) movie_snap(p, mv, (t + 1) / p->movout - 1, s);
             check(t, s);
         }
@@ -1607,18 +1629,24 @@ extern "C" int sfd_adjoint_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
     if ((rc = arm_unstable(p, st))) return rc;
     CKC(cudaEventRecord(p->ev0, st));
     int rcl = run_loop(p, p->gadj, key.s, st, [&](cudaStream_t s) {
+        // the sources a step takes out of the reconstructed fields go with the
+        // next step's residuals, unless a movie films the fields between
+        int tsrc = -1;
         for (int t = p->cfg.tmax - 1; t > p->cfg.tmin; t--) {
             for (int w = 0; w < NW; w++)
                 a.bnd[w] = p->d_bnd[w] ? (const char *)p->d_bnd[w] + p->bnd_elem * (size_t)(t - 1) * g.nbnd : nullptr;
             if (g.freesurf) launch_surface_adj(g, p->f, a, p->d_surf_q, s);
-            launch_residuals(g, a, R, p->d_res, NT, t, omask, s);
+            launch_residuals(g, p->f, a, R, p->d_res, NT, t, omask, S, p->d_src, tsrc, s);
+            tsrc = -1;
             launch_update_adj(g, p->f, a, true, p->cfg.precision, s);
             launch_update_adj(g, p->f, a, false, p->cfg.precision, s);
-            launch_sources(g, p->f, S, p->d_src, NT, t, -1, s);
+            if (mv.n) launch_sources(g, p->f, S, p->d_src, NT, t, -1, s);
+            else tsrc = t;
             if (mv.n && t % p->movout == 0) movie_snap(p, mv, (t + 1) / p->movout - 1, s);
             if (t % FINITE_CHECK_EVERY == 0 || t == p->cfg.tmin + 1)
                 launch_finite_check(g, chk, nchk, t, p->d_unstable, s);
         }
+        if (tsrc >= 0) launch_sources(g, p->f, S, p->d_src, NT, tsrc, -1, s);
     });
     if (rcl) return rcl;
     if (mv.n && (rc = movie_out(p, mv, st))) return rc;

@@ -311,13 +311,13 @@ __device__ __forceinline__ void taper_regs(const Grid &g, const float *taper, in
 __device__ __forceinline__ void cpml_v2d(const Grid &g, const Fields &f, int gz, int gx, float &sxx_x,
                                          float &szz_z, float &sxz_x, float &sxz_z)
 {
-    int F = g.F, NAB = g.nab, NZ = g.NZ, NX = g.NX;
-    if (gz > NZ - NAB - F - 1) {
+    int F = g.F, NAB = g.nab, NZ = g.NZl, NX = g.NX;
+    if (gz > NZ - NAB - F - 1 && gz < NZ - F) {
         int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
         i64 q = (i64)i * (2 * NAB) + k;
         cpml(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, sxz_z);
         cpml(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, szz_z);
-    } else if (!g.freesurf && gz - F < NAB) {
+    } else if (!g.freesurf && gz - F < NAB && gz < NZ - F) {
         int i = gx - F, k = gz - F;
         i64 q = (i64)i * (2 * NAB) + k;
         cpml(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], k, sxz_z);
@@ -341,13 +341,13 @@ __device__ __forceinline__ void cpml_v2d(const Grid &g, const Fields &f, int gz,
 __device__ __forceinline__ void cpml_s2d(const Grid &g, const Fields &f, int gz, int gx, float &vxx, float &vxz,
                                          float &vzx, float &vzz)
 {
-    int F = g.F, NAB = g.nab, NZ = g.NZ, NX = g.NX;
-    if (gz > NZ - NAB - F - 1) {
+    int F = g.F, NAB = g.nab, NZ = g.NZl, NX = g.NX;
+    if (gz > NZ - NAB - F - 1 && gz < NZ - F) {
         int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
         i64 q = (i64)i * (2 * NAB) + k;
         cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vxz);
         cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, vzz);
-    } else if (!g.freesurf && gz - F < NAB) {
+    } else if (!g.freesurf && gz - F < NAB && gz < NZ - F) {
         int i = gx - F, k = gz - F;
         i64 q = (i64)i * (2 * NAB) + k;
         cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], k, vxz);
@@ -431,6 +431,22 @@ __device__ __forceinline__ float surf2d_h(const Surf2d &s, float vxx, float vzz)
 __device__ __forceinline__ float surf2d_hr(const Surf2d &s, float b, float vxx, float vzz)
 {
     return __fmul_rn(b, __fsub_rn(__fmul_rn(s.c, vxx), __fmul_rn(s.de, vzz)));
+}
+
+// elastic P-SV gradient terms of a cell: forward stresses, adjoint increments
+struct Adj2dGrad {
+    float M, mu;
+};
+__device__ __forceinline__ Adj2dGrad adj2d_grad(int restype, float M, float mu, float sxx, float szz, float sxz,
+                                                float lsxx, float lszz, float lsxz)
+{
+    const float p = __fadd_rn(sxx, szz), lp = __fadd_rn(lsxx, lszz);
+    if (restype != 0) return Adj2dGrad{-__fmul_rn(p, lp), 0.0f};
+    const float q = __fmul_rn(2.0f, __fsub_rn(M, mu));
+    const float c1 = __fdiv_rn(1.0f, __fmul_rn(q, q)), c3 = __fdiv_rn(1.0f, __fmul_rn(mu, mu));
+    const float dM = __fmul_rn(__fmul_rn(c1, p), lp);
+    const float sh = __fmaf_rn(-c3, __fmul_rn(sxz, lsxz), dM);
+    return Adj2dGrad{-dM, __fmaf_rn(-__fmul_rn(0.25f, c3), __fmul_rn(__fsub_rn(sxx, szz), __fsub_rn(lsxx, lszz)), sh)};
 }
 
 }  // namespace sfd

@@ -15,6 +15,7 @@
 //   boundary  src/savebnd{2D,3D}.cl, src/header_injectbnd.cl
 // Arithmetic is FP32 with FMA; gradients accumulate in FP64.
 #include <algorithm>
+#include <cstring>
 #include <cstdlib>
 #include <utility>
 #include <type_traits>
@@ -847,8 +848,8 @@ __global__ void __launch_bounds__(256) k_adjv2d(Grid g, Fields f, AdjFields a)
         float szz_z = dfw<F>(f.w[SZZ], iv, 1, hc);
         float sxz_z = dbw<F>(f.w[SXZ], iv, 1, hc);
         float sxz_x = dbw<F>(f.w[SXZ], iv, g.NZ, hc);
-        vx = f.w[VX][iv] - (sxx_x + sxz_z) * rip;
-        vz = f.w[VZ][iv] - (szz_z + sxz_x) * rkp;
+        vx = __fmaf_rn(-__fadd_rn(sxx_x, sxz_z), rip, f.w[VX][iv]);
+        vz = __fmaf_rn(-__fadd_rn(szz_z, sxz_x), rkp, f.w[VZ][iv]);
         int m = inject_ind2d(g, gz, gx);
         if (m != -1) {
             vx = bnd_at<T>(g, a, VX, m);
@@ -862,15 +863,15 @@ __global__ void __launch_bounds__(256) k_adjv2d(Grid g, Fields f, AdjFields a)
     float sxz_zr = dbw<F>(a.wr[SXZ], iv, 1, hc);
     float sxz_xr = dbw<F>(a.wr[SXZ], iv, g.NZ, hc);
     if (g.abs_type == 1) cpml_v2d(g, f, gz, gx, sxx_xr, szz_zr, sxz_xr, sxz_zr);
-    float lvx = (sxx_xr + sxz_zr) * rip;
-    float lvz = (szz_zr + sxz_xr) * rkp;
+    float lvx = __fmul_rn(__fadd_rn(sxx_xr, sxz_zr), rip);
+    float lvz = __fmul_rn(__fadd_rn(szz_zr, sxz_xr), rkp);
     a.wr[VX][iv] += lvx;
     a.wr[VZ][iv] += lvz;
     if (g.abs_type == 2) {
         float *fs[2] = {a.wr[VX], a.wr[VZ]};
         apply_taper<2>(g, f.taper, gz, 0, gx, fs, iv);
     }
-    if (!g.bp2) a.grad[GRHO][ip] += (double)(-vx * lvx - vz * lvz);
+    if (!g.bp2) a.grad[GRHO][ip] += (double)__fmaf_rn(-vz, lvz, -__fmul_rn(vx, lvx));
 }
 
 template <int F, typename T>
@@ -912,9 +913,10 @@ __global__ void __launch_bounds__(256) k_adjs2d(Grid g, Fields f, AdjFields a)
         sxx = fwd_at<T>(g, a, SXX, iv); szz = fwd_at<T>(g, a, SZZ, iv); sxz = fwd_at<T>(g, a, SXZ, iv);
     } else if (L == 0) {
         sxx = f.w[SXX][iv]; szz = f.w[SZZ][iv]; sxz = f.w[SXZ][iv];
-        sxz -= fipkp * (vxz + vzx);
-        sxx -= gm * (vxx + vzz) - fm * vzz;
-        szz -= gm * (vxx + vzz) - fm * vxx;
+        const float tr = __fadd_rn(vxx, vzz);
+        sxz = __fmaf_rn(-fipkp, __fadd_rn(vxz, vzx), sxz);
+        sxx = __fsub_rn(sxx, s2d_normal(gm, tr, fm, vzz));
+        szz = __fsub_rn(szz, s2d_normal(gm, tr, fm, vxx));
     } else {
         sxx = f.w[SXX][iv]; szz = f.w[SZZ][iv]; sxz = f.w[SXZ][iv];
         float *rxx = f.r[RXX], *rzz = f.r[RZZ], *rxz = f.r[RXZ];
@@ -950,9 +952,10 @@ __global__ void __launch_bounds__(256) k_adjs2d(Grid g, Fields f, AdjFields a)
     if (g.abs_type == 1) cpml_s2d(g, f, gz, gx, vxxr, vxzr, vzxr, vzzr);
     float lsxz, lsxx, lszz;
     if (L == 0) {
-        lsxz = fipkp * (vxzr + vzxr);
-        lsxx = gm * (vxxr + vzzr) - fm * vzzr;
-        lszz = gm * (vxxr + vzzr) - fm * vxxr;
+        const float tr = __fadd_rn(vxxr, vzzr);
+        lsxz = __fmul_rn(fipkp, __fadd_rn(vxzr, vzxr));
+        lsxx = s2d_normal(gm, tr, fm, vzzr);
+        lszz = s2d_normal(gm, tr, fm, vxxr);
         a.wr[SXZ][iv] += lsxz;
         a.wr[SXX][iv] += lsxx;
         a.wr[SZZ][iv] += lszz;
@@ -986,21 +989,21 @@ __global__ void __launch_bounds__(256) k_adjs2d(Grid g, Fields f, AdjFields a)
     }
     if (g.bp2) {
     } else if (g.restype == 0) {
-        float c1 = 1.0f / ((2.0f * lM - 2.0f * lmu) * (2.0f * lM - 2.0f * lmu));
-        float c3 = 1.0f / (lmu * lmu);
-        float c5 = 0.25f * c3;
-        float dM = c1 * (sxx + szz) * (lsxx + lszz);
-        a.grad[GM][ip] += (double)(-dM);
-        a.grad[GMU][ip] += (double)(-c3 * (sxz * lsxz) + dM - c5 * ((sxx - szz) * (lsxx - lszz)));
+        const Adj2dGrad q = adj2d_grad(0, lM, lmu, sxx, szz, sxz, lsxx, lszz, lsxz);
+        a.grad[GM][ip] += (double)q.M;
+        a.grad[GMU][ip] += (double)q.mu;
         if (g.hout) {
+            float c1 = 1.0f / ((2.0f * lM - 2.0f * lmu) * (2.0f * lM - 2.0f * lmu));
+            float c3 = 1.0f / (lmu * lmu);
+            float c5 = 0.25f * c3;
+            const float dM = -q.M;
             // update_adjs2D.cl:453-457 (the mu term subtracts the gradient's dM)
             float dMH = c1 * (sxx + szz) * (sxx + szz);
             a.hess[GM][ip] += (double)dMH;
             a.hess[GMU][ip] += (double)(c3 * sxz * sxz - dM + c5 * (sxx - szz) * (sxx - szz));
         }
     } else {
-        float dM = (sxx + szz) * (lsxx + lszz);
-        a.grad[GM][ip] += (double)(-dM);
+        a.grad[GM][ip] += (double)adj2d_grad(1, lM, lmu, sxx, szz, sxz, lsxx, lszz, lsxz).M;
         if (g.hout) a.hess[GM][ip] += (double)((sxx + szz) * (sxx + szz));
     }
 }
@@ -1365,6 +1368,24 @@ __global__ void k_record(Fields f, PointSet r, float *out, int nt_total, int t, 
     if (gid < r.n) record_point<T, false>(f, r, out, nt_total, t, outmask, nd, ws, gid);
 }
 
+// receivers of step t and sources of step tsrc, for shots without a receiver
+// on a source's cell: the first `rblocks` blocks record, the rest inject
+template <class T = float>
+__global__ void k_record_sources(Fields f, PointSet r, float *out, int nt_total, int t, unsigned outmask, int nd,
+                                 WScale ws, unsigned rblocks, PointSet s, const float *src, int tsrc, float dt,
+                                 int freesurf, int F)
+{
+    pdl_trigger();
+    pdl_wait();
+    if (blockIdx.x < rblocks) {
+        const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+        if (gid < r.n) record_point<T, false>(f, r, out, nt_total, t, outmask, nd, ws, gid);
+    } else {
+        const int gid = (blockIdx.x - rblocks) * blockDim.x + threadIdx.x;
+        if (gid < s.n) source_point<T>(f, s, src, nt_total, tsrc, 1, dt, freesurf, F, ws, gid);
+    }
+}
+
 // ---------------------------------------------- fused 2D forward step tail
 // The stress kernel of a fused 2D step ends with the receivers of step t
 // and the sources of step t+1 (time_stepping.c:783-816 order: sources,
@@ -1425,8 +1446,17 @@ __global__ void __launch_bounds__(256) k_s2d_acc_step(Grid g, Fields f, StepTail
 }
 
 // src/automatic_kernels.c:631-836; res is [nsel][nrec][NT]
-__global__ void k_residuals(AdjFields a, PointSet r, const float *res, int nt_total, int t, unsigned outmask, int nd)
+// (into the adjoint fields); the blocks after the first `rblocks` take the
+// sources of step tsrc out of the forward fields
+__global__ void k_residuals(AdjFields a, PointSet r, const float *res, int nt_total, int t, unsigned outmask, int nd,
+                            unsigned rblocks, Fields f, PointSet s, const float *src, int tsrc, float dt, int freesurf,
+                            int F, WScale ws)
 {
+    if (blockIdx.x >= rblocks) {
+        const int q = (blockIdx.x - rblocks) * blockDim.x + threadIdx.x;
+        if (q < s.n) source_point<float>(f, s, src, nt_total, tsrc, -1, dt, freesurf, F, ws, q);
+        return;
+    }
     int gid = blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= r.n) return;
     i64 cell = r.cell[gid];
@@ -1500,6 +1530,8 @@ void launch_update_v(const Grid &g, const Fields &f, cudaStream_t st)
             return;
         }
         DISPATCH_F(g.F, MB_DISPATCH(g, k_v3d<FF, MBV><<<gr, b, 0, st>>>(g, f)));
+    } else if (quad2d_ok(g)) {
+        launch_quad2d_v(g, f, st);
     } else {
         dim3 b(32, 8), gr(cdiv(g.nz, 32), cdiv(g.nx, 8), g.nb);
         if (g.fhalf) DISPATCH_F(g.F, k_v2d<FF, __half><<<gr, b, 0, st>>>(g, f))
@@ -1549,6 +1581,12 @@ bool launch_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool fold_
             return false;
         }
         DISPATCH_F(g.F, MB_DISPATCH(g, k_s3d<FF, MBV><<<gr, b, 0, st>>>(g, f)));
+    } else if (quad2d_ok(g)) {
+        BndSlot none;
+        memset(&none, 0, sizeof none);
+        const bool fold = fold_surface && g.freesurf;
+        launch_quad2d_s(g, f, none, SFD_PREC_FP32, 0, fold, st);
+        return fold;
     } else {
         dim3 b(32, 8), gr(cdiv(g.nz, 32), cdiv(g.nx, 8), g.nb);
         if (g.fhalf) DISPATCH_F(g.F, k_s2d<FF, __half><<<gr, b, 0, st>>>(g, f))
@@ -1723,6 +1761,7 @@ void launch_update_adj(const Grid &g, const Fields &f, const AdjFields &a, bool 
         else quad_update_adj<2>(g, f, a, stress, prec, st);
         return;
     }
+    if (launch_quad2d_adj(g, f, a, stress, prec, st)) return;
     if (prec == SFD_PREC_FP16) launch_adj_t<__half>(g, f, a, stress, st);
     else if (prec == SFD_PREC_BF16) launch_adj_t<__nv_bfloat16>(g, f, a, stress, st);
     else launch_adj_t<float>(g, f, a, stress, st);
@@ -1762,11 +1801,28 @@ void launch_record(const Grid &g, const Fields &f, const PointSet &r, float *out
     else launch_maybe_pdl(pdl, k_record<float>, gr, b, st, f, r, out, nt_total, t, outmask, g.nd, g.ws);
 }
 
-void launch_residuals(const Grid &g, const AdjFields &a, const PointSet &r, const float *res, int nt_total, int t,
-                      unsigned outmask, cudaStream_t st)
+void launch_record_sources(const Grid &g, const Fields &f, const PointSet &r, float *out, int nt_total, int t,
+                           unsigned outmask, const PointSet &s, const float *src, int tsrc, cudaStream_t st)
 {
-    if (r.n == 0 || outmask == 0) return;
-    k_residuals<<<cdiv(r.n, 128), 128, 0, st>>>(a, r, res, nt_total, t, outmask, g.nd);
+    const unsigned rb = outmask ? cdiv(r.n, 128) : 0, sb = tsrc >= 0 ? cdiv(s.n, 128) : 0;
+    if (rb + sb == 0) return;
+    const bool pdl = g.nd == 3 && g.nb == 1 && pdl_enabled();
+    if (g.fhalf)
+        launch_maybe_pdl(pdl, k_record_sources<__half>, dim3(rb + sb), dim3(128), st, f, r, out, nt_total, t, outmask, g.nd,
+                         g.ws, rb, s, src, tsrc, g.dt, g.freesurf, g.F);
+    else
+        launch_maybe_pdl(pdl, k_record_sources<float>, dim3(rb + sb), dim3(128), st, f, r, out, nt_total, t, outmask, g.nd,
+                         g.ws, rb, s, src, tsrc, g.dt, g.freesurf, g.F);
+}
+
+void launch_residuals(const Grid &g, const Fields &f, const AdjFields &a, const PointSet &r, const float *res,
+                      int nt_total, int t, unsigned outmask, const PointSet &s, const float *src, int tsrc,
+                      cudaStream_t st)
+{
+    const unsigned rb = outmask ? cdiv(r.n, 128) : 0, sb = tsrc >= 0 ? cdiv(s.n, 128) : 0;
+    if (rb + sb == 0) return;
+    k_residuals<<<rb + sb, 128, 0, st>>>(a, r, res, nt_total, t, outmask, g.nd, rb, f, s, src, tsrc, g.dt, g.freesurf, g.F,
+                                        g.ws);
 }
 
 }  // namespace sfd

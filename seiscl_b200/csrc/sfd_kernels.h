@@ -52,6 +52,14 @@ void launch_surface(const Grid &g, const Fields &f, int pdir, cudaStream_t st);
 // 2D P-SV and acoustic forward: stress update, free surface, receivers of
 // step tl.t and sources of step tl.tsrc in one launch (false: not 2D)
 bool launch_update_s_step(const Grid &g, const Fields &f, const StepTail &tl, cudaStream_t st);
+// 4-cell vectorised 2D P-SV kernels (sfd_quad2d.cu).  The stress update saves
+// the boundary shells in b (nfield = 0: none) at offset tofs and then, with
+// surf, applies the free surface; the adjoint launcher returns false where it
+// does not apply (memory variables, Hessian)
+bool quad2d_ok(const Grid &g);
+void launch_quad2d_v(const Grid &g, const Fields &f, cudaStream_t st);
+void launch_quad2d_s(const Grid &g, const Fields &f, const BndSlot &b, int prec, int64_t tofs, bool surf, cudaStream_t st);
+bool launch_quad2d_adj(const Grid &g, const Fields &f, const AdjFields &a, bool stress, int prec, cudaStream_t st);
 // 2D P-SV modelling with the wave fields resident on chip (sfd_resident2d.cu)
 struct Res2d {              // tiles of a launch: ctas = ntz x ntx x shots, 0 where it does not apply
     int ntz, ntx, tz, tx;   // tiles along z and x, the largest tile
@@ -82,8 +90,15 @@ void launch_sources(const Grid &g, const Fields &f, const PointSet &s, const flo
                     int pdir, cudaStream_t st);
 void launch_record(const Grid &g, const Fields &f, const PointSet &r, float *out, int nt_total, int t,
                    unsigned outmask, cudaStream_t st);
-void launch_residuals(const Grid &g, const AdjFields &a, const PointSet &r, const float *res, int nt_total, int t,
-                      unsigned outmask, cudaStream_t st);
+// receivers of step t and sources of step tsrc (-1: none) in one launch, for
+// shots without a receiver on a source's cell
+void launch_record_sources(const Grid &g, const Fields &f, const PointSet &r, float *out, int nt_total, int t,
+                           unsigned outmask, const PointSet &s, const float *src, int tsrc, cudaStream_t st);
+// adjoint sources of step t into the adjoint fields and, in the same launch,
+// the sources of step tsrc (-1: none) out of the forward fields
+void launch_residuals(const Grid &g, const Fields &f, const AdjFields &a, const PointSet &r, const float *res,
+                      int nt_total, int t, unsigned outmask, const PointSet &s, const float *src, int tsrc,
+                      cudaStream_t st);
 
 // instability detection: if any of the n values of a wave field (FP32, or
 // FP16 when g.fhalf) is not finite, *first = min(*first, t)

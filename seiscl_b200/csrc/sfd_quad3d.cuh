@@ -79,6 +79,16 @@ __device__ __forceinline__ Q4 ldq_p(const __half *p)
     else return ldq_rw(p);
 }
 
+// add a quad to its FP64 sums
+__device__ __forceinline__ void grad_add4(double *g, i64 ip, const float (&d)[4])
+{
+    double2 *p = reinterpret_cast<double2 *>(g + ip);
+    double2 a = p[0], b = p[1];
+    a.x += (double)d[0]; a.y += (double)d[1]; b.x += (double)d[2]; b.y += (double)d[3];
+    p[0] = a;
+    p[1] = b;
+}
+
 // memory variables of four cells in storage type TR: with TR FP16 under
 // FP32 wave fields (Grid::rhalf) they are stored times g.rsc
 template <class T, class TR>
@@ -190,9 +200,9 @@ __device__ __forceinline__ void cpml_q(float *psi, i64 q, const float *Ki, const
     Q4 p = ldq_rw(psi + q);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        float ps = bb * p.v[j] + aa * d.v[j];
+        const float ps = cpml_psi(p.v[j], aa, bb, d.v[j]);
         p.v[j] = ps;
-        d.v[j] = d.v[j] * ki + ps;
+        d.v[j] = __fmaf_rn(d.v[j], ki, ps);
     }
     stq(psi + q, p);
 }
@@ -207,9 +217,9 @@ __device__ __forceinline__ void cpml_zq(float *psi, i64 q, const float *Ki, cons
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         const int ci = ci0 + step * j;
-        float ps = __ldg(b + ci) * p.v[j] + __ldg(a + ci) * d.v[j];
+        const float ps = cpml_psi(p.v[j], __ldg(a + ci), __ldg(b + ci), d.v[j]);
         p.v[j] = ps;
-        d.v[j] = d.v[j] * __ldg(Ki + ci) + ps;
+        d.v[j] = __fmaf_rn(d.v[j], __ldg(Ki + ci), ps);
     }
     stq(psi + q, p);
 }

@@ -11,15 +11,6 @@ namespace sfd {
 // same per-cell arithmetic: backpropagation of the forward field (not for
 // the DFT gradient, g.bp2), saved-boundary injection per cell, the adjoint
 // update with CPML, and the on-the-fly gradient accumulated in FP64.
-__device__ __forceinline__ void grad_add4(double *g, i64 ip, const float (&d)[4])
-{
-    double2 *p = reinterpret_cast<double2 *>(g + ip);
-    double2 a = p[0], b = p[1];
-    a.x += (double)d[0]; a.y += (double)d[1]; b.x += (double)d[2]; b.y += (double)d[3];
-    p[0] = a;
-    p[1] = b;
-}
-
 // L2 prefetch of one quad's cell in a per-cell stream
 __device__ __forceinline__ void pf_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 

@@ -95,6 +95,7 @@ __device__ __forceinline__ Slab slab_of(const Grid &g, const float *const *c, co
     Slab s = {1.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, -1};
     if (g.abs_type != 1) return s;
     int f, h;   // profile indices of the full and half nodes
+    if (i >= n) return s;   // a dummy row
     if (i >= n - g.nab) { s.at = i - n + 2 * g.nab; f = 2 * g.nab - s.at; h = f - 1; }
     else if (lo && i < g.nab) { s.at = f = h = i; }
     else return s;
@@ -218,7 +219,7 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_resident2d(const __grid_const
         else mat[i] = s2d_visco(L, g.dt, f.p[PM][ip], f.p[PMU][ip], f.p[PMUIPKP][ip], f.p[PTAUP][ip], f.p[PTAUS][ip],
                                 f.p[PTAUSIPKP][ip]);
         sx_at[i] = s_sx[on[i] ? xb + i : 0].at;
-        if (i == 0) sz = slab_of(g, f.cz, f.kinv[2], zz - F, g.nz, !g.freesurf);
+        if (i == 0) sz = slab_of(g, f.cz, f.kinv[2], zz - F, g.nz - g.zpad, !g.freesurf);
         psi_sxx[i] = psi_sxzx[i] = psi_szz[i] = psi_sxzz[i] = psi_vxx[i] = psi_vzx[i] = psi_vzz[i] = psi_vxz[i] = 0.0f;
         if (sx_at[i] >= 0) {
             const i64 q = (i64)sx_at[i] * g.nz + (zz - F);
@@ -573,7 +574,7 @@ Res2d resident2d_shape(const Grid &g, int nb, int npoints)
     memset(&best, 0, sizeof best);
     const int F = g.F;
     if (g.nd != 2 || g.fhalf || g.kernels != 0 || (F != 2 && F != 4) || g.L > 3 || g.abs_type == 2) return best;
-    if (g.abs_type == 1 && (g.nx < 2 * g.nab || g.nz < (g.freesurf ? 1 : 2) * g.nab)) return best;
+    if (g.abs_type == 1 && (g.nx < 2 * g.nab || g.nz - g.zpad < (g.freesurf ? 1 : 2) * g.nab)) return best;
     if (g.nz < F + 1 || g.nx < F + 1 || nb < 1 || npoints > R2_POINTS) return best;
     long bestc = 0;
     for (int nc = 1; nc <= 4; nc *= 2) {

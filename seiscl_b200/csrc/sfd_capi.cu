@@ -621,8 +621,9 @@ int alloc_ckpt(sfd_plan *p)
     cudaError_t e;
     p->d_snap = (char *)dalloc(p, z.snap * z.nseg, &e);
     if (!p->d_snap) return fail(p, SFD_ERR_MEMORY, "checkpoint snapshots do not fit in device memory");
-    p->d_seg = (char *)dalloc(p, z.seg, &e);
+    p->d_seg = (char *)dalloc(p, z.seg + field_slack(p->g), &e);
     if (!p->d_seg) return fail(p, SFD_ERR_MEMORY, "checkpoint segment store does not fit in device memory");
+    p->d_seg += z.elem * p->g.zshift;   // the alignment of the fields
     p->d_psi_adj = (float *)dalloc(p, sizeof(float) * std::max<int64_t>(z.psi, 1), &e);
     if (!p->d_psi_adj) return fail(p, SFD_ERR_MEMORY, "adjoint CPML allocation failed");
     p->snap_bytes = z.snap;
@@ -798,8 +799,7 @@ int adjoint_ckpt(sfd_plan *p, const PointSet &S, const PointSet &R, unsigned oma
                 ckpt_store(p, t - t0, s);
                 if (t == thi) break;
                 launch_update_v(g, p->f, s);
-                launch_update_s(g, p->f, s);
-                if (g.freesurf) launch_surface(g, p->f, 1, s);
+                if (!launch_update_s(g, p->f, s, true) && g.freesurf) launch_surface(g, p->f, 1, s);
             }
             for (int t = thi; t >= tlo; t--) {
                 ckpt_slot(p, t - t0, a);
@@ -1179,7 +1179,7 @@ extern "C" int sfd_footprint(const sfd_config *cfg, int gradient, int nsrc, int6
             b += B * 4 * g.nvol * (nwave + (int64_t)nmem * g.L) + slack * (nwave + nmem);
             if (cfg->checkpoint > 0) {   // snapshots, segment store, adjoint CPML memory
                 const CkptSizes z = ckpt_sizes(g, *cfg);
-                b += (int64_t)(z.snap * z.nseg + z.seg) + 4 * std::max<int64_t>(z.psi, 1);
+                b += (int64_t)(z.snap * z.nseg + z.seg) + slack + 4 * std::max<int64_t>(z.psi, 1);
                 if (g.fhalf) b += 4 * npar * 8;   // the adjoint's unscaled moduli and buoyancies
             } else {
                 b += B * (int64_t)(cfg->precision == SFD_PREC_FP32 ? 4 : 2) * nt * g.nbnd * nwave;

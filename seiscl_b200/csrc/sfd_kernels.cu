@@ -1543,7 +1543,8 @@ bool launch_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool fold_
 {
     if (g.fhalf && g.nd == 3 && g.L <= 3) {   // FP16 storage: the vectorised or the streaming kernels
         if (q4_ok(g)) {
-            return g.F == 4 ? quad_update_s<4>(g, f, st, false) : quad_update_s<2>(g, f, st, false);
+            const bool surf = fold_surface && g.freesurf && g.nb == 1;
+            return g.F == 4 ? quad_update_s<4>(g, f, st, surf) : quad_update_s<2>(g, f, st, surf);
         }
         dim3 b(32, 4, 2), gr(cdiv(g.nz, 32), cdiv(g.ny, 4), cdiv(g.nx, 2) * g.nb);
         switch (g.L) {
@@ -1696,12 +1697,34 @@ void launch_surface(const Grid &g, const Fields &f, int pdir, cudaStream_t st)
 // S arrays (FP32 or FP16 wave fields) to T stores (pack) or FP32 arrays
 // back from T stores (unpack), value times scale; one grid row per array, a
 // grid-stride loop over its elements
+//
+// FP32 to FP32 moves as 128-bit words where source and destination are
+// equally aligned: 9 arrays of 1.2 M cells took 23.5 us one value at a time.
 template <class T, bool UNPACK, class S = float>
 __global__ void k_pack(PackSet ps)
 {
     const int q = blockIdx.y;
-    const i64 n = ps.n[q];
+    i64 n = ps.n[q];
     const float sc = ps.scale[q];
+    if constexpr (std::is_same<T, float>::value && std::is_same<S, float>::value) {
+        const float *src = (const float *)ps.src[q];
+        float *dst = (float *)ps.dst[q];
+        if ((((uintptr_t)src ^ (uintptr_t)dst) & 15) == 0) {
+            const int head = (int)((16 - ((uintptr_t)src & 15)) / 4) & 3;   // values before the first aligned word
+            const i64 words = n > head ? (n - head) / 4 : 0;
+            for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < words; i += (i64)gridDim.x * blockDim.x) {
+                float4 v = *reinterpret_cast<const float4 *>(src + head + 4 * i);
+                v.x *= sc; v.y *= sc; v.z *= sc; v.w *= sc;
+                *reinterpret_cast<float4 *>(dst + head + 4 * i) = v;
+            }
+            // the ends: at most three values each
+            if (blockIdx.x == 0 && threadIdx.x < 8) {
+                const i64 i = threadIdx.x < 4 ? threadIdx.x : head + 4 * words + threadIdx.x - 4;
+                if (i < n && (i < head || i >= head + 4 * words)) dst[i] = src[i] * sc;
+            }
+            return;
+        }
+    }
     for (i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
         if (UNPACK) ((float *)ps.dst[q])[i] = to_f<T>(((const T *)ps.src[q])[i]) * sc;
         else ((T *)ps.dst[q])[i] = from_f<T>(to_f<S>(((const S *)ps.src[q])[i]) * sc);

@@ -138,15 +138,6 @@ __device__ __forceinline__ void bnd_put(const Grid &g, const BndSlot &b, int w, 
     ((T *)b.p[w])[at] = from_f<T>(v * g.bsc[w]);
 }
 
-// saved values of slice t-1, or the stored forward field, of one field of a quad
-template <typename T>
-__device__ __forceinline__ Q4 fwd_q(const Grid &g, const AdjFields &a, int w, i64 iv)
-{
-    Q4 q;
-#pragma unroll
-    for (int j = 0; j < 4; j++) q.v[j] = fwd_at<T>(g, a, w, iv + j);
-    return q;
-}
 // shell indices of a quad's cells (-1: none); most quads are inside or outside
 __device__ __forceinline__ bool shell_quad(const Grid &g, int gz0, int gx, int (&m)[4])
 {
@@ -302,8 +293,8 @@ __global__ void __launch_bounds__(128) k_adjv2d_q4(Grid g, Fields f, AdjFields a
     const Q4 rip = ldq(f.p[PRIP] + ip), rkp = ldq(f.p[PRKP] + ip);
     Q4 vx = {{0, 0, 0, 0}}, vz = vx;
     if (g.ckpt) {
-        vx = fwd_q<T>(g, a, VX, iv);
-        vz = fwd_q<T>(g, a, VZ, iv);
+        vx = fwd_quad<T>(g, a, VX, iv);
+        vz = fwd_quad<T>(g, a, VZ, iv);
     } else if (!g.bp2) {   // backpropagate the forward velocities (update_adjv2D.cl:205-240)
         const Deriv d = stress_diff<F>(f.w, iv, sx, hc);
         vx = ldq_rw(f.w[VX] + iv); vz = ldq_rw(f.w[VZ] + iv);
@@ -355,7 +346,7 @@ __global__ void __launch_bounds__(128) k_adjs2d_q4(Grid g, Fields f, AdjFields a
     const Q4 qM = ldq(f.p[PM] + ip), qmu = ldq(f.p[PMU] + ip), qmuipkp = ldq(f.p[PMUIPKP] + ip);
     Q4 s[3] = {{{0, 0, 0, 0}}, {{0, 0, 0, 0}}, {{0, 0, 0, 0}}};   // forward sxx, szz, sxz
     if (g.ckpt) {
-        s[0] = fwd_q<T>(g, a, SXX, iv); s[1] = fwd_q<T>(g, a, SZZ, iv); s[2] = fwd_q<T>(g, a, SXZ, iv);
+        s[0] = fwd_quad<T>(g, a, SXX, iv); s[1] = fwd_quad<T>(g, a, SZZ, iv); s[2] = fwd_quad<T>(g, a, SXZ, iv);
     } else if (!g.bp2) {   // reconstruct the forward stresses (update_adjs2D.cl:222-278)
         const Deriv d = velocity_diff<F>(f.w, iv, sx, hc);
         s[0] = ldq_rw(f.w[SXX] + iv); s[1] = ldq_rw(f.w[SZZ] + iv); s[2] = ldq_rw(f.w[SXZ] + iv);

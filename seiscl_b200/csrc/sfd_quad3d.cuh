@@ -89,6 +89,26 @@ __device__ __forceinline__ void grad_add4(double *g, i64 ip, const float (&d)[4]
     p[1] = b;
 }
 
+// the stored forward field of a checkpointed adjoint, four cells (the segment
+// store has the fields' alignment)
+template <class T>
+__device__ __forceinline__ Q4 fwd_quad(const Grid &g, const AdjFields &a, int w, i64 iv)
+{
+    const T *p = (const T *)a.fwd[w] + iv;
+    Q4 q;
+    if constexpr (std::is_same<T, float>::value) {
+        q = ldq(p);
+    } else {
+        const uint2 u = __ldg(reinterpret_cast<const uint2 *>(p));
+        const T *h = reinterpret_cast<const T *>(&u);
+#pragma unroll
+        for (int j = 0; j < 4; j++) q.v[j] = to_f<T>(h[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; j++) q.v[j] *= g.bsci[w];
+    return q;
+}
+
 // memory variables of four cells in storage type TR: with TR FP16 under
 // FP32 wave fields (Grid::rhalf) they are stored times g.rsc
 template <class T, class TR>
@@ -853,8 +873,8 @@ static void quad_update_s_l(const Grid &g, const Fields &f, dim3 g4, dim3 b4, cu
         // FP16: ordinary launches; with programmatic serialization the FP16
         // velocities need plain loads, which cost this kernel more than
         // the overlap gives (0.510 against 0.489 ms at 256^3, L=2)
-        if (pf) k_s3d_q4_pf<F, L, __half><<<g4, b4, 0, st>>>(g, f, false);
-        else k_s3d_q4<F, L, __half><<<g4, b4, 0, st>>>(g, f, false);
+        if (pf) k_s3d_q4_pf<F, L, __half><<<g4, b4, 0, st>>>(g, f, surf);
+        else k_s3d_q4<F, L, __half><<<g4, b4, 0, st>>>(g, f, surf);
         return;
     }
     if constexpr (L > 0) {
@@ -868,7 +888,6 @@ template <int F>
 bool quad_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool surf)
 {
     const dim3 b4 = q4_block(g, 16, 8, 1), g4 = q4_grid(g, b4);  // 0.70 ms vs 0.71 (32 x 2 x 2)
-    if (g.fhalf) surf = false;
     switch (g.L) {
     case 0: quad_update_s_l<F, 0>(g, f, g4, b4, st, surf); break;
     case 1: quad_update_s_l<F, 1>(g, f, g4, b4, st, surf); break;

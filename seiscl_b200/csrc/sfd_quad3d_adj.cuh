@@ -11,6 +11,29 @@ namespace sfd {
 // same per-cell arithmetic: backpropagation of the forward field (not for
 // the DFT gradient, g.bp2), saved-boundary injection per cell, the adjoint
 // update with CPML, and the on-the-fly gradient accumulated in FP64.
+// shell indices of a quad's cells (-1: none).  Most quads lie wholly inside
+// or outside the shell: one comparison per axis settles them, against some
+// forty integer operations a cell.
+__device__ __forceinline__ void shell_quad3d(const Grid &g, int gz0, int gy, int gx, int (&m)[4])
+{
+    const BndDims b = bnd_dims(g);
+    const int F = g.F, i = gx - b.lbnd, j = gy - b.lbnd, k = gz0 - b.lbnds;
+    if (i < 0 || i >= b.NXbnd || j < 0 || j >= b.NYbnd || k + 3 < 0 || k >= b.NZbnd) return;
+    if (i >= F && i < b.NXbnd - F && j >= F && j < b.NYbnd - F && k >= F && k + 3 < b.NZbnd - F) return;
+#pragma unroll
+    for (int q = 0; q < 4; q++) m[q] = inject_ind3d(g, gz0 + q, gy, gx);
+}
+
+// The adjoint memory variables the stress update reads.  Nothing writes
+// them in 3D but the DFT adjoint, where they are the forward arrays (the
+// update stores its new values there, update_adjs3D.cl:566-583): elsewhere
+// they keep the zeros the adjoint starts from, and 6 L streams a cell need
+// not be read.
+__device__ __forceinline__ Q4 adj_memory(const Grid &g, const float *p)
+{
+    return g.bp2 ? ldq_rw(p) : Q4{{0.0f, 0.0f, 0.0f, 0.0f}};
+}
+
 // L2 prefetch of one quad's cell in a per-cell stream
 __device__ __forceinline__ void pf_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
@@ -37,12 +60,7 @@ __global__ void __launch_bounds__(128, PF ? 3 : 1) k_adjv3d_q4(Grid g, Fields f,
     const Q4 rip = ldq(f.p[PRIP] + ip), rjp = ldq(f.p[PRJP] + ip), rkp = ldq(f.p[PRKP] + ip);
     Q4 vx = {{0, 0, 0, 0}}, vy = vx, vz = vx;
     if (g.ckpt) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            vx.v[j] = fwd_at<T>(g, a, VX, iv + j);
-            vy.v[j] = fwd_at<T>(g, a, VY, iv + j);
-            vz.v[j] = fwd_at<T>(g, a, VZ, iv + j);
-        }
+        vx = fwd_quad<T>(g, a, VX, iv); vy = fwd_quad<T>(g, a, VY, iv); vz = fwd_quad<T>(g, a, VZ, iv);
     } else if (!g.bp2) {  // backpropagate the forward velocities (update_adjv3D.cl:297-340)
         Q4 szz_z = dfw_z<F>(ldw(f.w[SZZ], iv), hc);
         Q4 sxx_x = dfw_q<F>(f.w[SXX], iv, sx, hc);
@@ -54,12 +72,14 @@ __global__ void __launch_bounds__(128, PF ? 3 : 1) k_adjv3d_q4(Grid g, Fields f,
         Q4 sxy_x = dbw_q<F>(f.w[SXY], iv, sx, hc);
         Q4 sxy_y = dbw_q<F>(f.w[SXY], iv, sy, hc);
         vx = ldq_rw(f.w[VX] + iv); vy = ldq_rw(f.w[VY] + iv); vz = ldq_rw(f.w[VZ] + iv);
+        int mq[4] = {-1, -1, -1, -1};
+        shell_quad3d(g, gz0, gy, gx, mq);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             vx.v[j] = vx.v[j] - (sxx_x.v[j] + sxy_y.v[j] + sxz_z.v[j]) * rip.v[j];
             vy.v[j] = vy.v[j] - (syy_y.v[j] + sxy_x.v[j] + syz_z.v[j]) * rjp.v[j];
             vz.v[j] = vz.v[j] - (szz_z.v[j] + sxz_x.v[j] + syz_y.v[j]) * rkp.v[j];
-            const int m = inject_ind3d(g, gz0 + j, gy, gx);
+            const int m = mq[j];
             if (m != -1) {
                 vx.v[j] = bnd_at<T>(g, a, VX, m);
                 vy.v[j] = bnd_at<T>(g, a, VY, m);
@@ -194,10 +214,8 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
 #pragma unroll
         for (int l = 0; l < L; l++)
 #pragma unroll
-            for (int q = 0; q < NR; q++) {
-                pf_l2(a.rr[q] + l * g.nvol + iv);
+            for (int q = 0; q < NR; q++)
                 if (recon) pf_l2(f.r[q] + l * g.nvol + iv);
-            }
         constexpr int np = L > 0 ? 10 : 5;
         constexpr int pid[10] = {PM, PMU, PMUIPJP, PMUJPKP, PMUIPKP, PTAUP, PTAUS, PTAUSIPJP, PTAUSJPKP, PTAUSIPKP};
 #pragma unroll
@@ -208,10 +226,7 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
         }
     }
     int mq[4] = {-1, -1, -1, -1};
-    if (recon) {
-#pragma unroll
-        for (int j = 0; j < 4; j++) mq[j] = inject_ind3d(g, gz0 + j, gy, gx);
-    }
+    if (recon) shell_quad3d(g, gz0, gy, gx, mq);
     const float *hc = g.hc;
     // adjoint velocity derivatives, with CPML
     Q4 vzzr = dbw_z<F>(ldw(a.wr[VZ], iv), hc), vyzr = dfw_z<F>(ldw(a.wr[VY], iv), hc);
@@ -239,9 +254,7 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
         Q4 s3[3] = {{{0, 0, 0, 0}}, {{0, 0, 0, 0}}, {{0, 0, 0, 0}}};
         if (g.ckpt) {
 #pragma unroll
-            for (int c = 0; c < 3; c++)
-#pragma unroll
-                for (int j = 0; j < 4; j++) s3[c].v[j] = fwd_at<T>(g, a, wid[c], iv + j);
+            for (int c = 0; c < 3; c++) s3[c] = fwd_quad<T>(g, a, wid[c], iv);
         } else if (!g.bp2) {
             const Q4 vzz = dbw_z<F>(ldw(f.w[VZ], iv), hc);
             const Q4 vyy = dbw_q<F>(f.w[VY], iv, sy, hc);
@@ -305,7 +318,7 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
 #pragma unroll
             for (int c = 0; c < 3; c++)
 #pragma unroll
-                for (int l = 0; l < L; l++) rr[c][l] = ldq_rw(a.rr[rid[c]] + l * g.nvol + iv);
+                for (int l = 0; l < L; l++) rr[c][l] = adj_memory(g, a.rr[rid[c]] + l * g.nvol + iv);
         }
         Q4 w3[3];
 #pragma unroll
@@ -398,8 +411,7 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
         if (L > 0) qtauc = ldq(f.p[ptau] + ip);
         Q4 sc = {{0, 0, 0, 0}};
         if (g.ckpt) {
-#pragma unroll
-            for (int j = 0; j < 4; j++) sc.v[j] = fwd_at<T>(g, a, wid, iv + j);
+            sc = fwd_quad<T>(g, a, wid, iv);
         } else if (!g.bp2) {
             Q4 d1, d2;   // forward derivative pair (vxy+vyx, vyz+vzy, vxz+vzx)
             if (c == 0) { d1 = dfw_q<F>(f.w[VX], iv, sy, hc); d2 = dfw_q<F>(f.w[VY], iv, sx, hc); }
@@ -442,7 +454,7 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
         Q4 rr[L > 0 ? L : 1];
         if constexpr (L > 0) {
 #pragma unroll
-            for (int l = 0; l < L; l++) rr[l] = ldq_rw(a.rr[rid] + l * g.nvol + iv);
+            for (int l = 0; l < L; l++) rr[l] = adj_memory(g, a.rr[rid] + l * g.nvol + iv);
         }
         Q4 wc = ldq_rw(a.wr[wid] + iv);
 #pragma unroll
@@ -479,8 +491,10 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
             }
         }
         if constexpr (L > 0) {
+            if (!g.ckpt) {   // as for the normal stresses
 #pragma unroll
-            for (int l = 0; l < L; l++) stq(f.r[rid] + l * g.nvol + iv, rr[l]);
+                for (int l = 0; l < L; l++) stq(f.r[rid] + l * g.nvol + iv, rr[l]);
+            }
         }
         if (g.abs_type == 2) {
 #pragma unroll

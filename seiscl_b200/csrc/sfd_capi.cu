@@ -76,13 +76,6 @@ void dfree(sfd_plan *p, void *ptr, size_t bytes)
 // cells of the plan's grid that a user sees (without dummy rows)
 int64_t user_cells(const Grid &g) { return (int64_t)(g.nz - g.zpad) * g.ny * g.nx; }
 
-// host array of a parameter [nx][(ny)][nz] -> device rows of g.nz
-cudaError_t upload_param(const Grid &g, float *dst, const float *src)
-{
-    const size_t w = sizeof(float) * (g.nz - g.zpad);
-    return cudaMemcpy2D(dst, sizeof(float) * g.nz, src, w, w, (size_t)g.ny * g.nx, cudaMemcpyHostToDevice);
-}
-
 // bytes added to every field allocation whose base is shifted
 size_t field_slack(const Grid &g) { return g.zshift ? 16 : 0; }
 
@@ -653,9 +646,10 @@ int prepare_adjoint_params(sfd_plan *p)
         if (!p->f.p[k] || param_exponent(k, 1) == 0) continue;
         float *dst = p->d_padj + npar * q++;
         if (!p->padj_valid)
-            CKC(upload_param(g, dst, p->hp[k].data()));
+            launch_scale(p->f.p[k], dst, npar, std::ldexp(1.0f, -param_exponent(k, p->kshift)), p->stream);
         p->padj[k] = dst;
     }
+    CKC(cudaStreamSynchronize(p->stream));
     p->padj_valid = true;
     return SFD_OK;
 }
@@ -1233,58 +1227,171 @@ extern "C" void sfd_plan_destroy(sfd_plan *p)
 
 extern "C" const char *sfd_last_error(const sfd_plan *p) { return p ? p->err.c_str() : "null plan"; }
 
-extern "C" int sfd_set_model(sfd_plan *p, const float *const *params)
+namespace {
+// A host copy of a transformed parameter [nx][(ny)][nz], unscaled
+int host_param(sfd_plan *p, int k, const float **out)
 {
-    if (!p || !params) return SFD_ERR_ARG;
-    const int nzu = p->g.nz - p->g.zpad;
-    int rc = transform_model(p->cfg, nzu, p->g.ny, p->g.nx, params, p->hp, p->err);
-    if (rc) return rc;
+    std::vector<float> &h = p->hp[k];
+    if (h.empty()) {
+        const Grid &g = p->g;
+        const size_t w = sizeof(float) * (g.nz - g.zpad);
+        h.resize(user_cells(g));
+        const cudaError_t e = cudaMemcpy2D(h.data(), w, p->f.p[k], sizeof(float) * g.nz, w, (size_t)g.ny * g.nx,
+                                           cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess) {
+            h.clear();
+            return fail(p, SFD_ERR_CUDA, std::string("parameter copy: ") + cudaGetErrorString(e));
+        }
+        const int ex = g.fhalf ? param_exponent(k, p->kshift) : 0;
+        if (ex)
+            for (float &v : h) v = std::ldexp(v, -ex);
+    }
+    *out = h.data();
+    return SFD_OK;
+}
+
+// log2 of the model's mean impedance sqrt(M / rip), from every step-th cell
+int impedance_shift(sfd_plan *p, char *scratch, int64_t bytes, int *shift)
+{
+    const Grid &g = p->g;
+    const int nzu = g.nz - g.zpad;
+    const int64_t n = user_cells(g), step = std::max<int64_t>(1, n / 4096);
+    std::vector<int64_t> at;
+    for (int64_t i = 0; i < n; i += step) at.push_back(i / nzu * g.nz + i % nzu);
+    const int cnt = (int)at.size();
+    if ((int64_t)cnt * (int64_t)(sizeof(int64_t) + 2 * sizeof(float)) > bytes) return fail(p, SFD_ERR_MEMORY, "scratch too small");
+    int64_t *d_at = (int64_t *)scratch;
+    float *d_v = (float *)(d_at + cnt);
+    std::vector<float> v(2 * cnt);
+    CKC(cudaMemcpyAsync(d_at, at.data(), sizeof(int64_t) * cnt, cudaMemcpyHostToDevice, p->stream));
+    launch_gather(p->f.p[PM], d_at, d_v, cnt, p->stream);
+    launch_gather(p->f.p[PRIP], d_at, d_v + cnt, cnt, p->stream);
+    CKC(cudaMemcpyAsync(v.data(), d_v, sizeof(float) * 2 * cnt, cudaMemcpyDeviceToHost, p->stream));
+    CKC(cudaStreamSynchronize(p->stream));
+    double acc = 0.0;
+    int64_t m = 0;
+    for (int i = 0; i < cnt; i++) {
+        const double z = std::sqrt((double)v[i] / (double)v[cnt + i]);
+        if (z > 0 && std::isfinite(z)) { acc += std::log2(z); m++; }
+    }
+    *shift = m ? (int)std::lround(acc / m) : 0;
+    return SFD_OK;
+}
+
+// checks, transforms and stores the model through `scratch` (room for `planes`
+// x planes of every input and the check record)
+int store_model(sfd_plan *p, const float *const in[5], char *scratch, int planes, int64_t bytes)
+{
+    const Grid &g = p->g;
+    const sfd_config &c = p->cfg;
+    cudaStream_t st = p->stream;
+    ModelIn m;
+    memset(&m, 0, sizeof m);
+    m.nd = g.nd;
+    m.nz = g.nz - g.zpad;
+    m.ny = g.ny;
+    m.nx = g.nx;
+    m.pitch = g.nz;
+    m.L = c.L;
+    m.par_type = c.param_type;
+    m.dt = c.dt;
+    m.dh = c.dh;
+    m.sumu = phase_weights(c, m.wl);
+    const int64_t plane = (int64_t)m.ny * m.nz;
+    ModelCheck *check = (ModelCheck *)scratch, found;
+    float *slab = (float *)(scratch + 256);
+    const float **dst[5] = {&m.a, &m.b, &m.rho, &m.taup, &m.taus};
+    auto upload = [&](int x0) {
+        m.x0 = x0;
+        const bool all = planes >= m.nx;
+        m.xs = all ? m.nx : std::min(planes - 1, m.nx - x0);
+        const int64_t n = plane * std::min(m.xs + 1, m.nx - x0);
+        float *q = slab;
+        for (int k = 0; k < 5; k++) {
+            *dst[k] = nullptr;
+            if (!in[k] || (k >= 3 && c.L == 0)) continue;
+            if (cudaError_t e = cudaMemcpyAsync(q, in[k] + plane * x0, sizeof(float) * n, cudaMemcpyHostToDevice, st)) return e;
+            *dst[k] = q;
+            q += plane * std::min(planes, m.nx);
+        }
+        return cudaSuccess;
+    };
+    CKC(cudaMemsetAsync(check, 0, sizeof *check, st));
+    for (int x0 = 0; x0 < m.nx; x0 += m.xs) {
+        CKC(upload(x0));
+        launch_model_check(m, check, st);
+    }
+    CKC(cudaMemcpyAsync(&found, check, sizeof found, cudaMemcpyDeviceToHost, st));
+    CKC(cudaStreamSynchronize(st));
+    if (found.bad_rho) return fail(p, SFD_ERR_ARG, "rho must be positive everywhere");
+    double mb, mub;
+    memcpy(&mb, &found.mb, sizeof mb);
+    memcpy(&mub, &found.mub, sizeof mub);
+    int rc;
+    if ((rc = check_cfl(c, mb, mub, p->err))) return rc;
+    // the model is accepted: from here on the old one is gone
     if (!p->model_set) {
         if ((rc = alloc_model(p))) return rc;
         if ((rc = upload_constants(p))) return rc;
     }
-    int64_t npar = user_cells(p->g);
-    // FP16 stores keep velocities as v * 2^b and stresses as s * 2^a with
-    // b - a ~ log2 of the impedance, so both stay near the same magnitude
-    {
-        double acc = 0.0;
-        int64_t n = 0, step = std::max<int64_t>(1, npar / 4096);
-        for (int64_t i = 0; i < npar; i += step) {
-            const double z = std::sqrt((double)p->hp[PM][i] / (double)p->hp[PRIP][i]);
-            if (z > 0 && std::isfinite(z)) { acc += std::log2(z); n++; }
-        }
-        p->bshift = n ? (int)std::lround(acc / n) : 0;
-    }
-    {
-        // the free-surface adjoint forms C^-1 at the top row with the factor
-        // 1 / (4 M mu - 4 mu^2) in 2D and 1 / (6 M mu - 8 mu^2) in 3D
-        // (surface2D_adj.cl, surface3D_adj.cl): undefined where mu = 0
-        p->surf_mu_zero = false;
-        const int64_t ncol = (int64_t)p->g.ny * p->g.nx;
-        for (int64_t c = 0; c < ncol && !p->surf_mu_zero; c++)
-            if (!(p->hp[PMU][c * nzu] > 0.0f)) p->surf_mu_zero = true;
-    }
-    if (p->g.fhalf) {
-        // FP16 wave fields: the moduli carry 2^-kshift and the buoyancies
-        // 2^kshift (exact power-of-two scalings of the FP32 parameters).
-        p->kshift = p->bshift;
-        const int up[3] = {PRIP, PRJP, PRKP}, down[5] = {PM, PMU, PMUIPKP, PMUIPJP, PMUJPKP};
-        std::vector<float> tmp(npar);
-        for (int k = 0; k < NPAR; k++) {
-            int e = 0;
-            for (int q : up) if (q == k) e = p->kshift;
-            for (int q : down) if (q == k) e = -p->kshift;
-            for (int64_t i = 0; i < npar; i++) tmp[i] = std::ldexp(p->hp[k][i], e);
-            CKC(upload_param(p->g, (float *)p->f.p[k], tmp.data()));
-        }
-    } else {
-        for (int k = 0; k < NPAR; k++)
-            CKC(upload_param(p->g, (float *)p->f.p[k], p->hp[k].data()));
-    }
-    p->model_set = true;
+    for (int k = 0; k < NPAR; k++) p->hp[k].clear();
     p->padj_valid = false;
     p->have_forward = false;
+    ModelOut o;
+    for (int k = 0; k < NPAR; k++) o.p[k] = (float *)p->f.p[k];
+    for (int x0 = 0; x0 < m.nx; x0 += m.xs) {
+        if (planes < m.nx) CKC(upload(x0));
+        launch_model_params(m, o, check, st);
+    }
+    CKC(cudaMemcpyAsync(&found, check, sizeof found, cudaMemcpyDeviceToHost, st));
+    CKC(cudaStreamSynchronize(st));
+    // the free-surface adjoint forms C^-1 at the top row with the factor
+    // 1 / (4 M mu - 4 mu^2) in 2D and 1 / (6 M mu - 8 mu^2) in 3D
+    // (surface2D_adj.cl, surface3D_adj.cl): undefined where mu = 0
+    p->surf_mu_zero = found.top_mu_zero != 0;
+    // FP16 stores keep velocities as v * 2^b and stresses as s * 2^a with
+    // b - a ~ log2 of the impedance, so both stay near the same magnitude
+    if ((rc = impedance_shift(p, scratch, bytes, &p->bshift))) return rc;
+    if (g.fhalf) {
+        // FP16 wave fields: the moduli carry 2^-kshift and the buoyancies
+        // 2^kshift (exact power-of-two scalings of the FP32 parameters)
+        p->kshift = p->bshift;
+        for (int k = 0; k < NPAR; k++)
+            if (const int ex = param_exponent(k, p->kshift))
+                launch_scale(o.p[k], o.p[k], (int64_t)g.nz * g.ny * g.nx, std::ldexp(1.0f, ex), st);
+        CKC(cudaStreamSynchronize(st));
+    }
+    CKC(cudaGetLastError());
+    p->model_set = true;
     return SFD_OK;
+}
+}  // namespace
+
+extern "C" int sfd_set_model(sfd_plan *p, const float *const *params)
+{
+    if (!p || !params) return SFD_ERR_ARG;
+    const sfd_config &c = p->cfg;
+    const Grid &g = p->g;
+    // SH reads only vs and rho, acoustic only vp and rho (assign_modeling_case.c:1004-1016)
+    const float *in[5] = {c.nd == 21 ? nullptr : params[0], c.nd == 22 ? nullptr : params[1], params[2],
+                          c.L > 0 ? params[3] : nullptr, c.L > 0 ? params[4] : nullptr};
+    if ((c.nd != 21 && !in[0]) || (c.nd == 21 && !in[1]) || !in[2])
+        return fail(p, SFD_ERR_ARG, c.nd == 21 ? "vs (or mu / Is) and rho are required" : "vp (or M / Ip) and rho are required");
+    if (!(in[2][0] > 0)) return fail(p, SFD_ERR_ARG, "rho must be positive everywhere");
+    if (c.param_type < 0 || c.param_type > 2) return fail(p, SFD_ERR_UNSUPPORTED, "param_type must be 0, 1 or 2");
+    if (c.L > 0 && (!in[3] || !in[4])) return fail(p, SFD_ERR_ARG, "taup and taus are required when L > 0");
+    // a slab of x planes at a time: the scratch stays below 100 MB (or two
+    // planes), and returns to the pool
+    const int64_t plane = (int64_t)(g.nz - g.zpad) * g.ny, narr = c.L > 0 ? 5 : 3;
+    const int planes = (int)std::min<int64_t>(g.nx, std::max<int64_t>(2, (5 << 20) / plane));
+    const int64_t bytes = 256 + std::max<int64_t>(sizeof(float) * narr * plane * planes, 8192 * 16);
+    cudaError_t e;
+    char *scratch = (char *)dalloc_raw(p, bytes, &e);
+    if (!scratch) return fail(p, SFD_ERR_MEMORY, "model staging does not fit in device memory");
+    const int rc = store_model(p, in, scratch, planes, bytes);
+    cudaStreamSynchronize(p->stream);
+    dfree(p, scratch, bytes);
+    return rc;
 }
 
 extern "C" int sfd_source_type_mask(const float *src_pos, int nsrc_all)
@@ -1708,9 +1815,13 @@ extern "C" int sfd_get_hessian(sfd_plan *p, int transform, float *const *out)
         // src/calc_grad.c:1004-1090 for the Hessian: the parameters rescaled
         // as for the gradient, no division by dt
         const double dt = p->cfg.dt, dh = p->cfg.dh;
+        const float *prho, *pM, *pmu;
+        int rc;
+        if (!p->model_set) return fail(p, SFD_ERR_STATE, "no model");
+        if ((rc = host_param(p, PRHO, &prho)) || (rc = host_param(p, PM, &pM)) || (rc = host_param(p, PMU, &pmu))) return rc;
         for (int64_t i = 0; i < n; i++) {
-            const double rho = 1.0 / p->hp[PRHO][i] * dt / dh;
-            const double M = p->hp[PM][i] * dh / dt, mu = p->hp[PMU][i] * dh / dt;
+            const double rho = 1.0 / prho[i] * dt / dh;
+            const double M = pM[i] * dh / dt, mu = pmu[i] * dh / dt;
             h[GRHO][i] += M / rho * h[GM][i];
             if (mu > 0) h[GRHO][i] += mu / rho * h[GMU][i];
             const double sM = pt == 0 ? std::sqrt(rho * M) : std::sqrt(M / rho);
@@ -1847,6 +1958,11 @@ extern "C" int sfd_residual_scale(sfd_plan *p, const sfd_shot *shot, const int *
     for (int o = 0; o < SFD_NOUT; o++) {
         if (!outsel || !outsel[o] || !res || !res[o]) continue;
         if (o != SFD_OUT_VX && o != SFD_OUT_VY && o != SFD_OUT_VZ && o != SFD_OUT_P) continue;
+        const int id = o == SFD_OUT_P ? PM : o == SFD_OUT_VX ? PRIP : (o == SFD_OUT_VY ? PRJP : PRKP);
+        const float *par, *pmu = nullptr;
+        if (int rc_ = host_param(p, id, &par)) return rc_;
+        if (o == SFD_OUT_P)
+            if (int rc_ = host_param(p, PMU, &pmu)) return rc_;
         for (int r = 0; r < shot->nrec; r++) {
             const float *rp = shot->rec_pos + 8 * r;
             int x, y, z;
@@ -1856,11 +1972,10 @@ extern "C" int sfd_residual_scale(sfd_plan *p, const sfd_shot *shot, const int *
             if (pos < 0 || pos >= npar) return fail(p, SFD_ERR_ARG, "residual scaling index outside the model");
             float *row = res[o] + (int64_t)r * NT;
             if (o == SFD_OUT_P) {
-                float parscal = -2.0 * (p->hp[PM][pos] - p->hp[PMU][pos]) * dh / dt;
+                float parscal = -2.0 * (par[pos] - pmu[pos]) * dh / dt;
                 for (int t = 0; t < tmax; t++) row[t] *= parscal * dt;
             } else {
-                int id = o == SFD_OUT_VX ? PRIP : (o == SFD_OUT_VY ? PRJP : PRKP);
-                float parscal = 1.0 / p->hp[id][pos] * dh / dt;
+                float parscal = 1.0 / par[pos] * dh / dt;
                 for (int t = 0; t < tmax; t++) row[t] *= 1.0 / parscal * dt;
             }
         }

@@ -145,7 +145,8 @@ struct sfd_plan {
     std::string err;
     double DH_lit;          // the reference's "%9.9f" dh literal
     double DT_lit;
-    // host copies of the transformed parameters (for transf_grad, res_scale)
+    // host copies of the transformed parameters, made when something asks
+    // (host_param); cleared with each new model
     std::vector<float> hp[sfd::NPAR];
     bool model_set;
     // device memory

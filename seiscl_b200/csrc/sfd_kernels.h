@@ -122,6 +122,25 @@ struct PackSet {
 };
 void launch_pack(const PackSet &ps, int prec, bool unpack, cudaStream_t st, bool half_src = false);
 
+// material parameters from raw inputs (sfd_model.cu)
+struct ModelIn {            // a slab of x planes x0 .. x0+xs-1 (and the next, where there is one)
+    const float *a, *b, *rho, *taup, *taus;   // raw inputs of the slab, [planes][ny][nz]; a or b may be null
+    int nd, nz, ny, nx, pitch;   // grid; row length of the stored parameters
+    int x0, xs, L, par_type;
+    double dt, dh, sumu, wl[8];
+};
+struct ModelOut {
+    float *p[NPAR];
+};
+struct ModelCheck {         // zeroed before use; mb, mub: bits of the largest M b, mu b
+    unsigned long long mb, mub;
+    int bad_rho, top_mu_zero;
+};
+void launch_model_check(const ModelIn &m, ModelCheck *out, cudaStream_t st);
+void launch_model_params(const ModelIn &m, const ModelOut &o, ModelCheck *check, cudaStream_t st);
+void launch_scale(const float *src, float *dst, int64_t n, float s, cudaStream_t st);
+void launch_gather(const float *src, const int64_t *at, float *out, int n, cudaStream_t st);
+
 // gradient sums -> gradient of the parameters (sfd_gradient.cu)
 struct GradOut {
     const double *sum[3];   // M, mu, rho: ncopy copies, `copy` apart, of rows of `pitch` with nz cells each

@@ -182,6 +182,21 @@ static void ave2(const std::vector<double> &in, std::vector<double> &out, int NZ
     }
 }
 
+// phase-velocity correction at f0 (assign_modeling_case.c:345-365, 414-437):
+// the weight of each mechanism and their sum
+double phase_weights(const sfd_config &c, double wl[8])
+{
+    const double ws = 2.0 * kPi * c.f0, dt = c.dt;
+    double sumu = 0.0;
+    for (int l = 0; l < c.L; l++) {
+        double eta = 2.0 * kPi * c.fl[l] * dt;
+        double pts = dt / eta;
+        wl[l] = ws * ws * pts * pts / (1.0 + ws * ws * pts * pts);
+        sumu += wl[l];
+    }
+    return sumu;
+}
+
 int transform_model(const sfd_config &c, int nz, int ny, int nx, const float *const *params,
                     std::vector<float> out[NPAR], std::string &err)
 {
@@ -213,15 +228,8 @@ int transform_model(const sfd_config &c, int nz, int ny, int nx, const float *co
         }
     }
     if (L > 0) {
-        // phase-velocity correction at f0 (assign_modeling_case.c:345-365, 414-437)
-        double ws = 2.0 * kPi * c.f0, sumu = 0.0;
-        std::vector<double> wl(L);
-        for (int l = 0; l < L; l++) {
-            double eta = 2.0 * kPi * c.fl[l] * dt;
-            double pts = dt / eta;
-            wl[l] = ws * ws * pts * pts / (1.0 + ws * ws * pts * pts);
-            sumu += wl[l];
-        }
+        double wl[8];
+        const double sumu = phase_weights(c, wl);
         for (int64_t i = 0; i < n; i++) {
             double sumpi = 0.0;
             for (int l = 0; l < L; l++) sumpi += wl[l] * taup[i];
@@ -258,12 +266,19 @@ int transform_model(const sfd_config &c, int nz, int ny, int nx, const float *co
         }
     }
     // stability: v = sqrt(M rho_b) dh / dt over the transformed model
-    double vmax = 0.0, vsmax = 0.0;
+    double mb = 0.0, mub = 0.0;
     for (int64_t i = 0; i < n; i++) {
-        vmax = std::max(vmax, std::sqrt(M[i] * brho[i]) / dt * dh);
-        vsmax = std::max(vsmax, std::sqrt(mu[i] * brho[i]) / dt * dh);
+        mb = std::max(mb, M[i] * brho[i]);
+        mub = std::max(mub, mu[i] * brho[i]);
     }
-    if (vmax == 0.0) vmax = vsmax;
+    return check_cfl(c, mb, mub, err);
+}
+
+int check_cfl(const sfd_config &c, double mb, double mub, std::string &err)
+{
+    const double dt = c.dt, dh = c.dh;
+    double vmax = std::sqrt(mb) / dt * dh;
+    if (vmax == 0.0) vmax = std::sqrt(mub) / dt * dh;
     double gamma;
     switch (c.fdorder) {
     case 2: gamma = 1.0; break;

@@ -18,6 +18,9 @@ void cerjan_taper(double abpc, int nab, float *taper);
 int nbnd_cells(int nd, int nz, int ny, int nx, int F, int nab, int freesurf);
 int transform_model(const sfd_config &c, int nz, int ny, int nx, const float *const *params,
                     std::vector<float> out[NPAR], std::string &err);
+double phase_weights(const sfd_config &c, double wl[8]);
+// time step against the stability limit; mb, mub: the model's largest M b and mu b
+int check_cfl(const sfd_config &c, double mb, double mub, std::string &err);
 int source_targets(int nd, int mask, int type, int fields[3], float div[3]);
 void point_cell(const float *pos, double DH, int F, int &i, int &j, int &k);
 

@@ -1558,9 +1558,8 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
     const bool bnd_shells = save_boundaries && !dft && !ckpt;
     // 2D P-SV runs whose wave fields fit on chip: the time loop in segments,
     // one cooperative launch each (sfd_resident2d.cu)
-    const Res2d rs = resident2d_shape(g, nshot, S.n + R.n);
+    const Res2d rs = resident2d_plan(g, nshot, S.n + R.n);
     const bool resident = rs.ctas > 0 && p->d_words && points.inside && !dft && !ckpt && !mv.n;
-    if (resident) CKC(cudaMemsetAsync(p->d_words, 0, sizeof(*p->d_words) * (size_t)resident2d_words(rs), st));
     LoopKey key;
     key.add(points.apart); key.add(mv.n); key.add(p->movout); key.add(p->d_mov); key.add(fuse2d); key.add(p->d_ticket); key.add(fuse3d);
     key.add(1); key.add(p->g); key.add(p->f); key.add_points(S); key.add_points(R); key.add(p->d_src);
@@ -1580,11 +1579,16 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
     int rcl = SFD_OK;
     if (resident) {
         if (tmax > 0) launch_sources(g, p->f, S, p->d_src, NT, 0, 1, st);
-        Res2dRun a{R, S, p->d_src, p->d_seis, omask, NT, 0, 0, tmax, bs, p->cfg.precision, p->d_words, p->d_unstable,
+        Res2dRun a{R, S, p->d_src, p->d_seis, omask, NT, 0, 0, tmax, 0, bs, p->cfg.precision, p->d_words, p->d_unstable,
                    p->d_unstable + 1};
-        for (a.t0 = 0; a.t0 < tmax; a.t0 = a.t1) {
-            a.t1 = std::min(a.t0 + RES2D_SEGMENT, tmax);
-            CKC(launch_resident2d(g, p->f, rs, a, p->device, st));
+        for (a.shot0 = 0; a.shot0 < nshot; a.shot0 += rs.shots) {
+            CKC(cudaMemsetAsync(p->d_words, 0, sizeof(*p->d_words) * (size_t)resident2d_words(rs), st));
+            Res2d r = rs;
+            r.ctas = r.ntz * r.ntx * std::min(rs.shots, nshot - a.shot0);
+            for (a.t0 = 0; a.t0 < tmax; a.t0 = a.t1) {
+                a.t1 = std::min(a.t0 + RES2D_SEGMENT, tmax);
+                CKC(launch_resident2d(g, p->f, r, a, p->device, st));
+            }
         }
     } else
     rcl = run_loop(p, p->gfwd, key.s, st, [&](cudaStream_t s) {

@@ -64,6 +64,7 @@ bool launch_quad2d_adj(const Grid &g, const Fields &f, const AdjFields &a, bool 
 struct Res2d {              // tiles of a launch: ctas = ntz x ntx x shots, 0 where it does not apply
     int ntz, ntx, tz, tx;   // tiles along z and x, the largest tile
     int side, ctas, F, nc;  // longer side of a tile, CTAs, half width, cells per thread
+    int shots;              // shots of a launch
     size_t smem;
 };
 struct Res2dRun {           // a segment of the time loop: steps t0 .. t1-1 of tmax
@@ -72,13 +73,14 @@ struct Res2dRun {           // a segment of the time loop: steps t0 .. t1-1 of t
     float *out;             // [nsel][nrec][nt_total]
     unsigned outmask;
     int nt_total, t0, t1, tmax;
+    int shot0;              // first shot of the launch
     BndSlot bnd;            // boundary shells to save (nfield = 0: none), in storage type prec
     int prec;
     unsigned long long *words;   // exchange words, zeroed before the run's first segment
     int *first_bad, *status;
 };
 constexpr int RES2D_SEGMENT = 256;   // steps of one launch: bounds how long it holds the SMs
-Res2d resident2d_shape(const Grid &g, int nb, int npoints);
+Res2d resident2d_plan(const Grid &g, int nb, int npoints);   // launches for the nb shots of a run
 int64_t resident2d_words(const Res2d &r);
 int64_t resident2d_bytes(const Grid &g, int batch);   // exchange words of launches of up to `batch` shots
 cudaError_t launch_resident2d(const Grid &g, const Fields &f, const Res2d &r, const Res2dRun &a, int device,

@@ -48,7 +48,7 @@ namespace {
 constexpr int R2_THREADS = 512;
 constexpr int R2_CTAS = 148;              // one CTA per SM
 constexpr int R2_SMEM = 200 * 1024;       // dynamic shared memory a CTA may take
-constexpr int R2_WORDS = 2;               // exchange words a thread receives in a half step
+constexpr int r2_words(int nc) { return nc == 4 ? 4 : 2; }   // most exchange words a thread receives in a half step
 constexpr int R2_POINTS = 4096;           // receivers and sources of a run
 constexpr long long R2_WAIT_NS = 2000000000LL;   // bound of one wait
 
@@ -143,10 +143,10 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_resident2d(const __grid_const
                                                               const __grid_constant__ Res2dRun a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int LL = L > 0 ? L : 1;
+    constexpr int LL = L > 0 ? L : 1, R2_WORDS = r2_words(NC);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ntile = r.ntz * r.ntx;
-    const int shot = blockIdx.x / ntile, tl = blockIdx.x % ntile;
+    const int shot = a.shot0 + blockIdx.x / ntile, tl = blockIdx.x % ntile;
     const int iz = tl % r.ntz, ix = tl / r.ntz;
     const int z0 = (int)((i64)iz * g.nz / r.ntz), tz = (int)((i64)(iz + 1) * g.nz / r.ntz) - z0;
     const int x0 = (int)((i64)ix * g.nx / r.ntx), tx = (int)((i64)(ix + 1) * g.nx / r.ntx) - x0;
@@ -561,14 +561,29 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_resident2d(const __grid_const
     }
 }
 
+// us per step of a resident launch, and of the ordinary launches
+// (sfd_quad2d.cu) of a run's nb shots: fits to a B200 (resident / ordinary:
+// 100 x 150 order 4 2.8 / 8.9; 300 x 400 order 8 4.7 / 11.0, L = 2 5.2 / 12.1;
+// 400 x 577 order 8 9.5 / 11.5, L = 3 11.6 / 15.7; ordinary alone: 600 x 1000
+// order 8 16.6, 602 x 1503 order 8 L = 2 28.8, 8 shots of 300 x 1000 order 4
+// 30.4).  4 shots of 300 x 400, L = 2: 20.2 one after the other, 17.7 together.
+static double resident2d_step_us(const Res2d &r, int L)
+{
+    return r.nc == 1 ? 3.2 : r.nc == 2 ? 4.7 + 0.25 * L : 9.3 + 0.8 * L;
+}
+static double ordinary2d_step_us(const Grid &g, int nb)
+{
+    return 9.0 + (g.F == 2 ? 0.9e-5 : 1.2e-5) * (1.0 + 0.4 * g.L) * nb * (double)g.nz * g.nx;
+}
+
 // Tiles of a resident launch of nb shots: ctas = 0 where it does not apply.
 // It takes FP32 fields, order 4 or 8, up to 3 relaxation mechanisms, CPML
 // slabs that do not overlap (or no absorbing layer); every tile is at least
 // F + 1 cells a side (its halo is one neighbour deep, and the surface images
-// of a column come from its own tile) and its halo at most R2_WORDS words a
+// of a column come from its own tile) and its halo at most r2_words words a
 // thread.  With one CTA per SM and up to 4 cells per thread that is about
 // 250,000 cells; larger grids fill the chip with ordinary launches.
-Res2d resident2d_shape(const Grid &g, int nb, int npoints)
+static Res2d resident2d_shape(const Grid &g, int nb, int npoints)
 {
     Res2d best;
     memset(&best, 0, sizeof best);
@@ -593,7 +608,7 @@ Res2d resident2d_shape(const Grid &g, int nb, int npoints)
             r.ctas = r.ntz * r.ntx * nb;
             r.side = std::max(r.tz, r.tx);
             const int words = 4 * F * (r.tz + r.tx);
-            if (r.ctas > R2_CTAS || words > R2_WORDS * R2_THREADS) continue;
+            if (r.ctas > R2_CTAS || words > r2_words(nc) * R2_THREADS) continue;
             const size_t field = sizeof(float) * (size_t)field_floats(F, nc) * R2_NF;
             r.smem = (field + 15) / 16 * 16 + (size_t)npoints * (sizeof(int4) + sizeof(float));
             // fewest cells a thread, then words a thread, then CTAs
@@ -602,6 +617,25 @@ Res2d resident2d_shape(const Grid &g, int nb, int npoints)
         }
         if (best.ctas) break;
     }
+    return best;
+}
+
+// Resident launches for the nb shots of a run: how many shots a launch takes
+// (r.shots; the launches follow one another), or ctas = 0 where the ordinary
+// launches take them all together in less time.
+Res2d resident2d_plan(const Grid &g, int nb, int npoints)
+{
+    Res2d best;
+    memset(&best, 0, sizeof best);
+    double best_us = 0.0;
+    for (int n = nb; n >= 1; n--) {
+        Res2d r = resident2d_shape(g, n, npoints);
+        if (!r.ctas) continue;
+        r.shots = n;
+        const double us = ((nb + n - 1) / n) * resident2d_step_us(r, g.L);
+        if (!best.ctas || us < best_us) { best = r; best_us = us; }
+    }
+    if (best.ctas && best_us > ordinary2d_step_us(g, nb)) best.ctas = 0;
     return best;
 }
 

@@ -1626,7 +1626,7 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
             // saved boundaries must see the stresses before it
             if (quads2d) {
                 launch_quad2d_s(g, p->f, bs, p->cfg.precision, (int64_t)t * g.nbnd, g.freesurf != 0, s);
-            } else {
+            } else if (!(bnd_shells && launch_update_s_bnd(g, p->f, bs, p->cfg.precision, (int64_t)t * g.nbnd, s))) {
                 const bool folded = launch_update_s(g, p->f, s, !bnd_shells);
                 if (bnd_shells) launch_savebnd(g, p->f, bs, p->cfg.precision, (int64_t)t * g.nbnd, s);
                 if (g.freesurf && !folded) launch_surface(g, p->f, 1, s);

@@ -1596,6 +1596,14 @@ bool launch_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool fold_
     return false;
 }
 
+bool launch_update_s_bnd(const Grid &g, const Fields &f, const BndSlot &b, int prec, int64_t tofs, cudaStream_t st)
+{
+    if (!q4_ok(g) || g.kernels != 0 || g.L > 0 || g.nb > 1 || g.fhalf || g.fused || g.vasync) return false;
+    if (g.F == 4) quad_update_s_bnd<4>(g, f, b, prec, tofs, g.freesurf != 0, st);
+    else quad_update_s_bnd<2>(g, f, b, prec, tofs, g.freesurf != 0, st);
+    return true;
+}
+
 // movie snapshot (time_stepping.c:272-350): padded field -> [nx][ny][nz]
 template <class T>
 __global__ void k_movie(Grid g, const T *fld, float inv_scale, float *dst)

@@ -27,6 +27,11 @@ int tma_take_status();      // 1 if a TMA stage of the last launches never arriv
 // 4-cell vectorised 3D kernels (sfd_quad3d.cuh), half width 2 or 4;
 // quad_update_s returns whether the launch applied the free surface
 template <int F> void quad_update_v(const Grid &g, const Fields &f, cudaStream_t st);
+// the elastic single-shot update that also saves the boundary shells
+template <int F>
+void quad_update_s_bnd(const Grid &g, const Fields &f, const BndSlot &b, int prec, int64_t tofs, bool surf, cudaStream_t st);
+// the same where it applies (false: not launched)
+bool launch_update_s_bnd(const Grid &g, const Fields &f, const BndSlot &b, int prec, int64_t tofs, cudaStream_t st);
 template <int F> bool quad_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool surf);
 template <int F>
 void quad_update_adj(const Grid &g, const Fields &f, const AdjFields &a, bool stress, int prec, cudaStream_t st);

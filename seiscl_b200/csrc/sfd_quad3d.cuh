@@ -432,7 +432,9 @@ __global__ void __launch_bounds__(128) k_v3d_q4(Grid g, Fields f)
     v3d_q4<F, T, MB>(g, f);
 }
 
-// The single-shot FP32 launch asks for 4 resident CTAs per SM (at most 128
+// The single-shot FP32 launch asks for NB resident CTAs per SM: 4, or 6 where
+// that (and not 4) holds the whole launch in one wave (72 x 64 x 80: 12.5 us
+// against 14.7).  4 (at most 128
 // registers, from 136, with a 36-byte spill): 0.333 ms against 0.345 at
 // 256^3 L=2 on a B200.  5 CTAs (102 registers) is slower again, and a
 // component-at-a-time update with 80 registers slower still (0.37 ms): the
@@ -444,8 +446,8 @@ __global__ void __launch_bounds__(128) k_v3d_q4(Grid g, Fields f)
 // Taking the x planes in the reverse of the stress kernel's order (each
 // kernel starting on the planes the other has just written) was measured
 // and is not faster: 16.96 against 17.00 Gcell/s at 256^3, L=2.
-template <int F, bool TRIG = false>
-__global__ void __launch_bounds__(128, 4) k_v3d_q4_b4(Grid g, Fields f)
+template <int F, int NB = 4, bool TRIG = false>
+__global__ void __launch_bounds__(128, NB) k_v3d_q4_b(Grid g, Fields f)
 {
     if constexpr (TRIG) pdl_trigger();
     constexpr bool MB = false;
@@ -577,9 +579,40 @@ __device__ __forceinline__ void cpml_s3d_q4(const Grid &g, const Fields &f, int 
 // forms them) and writes the images szz(F-m) = -szz(F+m) for m = 1..3 and
 // sxz(F-m) = -sxz(F+m-1), syz(F-m) = -syz(F+m-1) for m = 1..4; the quad at
 // gz0 = F+4 writes szz(F-4) = -szz(F+4).
-template <int F, int L, class T, class TR = T>
+// shell indices of a quad's cells (-1: none).  Most quads lie wholly inside
+// or outside the shell: one comparison per axis settles them, against some
+// forty integer operations a cell.
+__device__ __forceinline__ bool shell_quad3d(const Grid &g, int gz0, int gy, int gx, int (&m)[4])
+{
+    const BndDims b = bnd_dims(g);
+    const int F = g.F, i = gx - b.lbnd, j = gy - b.lbnd, k = gz0 - b.lbnds;
+    if (i < 0 || i >= b.NXbnd || j < 0 || j >= b.NYbnd || k + 3 < 0 || k >= b.NZbnd) return false;
+    if (i >= F && i < b.NXbnd - F && j >= F && j < b.NYbnd - F && k >= F && k + 3 < b.NZbnd - F) return false;
+#pragma unroll
+    for (int q = 0; q < 4; q++) m[q] = inject_ind3d(g, gz0 + q, gy, gx);
+    return true;
+}
+
+// the boundary shells a stress update saves: stores, offset of the step's
+// slice, shell indices of the quad's cells (none: the quad has none)
+struct BndQuad {
+    const BndSlot *b;
+    i64 at;
+    int m[4];
+    bool any;
+};
+template <class TB>
+__device__ __forceinline__ void bnd_save(const Grid &g, const BndQuad &q, int w, const Q4 &v)
+{
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        if (q.m[j] >= 0) ((TB *)q.b->p[w])[q.at + q.m[j]] = from_f<TB>(v.v[j] * g.bsc[w]);
+}
+
+template <int F, int L, class T, class TR = T, class TB = void>
 __device__ __forceinline__ void s_normal_q4(const Grid &g, const Fields &f, int gz0, int gy, int gx, i64 iv, i64 ip,
-                                            const Q4 &vxx, const Q4 &vyy, const Q4 &vzz, bool surf = false)
+                                            const Q4 &vxx, const Q4 &vyy, const Q4 &vzz, bool surf = false,
+                                            const BndQuad *bq = nullptr)
 {
     T *const ws[3] = {fld<T>(f.w[SXX]), fld<T>(f.w[SYY]), fld<T>(f.w[SZZ])};
     TR *const wr[3] = {fld<TR>(f.r[RXX]), fld<TR>(f.r[RYY]), fld<TR>(f.r[RZZ])};
@@ -634,6 +667,13 @@ __device__ __forceinline__ void s_normal_q4(const Grid &g, const Fields &f, int 
             for (int q = 0; q < 3; q++) sq[q].v[j] = v3[q];
         }
     }
+    if constexpr (!std::is_void<TB>::value) {   // before the free surface
+        if (bq->any) {
+            const int id[3] = {SXX, SYY, SZZ};
+#pragma unroll
+            for (int q = 0; q < 3; q++) bnd_save<TB>(g, *bq, id[q], sq[q]);
+        }
+    }
     if (F == 4 && surf && gz0 == F + 4) stv(ws[2] + iv - 8, -sq[2].v[0]);
     if (surf && gz0 == F) {
         // the arithmetic of k_surf3d, forward
@@ -674,9 +714,10 @@ __device__ __forceinline__ void s_normal_q4(const Grid &g, const Fields &f, int 
     for (int q = 0; q < 3; q++) stq(ws[q] + iv, sq[q]);
 }
 
-template <int F, int L, class T, class TR = T>
+template <int F, int L, class T, class TR = T, class TB = void>
 __device__ __forceinline__ void s_shear_q4(const Grid &g, const Fields &f, int gz0, int gy, int gx, i64 iv, i64 ip,
-                                           const Q4 &vxyyx, const Q4 &vyzzy, const Q4 &vxzzx, bool surf = false)
+                                           const Q4 &vxyyx, const Q4 &vyzzy, const Q4 &vxzzx, bool surf = false,
+                                           const BndQuad *bq = nullptr)
 {
     T *const ws[3] = {fld<T>(f.w[SXY]), fld<T>(f.w[SYZ]), fld<T>(f.w[SXZ])};
     TR *const wr[3] = {fld<TR>(f.r[RXY]), fld<TR>(f.r[RYZ]), fld<TR>(f.r[RXZ])};
@@ -729,6 +770,13 @@ __device__ __forceinline__ void s_shear_q4(const Grid &g, const Fields &f, int g
             for (int q = 0; q < 3; q++) sq[q].v[j] = v3[q];
         }
     }
+    if constexpr (!std::is_void<TB>::value) {
+        if (bq->any) {
+            const int id[3] = {SXY, SYZ, SXZ};
+#pragma unroll
+            for (int q = 0; q < 3; q++) bnd_save<TB>(g, *bq, id[q], sq[q]);
+        }
+    }
     if (surf && gz0 == F) {
 #pragma unroll
         for (int m = 1; m <= F; m++) {
@@ -743,9 +791,9 @@ __device__ __forceinline__ void s_shear_q4(const Grid &g, const Fields &f, int g
 // stress update of the quad (gz0..gz0+3, gy, gx); LP: load policy of the
 // velocity reads; surf: free surface folded in (see s_normal_q4); PF: first
 // ask L2 for the quad's per-cell streams
-template <int F, int L, class T, int LP = 0, bool PF = false, bool PDL = false, class TR = T>
+template <int F, int L, class T, int LP = 0, bool PF = false, bool PDL = false, class TR = T, class TB = void>
 __device__ __forceinline__ void s3d_q4_at(const Grid &g, const Fields &f, int gz0, int gy, int gx, i64 iv, i64 ip,
-                                          bool surf = false)
+                                          bool surf = false, const BndQuad *bq = nullptr)
 {
     const i64 sx = (i64)g.NY * g.NZ, sy = g.NZ;
     const float *hc = g.hc;
@@ -780,17 +828,40 @@ __device__ __forceinline__ void s3d_q4_at(const Grid &g, const Fields &f, int gz
         vyzzy.v[j] = __fadd_rn(vyz.v[j], vzy.v[j]);
         vxzzx.v[j] = __fadd_rn(vxz.v[j], vzx.v[j]);
     }
-    s_normal_q4<F, L, T, TR>(g, f, gz0, gy, gx, iv, ip, vxx, vyy, vzz, surf);
-    s_shear_q4<F, L, T, TR>(g, f, gz0, gy, gx, iv, ip, vxyyx, vyzzy, vxzzx, surf);
+    s_normal_q4<F, L, T, TR, TB>(g, f, gz0, gy, gx, iv, ip, vxx, vyy, vzz, surf, bq);
+    s_shear_q4<F, L, T, TR, TB>(g, f, gz0, gy, gx, iv, ip, vxyyx, vyzzy, vxzzx, surf, bq);
 }
 
 // surf: the free surface of the step applied in the same launch (single-shot
-// modelling runs; see s_normal_q4)
+// modelling runs; see s_normal_q4).  Elastic launches ask for 6 CTAs per SM,
+// viscoelastic ones for 4: 100 x 200 x 200 elastic 115 us at 4, 109 at 5, 106
+// at 6; 128 x 160 x 160 84, 79, 79; 72 x 64 x 80 (6 make it one wave) 15.4 and
+// 12.6.
 template <int F, int L, class T, bool MB = false>
-__global__ void __launch_bounds__(128, 4) k_s3d_q4(Grid g, Fields f, bool surf)
+__global__ void __launch_bounds__(128, L == 0 && sizeof(T) == 4 ? 6 : 4) k_s3d_q4(Grid g, Fields f, bool surf)
 {
     CELL3D_Q4
     s3d_q4_at<F, L, T, 0>(g, f, gz0, gy, gx, iv, ip, surf);
+}
+
+// Elastic single-shot gradient runs: the update also saves the boundary
+// shells (stores b in type TB, step offset tofs) and then applies the free
+// surface, which the separate launches did in 15 + 15 us of a 237 us step at
+// 100 x 200 x 200.
+template <int F, class TB>
+__global__ void __launch_bounds__(128, 5) k_s3d_q4_bnd(Grid g, Fields f, BndSlot b, i64 tofs, bool surf)
+{
+    constexpr bool MB = false;
+    CELL3D_Q4
+    BndQuad bq;
+    bq.b = &b;
+    bq.at = tofs;
+    bq.any = shell_quad3d(g, gz0, gy, gx, bq.m);
+    if (bq.any) {
+#pragma unroll
+        for (int w = VX; w <= VZ; w++) bnd_save<TB>(g, bq, w, ldq(f.w[w] + iv));
+    }
+    s3d_q4_at<F, 0, float, 0, false, false, float, TB>(g, f, gz0, gy, gx, iv, ip, surf, &bq);
 }
 
 // Single-shot launches of the default selection: each thread first asks L2
@@ -817,14 +888,26 @@ __global__ void __launch_bounds__(128, 3) k_s3d_q4_pf(Grid g, Fields f, bool sur
 
 // ------------------------------------------------------------- launchers
 // CTA shape (quads x y rows x x planes) of a 4-cell launch: the preferred
-// shape, or half as many quads along z and twice the rows when that leaves
-// fewer threads without a quad (nz = 200: 50 quads per column fill 56 slots
-// of 8 instead of 64 of 16)
+// shape, half as many quads along z and twice the rows where that leaves fewer
+// threads without a quad, or -- where both leave more than 6 % -- rows of the
+// whole column or an even part of it.  nz = 100 (25 quads), 200 x 200,
+// elastic: velocity 93.7 us with 25 x 5 x 1 against 95.6 with 16 x 4 x 2, stress
+// 110 against 115, an adjoint step 478 against 519; 128 x 160 x 160 (32 quads)
+// keeps the preferred shape (adjoint step 361 against 366 with 16 x 8 x 1).
 static dim3 q4_block(const Grid &g, unsigned bx, unsigned by, unsigned bz)
 {
     const unsigned nq = (unsigned)(g.nz / 4);
-    if (bx >= 16 && cdiv(nq, bx / 2) * (bx / 2) < cdiv(nq, bx) * bx) return dim3(bx / 2, by * 2, bz);
-    return dim3(bx, by, bz);
+    dim3 b(bx, by, bz);
+    if (bx >= 16 && cdiv(nq, bx / 2) * (bx / 2) < cdiv(nq, bx) * bx) b = dim3(bx / 2, by * 2, bz);
+    const unsigned slots = cdiv(nq, b.x) * b.x, part = cdiv(nq, cdiv(nq, 32));
+    if (nq >= 12 && slots * 100 > nq * 106 && cdiv(nq, part) * part < slots) b = dim3(part, 128 / part, 1);
+    return b;
+}
+// whether a launch's threads fit the chip at once with `ctas` CTAs of 128
+// threads an SM
+static bool one_wave(const Grid &g, int ctas)
+{
+    return (int64_t)(g.nz / 4) * g.ny * g.nx * g.nb <= (int64_t)148 * 128 * ctas;
 }
 static dim3 q4_grid(const Grid &g, dim3 b)
 {
@@ -836,7 +919,7 @@ template <int F>
 void quad_update_v(const Grid &g, const Fields &f, cudaStream_t st)
 {
     if (g.fhalf) {
-        dim3 b(8, 4, 4), gr(cdiv(g.nz / 4, 8), cdiv(g.ny, 4), cdiv(g.nx, 4) * g.nb);
+        const dim3 b = q4_block(g, 8, 4, 4), gr = q4_grid(g, b);
         k_v3d_q4<F, __half><<<gr, b, 0, st>>>(g, f);
         return;
     }
@@ -850,8 +933,11 @@ void quad_update_v(const Grid &g, const Fields &f, cudaStream_t st)
     // then) that lets the stress kernel launch early; launched with
     // programmatic serialization itself it would need plain loads:
     // 1.0062 against 1.0038 ms per step at 256^3, L=2
-    else if (pdl_enabled()) k_v3d_q4_b4<F, true><<<gr, b, 0, st>>>(g, f);
-    else k_v3d_q4_b4<F><<<gr, b, 0, st>>>(g, f);
+    else if (one_wave(g, 6) && !one_wave(g, 4)) {
+        if (pdl_enabled()) k_v3d_q4_b<F, 6, true><<<gr, b, 0, st>>>(g, f);
+        else k_v3d_q4_b<F, 6><<<gr, b, 0, st>>>(g, f);
+    } else if (pdl_enabled()) k_v3d_q4_b<F, 4, true><<<gr, b, 0, st>>>(g, f);
+    else k_v3d_q4_b<F><<<gr, b, 0, st>>>(g, f);
 }
 
 // the FP32 stream-prefetch stress kernel; TR: storage type of the memory variables
@@ -895,6 +981,15 @@ bool quad_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool surf)
     default: quad_update_s_l<F, 3>(g, f, g4, b4, st, surf); break;
     }
     return surf;
+}
+
+template <int F>
+void quad_update_s_bnd(const Grid &g, const Fields &f, const BndSlot &b, int prec, int64_t tofs, bool surf, cudaStream_t st)
+{
+    const dim3 b4 = q4_block(g, 16, 8, 1), g4 = q4_grid(g, b4);
+    if (prec == SFD_PREC_FP16) k_s3d_q4_bnd<F, __half><<<g4, b4, 0, st>>>(g, f, b, tofs, surf);
+    else if (prec == SFD_PREC_BF16) k_s3d_q4_bnd<F, __nv_bfloat16><<<g4, b4, 0, st>>>(g, f, b, tofs, surf);
+    else k_s3d_q4_bnd<F, float><<<g4, b4, 0, st>>>(g, f, b, tofs, surf);
 }
 
 }  // namespace sfd

@@ -11,19 +11,6 @@ namespace sfd {
 // same per-cell arithmetic: backpropagation of the forward field (not for
 // the DFT gradient, g.bp2), saved-boundary injection per cell, the adjoint
 // update with CPML, and the on-the-fly gradient accumulated in FP64.
-// shell indices of a quad's cells (-1: none).  Most quads lie wholly inside
-// or outside the shell: one comparison per axis settles them, against some
-// forty integer operations a cell.
-__device__ __forceinline__ void shell_quad3d(const Grid &g, int gz0, int gy, int gx, int (&m)[4])
-{
-    const BndDims b = bnd_dims(g);
-    const int F = g.F, i = gx - b.lbnd, j = gy - b.lbnd, k = gz0 - b.lbnds;
-    if (i < 0 || i >= b.NXbnd || j < 0 || j >= b.NYbnd || k + 3 < 0 || k >= b.NZbnd) return;
-    if (i >= F && i < b.NXbnd - F && j >= F && j < b.NYbnd - F && k >= F && k + 3 < b.NZbnd - F) return;
-#pragma unroll
-    for (int q = 0; q < 4; q++) m[q] = inject_ind3d(g, gz0 + q, gy, gx);
-}
-
 // The adjoint memory variables the stress update reads.  Nothing writes
 // them in 3D but the DFT adjoint, where they are the forward arrays (the
 // update stores its new values there, update_adjs3D.cl:566-583): elsewhere
@@ -39,10 +26,11 @@ __device__ __forceinline__ void pf_l2(const void *p) { asm volatile("prefetch.gl
 
 // PF (single-shot launches of the default selection): the thread first asks
 // L2 for its quad's per-cell streams -- the forward and adjoint velocities,
-// the buoyancies and the density gradient sum -- and the launch takes 3 CTAs
-// per SM, as k_s3d_q4_pf does for the forward stress update.
+// the buoyancies and the density gradient sum -- and the launch takes 4 CTAs
+// per SM (an adjoint step of 100 x 200 x 200: 511 us against 519 with 3, 528
+// with 5).
 template <int F, typename T, bool MB = false, bool PF = false>
-__global__ void __launch_bounds__(128, PF ? 3 : 1) k_adjv3d_q4(Grid g, Fields f, AdjFields a)
+__global__ void __launch_bounds__(128, PF ? 4 : 1) k_adjv3d_q4(Grid g, Fields f, AdjFields a)
 {
     CELL3D_Q4
     if (MB) shot_adj(g, a, shot);
@@ -244,6 +232,7 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
     }
     const Q4 qM = ldq(f.p[PM] + ip), qmu = ldq(f.p[PMU] + ip);
     float gM[4] = {0, 0, 0, 0}, gmu[4] = {0, 0, 0, 0};
+    Q4 qc3 = {{0, 0, 0, 0}};
 
     // ---- normal stresses (sxx, syy, szz) with rxx, ryy, rzz: the forward
     // reconstruction of the quad, then its adjoint update
@@ -297,7 +286,7 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
 #pragma unroll
                         for (int l = 0; l < L; l++) {
                             const float el = g.eta[l];
-                            const float b = 1.0f / (1.0f + el * 0.5f), cc = 1.0f - el * 0.5f;
+                            const float b = g.eta_b[l], cc = g.eta_c[l];
                             aa += b * (rf[c][l].v[j] * cc - el * dc[c]);
                         }
                         s3[c].v[j] -= ls + g.dt2 * aa;
@@ -353,7 +342,7 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
 #pragma unroll
                     for (int l = 0; l < L; l++) {
                         const float el = g.eta[l];
-                        const float b = 1.0f / (1.0f + el * 0.5f), cc = 1.0f - el * 0.5f;
+                        const float b = g.eta_b[l], cc = g.eta_c[l];
                         const float n = b * (rr[c][l].v[j] * cc - el * dc[c]);
                         aa = g.bp2 ? n : rr[c][l].v[j];
                         rr[c][l].v[j] = n;
@@ -363,7 +352,8 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
             }
             if (!g.bp2 && g.restype == 0) {
                 const float c1 = 1.0f / (3.0f * lM - 4.0f * lmu) / (3.0f * lM - 4.0f * lmu);
-                const float c3 = 1.0f / lmu / lmu;
+                const float c3 = 1.0f / lmu / lmu;   // kept for the shear stresses
+                qc3.v[j] = c3;
                 const float c5 = 1.0f / 6.0f * c3;
                 const float sxx = s3[0].v[j], syy = s3[1].v[j], szz = s3[2].v[j];
                 const float dM = c1 * (sxx + syy + szz) * (ls[0] + ls[1] + ls[2]);
@@ -440,7 +430,7 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
 #pragma unroll
                     for (int l = 0; l < L; l++) {
                         const float el = g.eta[l];
-                        const float b = 1.0f / (1.0f + el * 0.5f), cc = 1.0f - el * 0.5f;
+                        const float b = g.eta_b[l], cc = g.eta_c[l];
                         aa += b * (rf[l].v[j] * cc - el * (dc * fsum));
                     }
                     sc.v[j] -= ls + g.dt2 * aa;
@@ -477,7 +467,7 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
 #pragma unroll
                 for (int l = 0; l < L; l++) {
                     const float el = g.eta[l];
-                    const float b = 1.0f / (1.0f + el * 0.5f), cc = 1.0f - el * 0.5f;
+                    const float b = g.eta_b[l], cc = g.eta_c[l];
                     const float n = b * (rr[l].v[j] * cc - el * (dc * rsum.v[j]));
                     aa = g.bp2 ? n : rr[l].v[j];
                     rr[l].v[j] = n;
@@ -485,9 +475,7 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
                 wc.v[j] += ls + g.dt2 * aa;
             }
             if (!g.bp2 && g.restype == 0) {
-                const float lmu = qmu.v[j];
-                const float c3 = 1.0f / lmu / lmu;
-                gmu[j] += -c3 * (sc.v[j] * ls);
+                gmu[j] += -qc3.v[j] * (sc.v[j] * ls);
             }
         }
         if constexpr (L > 0) {
@@ -534,7 +522,7 @@ static void quad_adj_t(const Grid &g, const Fields &f, const AdjFields &a, bool 
         }
         return;
     }
-    dim3 b(8, 4, 4), gr(cdiv(g.nz / 4, 8), cdiv(g.ny, 4), cdiv(g.nx, 4) * g.nb);
+    const dim3 b = q4_block(g, 8, 4, 4), gr = q4_grid(g, b);
     if (g.kernels == 0 && g.nb == 1) k_adjv3d_q4<F, T, false, true><<<gr, b, 0, st>>>(g, f, a);
     else MB_DISPATCH(g, k_adjv3d_q4<F, T, MBV><<<gr, b, 0, st>>>(g, f, a))
 }

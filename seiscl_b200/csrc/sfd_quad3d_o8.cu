@@ -5,5 +5,6 @@ namespace sfd {
 
 template void quad_update_v<4>(const Grid &, const Fields &, cudaStream_t);
 template bool quad_update_s<4>(const Grid &, const Fields &, cudaStream_t, bool);
+template void quad_update_s_bnd<4>(const Grid &, const Fields &, const BndSlot &, int, int64_t, bool, cudaStream_t);
 
 }  // namespace sfd

@@ -230,11 +230,6 @@ int upload_shots(sfd_plan *p, int nshot, const sfd_shot *shots, int mask, PointS
     return SFD_OK;
 }
 
-int upload_shot(sfd_plan *p, const sfd_shot *shot, int mask, PointSet &S, PointSet &R, cudaStream_t st)
-{
-    return upload_shots(p, 1, shot, mask, S, R, st);
-}
-
 // bytes per stored wave-field / memory-variable value
 size_t wave_elem(const Grid &g) { return g.fhalf ? 2 : sizeof(float); }
 size_t mem_elem(const Grid &g) { return g.fhalf || g.rhalf ? 2 : sizeof(float); }
@@ -1023,9 +1018,11 @@ void init_grid(const sfd_config &c, Grid &g)
     if (c.nd == 3) { g.ny = c.n[1]; g.nx = c.n[2]; }
     else { g.ny = 1; g.nx = c.n[1]; }
     // grids of the default selection take the 4-cell kernels at orders 4
-    // and 8 whatever nz: rows of 4 n + 2 cells get two dummy rows, and at
-    // order 4 the fields' base moves by two elements.  One-cell streaming
-    // kernels on the same grids were 1.7-2.4 times slower.
+    // and 8 whatever nz: columns are filled up with at most 3 dummy cells,
+    // and at order 4 the fields' base moves by two elements.  us per step on
+    // a B200, one-cell streaming kernels / these: 130 x 121 x 147, order 4,
+    // elastic 262 / 131; 122 x 131 x 117, order 8, L = 1 231 / 142 (so the dummy
+    // cells pay down to the smallest grids, where both are launch-bound).
     g.zpad = g.zshift = 0;
     if ((c.nd == 3 || (c.nd == 2 && c.field_precision == 0)) && c.kernels == 0 && (g.F == 2 || g.F == 4) && c.L <= 3) {
         g.zpad = (4 - g.nz % 4) % 4;
@@ -1582,7 +1579,7 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
         Res2dRun a{R, S, p->d_src, p->d_seis, omask, NT, 0, 0, tmax, 0, bs, p->cfg.precision, p->d_words, p->d_unstable,
                    p->d_unstable + 1};
         for (a.shot0 = 0; a.shot0 < nshot; a.shot0 += rs.shots) {
-            CKC(cudaMemsetAsync(p->d_words, 0, sizeof(*p->d_words) * (size_t)resident2d_words(rs), st));
+            CKC(cudaMemsetAsync(p->d_words, 0, sizeof(*p->d_words) * (size_t)resident2d_words(rs, false), st));
             Res2d r = rs;
             r.ctas = r.ntz * r.ntx * std::min(rs.shots, nshot - a.shot0);
             for (a.t0 = 0; a.t0 < tmax; a.t0 = a.t1) {
@@ -1697,7 +1694,8 @@ extern "C" int sfd_adjoint_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
     unsigned omask = outmask_of(outsel, g.nd, &nsel);
     if ((rc = ensure_shot_buffers(p, sb.nsrc, sb.nrec, nsel))) return rc;
     PointSet S, R;
-    if ((rc = upload_shots(p, nshot, shots, mask, S, R, st))) return rc;
+    PointLayout points;
+    if ((rc = upload_shots(p, nshot, shots, mask, S, R, st, &points))) return rc;
     const int NT = p->cfg.nt;
     int slot = 0;
     for (int o = 0; o < SFD_NOUT; o++) {
@@ -1739,7 +1737,26 @@ extern "C" int sfd_adjoint_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
     const int64_t nchk = g.nvol * g.nb;
     if ((rc = arm_unstable(p, st))) return rc;
     CKC(cudaEventRecord(p->ev0, st));
-    int rcl = run_loop(p, p->gadj, key.s, st, [&](cudaStream_t s) {
+    // shots whose forward and adjoint fields fit on chip: the loop in
+    // segments, one cooperative launch each (sfd_resident2d.cu)
+    const Res2d rs = resident2d_adj_plan(g, nshot, S.n + R.n);
+    const int tmax = p->cfg.tmax, tmin = p->cfg.tmin;
+    int rcl = SFD_OK;
+    if (rs.ctas > 0 && p->d_words && points.inside && !mv.n) {
+        for (int w = 0; w < NW; w++) a.bnd[w] = p->d_bnd[w];
+        if (tmax - 1 > tmin) launch_residuals(g, p->f, a, R, p->d_res, NT, tmax - 1, omask, S, p->d_src, -1, st);
+        Res2dAdj q{R, S, p->d_src, p->d_res, omask, NT, 0, 0, tmax, tmin, 0, p->d_words, p->d_unstable, p->d_unstable + 1};
+        for (q.shot0 = 0; q.shot0 < nshot; q.shot0 += rs.shots) {
+            CKC(cudaMemsetAsync(p->d_words, 0, sizeof(*p->d_words) * (size_t)resident2d_words(rs, true), st));
+            Res2d r = rs;
+            r.ctas = r.ntz * r.ntx * std::min(rs.shots, nshot - q.shot0);
+            for (q.t0 = tmax - 1; q.t0 > tmin; q.t0 = q.t1) {
+                q.t1 = std::max(q.t0 - RES2D_SEGMENT, tmin);
+                CKC(launch_resident2d_adj(g, p->f, a, r, q, p->cfg.precision, p->device, st));
+            }
+        }
+    } else
+    rcl = run_loop(p, p->gadj, key.s, st, [&](cudaStream_t s) {
         // the sources a step takes out of the reconstructed fields go with the
         // next step's residuals, unless a movie films the fields between
         int tsrc = -1;

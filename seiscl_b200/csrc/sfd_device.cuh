@@ -433,20 +433,32 @@ __device__ __forceinline__ float surf2d_hr(const Surf2d &s, float b, float vxx, 
     return __fmul_rn(b, __fsub_rn(__fmul_rn(s.c, vxx), __fmul_rn(s.de, vzz)));
 }
 
-// elastic P-SV gradient terms of a cell: forward stresses, adjoint increments
+// elastic P-SV gradient terms of a cell: coefficients of its material, then
+// the terms from the forward stresses and the adjoint increments
+struct Adj2dCoef {
+    float c1, c3;
+};
+__device__ __forceinline__ Adj2dCoef adj2d_coef(float M, float mu)
+{
+    const float q = __fmul_rn(2.0f, __fsub_rn(M, mu));
+    return Adj2dCoef{__fdiv_rn(1.0f, __fmul_rn(q, q)), __fdiv_rn(1.0f, __fmul_rn(mu, mu))};
+}
 struct Adj2dGrad {
     float M, mu;
 };
-__device__ __forceinline__ Adj2dGrad adj2d_grad(int restype, float M, float mu, float sxx, float szz, float sxz,
-                                                float lsxx, float lszz, float lsxz)
+__device__ __forceinline__ Adj2dGrad adj2d_terms(int restype, Adj2dCoef k, float sxx, float szz, float sxz, float lsxx,
+                                                 float lszz, float lsxz)
 {
     const float p = __fadd_rn(sxx, szz), lp = __fadd_rn(lsxx, lszz);
     if (restype != 0) return Adj2dGrad{-__fmul_rn(p, lp), 0.0f};
-    const float q = __fmul_rn(2.0f, __fsub_rn(M, mu));
-    const float c1 = __fdiv_rn(1.0f, __fmul_rn(q, q)), c3 = __fdiv_rn(1.0f, __fmul_rn(mu, mu));
-    const float dM = __fmul_rn(__fmul_rn(c1, p), lp);
-    const float sh = __fmaf_rn(-c3, __fmul_rn(sxz, lsxz), dM);
-    return Adj2dGrad{-dM, __fmaf_rn(-__fmul_rn(0.25f, c3), __fmul_rn(__fsub_rn(sxx, szz), __fsub_rn(lsxx, lszz)), sh)};
+    const float dM = __fmul_rn(__fmul_rn(k.c1, p), lp);
+    const float sh = __fmaf_rn(-k.c3, __fmul_rn(sxz, lsxz), dM);
+    return Adj2dGrad{-dM, __fmaf_rn(-__fmul_rn(0.25f, k.c3), __fmul_rn(__fsub_rn(sxx, szz), __fsub_rn(lsxx, lszz)), sh)};
+}
+__device__ __forceinline__ Adj2dGrad adj2d_grad(int restype, float M, float mu, float sxx, float szz, float sxz,
+                                                float lsxx, float lszz, float lsxz)
+{
+    return adj2d_terms(restype, adj2d_coef(M, mu), sxx, szz, sxz, lsxx, lszz, lsxz);
 }
 
 }  // namespace sfd

@@ -86,8 +86,20 @@ struct Res2dRun {           // a segment of the time loop: steps t0 .. t1-1 of t
 };
 constexpr int RES2D_SEGMENT = 256;   // steps of one launch: bounds how long it holds the SMs
 Res2d resident2d_plan(const Grid &g, int nb, int npoints);   // launches for the nb shots of a run
-int64_t resident2d_words(const Res2d &r);
+Res2d resident2d_adj_plan(const Grid &g, int nb, int npoints);
+int64_t resident2d_words(const Res2d &r, bool adjoint);
 int64_t resident2d_bytes(const Grid &g, int batch);   // exchange words of launches of up to `batch` shots
+struct Res2dAdj {           // a segment of the adjoint loop: steps t0, t0-1 .. t1+1 of tmax-1 .. tmin+1
+    PointSet rec, src;
+    const float *stf, *res; // [nsrc][nt_total], [nsel][nrec][nt_total]
+    unsigned outmask;
+    int nt_total, t0, t1, tmax, tmin, shot0;
+    unsigned long long *words;
+    int *first_bad, *status;
+};
+// q.bnd: the saved boundaries from step 0
+cudaError_t launch_resident2d_adj(const Grid &g, const Fields &f, const AdjFields &q, const Res2d &r, const Res2dAdj &a,
+                                  int prec, int device, cudaStream_t st);
 cudaError_t launch_resident2d(const Grid &g, const Fields &f, const Res2d &r, const Res2dRun &a, int device,
                               cudaStream_t st);
 void launch_savebnd(const Grid &g, const Fields &f, const BndSlot &b, int prec, int64_t tofs, cudaStream_t st);

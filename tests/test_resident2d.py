@@ -1,7 +1,8 @@
 """2D P-SV modelling with the wave fields resident on chip
 (sfd_resident2d.cu) against the one-launch-per-kernel loop (kernels
 "general"), bit for bit: seismograms, final wave fields and memory
-variables, and the gradient from the boundary shells it saves.  Grids from
+variables, the gradient from the boundary shells it saves, and the adjoint
+loop of elastic media without a free surface.  Grids from
 one tile to the whole chip, ragged tiles, every order, more points in a tile
 than its list holds, several sources in one cell, points in the padding."""
 import dataclasses
@@ -95,6 +96,39 @@ def test_resident_batch_and_shells(nz, nx, nb, prec, cuda_device):
         p.zero_gradient()
         p.adjoint_batch(shots, d)
         got.append({**{"%s%d" % (k, i): v for i, s in enumerate(d) for k, v in s.items()}, **p.gradient(transform=False)})
+    assert np.abs(got[1]["M"]).max() > 0
+    _same(*got)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kw,nb,prec,sel", [
+    (dict(nz=20, nx=33, nt=60, nab=4, fdorder=4), 1, "fp32", ["vx", "vz"]),
+    (dict(nz=100, nx=150, nt=90, nab=16, fdorder=4, src_type=2), 1, "fp32", ["p"]),
+    (dict(nz=38, nx=301, nt=300, nab=8, fdorder=8), 1, "bf16", ["vx", "vz", "p", "sxz"]),     # two segments
+    (dict(nz=302, nx=391, nt=70, nab=20, fdorder=8), 1, "fp32", ["vx", "vz"]),                # two cells a thread
+    (dict(nz=102, nx=95, nt=80, nab=9, fdorder=8, src_type=0), 5, "fp16", ["vx", "p"]),
+    (dict(nz=120, nx=90, nt=70, nab=12, fdorder=4), 16, "fp32", ["vx", "vz"]),                # groups of shots
+    (dict(nz=60, nx=70, nt=60, nab=6, fdorder=8, tmin=10, tmax=50), 1, "fp32", ["vx", "vz"]),
+    (dict(nz=96, nx=90, nt=60, nab=9, fdorder=8, abs_type=2), 2, "fp32", ["vx", "vz"]),       # left to the ordinary loop
+], ids=lambda k: "%dx%d-o%d" % (k["nz"], k["nx"], k["fdorder"]) if isinstance(k, dict) else None)
+def test_resident_adjoint_matches_general(kw, nb, prec, sel, cuda_device):
+    """The resident adjoint loop: gradient sums, reconstructed fields and
+    memory variables left by the last step, bit for bit.  Two sources, the
+    second in the cell of a receiver."""
+    steps = {k: kw[k] for k in ("tmin", "tmax") if k in kw}
+    cfg, model, acq = make_case(nd=2, freesurf=0, **{k: v for k, v in kw.items() if k not in steps})
+    shots = []
+    for b in range(nb):
+        sp = np.repeat(acq["src_pos"], 2, 0)
+        sp[0, 0] += 10.0 * (b % 5)
+        sp[1, :3] = acq["rec_pos"][0, :3]
+        shots.append((sp, np.repeat(acq["src"], 2, 0) * (1 + b), acq["rec_pos"]))
+    got = []
+    for p in _plans(cfg, model, batch=nb, precision=prec, **steps):
+        d = p.forward_batch(shots, sel, save_boundaries=True)
+        p.zero_gradient()
+        p.adjoint_batch(shots, d)
+        got.append({**p.gradient(transform=False), **_states(p, cfg)})
     assert np.abs(got[1]["M"]).max() > 0
     _same(*got)
 

@@ -77,7 +77,7 @@ void dfree(sfd_plan *p, void *ptr, size_t bytes)
 int64_t user_cells(const Grid &g) { return (int64_t)(g.nz - g.zpad) * g.ny * g.nx; }
 
 // bytes added to every field allocation whose base is shifted
-size_t field_slack(const Grid &g) { return g.zshift ? 16 : 0; }
+size_t field_slack(const Grid &g) { return g.zshift ? 128 : 0; }
 
 // allocation owned by the plan (freed with it)
 void *dalloc(sfd_plan *p, size_t bytes, cudaError_t *err)
@@ -1027,6 +1027,12 @@ void init_grid(const sfd_config &c, Grid &g)
     if ((c.nd == 3 || (c.nd == 2 && c.field_precision == 0)) && c.kernels == 0 && (g.F == 2 || g.F == 4) && c.L <= 3) {
         g.zpad = (4 - g.nz % 4) % 4;
         g.zshift = (4 - g.F) % 4;
+        // viscoelastic 3D: the first interior cell on a 128-byte line, so that
+        // the rows of a grid with NZ % 8 == 0 all start on a 32-byte sector
+        // and a warp's accesses touch no more sectors than they fill.  256^3,
+        // L = 2 on a B200: stress 638 us against 654, velocity 285 against
+        // 289; elastic 256^3 was slower with it, 644 us a step against 633.
+        if (c.nd == 3 && c.L > 0 && c.field_precision == 0) g.zshift = 32 - g.F;
     }
     g.NZl = g.nz + 2 * g.F;
     g.nz += g.zpad;

@@ -52,6 +52,7 @@ struct Grid {
     int zpad, zshift;       // 3D, 4-cell kernels: dummy z rows at the bottom that fill nz up to whole quads (nz and NZ
                             // count them; parameters are zero there), and the elements by which the fields'
                             // base is moved so that every row's first physical cell is 16-byte aligned
+                            // (viscoelastic: 128-byte in the first row)
     int NZl;                // NZ without the dummy rows
     int nab, L, freesurf, abs_type;
     int64_t nvol;           // padded cell count

@@ -1482,7 +1482,7 @@ __global__ void k_residuals(AdjFields a, PointSet r, const float *res, int nt_to
 // first cell is aligned, see init_grid)
 static inline bool q4_ok(const Grid &g)
 {
-    return g.nd == 3 && g.nz % 4 == 0 && (g.F == 4 || (g.F == 2 && g.zshift == 2));
+    return g.nd == 3 && g.nz % 4 == 0 && (g.F == 4 || g.F == 2) && (g.F + g.zshift) % 4 == 0;
 }
 
 #define DISPATCH_F(F, ...)                                                      \
@@ -1664,7 +1664,7 @@ int stress_family(const Grid &g, const Fields &f)
     // the same selection as launch_update_s; 4-cell kernels on a grid that
     // needs padded rows (Grid::zpad) or a shifted base (Grid::zshift) count as
     // the streaming family's form for that grid
-    const bool plain = q4_ok(g) && g.zpad == 0 && g.zshift == 0;
+    const bool plain = q4_ok(g) && g.zpad == 0 && g.F == 4;
     if (g.nd != 3) return 0;
     if (g.fhalf && g.L <= 3) return plain ? 5 : 4;
     if (g.kernels == 3 && tma_ready(g, f)) return 3;

@@ -22,7 +22,7 @@ namespace sfd {
 // DRAM bytes.  Every row's first physical cell must lie on a 16-byte boundary
 // and rows must be whole quads: Grid::zpad fills rows of 4 n + 2 cells up with
 // dummy cells (zero parameters, so their fields stay zero), Grid::zshift
-// moves the fields' base for F = 2.  Same operation order per cell as k_v3d.
+// moves the fields' base for F = 2 and L > 0.  Same operation order per cell as k_v3d.
 struct Q4 {
     float v[4];
 };

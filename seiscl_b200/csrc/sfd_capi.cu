@@ -1032,7 +1032,7 @@ void init_grid(const sfd_config &c, Grid &g)
         // and a warp's accesses touch no more sectors than they fill.  256^3,
         // L = 2 on a B200: stress 638 us against 654, velocity 285 against
         // 289; elastic 256^3 was slower with it, 644 us a step against 633.
-        if (c.nd == 3 && c.L > 0 && c.field_precision == 0) g.zshift = 32 - g.F;
+        if (c.nd == 3 && c.L > 0) g.zshift = 32 - g.F;
     }
     g.NZl = g.nz + 2 * g.F;
     g.nz += g.zpad;

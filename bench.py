@@ -763,13 +763,13 @@ def main():
     h2d = sp.nbytes + src.nbytes + rp.nbytes
     d2h = len(outs) * rp.shape[0] * w["nt"] * 4
     checks = (w["nt"] + 63) // 64   # finite checks of the instability detection
-    if w["nd"] == 3 and fused:      # sources, fused step, receivers
-        launches_per_shot = 3 * w["nt"] + checks
-    elif w["nd"] == 3:   # sources, velocity, stress (FP32 4-cell: with the free surface), [surface], receivers
-        sep_surface = w["freesurf"] and (fam != "vector" or args.fields == "fp16")
-        launches_per_shot = w["nt"] * (4 + (1 if sep_surface else 0)) + checks
-    else:   # 2D modelling: update_v and the fused stress/surface/receiver/source launch
-        launches_per_shot = 2 * w["nt"] + 1 + checks
+    if w["nd"] == 3:   # first sources; velocity and stress (or the fused step), [surface], receivers with the next sources
+        sep_surface = 1 if w["freesurf"] and fam != "vector" and not fused else 0
+        launches_per_shot = 1 + w["nt"] * ((1 if fused else 2) + sep_surface + 1) + checks
+    elif args.kernels == "fast" and args.fields == "fp32" and cells <= 250000:   # first sources; segments of 256 resident steps
+        launches_per_shot = 1 + (w["nt"] + 255) // 256
+    else:   # first sources; velocity, stress with the surface, receivers with the next sources
+        launches_per_shot = 1 + 3 * w["nt"] + checks
     field_gb = cells * 4 * (9 + 6 * w["L"]) / 1e9 if w["nd"] == 3 else cells * 4 * (5 + 3 * w["L"]) / 1e9
     l2 = ("inputs larger than L2 (%.2f GB of fields)" % field_gb if field_gb > 0.126 else
           "working set L2-resident by design (%.1f MB of fields, reread every time step); no flush" % (field_gb * 1e3))

@@ -77,12 +77,14 @@ typedef struct sfd_config {
     int param_type;    /* 0: vp,vs,rho  1: M,mu,rho  2: Ip,Is,rho */
     int restype;       /* 0: L2 (full gradient), 1: M only */
     int precision;     /* SFD_PREC_*: storage of the saved boundaries */
-    int kernels;       /* 0: fastest measured: in 3D the 4-cell vectorised kernels where
-                             they apply (8th order, nz a multiple of 4, L <= 3), else the
-                             streaming ones; in 2D (P-SV, acoustic) modelling runs
-                             without saved boundaries, DFT or movie, two launches per
-                             step (the stress update carries the free surface, the
-                             receivers and the next step's sources),
+    int kernels;       /* 0: fastest measured: 4-cell vectorised kernels (3D and 2D P-SV,
+                             4th and 8th order, L <= 3; rows that are no multiple of 4
+                             carry up to 3 dummy cells on the device), else streaming
+                             (3D) or one-cell (2D) ones; 2D P-SV runs whose wave fields
+                             fit on chip take segments of time steps in one cooperative
+                             launch; 2D acoustic modelling runs without saved boundaries,
+                             DFT or movie, two launches per step (the stress update
+                             carries the receivers and the next step's sources),
                           1: general one-thread-per-cell kernels only, one launch per
                              reference kernel,
                           2: register-blocked 3D kernels where available,
@@ -348,8 +350,9 @@ int sfd_plan_info(const sfd_plan *plan, int64_t *out8);
 int sfd_plan_uses_tma(const sfd_plan *plan);
 
 /* Kernel family of the plan's 3D stress update (after sfd_set_model): 0 not
- * 3D, 1 general, 2 register-blocked, 3 TMA-pipelined, 4 streaming, 5 4-cell
- * vectorised; negative on error.  No counterpart in the reference. */
+ * 3D, 1 general, 2 register-blocked, 3 TMA-pipelined, 4 streaming (and grids
+ * whose rows are padded or shifted on the device for the 4-cell kernels), 5
+ * 4-cell vectorised; negative on error.  No counterpart in the reference. */
 int sfd_plan_kernel_family(const sfd_plan *plan);
 
 /* Copy a device array of the plan to the host (tests): kind 0 wave field,

@@ -150,7 +150,7 @@ class Config:
     param_type: int = 0
     restype: int = 0
     precision: str = "fp32"
-    kernels: str = "fast"  # "fast" (3D: 4-cell vectorised where eligible, else streaming), "general",
+    kernels: str = "fast"  # "fast" (the measured fastest: 4-cell vectorised where eligible), "general",
     #                        "register", "tma", "stream", "vector", "fused" ("fast" plus the fused
     #                        one-launch modelling step)
     adjoint_reset_psi: bool = False  # True: the adjoint starts from zeroed CPML memory (not the reference's)
@@ -471,7 +471,8 @@ class Plan:
     @property
     def kernel_family(self) -> str:
         """Kernel family of the 3D stress update ("general", "register",
-        "tma", "stream", "vector"; "2d" for 2D plans)."""
+        "tma", "stream", "vector"; "2d" for 2D plans).  "stream" covers the
+        grids whose rows are padded on the device for the 4-cell kernels."""
         rc = int(self.lib.sfd_plan_kernel_family(self.h))
         if rc < 0:
             self._check(rc)

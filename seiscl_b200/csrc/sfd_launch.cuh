@@ -19,17 +19,14 @@ static inline unsigned cdiv(long a, long b) { return (unsigned)((a + b - 1) / b)
     if ((g).nb > 1) { constexpr bool MBV = true; __VA_ARGS__; }                  \
     else { constexpr bool MBV = false; __VA_ARGS__; }
 
-// Programmatic dependent launch for the single-shot 3D loop: the stress
-// kernel, the sources and the receivers are launched with programmatic
-// stream serialization, so each may be resident while the previous one
-// drains its last wave (and the stress kernel asks L2 for its own streams
-// meanwhile); every one of them waits (pdl_wait) before it reads or writes
-// anything the previous kernels touch, and reads those fields with plain
-// loads (a read-only-path load may be hoisted above the wait).  The
-// velocity kernel is an ordinary launch that triggers its dependents
-// early.  256^3, L=2: 1.004 against 1.015 ms per step.  The same for the
-// 2D P-SV loop (velocity and fused stress-step kernels, 300 x 400) was
-// slower, 7.17 against 7.39 Gcell/s, and is not done.  On unless the
+// Programmatic dependent launch for the single-shot 3D loop: the receivers
+// and the sources are launched with programmatic stream serialization, so
+// they may be resident while the previous kernel drains its last wave; they
+// wait (pdl_wait) before they read or write anything the previous kernels
+// touch, and read those fields with plain loads (a read-only-path load may be
+// hoisted above the wait).  The velocity and stress kernels are ordinary
+// launches: their stencils are faster through the read-only path than any
+// overlap gains (256^3, L=2: 911 against 919 us per step).  On unless the
 // environment sets SEISCL_B200_PDL=0.
 static bool pdl_enabled()
 {

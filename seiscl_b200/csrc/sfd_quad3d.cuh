@@ -58,25 +58,22 @@ __device__ __forceinline__ void stq(__half *p, const Q4 &q)
     *reinterpret_cast<uint2 *>(p) = u;
 }
 // Load policy of the stencil reads (template parameter LP): 0 the read-only
-// path (__ldg; arrays no thread writes during the launch), 1 a plain global
-// load (arrays that other CTAs write later in the same launch, read before
-// they do), 2 L2 only (__ldcg: values other CTAs wrote earlier in the same
-// launch, which a stale L1 line must not hide).
+// path (__ldg; arrays no thread writes during the launch), 2 L2 only (__ldcg:
+// values other CTAs wrote earlier in the same launch, which a stale L1 line
+// must not hide).
 template <int LP>
 __device__ __forceinline__ Q4 ldq_p(const float *p)
 {
     float4 t;
     if constexpr (LP == 0) t = __ldg(reinterpret_cast<const float4 *>(p));
-    else if constexpr (LP == 1) t = *reinterpret_cast<const float4 *>(p);
     else t = __ldcg(reinterpret_cast<const float4 *>(p));
     return Q4{{t.x, t.y, t.z, t.w}};
 }
 template <int LP>
 __device__ __forceinline__ Q4 ldq_p(const __half *p)
 {
-    static_assert(LP == 0 || LP == 1, "FP16 fields are read through the read-only path or plainly");
-    if constexpr (LP == 0) return ldq(p);
-    else return ldq_rw(p);
+    static_assert(LP == 0, "FP16 fields are read through the read-only path");
+    return ldq(p);
 }
 
 // add a quad to its FP64 sums
@@ -434,22 +431,17 @@ __global__ void __launch_bounds__(128) k_v3d_q4(Grid g, Fields f)
 
 // The single-shot FP32 launch asks for NB resident CTAs per SM: 4, or 6 where
 // that (and not 4) holds the whole launch in one wave (72 x 64 x 80: 12.5 us
-// against 14.7).  4 (at most 128
-// registers, from 136, with a 36-byte spill): 0.333 ms against 0.345 at
-// 256^3 L=2 on a B200.  5 CTAs (102 registers) is slower again, and a
-// component-at-a-time update with 80 registers slower still (0.37 ms): the
-// kernel is bound by the stencil loads each thread keeps in flight.
-// TRIG: an ordinary launch that lets the next kernel (the stress update,
-// launched with programmatic stream serialization) launch early.  Launched
-// that way itself, the kernel would have to read the stresses with plain
-// loads (see k_s3d_q4_pf), which cost it more than the overlap gives.
+// against 14.7).  4 (at most 128 registers, from 136, with a 24-byte spill):
+// 0.333 ms against 0.345 at 256^3 L=2 on a B200, 0.285 since.  5 CTAs (102
+// registers) is slower again, and a component-at-a-time update with 80
+// registers slower still (0.37 ms): the kernel is bound by the stencil loads
+// each thread keeps in flight.  CTAs of 256 or 512 threads: 0.323-0.343 ms.
 // Taking the x planes in the reverse of the stress kernel's order (each
 // kernel starting on the planes the other has just written) was measured
 // and is not faster: 16.96 against 17.00 Gcell/s at 256^3, L=2.
-template <int F, int NB = 4, bool TRIG = false>
+template <int F, int NB = 4>
 __global__ void __launch_bounds__(128, NB) k_v3d_q4_b(Grid g, Fields f)
 {
-    if constexpr (TRIG) pdl_trigger();
     constexpr bool MB = false;
     CELL3D_Q4
     v3d_q4_at<F, float, 0>(g, f, gz0, gy, gx, iv, ip);
@@ -791,7 +783,7 @@ __device__ __forceinline__ void s_shear_q4(const Grid &g, const Fields &f, int g
 // stress update of the quad (gz0..gz0+3, gy, gx); LP: load policy of the
 // velocity reads; surf: free surface folded in (see s_normal_q4); PF: first
 // ask L2 for the quad's per-cell streams
-template <int F, int L, class T, int LP = 0, bool PF = false, bool PDL = false, class TR = T, class TB = void>
+template <int F, int L, class T, int LP = 0, bool PF = false, class TR = T, class TB = void>
 __device__ __forceinline__ void s3d_q4_at(const Grid &g, const Fields &f, int gz0, int gy, int gx, i64 iv, i64 ip,
                                           bool surf = false, const BndQuad *bq = nullptr)
 {
@@ -810,9 +802,6 @@ __device__ __forceinline__ void s3d_q4_at(const Grid &g, const Fields &f, int gz
 #pragma unroll
         for (int k = 0; k < np; k++) asm volatile("prefetch.global.L2 [%0];" ::"l"(f.p[pid[k]] + ip));
     }
-    // launched early (programmatic dependent launch): everything the
-    // previous kernels write is read from here on
-    if constexpr (PDL) pdl_wait();
     const T *Vx = fld<T>(f.w[VX]), *Vy = fld<T>(f.w[VY]), *Vz = fld<T>(f.w[VZ]);
     Q4 vzz = dbw_z<F>(ldw<T, LP>(Vz, iv), hc);
     Q4 vyz = dfw_z<F>(ldw<T, LP>(Vy, iv), hc);
@@ -861,7 +850,7 @@ __global__ void __launch_bounds__(128, 5) k_s3d_q4_bnd(Grid g, Fields f, BndSlot
 #pragma unroll
         for (int w = VX; w <= VZ; w++) bnd_save<TB>(g, bq, w, ldq(f.w[w] + iv));
     }
-    s3d_q4_at<F, 0, float, 0, false, false, float, TB>(g, f, gz0, gy, gx, iv, ip, surf, &bq);
+    s3d_q4_at<F, 0, float, 0, false, float, TB>(g, f, gz0, gy, gx, iv, ip, surf, &bq);
 }
 
 // Single-shot launches of the default selection: each thread first asks L2
@@ -872,18 +861,21 @@ __global__ void __launch_bounds__(128, 5) k_s3d_q4_bnd(Grid g, Fields f, BndSlot
 // 0.651 ms against 0.695 for k_s3d_q4 (0.571 against 0.601 without
 // absorbing boundary); the prefetch at 4 CTAs per SM gave 0.674, 3 CTAs
 // without it 0.713.
-// PDL: launched with programmatic stream serialization (launch_pdl).  The
-// velocities then come through plain loads: a read-only-path (ld.global.nc)
-// load counts as invariant, and the compiler may move it above the wait.
+// An ordinary launch that lets the receivers' kernel launch early.  Launched
+// with programmatic serialization itself, with the prefetch ahead of its
+// wait, it has to read the velocities with plain loads (a read-only-path load
+// counts as invariant, and the compiler may move it above the wait): 0.637 ms
+// against 0.622, and 919 us a step against 911; 122 x 131 x 117, L = 1 143.9
+// against 142.9.  256 and 384 threads a CTA: 0.686-0.721 ms.
 // TR: storage type of the memory variables (FP16 under FP32 wave fields
 // with Grid::rhalf)
-template <int F, int L, class T, bool PDL = false, class TR = T>
+template <int F, int L, class T, class TR = T>
 __global__ void __launch_bounds__(128, 3) k_s3d_q4_pf(Grid g, Fields f, bool surf)
 {
     constexpr bool MB = false;
-    if constexpr (PDL) pdl_trigger();
+    pdl_trigger();
     CELL3D_Q4
-    s3d_q4_at<F, L, T, PDL ? 1 : 0, true, PDL, TR>(g, f, gz0, gy, gx, iv, ip, surf);
+    s3d_q4_at<F, L, T, 0, true, TR>(g, f, gz0, gy, gx, iv, ip, surf);
 }
 
 // ------------------------------------------------------------- launchers
@@ -929,23 +921,8 @@ void quad_update_v(const Grid &g, const Fields &f, cudaStream_t st)
     // 4, 0.284 for 8 x 2 x 8 and 0.34 for 4 x 8 x 4 quads x y x x
     const dim3 b = q4_block(g, 16, 4, 2), gr = q4_grid(g, b);
     if (g.nb > 1) k_v3d_q4<F, float, true><<<gr, b, 0, st>>>(g, f);
-    // an ordinary launch (after the sources, which are complete by
-    // then) that lets the stress kernel launch early; launched with
-    // programmatic serialization itself it would need plain loads:
-    // 1.0062 against 1.0038 ms per step at 256^3, L=2
-    else if (one_wave(g, 6) && !one_wave(g, 4)) {
-        if (pdl_enabled()) k_v3d_q4_b<F, 6, true><<<gr, b, 0, st>>>(g, f);
-        else k_v3d_q4_b<F, 6><<<gr, b, 0, st>>>(g, f);
-    } else if (pdl_enabled()) k_v3d_q4_b<F, 4, true><<<gr, b, 0, st>>>(g, f);
+    else if (one_wave(g, 6) && !one_wave(g, 4)) k_v3d_q4_b<F, 6><<<gr, b, 0, st>>>(g, f);
     else k_v3d_q4_b<F><<<gr, b, 0, st>>>(g, f);
-}
-
-// the FP32 stream-prefetch stress kernel; TR: storage type of the memory variables
-template <int F, int L, class TR>
-static void launch_s_pf(const Grid &g, const Fields &f, dim3 g4, dim3 b4, cudaStream_t st, bool surf)
-{
-    if (pdl_enabled()) launch_pdl(k_s3d_q4_pf<F, L, float, true, TR>, g4, b4, st, g, f, surf);
-    else k_s3d_q4_pf<F, L, float, false, TR><<<g4, b4, 0, st>>>(g, f, surf);
 }
 
 template <int F, int L>
@@ -956,16 +933,13 @@ static void quad_update_s_l(const Grid &g, const Fields &f, dim3 g4, dim3 b4, cu
     // 0.376 against 0.366 without it.  kernels 5 keeps k_s3d_q4.
     const bool pf = g.nb == 1 && g.kernels == 0 && L > 0;
     if (g.fhalf) {
-        // FP16: ordinary launches; with programmatic serialization the FP16
-        // velocities need plain loads, which cost this kernel more than
-        // the overlap gives (0.510 against 0.489 ms at 256^3, L=2)
         if (pf) k_s3d_q4_pf<F, L, __half><<<g4, b4, 0, st>>>(g, f, surf);
         else k_s3d_q4<F, L, __half><<<g4, b4, 0, st>>>(g, f, surf);
         return;
     }
     if constexpr (L > 0) {
-        if (pf && g.rhalf) { launch_s_pf<F, L, __half>(g, f, g4, b4, st, surf); return; }
-        if (pf) { launch_s_pf<F, L, float>(g, f, g4, b4, st, surf); return; }
+        if (pf && g.rhalf) { k_s3d_q4_pf<F, L, float, __half><<<g4, b4, 0, st>>>(g, f, surf); return; }
+        if (pf) { k_s3d_q4_pf<F, L, float><<<g4, b4, 0, st>>>(g, f, surf); return; }
     }
     MB_DISPATCH(g, k_s3d_q4<F, L, float, MBV><<<g4, b4, 0, st>>>(g, f, surf))
 }

@@ -265,6 +265,10 @@ float *dalloc_field(sfd_plan *p, size_t elem, int64_t n, cudaError_t *e)
     return (float *)(q + elem * p->g.zshift);
 }
 
+// CPML profiles, taper and reciprocals of K: 6 nc doubles, then floats, up to a
+// multiple of 8 bytes
+size_t const_bytes(int nc) { return sizeof(double) * (6 * nc + (3 * NC * nc + nc + 6 * nc + 1) / 2); }
+
 int alloc_model(sfd_plan *p)
 {
     const Grid &g = p->g;
@@ -296,8 +300,9 @@ int alloc_model(sfd_plan *p)
         if (g.zpad) CKC(cudaMemset((void *)p->f.p[k], 0, sizeof(float) * npar));   // dummy rows
     }
     int nc = std::max(2 * g.nab, 1);
-    float *cst = (float *)dalloc(p, sizeof(float) * (3 * NC * nc + nc + 6 * nc), &e);
+    double *kq = (double *)dalloc(p, const_bytes(nc), &e);
     if (e) return fail(p, SFD_ERR_MEMORY, "constant allocation failed");
+    float *cst = (float *)(kq + 6 * nc);
     for (int k = 0; k < NC; k++) {
         p->f.cx[k] = cst + (0 * NC + k) * nc;
         p->f.cy[k] = cst + (1 * NC + k) * nc;
@@ -321,7 +326,10 @@ int alloc_model(sfd_plan *p)
         if (e) return fail(p, SFD_ERR_MEMORY, "fused-step flag allocation failed");
     }
     for (int ax = 0; ax < 3; ax++)
-        for (int h = 0; h < 2; h++) p->f.kinv[ax][h] = cst + 3 * NC * nc + nc + (2 * ax + h) * nc;
+        for (int h = 0; h < 2; h++) {
+            p->f.kq[ax][h] = kq + (2 * ax + h) * nc;
+            p->f.kinv[ax][h] = cst + 3 * NC * nc + nc + (2 * ax + h) * nc;
+        }
     return SFD_OK;
 }
 
@@ -330,24 +338,29 @@ int upload_constants(sfd_plan *p)
     const Grid &g = p->g;
     const sfd_config &c = p->cfg;
     int nc = std::max(2 * g.nab, 1);
-    std::vector<float> h(3 * NC * nc + nc + 6 * nc, 0.0f);
+    std::vector<double> all(const_bytes(nc) / sizeof(double), 0.0);
+    double *const kq = all.data();
+    float *const h = (float *)(kq + 6 * nc);
     if (g.abs_type == 1 && g.nab > 0) {
         for (int ax = 0; ax < 3; ax++) {
-            float *b = h.data() + ax * NC * nc;
+            float *b = h + ax * NC * nc;
             if (!cpml_profiles(c.npower, c.k_max_cpml, c.fpml, c.vppml, c.dh, c.dt, g.nab, b + CK * nc, b + CA * nc,
                                b + CB * nc, b + CKH * nc, b + CAH * nc, b + CBH * nc))
                 return fail(p, SFD_ERR_ARG, "invalid CPML parameters");
         }
     }
-    if (g.abs_type == 2) cerjan_taper(c.abpc, g.nab, h.data() + 3 * NC * nc);
+    if (g.abs_type == 2) cerjan_taper(c.abpc, g.nab, h + 3 * NC * nc);
     // reciprocals of K and K_half for kernels that multiply instead of divide
     for (int ax = 0; ax < 3; ax++)
         for (int hh = 0; hh < 2; hh++) {
-            const float *K = h.data() + ax * NC * nc + (hh ? CKH : CK) * nc;
-            float *ki = h.data() + 3 * NC * nc + nc + (2 * ax + hh) * nc;
-            for (int i = 0; i < nc; i++) ki[i] = K[i] != 0.0f ? 1.0f / K[i] : 0.0f;
+            const float *K = h + ax * NC * nc + (hh ? CKH : CK) * nc;
+            float *ki = h + 3 * NC * nc + nc + (2 * ax + hh) * nc;
+            for (int i = 0; i < nc; i++) {
+                ki[i] = K[i] != 0.0f ? 1.0f / K[i] : 0.0f;
+                kq[(2 * ax + hh) * nc + i] = K[i] != 0.0f ? 1.0 / (double)K[i] : 0.0;
+            }
         }
-    CKC(cudaMemcpy((void *)p->f.cx[0], h.data(), sizeof(float) * h.size(), cudaMemcpyHostToDevice));
+    CKC(cudaMemcpy((void *)p->f.kq[0][0], kq, const_bytes(nc), cudaMemcpyHostToDevice));
     return SFD_OK;
 }
 
@@ -788,7 +801,7 @@ int adjoint_ckpt(sfd_plan *p, const PointSet &S, const PointSet &R, unsigned oma
                 ckpt_store(p, t - t0, s);
                 if (t == thi) break;
                 launch_update_v(g, p->f, s);
-                if (!launch_update_s(g, p->f, s, true) && g.freesurf) launch_surface(g, p->f, 1, s);
+                if (!launch_update_s(g, p->f, s, SURF_APART) && g.freesurf) launch_surface(g, p->f, 1, s);
             }
             for (int t = thi; t >= tlo; t--) {
                 ckpt_slot(p, t - t0, a);
@@ -1155,7 +1168,7 @@ extern "C" int sfd_footprint(const sfd_config *cfg, int gradient, int nsrc, int6
     const int64_t slack = (int64_t)field_slack(g);
     int64_t b = B * ((int64_t)wave_elem(g) * g.nvol * nwave + (int64_t)mem_elem(g) * g.nvol * nmem * g.L +
                      4 * psi_sizes(g, psz)) + slack * (nwave + nmem) +
-                4 * npar * NPAR + 4 * (3 * NC * nc + nc + 6 * nc);
+                4 * npar * NPAR + (int64_t)const_bytes((int)nc);
     // ensure_shot_buffers: source maps and signatures, receiver maps, seismograms and residuals
     const int64_t cs = std::max<int64_t>(nsrc, 16), cr = std::max<int64_t>(nrec_sel, 16);
     b += cs * (8 + 4 + 12 + 4 + 12 + 4 * nt) + cr * (8 + 8 * nt);
@@ -1630,7 +1643,7 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
             if (quads2d) {
                 launch_quad2d_s(g, p->f, bs, p->cfg.precision, (int64_t)t * g.nbnd, g.freesurf != 0, s);
             } else if (!(bnd_shells && launch_update_s_bnd(g, p->f, bs, p->cfg.precision, (int64_t)t * g.nbnd, s))) {
-                const bool folded = launch_update_s(g, p->f, s, !bnd_shells);
+                const bool folded = launch_update_s(g, p->f, s, bnd_shells ? SURF_NONE : SURF_FOLD);
                 if (bnd_shells) launch_savebnd(g, p->f, bs, p->cfg.precision, (int64_t)t * g.nbnd, s);
                 if (g.freesurf && !folded) launch_surface(g, p->f, 1, s);
             }

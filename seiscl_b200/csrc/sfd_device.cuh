@@ -94,19 +94,32 @@ __device__ __forceinline__ float dbw_rwT(const T *v, i64 i, i64 st, const float 
     return acc;
 }
 
-// psi = b psi + a d ; d = d/K + psi    (the CPML recursion of every kernel).
-// Ki: 1/K, rounded to FP32 on the host (Fields::kinv): within one rounding of
-// the quotient, without a division on the path of every absorbing cell
+// psi = b psi + a d ; d = d/K + psi    (the CPML recursion).  The 4-cell
+// kernels of 3D grids whose rows are whole quads multiply by 1/K in FP32
+// instead (cpml_q); everything else takes the quotient.
 __device__ __forceinline__ float cpml_psi(float psi, float a, float b, float d)
 {
     return __fmaf_rn(b, psi, __fmul_rn(a, d));
 }
-__device__ __forceinline__ void cpml(float *psi, i64 q, const float *Ki, const float *a, const float *b, int ci,
-                                     float &d)
+struct KTab {           // 1/K of a profile: of the FP32 value in FP64, and in FP32
+    const double *kq;
+    const float *kinv;
+};
+__device__ __forceinline__ KTab ktab(const Fields &f, int axis, int half) { return KTab{f.kq[axis][half], f.kinv[axis][half]}; }
+// d / K + psi with the bits of FP32 division: the FP64 product is within 2^-52
+// of the quotient, and a quotient of two 24-bit significands is 2^-49 or more
+// away from where its rounding to FP32 would change.  With division
+// instructions instead, a run of 130 x 121 x 147, order 4, took 39 ms against
+// 26, and one of 100 x 150 2.2 against 1.6.
+__device__ __forceinline__ float cpml_quot(float d, double kq, float psi)
+{
+    return __fadd_rn(__double2float_rn(__dmul_rn((double)d, kq)), psi);
+}
+__device__ __forceinline__ void cpml(float *psi, i64 q, KTab k, const float *a, const float *b, int ci, float &d)
 {
     const float ps = cpml_psi(psi[q], __ldg(a + ci), __ldg(b + ci), d);
     psi[q] = ps;
-    d = __fmaf_rn(d, __ldg(Ki + ci), ps);
+    d = cpml_quot(d, __ldg(k.kq + ci), ps);
 }
 
 template <typename T> __device__ __forceinline__ float to_f(T v);
@@ -315,25 +328,25 @@ __device__ __forceinline__ void cpml_v2d(const Grid &g, const Fields &f, int gz,
     if (gz > NZ - NAB - F - 1 && gz < NZ - F) {
         int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
         i64 q = (i64)i * (2 * NAB) + k;
-        cpml(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, sxz_z);
-        cpml(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, szz_z);
+        cpml(f.psi[PSXZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, sxz_z);
+        cpml(f.psi[PSZZ_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, szz_z);
     } else if (!g.freesurf && gz - F < NAB && gz < NZ - F) {
         int i = gx - F, k = gz - F;
         i64 q = (i64)i * (2 * NAB) + k;
-        cpml(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], k, sxz_z);
-        cpml(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], k, szz_z);
+        cpml(f.psi[PSXZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], k, sxz_z);
+        cpml(f.psi[PSZZ_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], k, szz_z);
     }
     if (gx - F < NAB) {
         int i = gx - F, k = gz - F;
         i64 q = (i64)i * g.nz + k;
-        cpml(f.psi[PSXX_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], i, sxx_x);
-        cpml(f.psi[PSXZ_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], i, sxz_x);
+        cpml(f.psi[PSXX_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], i, sxx_x);
+        cpml(f.psi[PSXZ_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], i, sxz_x);
     }
     if (gx > NX - NAB - F - 1) {
         int i = gx - NX + NAB + F + NAB, k = gz - F, ind = 2 * NAB - 1 - i;
         i64 q = (i64)i * g.nz + k;
-        cpml(f.psi[PSXX_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, sxx_x);
-        cpml(f.psi[PSXZ_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, sxz_x);
+        cpml(f.psi[PSXX_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ind, sxx_x);
+        cpml(f.psi[PSXZ_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], ind + 1, sxz_x);
     }
 }
 
@@ -345,25 +358,25 @@ __device__ __forceinline__ void cpml_s2d(const Grid &g, const Fields &f, int gz,
     if (gz > NZ - NAB - F - 1 && gz < NZ - F) {
         int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
         i64 q = (i64)i * (2 * NAB) + k;
-        cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vxz);
-        cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, vzz);
+        cpml(f.psi[PVX_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, vxz);
+        cpml(f.psi[PVZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, vzz);
     } else if (!g.freesurf && gz - F < NAB && gz < NZ - F) {
         int i = gx - F, k = gz - F;
         i64 q = (i64)i * (2 * NAB) + k;
-        cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], k, vxz);
-        cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], k, vzz);
+        cpml(f.psi[PVX_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], k, vxz);
+        cpml(f.psi[PVZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], k, vzz);
     }
     if (gx - F < NAB) {
         int i = gx - F, k = gz - F;
         i64 q = (i64)i * g.nz + k;
-        cpml(f.psi[PVX_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], i, vxx);
-        cpml(f.psi[PVZ_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], i, vzx);
+        cpml(f.psi[PVX_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], i, vxx);
+        cpml(f.psi[PVZ_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], i, vzx);
     }
     if (gx > NX - NAB - F - 1) {
         int i = gx - NX + NAB + F + NAB, k = gz - F, ind = 2 * NAB - 1 - i;
         i64 q = (i64)i * g.nz + k;
-        cpml(f.psi[PVX_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, vxx);
-        cpml(f.psi[PVZ_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, vzx);
+        cpml(f.psi[PVX_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], ind + 1, vxx);
+        cpml(f.psi[PVZ_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ind, vzx);
     }
 }
 
@@ -409,28 +422,34 @@ __device__ __forceinline__ float s2d_add(float s, float rate, float dt2, float a
 {
     return __fadd_rn(s, __fmaf_rn(dt2, a, rate));
 }
-// free surface (surface2D.cl): what a column's correction of sxx (h) and of
-// its memory variables (b hr) needs of its material and mechanisms
+// free surface (surface2D.cl, surface3D.cl): what a column's correction of sxx
+// (h) and of its memory variables (b hr) needs of its material and mechanisms
 struct Surf2d {
-    float q, a, c, de;   // gm - fm, (gm - fm)^2 / gm, (d - e)(fm / gm - 1), d - e
+    float q, qq, gm, c, de;   // gm - fm, its square, gm, (d - e)(fm / gm - 1), d - e
 };
 __device__ __forceinline__ Surf2d surf2d_of(const S2dMat &m)
 {
     Surf2d s;
     s.q = __fsub_rn(m.gm, m.fm);
-    s.a = __fdiv_rn(__fmul_rn(s.q, s.q), m.gm);
+    s.qq = __fmul_rn(s.q, s.q);
+    s.gm = m.gm;
     s.de = __fsub_rn(m.d, m.e);
     s.c = __fmul_rn(s.de, __fsub_rn(__fdiv_rn(m.fm, m.gm), 1.0f));
     return s;
 }
 __device__ __forceinline__ float surf2d_b(float eta) { return __fdiv_rn(eta, __fmaf_rn(eta, 0.5f, 1.0f)); }
+// FMA: whether the second product is added in one rounding: elastic media, and
+// the surface folded into the 3D stress update of whole rows
+template <bool FMA>
 __device__ __forceinline__ float surf2d_h(const Surf2d &s, float vxx, float vzz)
 {
-    return __fsub_rn(-__fmul_rn(s.a, vxx), __fmul_rn(s.q, vzz));
+    const float t = __fdiv_rn(__fmul_rn(s.qq, vxx), s.gm);
+    return FMA ? __fmaf_rn(-s.q, vzz, -t) : __fsub_rn(-t, __fmul_rn(s.q, vzz));
 }
-__device__ __forceinline__ float surf2d_hr(const Surf2d &s, float b, float vxx, float vzz)
+// what a mechanism's memory variable gains is b (surf2d_b) times this
+__device__ __forceinline__ float surf2d_hr(const Surf2d &s, float vxx, float vzz)
 {
-    return __fmul_rn(b, __fsub_rn(__fmul_rn(s.c, vxx), __fmul_rn(s.de, vzz)));
+    return __fmaf_rn(s.c, vxx, -__fmul_rn(s.de, vzz));
 }
 
 // elastic P-SV gradient terms of a cell: coefficients of its material, then

@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(128, 2) k_v3d_async(Grid g, Fields f)
             Q4 syy_y = dfw_s(H0 + 0 * HP + hrow + 4, AHZ, hc);
             Q4 sxy_y = dbw_s(H0 + 3 * HP + hrow + 4, AHZ, hc);
             if (g.abs_type == 1)
-                cpml_v3d_q4(g, f, gz0, gy, gx, sxx_x, syy_y, szz_z, sxy_y, sxy_x, syz_y, syz_z, sxz_x, sxz_z);
+                cpml_v3d_q4<false>(g, f, gz0, gy, gx, sxx_x, syy_y, szz_z, sxy_y, sxy_x, syz_y, syz_z, sxz_x, sxz_z);
 #pragma unroll
             for (int j = 0; j < 4; j++) {
                 float v3[3] = {vx.v[j] + (sxx_x.v[j] + sxy_y.v[j] + sxz_z.v[j]) * rip.v[j],
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(128, 4) k_fused3d_q4(Grid g, Fields f, FusedSy
     const int gx = F + c;
     const i64 iv = gx * sx + (i64)gy * sy + gz0;
     const i64 ip = ((i64)(gx - F) * g.ny + (gy - F)) * g.nz + (gz0 - F);
-    s3d_q4_at<4, L, float, 2>(g, f, gz0, gy, gx, iv, ip, g.freesurf != 0);
+    s3d_q4_at<4, L, float, 2>(g, f, gz0, gy, gx, iv, ip, g.freesurf ? SURF_FOLD : SURF_NONE);
 }
 
 FusedShape fused_shape(const Grid &g)

@@ -95,6 +95,7 @@ struct Fields {
     const float *cx[NC], *cy[NC], *cz[NC];
     const float *kinv[3][2];  // 1/K and 1/K_half per axis (x, y, z), FP32-rounded on the host
     const float *taper;
+    const double *kq[3][2];   // kinv in FP64
 };
 
 struct AdjFields {

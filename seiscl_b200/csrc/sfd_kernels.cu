@@ -130,27 +130,27 @@ __device__ __forceinline__ void surf2d_column(const Grid &g, const Fields &f, in
     if (g.abs_type == 1) {
         if (gx - F < NAB) {
             int i = gx - F;
-            vxx = __fmaf_rn(vxx, f.kinv[0][0][i], f.psi[PVX_X][(i64)i * g.nz + (gz - F)]);
+            vxx = cpml_quot(vxx, f.kq[0][0][i], f.psi[PVX_X][(i64)i * g.nz + (gz - F)]);
         }
         if (gx > g.NX - NAB - F - 1) {
             int i = gx - g.NX + NAB + F + NAB, ind = 2 * NAB - 1 - i;
-            vxx = __fmaf_rn(vxx, f.kinv[0][0][ind + 1], f.psi[PVX_X][(i64)i * g.nz + (gz - F)]);
+            vxx = cpml_quot(vxx, f.kq[0][0][ind + 1], f.psi[PVX_X][(i64)i * g.nz + (gz - F)]);
         }
     }
     const float sg = (float)pdir;
     if (L == 0) {
         const S2dMat m = s2d_elastic(f.p[PM][ip], f.p[PMU][ip], 0.0f);
-        stv(sxx + iv, __fmaf_rn(sg, surf2d_h(surf2d_of(m), vxx, vzz), ldv(sxx + iv)));
+        stv(sxx + iv, __fmaf_rn(sg, surf2d_h<true>(surf2d_of(m), vxx, vzz), ldv(sxx + iv)));
     } else {
         const S2dMat m = s2d_visco(L, g.dt, f.p[PM][ip], f.p[PMU][ip], 0.0f, f.p[PTAUP][ip], f.p[PTAUS][ip], 0.0f);
         float sump = 0;
         for (int l = 0; l < L; l++) sump += ldv(rxx + l * g.nvol + iv);
         const Surf2d su = surf2d_of(m);
-        const float h = __fmaf_rn(-g.dt2, sump, surf2d_h(su, vxx, vzz));
+        const float h = __fmaf_rn(-g.dt2, sump, surf2d_h<false>(su, vxx, vzz));
         stv(sxx + iv, __fmaf_rn(sg, h, ldv(sxx + iv)));
         sump = 0;
         for (int l = 0; l < L; l++) {
-            const float hh = surf2d_hr(su, surf2d_b(g.eta[l]), vxx, vzz);
+            const float hh = __fmul_rn(surf2d_b(g.eta[l]), surf2d_hr(su, vxx, vzz));
             float r = __fmaf_rn(sg, hh, ldv(rxx + l * g.nvol + iv));
             stv(rxx + l * g.nvol + iv, r);
             sump += r;
@@ -188,44 +188,44 @@ __device__ __forceinline__ void cpml_v3d(const Grid &g, const Fields &f, int gz,
         i64 i = gx - F, j = gy - F, k = gz - NZ + NAB + F + NAB;
         int ind = 2 * NAB - 1 - (int)k;
         i64 q = (i * ny + j) * (2 * NAB) + k;
-        cpml(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, sxz_z);
-        cpml(f.psi[PSYZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, syz_z);
-        cpml(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, szz_z);
+        cpml(f.psi[PSXZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, sxz_z);
+        cpml(f.psi[PSYZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, syz_z);
+        cpml(f.psi[PSZZ_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, szz_z);
     } else if (!g.freesurf && gz - F < NAB) {
         i64 i = gx - F, j = gy - F, k = gz - F;
         i64 q = (i * ny + j) * (2 * NAB) + k;
-        cpml(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, sxz_z);
-        cpml(f.psi[PSYZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, syz_z);
-        cpml(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, szz_z);
+        cpml(f.psi[PSXZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], (int)k, sxz_z);
+        cpml(f.psi[PSYZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], (int)k, syz_z);
+        cpml(f.psi[PSZZ_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], (int)k, szz_z);
     }
     if (gy - F < NAB) {
         i64 i = gx - F, j = gy - F, k = gz - F;
         i64 q = (i * (2 * NAB) + j) * nz + k;
-        cpml(f.psi[PSXY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], (int)j, sxy_y);
-        cpml(f.psi[PSYY_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], (int)j, syy_y);
-        cpml(f.psi[PSYZ_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], (int)j, syz_y);
+        cpml(f.psi[PSXY_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], (int)j, sxy_y);
+        cpml(f.psi[PSYY_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], (int)j, syy_y);
+        cpml(f.psi[PSYZ_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], (int)j, syz_y);
     } else if (gy > NY - NAB - F - 1) {
         i64 i = gx - F, j = gy - NY + NAB + F + NAB, k = gz - F;
         int ind = 2 * NAB - 1 - (int)j;
         i64 q = (i * (2 * NAB) + j) * nz + k;
-        cpml(f.psi[PSXY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], ind + 1, sxy_y);
-        cpml(f.psi[PSYY_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ind, syy_y);
-        cpml(f.psi[PSYZ_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], ind + 1, syz_y);
+        cpml(f.psi[PSXY_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], ind + 1, sxy_y);
+        cpml(f.psi[PSYY_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], ind, syy_y);
+        cpml(f.psi[PSYZ_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], ind + 1, syz_y);
     }
     if (gx - F < NAB) {
         i64 i = gx - F, j = gy - F, k = gz - F;
         i64 q = (i * ny + j) * nz + k;
-        cpml(f.psi[PSXX_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], (int)i, sxx_x);
-        cpml(f.psi[PSXY_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], (int)i, sxy_x);
-        cpml(f.psi[PSXZ_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], (int)i, sxz_x);
+        cpml(f.psi[PSXX_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], (int)i, sxx_x);
+        cpml(f.psi[PSXY_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], (int)i, sxy_x);
+        cpml(f.psi[PSXZ_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], (int)i, sxz_x);
     }
     if (gx > NX - NAB - F - 1) {
         i64 i = gx - NX + NAB + F + NAB, j = gy - F, k = gz - F;
         int ind = 2 * NAB - 1 - (int)i;
         i64 q = (i * ny + j) * nz + k;
-        cpml(f.psi[PSXX_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, sxx_x);
-        cpml(f.psi[PSXY_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, sxy_x);
-        cpml(f.psi[PSXZ_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, sxz_x);
+        cpml(f.psi[PSXX_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ind, sxx_x);
+        cpml(f.psi[PSXY_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], ind + 1, sxy_x);
+        cpml(f.psi[PSXZ_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], ind + 1, sxz_x);
     }
 }
 
@@ -242,47 +242,47 @@ __device__ __forceinline__ void cpml_s3d(const Grid &g, const Fields &f, int gz,
         i64 i = gx - F, j = gy - F, k = gz - NZ + NAB + F + NAB;
         int ind = 2 * NAB - 1 - (int)k;
         i64 q = (i * ny + j) * (2 * NAB) + k;
-        cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vxz);
-        cpml(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vyz);
-        cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, vzz);
+        cpml(f.psi[PVX_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, vxz);
+        cpml(f.psi[PVY_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, vyz);
+        cpml(f.psi[PVZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, vzz);
     }
     if (!g.freesurf && gz - F < NAB && !(adjoint_form && zb)) {
         i64 i = gx - F, j = gy - F, k = gz - F;
         i64 q = (i * ny + j) * (2 * NAB) + k;
-        cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, vxz);
-        cpml(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, vyz);
-        cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, vzz);
+        cpml(f.psi[PVX_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], (int)k, vxz);
+        cpml(f.psi[PVY_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], (int)k, vyz);
+        cpml(f.psi[PVZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], (int)k, vzz);
     }
     bool yb = gy - F < NAB;
     if (yb) {
         i64 i = gx - F, j = gy - F, k = gz - F;
         i64 q = (i * (2 * NAB) + j) * nz + k;
-        cpml(f.psi[PVX_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], (int)j, vxy);
-        cpml(f.psi[PVY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], (int)j, vyy);
-        cpml(f.psi[PVZ_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], (int)j, vzy);
+        cpml(f.psi[PVX_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], (int)j, vxy);
+        cpml(f.psi[PVY_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], (int)j, vyy);
+        cpml(f.psi[PVZ_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], (int)j, vzy);
     }
     if (gy > NY - NAB - F - 1 && !(adjoint_form && yb)) {
         i64 i = gx - F, j = gy - NY + NAB + F + NAB, k = gz - F;
         int ind = 2 * NAB - 1 - (int)j;
         i64 q = (i * (2 * NAB) + j) * nz + k;
-        cpml(f.psi[PVX_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ind, vxy);
-        cpml(f.psi[PVY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], ind + 1, vyy);
-        cpml(f.psi[PVZ_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ind, vzy);
+        cpml(f.psi[PVX_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], ind, vxy);
+        cpml(f.psi[PVY_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], ind + 1, vyy);
+        cpml(f.psi[PVZ_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], ind, vzy);
     }
     if (gx - F < NAB) {
         i64 i = gx - F, j = gy - F, k = gz - F;
         i64 q = (i * ny + j) * nz + k;
-        cpml(f.psi[PVX_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], (int)i, vxx);
-        cpml(f.psi[PVY_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], (int)i, vyx);
-        cpml(f.psi[PVZ_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], (int)i, vzx);
+        cpml(f.psi[PVX_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], (int)i, vxx);
+        cpml(f.psi[PVY_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], (int)i, vyx);
+        cpml(f.psi[PVZ_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], (int)i, vzx);
     }
     if (gx > NX - NAB - F - 1) {
         i64 i = gx - NX + NAB + F + NAB, j = gy - F, k = gz - F;
         int ind = 2 * NAB - 1 - (int)i;
         i64 q = (i * ny + j) * nz + k;
-        cpml(f.psi[PVX_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, vxx);
-        cpml(f.psi[PVY_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, vyx);
-        cpml(f.psi[PVZ_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, vzx);
+        cpml(f.psi[PVX_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], ind + 1, vxx);
+        cpml(f.psi[PVY_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ind, vyx);
+        cpml(f.psi[PVZ_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ind, vzx);
     }
 }
 
@@ -578,12 +578,12 @@ __global__ void k_surf3d(Grid g, Fields f, int pdir)
     const float vh = __fadd_rn(vxx, vyy), sg = (float)pdir;
     if (L == 0) {
         // the reference adds h without the propagation direction (surface3D.cl:172-173)
-        const float h = surf2d_h(surf2d_of(s2d_elastic(f.p[PM][ip], f.p[PMU][ip], 0.0f)), vh, vzz);
+        const float h = surf2d_h<true>(surf2d_of(s2d_elastic(f.p[PM][ip], f.p[PMU][ip], 0.0f)), vh, vzz);
         stv(sxx + iv, __fadd_rn(ldv(sxx + iv), h));
         stv(syy + iv, __fadd_rn(ldv(syy + iv), h));
     } else {
         const Surf2d su = surf2d_of(s2d_visco(L, g.dt, f.p[PM][ip], f.p[PMU][ip], 0.0f, f.p[PTAUP][ip], f.p[PTAUS][ip], 0.0f));
-        const float h = surf2d_h(su, vh, vzz);
+        const float h = surf2d_h<false>(su, vh, vzz);
         float sumx = 0, sumy = 0;
         for (int l = 0; l < L; l++) {
             sumx += ldv(rxx + l * g.nvol + iv) * g.rsci;
@@ -593,8 +593,9 @@ __global__ void k_surf3d(Grid g, Fields f, int pdir)
         stv(syy + iv, __fmaf_rn(sg, __fmaf_rn(-g.dt2, sumy, h), ldv(syy + iv)));
         sumx = 0; sumy = 0;
         for (int l = 0; l < L; l++) {
-            const float hh = surf2d_hr(su, surf2d_b(g.eta[l]), vh, vzz);
-            float rx = ldv(rxx + l * g.nvol + iv) * g.rsci + hh, ry = ldv(ryy + l * g.nvol + iv) * g.rsci + hh;
+            const float b = surf2d_b(g.eta[l]), hr = surf2d_hr(su, vh, vzz);
+            const float x = __fmul_rn(ldv(rxx + l * g.nvol + iv), g.rsci), y = __fmul_rn(ldv(ryy + l * g.nvol + iv), g.rsci);
+            const float rx = sizeof(T) == 2 ? __fmaf_rn(b, hr, x) : __fadd_rn(x, __fmul_rn(b, hr)), ry = __fmaf_rn(b, hr, y);
             stv(rxx + l * g.nvol + iv, rx * g.rsc);
             stv(ryy + l * g.nvol + iv, ry * g.rsc);
             sumx += rx; sumy += ry;
@@ -623,18 +624,18 @@ __global__ void __launch_bounds__(256) k_v2d_acc(Grid g, Fields f)
     if (g.abs_type == 1) {
         if (gz > NZ - NAB - F - 1) {
             int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
-            cpml(f.psi[PSZZ_Z], (i64)i * (2 * NAB) + k, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, p_z);
+            cpml(f.psi[PSZZ_Z], (i64)i * (2 * NAB) + k, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, p_z);
         } else if (!g.freesurf && gz - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PSZZ_Z], (i64)i * (2 * NAB) + k, f.kinv[2][1], f.cz[CAH], f.cz[CBH], k, p_z);
+            cpml(f.psi[PSZZ_Z], (i64)i * (2 * NAB) + k, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], k, p_z);
         }
         if (gx - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PSXX_X], (i64)i * g.nz + k, f.kinv[0][1], f.cx[CAH], f.cx[CBH], i, p_x);
+            cpml(f.psi[PSXX_X], (i64)i * g.nz + k, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], i, p_x);
         }
         if (gx > NX - NAB - F - 1) {
             int i = gx - NX + NAB + F + NAB, k = gz - F, ind = 2 * NAB - 1 - i;
-            cpml(f.psi[PSXX_X], (i64)i * g.nz + k, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, p_x);
+            cpml(f.psi[PSXX_X], (i64)i * g.nz + k, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ind, p_x);
         }
     }
     float vx = f.w[VX][iv] + p_x * __ldg(f.p[PRIP] + ip);
@@ -662,18 +663,18 @@ __device__ __forceinline__ void s2d_acc_cell(const Grid &g, const Fields &f, int
     if (g.abs_type == 1) {
         if (gz > NZ - NAB - F - 1) {
             int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
-            cpml(f.psi[PVZ_Z], (i64)i * (2 * NAB) + k, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, vzz);
+            cpml(f.psi[PVZ_Z], (i64)i * (2 * NAB) + k, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, vzz);
         } else if (!g.freesurf && gz - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PVZ_Z], (i64)i * (2 * NAB) + k, f.kinv[2][0], f.cz[CA], f.cz[CB], k, vzz);
+            cpml(f.psi[PVZ_Z], (i64)i * (2 * NAB) + k, ktab(f, 2, 0), f.cz[CA], f.cz[CB], k, vzz);
         }
         if (gx - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PVX_X], (i64)i * g.nz + k, f.kinv[0][0], f.cx[CA], f.cx[CB], i, vxx);
+            cpml(f.psi[PVX_X], (i64)i * g.nz + k, ktab(f, 0, 0), f.cx[CA], f.cx[CB], i, vxx);
         }
         if (gx > NX - NAB - F - 1) {
             int i = gx - NX + NAB + F + NAB, k = gz - F, ind = 2 * NAB - 1 - i;
-            cpml(f.psi[PVX_X], (i64)i * g.nz + k, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, vxx);
+            cpml(f.psi[PVX_X], (i64)i * g.nz + k, ktab(f, 0, 0), f.cx[CA], f.cx[CB], ind + 1, vxx);
         }
     }
     float p = f.w[SXX][iv];
@@ -734,18 +735,18 @@ __global__ void __launch_bounds__(256) k_v2d_sh(Grid g, Fields f)
     if (g.abs_type == 1) {
         if (gz > NZ - NAB - F - 1) {
             int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
-            cpml(f.psi[PSYZ_Z], (i64)i * (2 * NAB) + k, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, syz_z);
+            cpml(f.psi[PSYZ_Z], (i64)i * (2 * NAB) + k, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, syz_z);
         } else if (!g.freesurf && gz - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PSYZ_Z], (i64)i * (2 * NAB) + k, f.kinv[2][0], f.cz[CA], f.cz[CB], k, syz_z);
+            cpml(f.psi[PSYZ_Z], (i64)i * (2 * NAB) + k, ktab(f, 2, 0), f.cz[CA], f.cz[CB], k, syz_z);
         }
         if (gx - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PSXY_X], (i64)i * g.nz + k, f.kinv[0][0], f.cx[CA], f.cx[CB], i, sxy_x);
+            cpml(f.psi[PSXY_X], (i64)i * g.nz + k, ktab(f, 0, 0), f.cx[CA], f.cx[CB], i, sxy_x);
         }
         if (gx > NX - NAB - F - 1) {
             int i = gx - NX + NAB + F + NAB, k = gz - F, ind = 2 * NAB - 1 - i;
-            cpml(f.psi[PSXY_X], (i64)i * g.nz + k, f.kinv[0][0], f.cx[CA], f.cx[CB], ind, sxy_x);
+            cpml(f.psi[PSXY_X], (i64)i * g.nz + k, ktab(f, 0, 0), f.cx[CA], f.cx[CB], ind, sxy_x);
         }
     }
     float vy = f.w[VY][iv] + (sxy_x + syz_z) * __ldg(f.p[PRHO] + ip);
@@ -774,18 +775,18 @@ __global__ void __launch_bounds__(256) k_s2d_sh(Grid g, Fields f)
     if (g.abs_type == 1) {
         if (gz > NZ - NAB - F - 1) {
             int i = gx - F, k = gz - NZ + NAB + F + NAB, ind = 2 * NAB - 1 - k;
-            cpml(f.psi[PVY_Z], (i64)i * (2 * NAB) + k, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vyz);
+            cpml(f.psi[PVY_Z], (i64)i * (2 * NAB) + k, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, vyz);
         } else if (!g.freesurf && gz - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PVY_Z], (i64)i * (2 * NAB) + k, f.kinv[2][1], f.cz[CAH], f.cz[CBH], k, vyz);
+            cpml(f.psi[PVY_Z], (i64)i * (2 * NAB) + k, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], k, vyz);
         }
         if (gx - F < NAB) {
             int i = gx - F, k = gz - F;
-            cpml(f.psi[PVY_X], (i64)i * g.nz + k, f.kinv[0][1], f.cx[CAH], f.cx[CBH], i, vyx);
+            cpml(f.psi[PVY_X], (i64)i * g.nz + k, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], i, vyx);
         }
         if (gx > NX - NAB - F - 1) {
             int i = gx - NX + NAB + F + NAB, k = gz - F, ind = 2 * NAB - 1 - i;
-            cpml(f.psi[PVY_X], (i64)i * g.nz + k, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, vyx);
+            cpml(f.psi[PVY_X], (i64)i * g.nz + k, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ind, vyx);
         }
     }
     float mu = __ldg(f.p[PMU] + ip);
@@ -871,7 +872,7 @@ __global__ void __launch_bounds__(256) k_adjv2d(Grid g, Fields f, AdjFields a)
         float *fs[2] = {a.wr[VX], a.wr[VZ]};
         apply_taper<2>(g, f.taper, gz, 0, gx, fs, iv);
     }
-    if (!g.bp2) a.grad[GRHO][ip] += (double)__fmaf_rn(-vz, lvz, -__fmul_rn(vx, lvx));
+    if (!g.bp2) a.grad[GRHO][ip] += (double)__fmaf_rn(-vx, lvx, -__fmul_rn(vz, lvz));
 }
 
 template <int F, typename T>
@@ -1485,6 +1486,12 @@ static inline bool q4_ok(const Grid &g)
     return g.nd == 3 && g.nz % 4 == 0 && (g.F == 4 || g.F == 2) && (g.F + g.zshift) % 4 == 0;
 }
 
+// the instances of a grid's rows (grids that q4_ok accepts)
+#define ROWS_DISPATCH(g, ...)                                                   \
+    if ((g).F != 4) { constexpr int R = ROWS_O4; __VA_ARGS__; }                  \
+    else if ((g).zpad) { constexpr int R = ROWS_FILLED; __VA_ARGS__; }           \
+    else { constexpr int R = ROWS_WHOLE; __VA_ARGS__; }
+
 #define DISPATCH_F(F, ...)                                                      \
     switch (F) {                                                               \
     case 1: { constexpr int FF = 1; __VA_ARGS__; } break;                      \
@@ -1500,7 +1507,7 @@ void launch_update_v(const Grid &g, const Fields &f, cudaStream_t st)
 {
     if (g.fhalf && g.nd == 3) {   // FP16 storage: the vectorised or the streaming kernels
         if (q4_ok(g)) {
-            g.F == 4 ? quad_update_v<4>(g, f, st) : quad_update_v<2>(g, f, st);
+            ROWS_DISPATCH(g, quad_update_v<R>(g, f, st))
             return;
         }
         dim3 b(32, 4, 2), gr(cdiv(g.nz, 32), cdiv(g.ny, 4), cdiv(g.nx, 2) * g.nb);
@@ -1521,7 +1528,7 @@ void launch_update_v(const Grid &g, const Fields &f, cudaStream_t st)
     }
     if (g.nd == 3) {
         if ((g.kernels == 0 || g.kernels == 5) && q4_ok(g)) {
-            g.F == 4 ? quad_update_v<4>(g, f, st) : quad_update_v<2>(g, f, st);
+            ROWS_DISPATCH(g, quad_update_v<R>(g, f, st))
             return;
         }
         dim3 b(32, 4, 2), gr(cdiv(g.nz, 32), cdiv(g.ny, 4), cdiv(g.nx, 2) * g.nb);
@@ -1539,12 +1546,12 @@ void launch_update_v(const Grid &g, const Fields &f, cudaStream_t st)
     }
 }
 
-bool launch_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool fold_surface)
+bool launch_update_s(const Grid &g, const Fields &f, cudaStream_t st, Surf fold)
 {
     if (g.fhalf && g.nd == 3 && g.L <= 3) {   // FP16 storage: the vectorised or the streaming kernels
         if (q4_ok(g)) {
-            const bool surf = fold_surface && g.freesurf && g.nb == 1;
-            return g.F == 4 ? quad_update_s<4>(g, f, st, surf) : quad_update_s<2>(g, f, st, surf);
+            const Surf surf = g.freesurf && g.nb == 1 ? fold : SURF_NONE;
+            ROWS_DISPATCH(g, return quad_update_s<R>(g, f, st, surf))
         }
         dim3 b(32, 4, 2), gr(cdiv(g.nz, 32), cdiv(g.ny, 4), cdiv(g.nx, 2) * g.nb);
         switch (g.L) {
@@ -1560,7 +1567,7 @@ bool launch_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool fold_
     if (g.kernels == 3 && launch_update_s_tma(g, f, st)) return false;
     if (g.kernels == 2 && launch_update_s_fast(g, f, st)) return false;
     // single-shot FP32 4-cell kernels apply the free surface in the same launch
-    const bool surf = fold_surface && g.freesurf && g.nb == 1;
+    const Surf surf = g.freesurf && g.nb == 1 ? fold : SURF_NONE;
     if (g.nd == 21 || g.nd == 22) {
         dim3 b(32, 8), gr(cdiv(g.nz, 32), cdiv(g.nx, 8), g.nb);
         if (g.nd == 21) DISPATCH_F(g.F, k_s2d_sh<FF><<<gr, b, 0, st>>>(g, f))
@@ -1570,7 +1577,7 @@ bool launch_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool fold_
     if (g.nd == 3) {
         dim3 b(32, 4, 2), gr(cdiv(g.nz, 32), cdiv(g.ny, 4), cdiv(g.nx, 2) * g.nb);
         if ((g.kernels == 0 || g.kernels == 5) && q4_ok(g) && g.L <= 3) {
-            return g.F == 4 ? quad_update_s<4>(g, f, st, surf) : quad_update_s<2>(g, f, st, surf);
+            ROWS_DISPATCH(g, return quad_update_s<R>(g, f, st, surf))
         }
         if ((g.kernels == 0 || g.kernels == 4 || g.kernels == 5) && g.L <= 3) {
             switch (g.L) {
@@ -1585,9 +1592,9 @@ bool launch_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool fold_
     } else if (quad2d_ok(g)) {
         BndSlot none;
         memset(&none, 0, sizeof none);
-        const bool fold = fold_surface && g.freesurf;
-        launch_quad2d_s(g, f, none, SFD_PREC_FP32, 0, fold, st);
-        return fold;
+        const bool surf2d = fold != SURF_NONE && g.freesurf;
+        launch_quad2d_s(g, f, none, SFD_PREC_FP32, 0, surf2d, st);
+        return surf2d;
     } else {
         dim3 b(32, 8), gr(cdiv(g.nz, 32), cdiv(g.nx, 8), g.nb);
         if (g.fhalf) DISPATCH_F(g.F, k_s2d<FF, __half><<<gr, b, 0, st>>>(g, f))
@@ -1599,8 +1606,7 @@ bool launch_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool fold_
 bool launch_update_s_bnd(const Grid &g, const Fields &f, const BndSlot &b, int prec, int64_t tofs, cudaStream_t st)
 {
     if (!q4_ok(g) || g.kernels != 0 || g.L > 0 || g.nb > 1 || g.fhalf || g.fused || g.vasync) return false;
-    if (g.F == 4) quad_update_s_bnd<4>(g, f, b, prec, tofs, g.freesurf != 0, st);
-    else quad_update_s_bnd<2>(g, f, b, prec, tofs, g.freesurf != 0, st);
+    ROWS_DISPATCH(g, quad_update_s_bnd<R>(g, f, b, prec, tofs, g.freesurf != 0, st))
     return true;
 }
 
@@ -1788,8 +1794,7 @@ static void launch_adj_t(const Grid &g, const Fields &f, const AdjFields &a, boo
 void launch_update_adj(const Grid &g, const Fields &f, const AdjFields &a, bool stress, int prec, cudaStream_t st)
 {
     if (g.nd == 3 && (g.kernels == 0 || g.kernels == 5) && q4_ok(g) && g.L <= 3) {
-        if (g.F == 4) quad_update_adj<4>(g, f, a, stress, prec, st);
-        else quad_update_adj<2>(g, f, a, stress, prec, st);
+        ROWS_DISPATCH(g, quad_update_adj<R>(g, f, a, stress, prec, st))
         return;
     }
     if (launch_quad2d_adj(g, f, a, stress, prec, st)) return;

@@ -22,23 +22,34 @@ bool launch_update_v_tma(const Grid &g, const Fields &f, cudaStream_t st);
 bool launch_update_s_tma(const Grid &g, const Fields &f, cudaStream_t st);
 bool tma_ready(const Grid &g, const Fields &f);  // the TMA kernels will run for this plan
 int tma_take_status();      // 1 if a TMA stage of the last launches never arrived (and clears it)
-// 3D stress-update family of a plan: 0 not 3D, 1 general, 2 register-blocked,
-// 3 TMA-pipelined, 4 streaming, 5 4-cell vectorised
-// 4-cell vectorised 3D kernels (sfd_quad3d.cuh), half width 2 or 4;
+// Free surface in a stress update's launch: not at all, in the form whose
+// products are added in one rounding, or with the roundings of the separate
+// launch (k_surf3d: checkpoint recomputation, boundary saving, FP16 fields,
+// rows that are no whole quads).  The two differ in the last bits of
+// viscoelastic 3D runs only.
+enum Surf { SURF_NONE = 0, SURF_FOLD, SURF_APART };
+// kinds of rows of the 4-cell 3D kernels, each with its own instances: order 4;
+// order 8 in whole quads; order 8 filled up with dummy cells
+constexpr int ROWS_O4 = 2, ROWS_WHOLE = 4, ROWS_FILLED = 5;
+__host__ __device__ constexpr int half_width(int rows) { return rows & ~1; }
+__host__ __device__ constexpr bool whole_rows(int rows) { return rows == ROWS_WHOLE; }
+// 4-cell vectorised 3D kernels (sfd_quad3d.cuh);
 // quad_update_s returns whether the launch applied the free surface
-template <int F> void quad_update_v(const Grid &g, const Fields &f, cudaStream_t st);
+template <int R> void quad_update_v(const Grid &g, const Fields &f, cudaStream_t st);
 // the elastic single-shot update that also saves the boundary shells
-template <int F>
+template <int R>
 void quad_update_s_bnd(const Grid &g, const Fields &f, const BndSlot &b, int prec, int64_t tofs, bool surf, cudaStream_t st);
 // the same where it applies (false: not launched)
 bool launch_update_s_bnd(const Grid &g, const Fields &f, const BndSlot &b, int prec, int64_t tofs, cudaStream_t st);
-template <int F> bool quad_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool surf);
-template <int F>
+template <int R> bool quad_update_s(const Grid &g, const Fields &f, cudaStream_t st, Surf surf);
+template <int R>
 void quad_update_adj(const Grid &g, const Fields &f, const AdjFields &a, bool stress, int prec, cudaStream_t st);
+// 3D stress-update family of a plan: 0 not 3D, 1 general, 2 register-blocked,
+// 3 TMA-pipelined, 4 streaming, 5 4-cell vectorised
 int stress_family(const Grid &g, const Fields &f);
-// fold_surface: single-shot FP32 4-cell kernels may apply the free surface in
-// the same launch (true returned: the caller skips launch_surface)
-bool launch_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool fold_surface = false);
+// fold: single-shot 4-cell kernels may apply the free surface in the same
+// launch (true returned: the caller skips launch_surface)
+bool launch_update_s(const Grid &g, const Fields &f, cudaStream_t st, Surf fold = SURF_NONE);
 // Fused 3D forward step (velocity, stress, free surface in one launch; see
 // sfd_kernels.cu).  Work units = ntz x nty x nchunk; units = 0 when the plan's
 // grid does not take it (sfd_config.kernels 6; 3D, 8th order, nz % 4 == 0,

@@ -41,24 +41,24 @@ __device__ __forceinline__ void cpml2d_z(const Grid &g, const Fields &f, int gz0
     const i64 row = (i64)(gx - F) * (2 * NAB);
     if (zq && !g.zpad && gz0 > NZ - NAB - F - 1) {
         const int k = gz0 - NZ + 2 * NAB + F;
-        cpml_zq(pf, row + k, f.kinv[2][0], f.cz[CA], f.cz[CB], 2 * NAB - k, -1, df);
-        cpml_zq(ph, row + k, f.kinv[2][1], f.cz[CAH], f.cz[CBH], 2 * NAB - 1 - k, -1, dh);
+        cpml_zq<true>(pf, row + k, ktab(f, 2, 0), f.cz[CA], f.cz[CB], 2 * NAB - k, -1, df);
+        cpml_zq<true>(ph, row + k, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], 2 * NAB - 1 - k, -1, dh);
     } else if (zq && !g.freesurf && gz0 - F < NAB) {
         const int k = gz0 - F;
-        cpml_zq(pf, row + k, f.kinv[2][0], f.cz[CA], f.cz[CB], k, 1, df);
-        cpml_zq(ph, row + k, f.kinv[2][1], f.cz[CAH], f.cz[CBH], k, 1, dh);
+        cpml_zq<true>(pf, row + k, ktab(f, 2, 0), f.cz[CA], f.cz[CB], k, 1, df);
+        cpml_zq<true>(ph, row + k, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], k, 1, dh);
     } else if (gz0 + 3 > NZ - NAB - F - 1 || (!zq && !g.freesurf && gz0 - F < NAB)) {
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const int gz = gz0 + j;
             if (gz > NZ - NAB - F - 1 && gz < NZ - F) {
                 const int k = gz - NZ + 2 * NAB + F;
-                cpml(pf, row + k, f.kinv[2][0], f.cz[CA], f.cz[CB], 2 * NAB - k, df.v[j]);
-                cpml(ph, row + k, f.kinv[2][1], f.cz[CAH], f.cz[CBH], 2 * NAB - 1 - k, dh.v[j]);
+                cpml(pf, row + k, ktab(f, 2, 0), f.cz[CA], f.cz[CB], 2 * NAB - k, df.v[j]);
+                cpml(ph, row + k, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], 2 * NAB - 1 - k, dh.v[j]);
             } else if (!g.freesurf && gz - F < NAB && gz < NZ - F) {
                 const int k = gz - F;
-                cpml(pf, row + k, f.kinv[2][0], f.cz[CA], f.cz[CB], k, df.v[j]);
-                cpml(ph, row + k, f.kinv[2][1], f.cz[CAH], f.cz[CBH], k, dh.v[j]);
+                cpml(pf, row + k, ktab(f, 2, 0), f.cz[CA], f.cz[CB], k, df.v[j]);
+                cpml(ph, row + k, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], k, dh.v[j]);
             }
         }
     }
@@ -71,14 +71,14 @@ __device__ __forceinline__ void cpml2d_x(const Grid &g, const Fields &f, int gz0
     if (gx - F < NAB) {
         const int i = gx - F;
         const i64 q = (i64)i * g.nz + (gz0 - F);
-        cpml_q(pf, q, f.kinv[0][0], f.cx[CA], f.cx[CB], i, df);
-        cpml_q(ph, q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], i, dh);
+        cpml_q<true>(pf, q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], i, df);
+        cpml_q<true>(ph, q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], i, dh);
     }
     if (gx > g.NX - NAB - F - 1) {
         const int i = gx - g.NX + 2 * NAB + F;
         const i64 q = (i64)i * g.nz + (gz0 - F);
-        cpml_q(pf, q, f.kinv[0][0], f.cx[CA], f.cx[CB], 2 * NAB - i, df);
-        cpml_q(ph, q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], 2 * NAB - 1 - i, dh);
+        cpml_q<true>(pf, q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], 2 * NAB - i, df);
+        cpml_q<true>(ph, q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], 2 * NAB - 1 - i, dh);
     }
 }
 
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(128) k_s2d_q4(Grid g, Fields f, BndSlot b, i64
         if (F == 4 && gz0 == F + 4) f.w[SZZ][iv - 8] = -s[1].v[0];
         if (gz0 == F) {
             const Surf2d su = surf2d_of(m0);
-            const float vxx = d.xx.v[0], vzz = d.zz.v[0], h = surf2d_h(su, vxx, vzz);
+            const float vxx = d.xx.v[0], vzz = d.zz.v[0], h = surf2d_h<L == 0>(su, vxx, vzz);
             s[1].v[0] = 0.0f;
             if constexpr (L == 0) {
                 s[0].v[0] = __fadd_rn(h, s[0].v[0]);
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(128) k_s2d_q4(Grid g, Fields f, BndSlot b, i64
                 sump = 0;
 #pragma unroll
                 for (int l = 0; l < L; l++) {
-                    r[0][l].v[0] = __fadd_rn(surf2d_hr(su, surf2d_b(g.eta[l]), vxx, vzz), r[0][l].v[0]);
+                    r[0][l].v[0] = __fadd_rn(__fmul_rn(surf2d_b(g.eta[l]), surf2d_hr(su, vxx, vzz)), r[0][l].v[0]);
                     sump += r[0][l].v[0];
                 }
                 s[0].v[0] = __fadd_rn(__fmul_rn(g.dt2, sump), s[0].v[0]);
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(128) k_adjv2d_q4(Grid g, Fields f, AdjFields a
         const float lvz = __fmul_rn(__fadd_rn(d.zz.v[j], d.x.v[j]), rkp.v[j]);
         wx.v[j] = __fadd_rn(wx.v[j], lvx);
         wz.v[j] = __fadd_rn(wz.v[j], lvz);
-        gr[j] = __fmaf_rn(-vz.v[j], lvz, -__fmul_rn(vx.v[j], lvx));
+        gr[j] = __fmaf_rn(-vx.v[j], lvx, -__fmul_rn(vz.v[j], lvz));
     }
     if (g.abs_type == 2) {
         Q4 *const q[2] = {&wx, &wz};

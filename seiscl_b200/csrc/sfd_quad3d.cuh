@@ -1,5 +1,5 @@
 // sfd_quad3d.cuh -- 4-cell vectorised 3D kernels (forward and adjoint) and
-// their launchers, templates on the stencil half width F (2 or 4).  The
+// their launchers, templates on the kind of rows R (sfd_kernels.h).  The
 // instantiations live in sfd_quad3d_*.cu, one translation unit per half
 // width and direction.
 #pragma once
@@ -206,28 +206,46 @@ __device__ __forceinline__ Q4 dbw_z(const W12 &w, const float *hc)
 
 // CPML recursion on four consecutive z cells sharing one profile index
 // (y and x slabs: the psi arrays are z-fastest and 16-byte aligned there).
-// cpml()'s recursion, with the division by K replaced by a multiplication by
-// 1/K (Fields::kinv, rounded to FP32 on the host): within one rounding of
-// the quotient per cell, and cheaper -- the FP32 divisions had cost the
-// velocity update at 256^3 with 20-cell slabs 0.031 ms of its 0.306.
-__device__ __forceinline__ void cpml_q(float *psi, i64 q, const float *Ki, const float *a, const float *b, int ci,
+// DIV: cpml()'s recursion with its division by K, so that grids that reach
+// these kernels by dummy rows or a shifted base, and 2D ones, have the bits of
+// the one-cell kernels.  Otherwise (whole rows at order 8) d is multiplied by
+// 1/K (Fields::kinv, rounded to FP32 on the host): within one rounding of the
+// quotient per cell, and cheaper -- the FP32 divisions had cost the velocity
+// update at 256^3 with 20-cell slabs 0.031 ms of its 0.306.  A run keeps one
+// of the two: where shells are saved under a free surface, the adjoint's
+// surface amplifies a difference of one rounding a thousandfold and more.
+template <bool DIV> struct KVal;   // 1/K of one node
+template <> struct KVal<true> {
+    double k;
+    __device__ __forceinline__ KVal(const KTab &t, int ci) : k(__ldg(t.kq + ci)) {}
+    __device__ __forceinline__ float operator()(float d, float psi) const { return cpml_quot(d, k, psi); }
+};
+template <> struct KVal<false> {
+    float k;
+    __device__ __forceinline__ KVal(const KTab &t, int ci) : k(__ldg(t.kinv + ci)) {}
+    __device__ __forceinline__ float operator()(float d, float psi) const { return __fmaf_rn(d, k, psi); }
+};
+template <bool DIV>
+__device__ __forceinline__ void cpml_q(float *psi, i64 q, KTab t, const float *a, const float *b, int ci,
                                        Q4 &d)
 {
-    const float ki = __ldg(Ki + ci), aa = __ldg(a + ci), bb = __ldg(b + ci);
+    const KVal<DIV> k(t, ci);
+    const float aa = __ldg(a + ci), bb = __ldg(b + ci);
     Q4 p = ldq_rw(psi + q);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         const float ps = cpml_psi(p.v[j], aa, bb, d.v[j]);
         p.v[j] = ps;
-        d.v[j] = __fmaf_rn(d.v[j], ki, ps);
+        d.v[j] = k(d.v[j], ps);
     }
     stq(psi + q, p);
 }
 
 // z-slab CPML on a quad that lies entirely inside the slab: the psi cells
 // are consecutive (z-type psi is [nx][ny][2 nab], k fastest), the profile
-// index differs per cell (ci0 + step * j); multiplies by 1/K as cpml_q
-__device__ __forceinline__ void cpml_zq(float *psi, i64 q, const float *Ki, const float *a, const float *b, int ci0,
+// index differs per cell (ci0 + step * j)
+template <bool DIV>
+__device__ __forceinline__ void cpml_zq(float *psi, i64 q, KTab t, const float *a, const float *b, int ci0,
                                         int step, Q4 &d)
 {
     Q4 p = ldq_rw(psi + q);
@@ -236,7 +254,7 @@ __device__ __forceinline__ void cpml_zq(float *psi, i64 q, const float *Ki, cons
         const int ci = ci0 + step * j;
         const float ps = cpml_psi(p.v[j], __ldg(a + ci), __ldg(b + ci), d.v[j]);
         p.v[j] = ps;
-        d.v[j] = __fmaf_rn(d.v[j], __ldg(Ki + ci), ps);
+        d.v[j] = KVal<DIV>(t, ci)(d.v[j], ps);
     }
     stq(psi + q, p);
 }
@@ -250,11 +268,15 @@ __device__ __forceinline__ bool cpml_slabs_apart(const Grid &g)
 {
     return g.nab % 4 == 0 && g.nz - g.zpad >= 2 * g.nab + 4 && g.ny >= 2 * g.nab && g.nx >= 2 * g.nab;
 }
-// z slabs made of whole quads (the bottom one only without dummy rows), apart
+// z slabs made of whole quads (the bottom one only without dummy rows), apart.
+// zpad stays a run-time value in the corrections below, whatever the rows: the
+// instances of whole rows compiled without it were slower, 256^3, L = 2, 946
+// against 931 us a step, 72 x 64 x 80 28.5 against 26.9.
 __device__ __forceinline__ bool z_quads(const Grid &g) { return g.nab % 4 == 0 && g.nz - g.zpad >= 2 * g.nab + 4; }
 
 // The CPML corrections of cpml_v3d for a quad of z cells: z slabs per cell
 // (a quad may straddle a z-slab edge), y and x slabs per quad.
+template <bool DIV>
 __device__ __forceinline__ void cpml_v3d_q4(const Grid &g, const Fields &f, int gz0, int gy, int gx, Q4 &sxx_x,
                                             Q4 &syy_y, Q4 &szz_z, Q4 &sxy_y, Q4 &sxy_x, Q4 &syz_y, Q4 &syz_z,
                                             Q4 &sxz_x, Q4 &sxz_z)
@@ -264,32 +286,33 @@ __device__ __forceinline__ void cpml_v3d_q4(const Grid &g, const Fields &f, int 
     // side-merged forms where the slabs are apart: far-side profile indices are
     // 2 nab - k (integer grid) and 2 nab - 1 - k (half grid) of the slab-local
     // index k.  zq: a quad lies wholly inside or outside a z slab
-    const bool apart = cpml_slabs_apart(g), zq = z_quads(g);
+    const bool apart = cpml_slabs_apart(g), zq = DIV ? z_quads(g) : NAB % 4 == 0;
+    const int zpad = g.zpad;
     const i64 k0 = gz0 - F;
-    if (apart && !g.zpad) {
+    if (apart && !zpad) {
         const bool zhi = gz0 > NZ - NAB - F - 1, zlo = !g.freesurf && gz0 - F < NAB;
         if (zhi || zlo) {
             const int k = zhi ? gz0 - NZ + 2 * NAB + F : gz0 - F;
             const int st = zhi ? -1 : 1, cf = zhi ? 2 * NAB - k : k, ch = zhi ? 2 * NAB - 1 - k : k;
             const i64 q = ((i64)(gx - F) * ny + (gy - F)) * (2 * NAB) + k;
-            cpml_zq(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], cf, st, sxz_z);
-            cpml_zq(f.psi[PSYZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], cf, st, syz_z);
-            cpml_zq(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ch, st, szz_z);
+            cpml_zq<DIV>(f.psi[PSXZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], cf, st, sxz_z);
+            cpml_zq<DIV>(f.psi[PSYZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], cf, st, syz_z);
+            cpml_zq<DIV>(f.psi[PSZZ_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ch, st, szz_z);
         }
     } else {
-        if (zq && !g.zpad && gz0 > NZ - NAB - F - 1) {
+        if (zq && !zpad && gz0 > NZ - NAB - F - 1) {
             i64 i = gx - F, jj = gy - F, k = gz0 - NZ + NAB + F + NAB;
             int ind = 2 * NAB - 1 - (int)k;
             i64 q = (i * ny + jj) * (2 * NAB) + k;
-            cpml_zq(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, -1, sxz_z);
-            cpml_zq(f.psi[PSYZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, -1, syz_z);
-            cpml_zq(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, -1, szz_z);
+            cpml_zq<DIV>(f.psi[PSXZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, -1, sxz_z);
+            cpml_zq<DIV>(f.psi[PSYZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, -1, syz_z);
+            cpml_zq<DIV>(f.psi[PSZZ_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, -1, szz_z);
         } else if (zq && !g.freesurf && gz0 - F < NAB) {
             i64 i = gx - F, jj = gy - F, k = gz0 - F;
             i64 q = (i * ny + jj) * (2 * NAB) + k;
-            cpml_zq(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, 1, sxz_z);
-            cpml_zq(f.psi[PSYZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, 1, syz_z);
-            cpml_zq(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, 1, szz_z);
+            cpml_zq<DIV>(f.psi[PSXZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], (int)k, 1, sxz_z);
+            cpml_zq<DIV>(f.psi[PSYZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], (int)k, 1, syz_z);
+            cpml_zq<DIV>(f.psi[PSZZ_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], (int)k, 1, szz_z);
         } else if (gz0 + 3 > NZ - NAB - F - 1 || (!zq && !g.freesurf && gz0 - F < NAB)) {
 #pragma unroll
             for (int j = 0; j < 4; j++) {
@@ -298,15 +321,15 @@ __device__ __forceinline__ void cpml_v3d_q4(const Grid &g, const Fields &f, int 
                     i64 i = gx - F, jj = gy - F, k = gz - NZ + NAB + F + NAB;
                     int ind = 2 * NAB - 1 - (int)k;
                     i64 q = (i * ny + jj) * (2 * NAB) + k;
-                    cpml(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, sxz_z.v[j]);
-                    cpml(f.psi[PSYZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, syz_z.v[j]);
-                    cpml(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, szz_z.v[j]);
+                    cpml(f.psi[PSXZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, sxz_z.v[j]);
+                    cpml(f.psi[PSYZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, syz_z.v[j]);
+                    cpml(f.psi[PSZZ_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, szz_z.v[j]);
                 } else if (!g.freesurf && gz - F < NAB) {
                     i64 i = gx - F, jj = gy - F, k = gz - F;
                     i64 q = (i * ny + jj) * (2 * NAB) + k;
-                    cpml(f.psi[PSXZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, sxz_z.v[j]);
-                    cpml(f.psi[PSYZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, syz_z.v[j]);
-                    cpml(f.psi[PSZZ_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, szz_z.v[j]);
+                    cpml(f.psi[PSXZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], (int)k, sxz_z.v[j]);
+                    cpml(f.psi[PSYZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], (int)k, syz_z.v[j]);
+                    cpml(f.psi[PSZZ_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], (int)k, szz_z.v[j]);
                 }
             }
         }
@@ -317,49 +340,49 @@ __device__ __forceinline__ void cpml_v3d_q4(const Grid &g, const Fields &f, int 
             const int j = ylo ? gy - F : gy - NY + 2 * NAB + F;
             const int cf = ylo ? j : 2 * NAB - j, ch = ylo ? j : 2 * NAB - 1 - j;
             const i64 q = ((i64)(gx - F) * (2 * NAB) + j) * nz + k0;
-            cpml_q(f.psi[PSXY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], cf, sxy_y);
-            cpml_q(f.psi[PSYY_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ch, syy_y);
-            cpml_q(f.psi[PSYZ_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], cf, syz_y);
+            cpml_q<DIV>(f.psi[PSXY_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], cf, sxy_y);
+            cpml_q<DIV>(f.psi[PSYY_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], ch, syy_y);
+            cpml_q<DIV>(f.psi[PSYZ_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], cf, syz_y);
         }
         const bool xlo = gx - F < NAB, xhi = gx > NX - NAB - F - 1;
         if (xlo || xhi) {
             const int i = xlo ? gx - F : gx - NX + 2 * NAB + F;
             const int cf = xlo ? i : 2 * NAB - i, ch = xlo ? i : 2 * NAB - 1 - i;
             const i64 q = ((i64)i * ny + (gy - F)) * nz + k0;
-            cpml_q(f.psi[PSXX_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ch, sxx_x);
-            cpml_q(f.psi[PSXY_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], cf, sxy_x);
-            cpml_q(f.psi[PSXZ_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], cf, sxz_x);
+            cpml_q<DIV>(f.psi[PSXX_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ch, sxx_x);
+            cpml_q<DIV>(f.psi[PSXY_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], cf, sxy_x);
+            cpml_q<DIV>(f.psi[PSXZ_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], cf, sxz_x);
         }
         return;
     }
     if (gy - F < NAB) {
         i64 i = gx - F, j = gy - F;
         i64 q = (i * (2 * NAB) + j) * nz + k0;
-        cpml_q(f.psi[PSXY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], (int)j, sxy_y);
-        cpml_q(f.psi[PSYY_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], (int)j, syy_y);
-        cpml_q(f.psi[PSYZ_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], (int)j, syz_y);
+        cpml_q<DIV>(f.psi[PSXY_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], (int)j, sxy_y);
+        cpml_q<DIV>(f.psi[PSYY_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], (int)j, syy_y);
+        cpml_q<DIV>(f.psi[PSYZ_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], (int)j, syz_y);
     } else if (gy > NY - NAB - F - 1) {
         i64 i = gx - F, j = gy - NY + NAB + F + NAB;
         int ind = 2 * NAB - 1 - (int)j;
         i64 q = (i * (2 * NAB) + j) * nz + k0;
-        cpml_q(f.psi[PSXY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], ind + 1, sxy_y);
-        cpml_q(f.psi[PSYY_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ind, syy_y);
-        cpml_q(f.psi[PSYZ_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], ind + 1, syz_y);
+        cpml_q<DIV>(f.psi[PSXY_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], ind + 1, sxy_y);
+        cpml_q<DIV>(f.psi[PSYY_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], ind, syy_y);
+        cpml_q<DIV>(f.psi[PSYZ_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], ind + 1, syz_y);
     }
     if (gx - F < NAB) {
         i64 i = gx - F, j = gy - F;
         i64 q = (i * ny + j) * nz + k0;
-        cpml_q(f.psi[PSXX_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], (int)i, sxx_x);
-        cpml_q(f.psi[PSXY_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], (int)i, sxy_x);
-        cpml_q(f.psi[PSXZ_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], (int)i, sxz_x);
+        cpml_q<DIV>(f.psi[PSXX_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], (int)i, sxx_x);
+        cpml_q<DIV>(f.psi[PSXY_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], (int)i, sxy_x);
+        cpml_q<DIV>(f.psi[PSXZ_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], (int)i, sxz_x);
     }
     if (gx > NX - NAB - F - 1) {
         i64 i = gx - NX + NAB + F + NAB, j = gy - F;
         int ind = 2 * NAB - 1 - (int)i;
         i64 q = (i * ny + j) * nz + k0;
-        cpml_q(f.psi[PSXX_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, sxx_x);
-        cpml_q(f.psi[PSXY_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, sxy_x);
-        cpml_q(f.psi[PSXZ_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, sxz_x);
+        cpml_q<DIV>(f.psi[PSXX_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ind, sxx_x);
+        cpml_q<DIV>(f.psi[PSXY_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], ind + 1, sxy_x);
+        cpml_q<DIV>(f.psi[PSXZ_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], ind + 1, sxz_x);
     }
 }
 
@@ -382,9 +405,10 @@ __device__ __forceinline__ void cpml_v3d_q4(const Grid &g, const Fields &f, int 
 
 // velocity update of the quad (gz0..gz0+3, gy, gx); LP: load policy of the
 // stress reads
-template <int F, class T, int LP = 0>
+template <int R, class T, int LP = 0>
 __device__ __forceinline__ void v3d_q4_at(const Grid &g, const Fields &f, int gz0, int gy, int gx, i64 iv, i64 ip)
 {
+    constexpr int F = half_width(R);
     const i64 sx = (i64)g.NY * g.NZ, sy = g.NZ;
     const float *hc = g.hc;
     T *wvx = fld<T>(f.w[VX]), *wvy = fld<T>(f.w[VY]), *wvz = fld<T>(f.w[VZ]);
@@ -402,7 +426,8 @@ __device__ __forceinline__ void v3d_q4_at(const Grid &g, const Fields &f, int gz
     Q4 syy_y = dfw_q<F, T, LP>(Syy, iv, sy, hc);
     Q4 sxy_x = dbw_q<F, T, LP>(Sxy, iv, sx, hc);
     Q4 sxy_y = dbw_q<F, T, LP>(Sxy, iv, sy, hc);
-    if (g.abs_type == 1) cpml_v3d_q4(g, f, gz0, gy, gx, sxx_x, syy_y, szz_z, sxy_y, sxy_x, syz_y, syz_z, sxz_x, sxz_z);
+    if (g.abs_type == 1)
+        cpml_v3d_q4<!whole_rows(R)>(g, f, gz0, gy, gx, sxx_x, syy_y, szz_z, sxy_y, sxy_x, syz_y, syz_z, sxz_x, sxz_z);
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         float v3[3] = {__fmaf_rn(__fadd_rn(__fadd_rn(sxx_x.v[j], sxy_y.v[j]), sxz_z.v[j]), rip.v[j], vx.v[j]),
@@ -416,17 +441,19 @@ __device__ __forceinline__ void v3d_q4_at(const Grid &g, const Fields &f, int gz
     stq(wvz + iv, vz);
 }
 
-template <int F, class T, bool MB>
+template <int R, class T, bool MB>
 __device__ __forceinline__ void v3d_q4(const Grid &g, Fields f)
 {
+    constexpr int F = half_width(R);
     CELL3D_Q4
-    v3d_q4_at<F, T, 0>(g, f, gz0, gy, gx, iv, ip);
+    v3d_q4_at<R, T, 0>(g, f, gz0, gy, gx, iv, ip);
 }
 
-template <int F, class T, bool MB = false>
+template <int R, class T, bool MB = false>
 __global__ void __launch_bounds__(128) k_v3d_q4(Grid g, Fields f)
 {
-    v3d_q4<F, T, MB>(g, f);
+    constexpr int F = half_width(R);
+    v3d_q4<R, T, MB>(g, f);
 }
 
 // The single-shot FP32 launch asks for NB resident CTAs per SM: 4, or 6 where
@@ -439,15 +466,17 @@ __global__ void __launch_bounds__(128) k_v3d_q4(Grid g, Fields f)
 // Taking the x planes in the reverse of the stress kernel's order (each
 // kernel starting on the planes the other has just written) was measured
 // and is not faster: 16.96 against 17.00 Gcell/s at 256^3, L=2.
-template <int F, int NB = 4>
+template <int R, int NB = 4>
 __global__ void __launch_bounds__(128, NB) k_v3d_q4_b(Grid g, Fields f)
 {
+    constexpr int F = half_width(R);
     constexpr bool MB = false;
     CELL3D_Q4
-    v3d_q4_at<F, float, 0>(g, f, gz0, gy, gx, iv, ip);
+    v3d_q4_at<R, float, 0>(g, f, gz0, gy, gx, iv, ip);
 }
 
 // CPML corrections of cpml_s3d (forward form) for a quad of z cells
+template <bool DIV>
 __device__ __forceinline__ void cpml_s3d_q4(const Grid &g, const Fields &f, int gz0, int gy, int gx, Q4 &vxx,
                                             Q4 &vxy, Q4 &vxz, Q4 &vyx, Q4 &vyy, Q4 &vyz, Q4 &vzx, Q4 &vzy, Q4 &vzz)
 {
@@ -457,31 +486,32 @@ __device__ __forceinline__ void cpml_s3d_q4(const Grid &g, const Fields &f, int 
     // 2 nab - k (integer grid) and 2 nab - 1 - k (half grid) of the slab-local
     // index k.  zq: a quad lies wholly inside or outside a z slab
     const bool apart = cpml_slabs_apart(g), zq = z_quads(g);
+    const int zpad = g.zpad;
     const i64 k0 = gz0 - F;
-    if (apart && !g.zpad) {
+    if (apart && !zpad) {
         const bool zhi = gz0 > NZ - NAB - F - 1, zlo = !g.freesurf && gz0 - F < NAB;
         if (zhi || zlo) {
             const int k = zhi ? gz0 - NZ + 2 * NAB + F : gz0 - F;
             const int st = zhi ? -1 : 1, cf = zhi ? 2 * NAB - k : k, ch = zhi ? 2 * NAB - 1 - k : k;
             const i64 q = ((i64)(gx - F) * ny + (gy - F)) * (2 * NAB) + k;
-            cpml_zq(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ch, st, vxz);
-            cpml_zq(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ch, st, vyz);
-            cpml_zq(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], cf, st, vzz);
+            cpml_zq<DIV>(f.psi[PVX_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ch, st, vxz);
+            cpml_zq<DIV>(f.psi[PVY_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ch, st, vyz);
+            cpml_zq<DIV>(f.psi[PVZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], cf, st, vzz);
         }
     } else {
-        if (zq && !g.zpad && gz0 > NZ - NAB - F - 1) {
+        if (zq && !zpad && gz0 > NZ - NAB - F - 1) {
             i64 i = gx - F, jj = gy - F, k = gz0 - NZ + NAB + F + NAB;
             int ind = 2 * NAB - 1 - (int)k;
             i64 q = (i * ny + jj) * (2 * NAB) + k;
-            cpml_zq(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, -1, vxz);
-            cpml_zq(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, -1, vyz);
-            cpml_zq(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, -1, vzz);
+            cpml_zq<DIV>(f.psi[PVX_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, -1, vxz);
+            cpml_zq<DIV>(f.psi[PVY_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, -1, vyz);
+            cpml_zq<DIV>(f.psi[PVZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, -1, vzz);
         } else if (zq && !g.freesurf && gz0 - F < NAB) {
             i64 i = gx - F, jj = gy - F, k = gz0 - F;
             i64 q = (i * ny + jj) * (2 * NAB) + k;
-            cpml_zq(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, 1, vxz);
-            cpml_zq(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, 1, vyz);
-            cpml_zq(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, 1, vzz);
+            cpml_zq<DIV>(f.psi[PVX_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], (int)k, 1, vxz);
+            cpml_zq<DIV>(f.psi[PVY_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], (int)k, 1, vyz);
+            cpml_zq<DIV>(f.psi[PVZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], (int)k, 1, vzz);
         } else if (gz0 + 3 > NZ - NAB - F - 1 || (!zq && !g.freesurf && gz0 - F < NAB)) {
 #pragma unroll
             for (int j = 0; j < 4; j++) {
@@ -490,16 +520,16 @@ __device__ __forceinline__ void cpml_s3d_q4(const Grid &g, const Fields &f, int 
                     i64 i = gx - F, jj = gy - F, k = gz - NZ + NAB + F + NAB;
                     int ind = 2 * NAB - 1 - (int)k;
                     i64 q = (i * ny + jj) * (2 * NAB) + k;
-                    cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vxz.v[j]);
-                    cpml(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vyz.v[j]);
-                    cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, vzz.v[j]);
+                    cpml(f.psi[PVX_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, vxz.v[j]);
+                    cpml(f.psi[PVY_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, vyz.v[j]);
+                    cpml(f.psi[PVZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, vzz.v[j]);
                 }
                 if (!g.freesurf && gz - F < NAB) {
                     i64 i = gx - F, jj = gy - F, k = gz - F;
                     i64 q = (i * ny + jj) * (2 * NAB) + k;
-                    cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, vxz.v[j]);
-                    cpml(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, vyz.v[j]);
-                    cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, vzz.v[j]);
+                    cpml(f.psi[PVX_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], (int)k, vxz.v[j]);
+                    cpml(f.psi[PVY_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], (int)k, vyz.v[j]);
+                    cpml(f.psi[PVZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], (int)k, vzz.v[j]);
                 }
             }
         }
@@ -510,50 +540,50 @@ __device__ __forceinline__ void cpml_s3d_q4(const Grid &g, const Fields &f, int 
             const int j = ylo ? gy - F : gy - NY + 2 * NAB + F;
             const int cf = ylo ? j : 2 * NAB - j, ch = ylo ? j : 2 * NAB - 1 - j;
             const i64 q = ((i64)(gx - F) * (2 * NAB) + j) * nz + k0;
-            cpml_q(f.psi[PVX_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ch, vxy);
-            cpml_q(f.psi[PVY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], cf, vyy);
-            cpml_q(f.psi[PVZ_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ch, vzy);
+            cpml_q<DIV>(f.psi[PVX_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], ch, vxy);
+            cpml_q<DIV>(f.psi[PVY_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], cf, vyy);
+            cpml_q<DIV>(f.psi[PVZ_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], ch, vzy);
         }
         const bool xlo = gx - F < NAB, xhi = gx > NX - NAB - F - 1;
         if (xlo || xhi) {
             const int i = xlo ? gx - F : gx - NX + 2 * NAB + F;
             const int cf = xlo ? i : 2 * NAB - i, ch = xlo ? i : 2 * NAB - 1 - i;
             const i64 q = ((i64)i * ny + (gy - F)) * nz + k0;
-            cpml_q(f.psi[PVX_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], cf, vxx);
-            cpml_q(f.psi[PVY_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ch, vyx);
-            cpml_q(f.psi[PVZ_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ch, vzx);
+            cpml_q<DIV>(f.psi[PVX_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], cf, vxx);
+            cpml_q<DIV>(f.psi[PVY_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ch, vyx);
+            cpml_q<DIV>(f.psi[PVZ_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ch, vzx);
         }
         return;
     }
     if (gy - F < NAB) {
         i64 i = gx - F, j = gy - F;
         i64 q = (i * (2 * NAB) + j) * nz + k0;
-        cpml_q(f.psi[PVX_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], (int)j, vxy);
-        cpml_q(f.psi[PVY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], (int)j, vyy);
-        cpml_q(f.psi[PVZ_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], (int)j, vzy);
+        cpml_q<DIV>(f.psi[PVX_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], (int)j, vxy);
+        cpml_q<DIV>(f.psi[PVY_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], (int)j, vyy);
+        cpml_q<DIV>(f.psi[PVZ_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], (int)j, vzy);
     }
     if (gy > NY - NAB - F - 1) {
         i64 i = gx - F, j = gy - NY + NAB + F + NAB;
         int ind = 2 * NAB - 1 - (int)j;
         i64 q = (i * (2 * NAB) + j) * nz + k0;
-        cpml_q(f.psi[PVX_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ind, vxy);
-        cpml_q(f.psi[PVY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], ind + 1, vyy);
-        cpml_q(f.psi[PVZ_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ind, vzy);
+        cpml_q<DIV>(f.psi[PVX_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], ind, vxy);
+        cpml_q<DIV>(f.psi[PVY_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], ind + 1, vyy);
+        cpml_q<DIV>(f.psi[PVZ_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], ind, vzy);
     }
     if (gx - F < NAB) {
         i64 i = gx - F, j = gy - F;
         i64 q = (i * ny + j) * nz + k0;
-        cpml_q(f.psi[PVX_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], (int)i, vxx);
-        cpml_q(f.psi[PVY_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], (int)i, vyx);
-        cpml_q(f.psi[PVZ_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], (int)i, vzx);
+        cpml_q<DIV>(f.psi[PVX_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], (int)i, vxx);
+        cpml_q<DIV>(f.psi[PVY_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], (int)i, vyx);
+        cpml_q<DIV>(f.psi[PVZ_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], (int)i, vzx);
     }
     if (gx > NX - NAB - F - 1) {
         i64 i = gx - NX + NAB + F + NAB, j = gy - F;
         int ind = 2 * NAB - 1 - (int)i;
         i64 q = (i * ny + j) * nz + k0;
-        cpml_q(f.psi[PVX_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, vxx);
-        cpml_q(f.psi[PVY_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, vyx);
-        cpml_q(f.psi[PVZ_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, vzx);
+        cpml_q<DIV>(f.psi[PVX_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], ind + 1, vxx);
+        cpml_q<DIV>(f.psi[PVY_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ind, vyx);
+        cpml_q<DIV>(f.psi[PVZ_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ind, vzx);
     }
 }
 
@@ -571,6 +601,40 @@ __device__ __forceinline__ void cpml_s3d_q4(const Grid &g, const Fields &f, int 
 // forms them) and writes the images szz(F-m) = -szz(F+m) for m = 1..3 and
 // sxz(F-m) = -sxz(F+m-1), syz(F-m) = -syz(F+m-1) for m = 1..4; the quad at
 // gz0 = F+4 writes szz(F-4) = -szz(F+4).
+// the strains (vxx, vyy, vzz) the free surface takes at the top cell iv, as
+// k_surf3d forms them: derivatives times 1/K plus the memory of this step
+template <int F, class T>
+__device__ __forceinline__ void surf_strain(const Grid &g, const Fields &f, int gy, int gx, i64 iv, float (&v)[3])
+{
+    const int NAB = g.nab;
+    v[0] = dbwT<F>(fld<T>(f.w[VX]), iv, (i64)g.NY * g.NZ, g.hc);
+    v[1] = dbwT<F>(fld<T>(f.w[VY]), iv, (i64)g.NZ, g.hc);
+    v[2] = dbwT<F>(fld<T>(f.w[VZ]), iv, 1, g.hc);
+    if (g.abs_type != 1) return;
+    const i64 nz = g.nz, ny = g.ny, i = gx - F, j = gy - F;
+    if (j < NAB) {
+        v[1] = __fmaf_rn(v[1], f.kinv[1][0][j], f.psi[PVY_Y][(i * (2 * NAB) + j) * nz]);
+    } else if (j >= ny - NAB) {
+        const i64 k = j - ny + 2 * NAB;
+        v[1] = __fmaf_rn(v[1], f.kinv[1][0][2 * NAB - k], f.psi[PVY_Y][(i * (2 * NAB) + k) * nz]);
+    }
+    if (i < NAB) v[0] = __fmaf_rn(v[0], f.kinv[0][0][i], f.psi[PVX_X][(i * ny + j) * nz]);
+    if (i >= g.nx - NAB) {
+        const i64 k = i - g.nx + 2 * NAB;
+        v[0] = __fmaf_rn(v[0], f.kinv[0][0][2 * NAB - k], f.psi[PVX_X][(k * ny + j) * nz]);
+    }
+}
+// whether a folded surface takes the roundings of the separate launch
+// (k_surf3d): where the call asks for it (SURF_APART), and on grids and
+// storage types that otherwise run that launch
+template <int R, class T>
+__device__ __forceinline__ bool surf_apart(Surf surf)
+{
+    return surf == SURF_APART || !whole_rows(R) || sizeof(T) == 2;
+}
+// a value as storage type T keeps it
+template <class T> __device__ __forceinline__ float stored(float v) { return to_f<T>(from_f<T>(v)); }
+
 // shell indices of a quad's cells (-1: none).  Most quads lie wholly inside
 // or outside the shell: one comparison per axis settles them, against some
 // forty integer operations a cell.
@@ -601,11 +665,12 @@ __device__ __forceinline__ void bnd_save(const Grid &g, const BndQuad &q, int w,
         if (q.m[j] >= 0) ((TB *)q.b->p[w])[q.at + q.m[j]] = from_f<TB>(v.v[j] * g.bsc[w]);
 }
 
-template <int F, int L, class T, class TR = T, class TB = void>
+template <int R, int L, class T, class TR = T, class TB = void>
 __device__ __forceinline__ void s_normal_q4(const Grid &g, const Fields &f, int gz0, int gy, int gx, i64 iv, i64 ip,
-                                            const Q4 &vxx, const Q4 &vyy, const Q4 &vzz, bool surf = false,
+                                            const Q4 &vxx, const Q4 &vyy, const Q4 &vzz, Surf surf = SURF_NONE,
                                             const BndQuad *bq = nullptr)
 {
+    constexpr int F = half_width(R);
     T *const ws[3] = {fld<T>(f.w[SXX]), fld<T>(f.w[SYY]), fld<T>(f.w[SZZ])};
     TR *const wr[3] = {fld<TR>(f.r[RXX]), fld<TR>(f.r[RYY]), fld<TR>(f.r[RZZ])};
     Q4 sq[3];
@@ -670,7 +735,19 @@ __device__ __forceinline__ void s_normal_q4(const Grid &g, const Fields &f, int 
     if (surf && gz0 == F) {
         // the arithmetic of k_surf3d, forward
         const Surf2d su = surf2d_of(m0);
-        const float vh = __fadd_rn(vxx.v[0], vyy.v[0]), vz0 = vzz.v[0], h = surf2d_h(su, vh, vz0);
+        float v1[3] = {vxx.v[0], vyy.v[0], vzz.v[0]};
+        // whole rows: the update's own CPML multiplies by 1/K
+        if constexpr (!whole_rows(R)) surf_strain<F, T>(g, f, gy, gx, iv, v1);
+        const float vh = __fadd_rn(v1[0], v1[1]), vz0 = v1[2], h = L == 0 || !surf_apart<R, T>(surf) ? surf2d_h<true>(su, vh, vz0) : surf2d_h<false>(su, vh, vz0);
+        // FP16 fields: k_surf3d reads what the update has stored
+        if constexpr (sizeof(T) == 2) {
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                sq[q].v[0] = stored<T>(sq[q].v[0]);
+#pragma unroll
+                for (int l = 0; l < L; l++) rq[q][l].v[0] = stored<T>(rq[q][l].v[0]);
+            }
+        }
         sq[2].v[0] = 0.0f;
         if constexpr (L == 0) {
             sq[0].v[0] = __fadd_rn(sq[0].v[0], h);
@@ -681,11 +758,12 @@ __device__ __forceinline__ void s_normal_q4(const Grid &g, const Fields &f, int 
                 float sum = 0;
 #pragma unroll
                 for (int l = 0; l < L; l++) sum += rq[q][l].v[0];
-                float t = __fadd_rn(sq[q].v[0], __fmaf_rn(-g.dt2, sum, h));
+                const float t = stored<T>(__fadd_rn(sq[q].v[0], __fmaf_rn(-g.dt2, sum, h)));
                 sum = 0;
 #pragma unroll
                 for (int l = 0; l < L; l++) {
-                    rq[q][l].v[0] = __fadd_rn(rq[q][l].v[0], surf2d_hr(su, surf2d_b(g.eta[l]), vh, vz0));
+                    const float b = surf2d_b(g.eta[l]), hr = surf2d_hr(su, vh, vz0);
+                    rq[q][l].v[0] = q == 0 && sizeof(T) == 4 && surf_apart<R, T>(surf) ? __fadd_rn(rq[q][l].v[0], __fmul_rn(b, hr)) : __fmaf_rn(b, hr, rq[q][l].v[0]);
                     sum += rq[q][l].v[0];
                 }
                 sq[q].v[0] = __fmaf_rn(g.dt2, sum, t);
@@ -706,11 +784,12 @@ __device__ __forceinline__ void s_normal_q4(const Grid &g, const Fields &f, int 
     for (int q = 0; q < 3; q++) stq(ws[q] + iv, sq[q]);
 }
 
-template <int F, int L, class T, class TR = T, class TB = void>
+template <int R, int L, class T, class TR = T, class TB = void>
 __device__ __forceinline__ void s_shear_q4(const Grid &g, const Fields &f, int gz0, int gy, int gx, i64 iv, i64 ip,
-                                           const Q4 &vxyyx, const Q4 &vyzzy, const Q4 &vxzzx, bool surf = false,
+                                           const Q4 &vxyyx, const Q4 &vyzzy, const Q4 &vxzzx, Surf surf = SURF_NONE,
                                            const BndQuad *bq = nullptr)
 {
+    constexpr int F = half_width(R);
     T *const ws[3] = {fld<T>(f.w[SXY]), fld<T>(f.w[SYZ]), fld<T>(f.w[SXZ])};
     TR *const wr[3] = {fld<TR>(f.r[RXY]), fld<TR>(f.r[RYZ]), fld<TR>(f.r[RXZ])};
     Q4 sq[3];
@@ -783,10 +862,11 @@ __device__ __forceinline__ void s_shear_q4(const Grid &g, const Fields &f, int g
 // stress update of the quad (gz0..gz0+3, gy, gx); LP: load policy of the
 // velocity reads; surf: free surface folded in (see s_normal_q4); PF: first
 // ask L2 for the quad's per-cell streams
-template <int F, int L, class T, int LP = 0, bool PF = false, class TR = T, class TB = void>
+template <int R, int L, class T, int LP = 0, bool PF = false, class TR = T, class TB = void>
 __device__ __forceinline__ void s3d_q4_at(const Grid &g, const Fields &f, int gz0, int gy, int gx, i64 iv, i64 ip,
-                                          bool surf = false, const BndQuad *bq = nullptr)
+                                          Surf surf = SURF_NONE, const BndQuad *bq = nullptr)
 {
+    constexpr int F = half_width(R);
     const i64 sx = (i64)g.NY * g.NZ, sy = g.NZ;
     const float *hc = g.hc;
     if constexpr (PF) {
@@ -809,7 +889,7 @@ __device__ __forceinline__ void s3d_q4_at(const Grid &g, const Fields &f, int gz
     Q4 vzx = dfw_q<F, T, LP>(Vz, iv, sx, hc), vzy = dfw_q<F, T, LP>(Vz, iv, sy, hc);
     Q4 vyx = dfw_q<F, T, LP>(Vy, iv, sx, hc), vyy = dbw_q<F, T, LP>(Vy, iv, sy, hc);
     Q4 vxx = dbw_q<F, T, LP>(Vx, iv, sx, hc), vxy = dfw_q<F, T, LP>(Vx, iv, sy, hc);
-    if (g.abs_type == 1) cpml_s3d_q4(g, f, gz0, gy, gx, vxx, vxy, vxz, vyx, vyy, vyz, vzx, vzy, vzz);
+    if (g.abs_type == 1) cpml_s3d_q4<!whole_rows(R)>(g, f, gz0, gy, gx, vxx, vxy, vxz, vyx, vyy, vyz, vzx, vzy, vzz);
     Q4 vxyyx, vyzzy, vxzzx;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -817,8 +897,8 @@ __device__ __forceinline__ void s3d_q4_at(const Grid &g, const Fields &f, int gz
         vyzzy.v[j] = __fadd_rn(vyz.v[j], vzy.v[j]);
         vxzzx.v[j] = __fadd_rn(vxz.v[j], vzx.v[j]);
     }
-    s_normal_q4<F, L, T, TR, TB>(g, f, gz0, gy, gx, iv, ip, vxx, vyy, vzz, surf, bq);
-    s_shear_q4<F, L, T, TR, TB>(g, f, gz0, gy, gx, iv, ip, vxyyx, vyzzy, vxzzx, surf, bq);
+    s_normal_q4<R, L, T, TR, TB>(g, f, gz0, gy, gx, iv, ip, vxx, vyy, vzz, surf, bq);
+    s_shear_q4<R, L, T, TR, TB>(g, f, gz0, gy, gx, iv, ip, vxyyx, vyzzy, vxzzx, surf, bq);
 }
 
 // surf: the free surface of the step applied in the same launch (single-shot
@@ -826,20 +906,22 @@ __device__ __forceinline__ void s3d_q4_at(const Grid &g, const Fields &f, int gz
 // viscoelastic ones for 4: 100 x 200 x 200 elastic 115 us at 4, 109 at 5, 106
 // at 6; 128 x 160 x 160 84, 79, 79; 72 x 64 x 80 (6 make it one wave) 15.4 and
 // 12.6.
-template <int F, int L, class T, bool MB = false>
-__global__ void __launch_bounds__(128, L == 0 && sizeof(T) == 4 ? 6 : 4) k_s3d_q4(Grid g, Fields f, bool surf)
+template <int R, int L, class T, bool MB = false>
+__global__ void __launch_bounds__(128, L == 0 && sizeof(T) == 4 ? 6 : 4) k_s3d_q4(Grid g, Fields f, Surf surf)
 {
+    constexpr int F = half_width(R);
     CELL3D_Q4
-    s3d_q4_at<F, L, T, 0>(g, f, gz0, gy, gx, iv, ip, surf);
+    s3d_q4_at<R, L, T, 0>(g, f, gz0, gy, gx, iv, ip, surf);
 }
 
 // Elastic single-shot gradient runs: the update also saves the boundary
 // shells (stores b in type TB, step offset tofs) and then applies the free
 // surface, which the separate launches did in 15 + 15 us of a 237 us step at
 // 100 x 200 x 200.
-template <int F, class TB>
-__global__ void __launch_bounds__(128, 5) k_s3d_q4_bnd(Grid g, Fields f, BndSlot b, i64 tofs, bool surf)
+template <int R, class TB>
+__global__ void __launch_bounds__(128, 5) k_s3d_q4_bnd(Grid g, Fields f, BndSlot b, i64 tofs, Surf surf)
 {
+    constexpr int F = half_width(R);
     constexpr bool MB = false;
     CELL3D_Q4
     BndQuad bq;
@@ -850,7 +932,7 @@ __global__ void __launch_bounds__(128, 5) k_s3d_q4_bnd(Grid g, Fields f, BndSlot
 #pragma unroll
         for (int w = VX; w <= VZ; w++) bnd_save<TB>(g, bq, w, ldq(f.w[w] + iv));
     }
-    s3d_q4_at<F, 0, float, 0, false, float, TB>(g, f, gz0, gy, gx, iv, ip, surf, &bq);
+    s3d_q4_at<R, 0, float, 0, false, float, TB>(g, f, gz0, gy, gx, iv, ip, surf, &bq);
 }
 
 // Single-shot launches of the default selection: each thread first asks L2
@@ -869,13 +951,14 @@ __global__ void __launch_bounds__(128, 5) k_s3d_q4_bnd(Grid g, Fields f, BndSlot
 // against 142.9.  256 and 384 threads a CTA: 0.686-0.721 ms.
 // TR: storage type of the memory variables (FP16 under FP32 wave fields
 // with Grid::rhalf)
-template <int F, int L, class T, class TR = T>
-__global__ void __launch_bounds__(128, 3) k_s3d_q4_pf(Grid g, Fields f, bool surf)
+template <int R, int L, class T, class TR = T>
+__global__ void __launch_bounds__(128, 3) k_s3d_q4_pf(Grid g, Fields f, Surf surf)
 {
+    constexpr int F = half_width(R);
     constexpr bool MB = false;
     pdl_trigger();
     CELL3D_Q4
-    s3d_q4_at<F, L, T, 0, true, TR>(g, f, gz0, gy, gx, iv, ip, surf);
+    s3d_q4_at<R, L, T, 0, true, TR>(g, f, gz0, gy, gx, iv, ip, surf);
 }
 
 // ------------------------------------------------------------- launchers
@@ -907,12 +990,12 @@ static dim3 q4_grid(const Grid &g, dim3 b)
 }
 
 
-template <int F>
+template <int R>
 void quad_update_v(const Grid &g, const Fields &f, cudaStream_t st)
 {
     if (g.fhalf) {
         const dim3 b = q4_block(g, 8, 4, 4), gr = q4_grid(g, b);
-        k_v3d_q4<F, __half><<<gr, b, 0, st>>>(g, f);
+        k_v3d_q4<R, __half><<<gr, b, 0, st>>>(g, f);
         return;
     }
     // 16 quads (64 z cells) x 4 y x 2 x per CTA: the y and x stencil
@@ -920,50 +1003,51 @@ void quad_update_v(const Grid &g, const Fields &f, cudaStream_t st)
     // timing at 256^3 on a B200: 0.268 ms, against 0.275 for 8 x 4 x
     // 4, 0.284 for 8 x 2 x 8 and 0.34 for 4 x 8 x 4 quads x y x x
     const dim3 b = q4_block(g, 16, 4, 2), gr = q4_grid(g, b);
-    if (g.nb > 1) k_v3d_q4<F, float, true><<<gr, b, 0, st>>>(g, f);
-    else if (one_wave(g, 6) && !one_wave(g, 4)) k_v3d_q4_b<F, 6><<<gr, b, 0, st>>>(g, f);
-    else k_v3d_q4_b<F><<<gr, b, 0, st>>>(g, f);
+    if (g.nb > 1) k_v3d_q4<R, float, true><<<gr, b, 0, st>>>(g, f);
+    else if (one_wave(g, 6) && !one_wave(g, 4)) k_v3d_q4_b<R, 6><<<gr, b, 0, st>>>(g, f);
+    else k_v3d_q4_b<R><<<gr, b, 0, st>>>(g, f);
 }
 
-template <int F, int L>
-static void quad_update_s_l(const Grid &g, const Fields &f, dim3 g4, dim3 b4, cudaStream_t st, bool surf)
+template <int R, int L>
+static void quad_update_s_l(const Grid &g, const Fields &f, dim3 g4, dim3 b4, cudaStream_t st, Surf surf)
 {
     // the stream prefetch pays where memory variables add per-cell
     // streams: 256^3, L=2: 0.654 ms against 0.706; elastic (L=0):
     // 0.376 against 0.366 without it.  kernels 5 keeps k_s3d_q4.
     const bool pf = g.nb == 1 && g.kernels == 0 && L > 0;
     if (g.fhalf) {
-        if (pf) k_s3d_q4_pf<F, L, __half><<<g4, b4, 0, st>>>(g, f, surf);
-        else k_s3d_q4<F, L, __half><<<g4, b4, 0, st>>>(g, f, surf);
+        if (pf) k_s3d_q4_pf<R, L, __half><<<g4, b4, 0, st>>>(g, f, surf);
+        else k_s3d_q4<R, L, __half><<<g4, b4, 0, st>>>(g, f, surf);
         return;
     }
     if constexpr (L > 0) {
-        if (pf && g.rhalf) { k_s3d_q4_pf<F, L, float, __half><<<g4, b4, 0, st>>>(g, f, surf); return; }
-        if (pf) { k_s3d_q4_pf<F, L, float><<<g4, b4, 0, st>>>(g, f, surf); return; }
+        if (pf && g.rhalf) { k_s3d_q4_pf<R, L, float, __half><<<g4, b4, 0, st>>>(g, f, surf); return; }
+        if (pf) { k_s3d_q4_pf<R, L, float><<<g4, b4, 0, st>>>(g, f, surf); return; }
     }
-    MB_DISPATCH(g, k_s3d_q4<F, L, float, MBV><<<g4, b4, 0, st>>>(g, f, surf))
+    MB_DISPATCH(g, k_s3d_q4<R, L, float, MBV><<<g4, b4, 0, st>>>(g, f, surf))
 }
 
-template <int F>
-bool quad_update_s(const Grid &g, const Fields &f, cudaStream_t st, bool surf)
+template <int R>
+bool quad_update_s(const Grid &g, const Fields &f, cudaStream_t st, Surf surf)
 {
     const dim3 b4 = q4_block(g, 16, 8, 1), g4 = q4_grid(g, b4);  // 0.70 ms vs 0.71 (32 x 2 x 2)
     switch (g.L) {
-    case 0: quad_update_s_l<F, 0>(g, f, g4, b4, st, surf); break;
-    case 1: quad_update_s_l<F, 1>(g, f, g4, b4, st, surf); break;
-    case 2: quad_update_s_l<F, 2>(g, f, g4, b4, st, surf); break;
-    default: quad_update_s_l<F, 3>(g, f, g4, b4, st, surf); break;
+    case 0: quad_update_s_l<R, 0>(g, f, g4, b4, st, surf); break;
+    case 1: quad_update_s_l<R, 1>(g, f, g4, b4, st, surf); break;
+    case 2: quad_update_s_l<R, 2>(g, f, g4, b4, st, surf); break;
+    default: quad_update_s_l<R, 3>(g, f, g4, b4, st, surf); break;
     }
-    return surf;
+    return surf != SURF_NONE;
 }
 
-template <int F>
-void quad_update_s_bnd(const Grid &g, const Fields &f, const BndSlot &b, int prec, int64_t tofs, bool surf, cudaStream_t st)
+template <int R>
+void quad_update_s_bnd(const Grid &g, const Fields &f, const BndSlot &b, int prec, int64_t tofs, bool surface, cudaStream_t st)
 {
+    const Surf surf = surface ? SURF_APART : SURF_NONE;
     const dim3 b4 = q4_block(g, 16, 8, 1), g4 = q4_grid(g, b4);
-    if (prec == SFD_PREC_FP16) k_s3d_q4_bnd<F, __half><<<g4, b4, 0, st>>>(g, f, b, tofs, surf);
-    else if (prec == SFD_PREC_BF16) k_s3d_q4_bnd<F, __nv_bfloat16><<<g4, b4, 0, st>>>(g, f, b, tofs, surf);
-    else k_s3d_q4_bnd<F, float><<<g4, b4, 0, st>>>(g, f, b, tofs, surf);
+    if (prec == SFD_PREC_FP16) k_s3d_q4_bnd<R, __half><<<g4, b4, 0, st>>>(g, f, b, tofs, surf);
+    else if (prec == SFD_PREC_BF16) k_s3d_q4_bnd<R, __nv_bfloat16><<<g4, b4, 0, st>>>(g, f, b, tofs, surf);
+    else k_s3d_q4_bnd<R, float><<<g4, b4, 0, st>>>(g, f, b, tofs, surf);
 }
 
 }  // namespace sfd

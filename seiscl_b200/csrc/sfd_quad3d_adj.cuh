@@ -1,5 +1,5 @@
 // sfd_quad3d_adj.cuh -- 4-cell vectorised 3D adjoint kernels and their
-// launchers, templates on the stencil half width F (2 or 4).
+// launchers, templates on the kind of rows R.
 #pragma once
 
 #include "sfd_quad3d.cuh"
@@ -29,9 +29,10 @@ __device__ __forceinline__ void pf_l2(const void *p) { asm volatile("prefetch.gl
 // the buoyancies and the density gradient sum -- and the launch takes 4 CTAs
 // per SM (an adjoint step of 100 x 200 x 200: 511 us against 519 with 3, 528
 // with 5).
-template <int F, typename T, bool MB = false, bool PF = false>
+template <int R, typename T, bool MB = false, bool PF = false>
 __global__ void __launch_bounds__(128, PF ? 4 : 1) k_adjv3d_q4(Grid g, Fields f, AdjFields a)
 {
+    constexpr int F = half_width(R);
     CELL3D_Q4
     if (MB) shot_adj(g, a, shot);
     if constexpr (PF) {
@@ -86,7 +87,7 @@ __global__ void __launch_bounds__(128, PF ? 4 : 1) k_adjv3d_q4(Grid g, Fields f,
     Q4 sxy_xr = dbw_q<F>(a.wr[SXY], iv, sx, hc);
     Q4 sxy_yr = dbw_q<F>(a.wr[SXY], iv, sy, hc);
     if (g.abs_type == 1)
-        cpml_v3d_q4(g, f, gz0, gy, gx, sxx_xr, syy_yr, szz_zr, sxy_yr, sxy_xr, syz_yr, syz_zr, sxz_xr, sxz_zr);
+        cpml_v3d_q4<!whole_rows(R)>(g, f, gz0, gy, gx, sxx_xr, syy_yr, szz_zr, sxy_yr, sxy_xr, syz_yr, syz_zr, sxz_xr, sxz_zr);
     Q4 wx = ldq_rw(a.wr[VX] + iv), wy = ldq_rw(a.wr[VY] + iv), wz = ldq_rw(a.wr[VZ] + iv);
     float gr[4];
 #pragma unroll
@@ -106,6 +107,7 @@ __global__ void __launch_bounds__(128, PF ? 4 : 1) k_adjv3d_q4(Grid g, Fields f,
 // CPML of the adjoint stress update (cpml_s3d with adjoint_form): as
 // cpml_s3d_q4, except that a cell in both z slabs or both y slabs takes
 // only the first (else-if), as update_adjs3D.cl does
+template <bool DIV>
 __device__ __forceinline__ void cpml_s3d_adj_q4(const Grid &g, const Fields &f, int gz0, int gy, int gx, Q4 &vxx,
                                                 Q4 &vxy, Q4 &vxz, Q4 &vyx, Q4 &vyy, Q4 &vyz, Q4 &vzx, Q4 &vzy,
                                                 Q4 &vzz)
@@ -113,23 +115,24 @@ __device__ __forceinline__ void cpml_s3d_adj_q4(const Grid &g, const Fields &f, 
     const int F = g.F, NAB = g.nab, NZ = g.NZl, NY = g.NY, NX = g.NX;
     const i64 nz = g.nz, ny = g.ny;
     if (cpml_slabs_apart(g)) {   // then no cell is in two slabs of an axis
-        cpml_s3d_q4(g, f, gz0, gy, gx, vxx, vxy, vxz, vyx, vyy, vyz, vzx, vzy, vzz);
+        cpml_s3d_q4<DIV>(g, f, gz0, gy, gx, vxx, vxy, vxz, vyx, vyy, vyz, vzx, vzy, vzz);
         return;
     }
     const bool zq = z_quads(g);
-    if (zq && !g.zpad && gz0 > NZ - NAB - F - 1) {
+    const int zpad = g.zpad;
+    if (zq && !zpad && gz0 > NZ - NAB - F - 1) {
         i64 i = gx - F, jj = gy - F, k = gz0 - NZ + NAB + F + NAB;
         int ind = 2 * NAB - 1 - (int)k;
         i64 q = (i * ny + jj) * (2 * NAB) + k;
-        cpml_zq(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, -1, vxz);
-        cpml_zq(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, -1, vyz);
-        cpml_zq(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, -1, vzz);
+        cpml_zq<DIV>(f.psi[PVX_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, -1, vxz);
+        cpml_zq<DIV>(f.psi[PVY_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, -1, vyz);
+        cpml_zq<DIV>(f.psi[PVZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, -1, vzz);
     } else if (zq && !g.freesurf && gz0 - F < NAB) {
         i64 i = gx - F, jj = gy - F, k = gz0 - F;
         i64 q = (i * ny + jj) * (2 * NAB) + k;
-        cpml_zq(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, 1, vxz);
-        cpml_zq(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, 1, vyz);
-        cpml_zq(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, 1, vzz);
+        cpml_zq<DIV>(f.psi[PVX_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], (int)k, 1, vxz);
+        cpml_zq<DIV>(f.psi[PVY_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], (int)k, 1, vyz);
+        cpml_zq<DIV>(f.psi[PVZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], (int)k, 1, vzz);
     } else if (gz0 + 3 > NZ - NAB - F - 1 || (!zq && !g.freesurf && gz0 - F < NAB)) {
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -139,15 +142,15 @@ __device__ __forceinline__ void cpml_s3d_adj_q4(const Grid &g, const Fields &f, 
                 i64 i = gx - F, jj = gy - F, k = gz - NZ + NAB + F + NAB;
                 int ind = 2 * NAB - 1 - (int)k;
                 i64 q = (i * ny + jj) * (2 * NAB) + k;
-                cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vxz.v[j]);
-                cpml(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], ind, vyz.v[j]);
-                cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], ind + 1, vzz.v[j]);
+                cpml(f.psi[PVX_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, vxz.v[j]);
+                cpml(f.psi[PVY_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], ind, vyz.v[j]);
+                cpml(f.psi[PVZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], ind + 1, vzz.v[j]);
             } else if (!g.freesurf && gz - F < NAB) {
                 i64 i = gx - F, jj = gy - F, k = gz - F;
                 i64 q = (i * ny + jj) * (2 * NAB) + k;
-                cpml(f.psi[PVX_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, vxz.v[j]);
-                cpml(f.psi[PVY_Z], q, f.kinv[2][1], f.cz[CAH], f.cz[CBH], (int)k, vyz.v[j]);
-                cpml(f.psi[PVZ_Z], q, f.kinv[2][0], f.cz[CA], f.cz[CB], (int)k, vzz.v[j]);
+                cpml(f.psi[PVX_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], (int)k, vxz.v[j]);
+                cpml(f.psi[PVY_Z], q, ktab(f, 2, 1), f.cz[CAH], f.cz[CBH], (int)k, vyz.v[j]);
+                cpml(f.psi[PVZ_Z], q, ktab(f, 2, 0), f.cz[CA], f.cz[CB], (int)k, vzz.v[j]);
             }
         }
     }
@@ -155,31 +158,31 @@ __device__ __forceinline__ void cpml_s3d_adj_q4(const Grid &g, const Fields &f, 
     if (gy - F < NAB) {
         i64 i = gx - F, j = gy - F;
         i64 q = (i * (2 * NAB) + j) * nz + k0;
-        cpml_q(f.psi[PVX_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], (int)j, vxy);
-        cpml_q(f.psi[PVY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], (int)j, vyy);
-        cpml_q(f.psi[PVZ_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], (int)j, vzy);
+        cpml_q<DIV>(f.psi[PVX_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], (int)j, vxy);
+        cpml_q<DIV>(f.psi[PVY_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], (int)j, vyy);
+        cpml_q<DIV>(f.psi[PVZ_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], (int)j, vzy);
     } else if (gy > NY - NAB - F - 1) {
         i64 i = gx - F, j = gy - NY + NAB + F + NAB;
         int ind = 2 * NAB - 1 - (int)j;
         i64 q = (i * (2 * NAB) + j) * nz + k0;
-        cpml_q(f.psi[PVX_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ind, vxy);
-        cpml_q(f.psi[PVY_Y], q, f.kinv[1][0], f.cy[CA], f.cy[CB], ind + 1, vyy);
-        cpml_q(f.psi[PVZ_Y], q, f.kinv[1][1], f.cy[CAH], f.cy[CBH], ind, vzy);
+        cpml_q<DIV>(f.psi[PVX_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], ind, vxy);
+        cpml_q<DIV>(f.psi[PVY_Y], q, ktab(f, 1, 0), f.cy[CA], f.cy[CB], ind + 1, vyy);
+        cpml_q<DIV>(f.psi[PVZ_Y], q, ktab(f, 1, 1), f.cy[CAH], f.cy[CBH], ind, vzy);
     }
     if (gx - F < NAB) {
         i64 i = gx - F, j = gy - F;
         i64 q = (i * ny + j) * nz + k0;
-        cpml_q(f.psi[PVX_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], (int)i, vxx);
-        cpml_q(f.psi[PVY_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], (int)i, vyx);
-        cpml_q(f.psi[PVZ_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], (int)i, vzx);
+        cpml_q<DIV>(f.psi[PVX_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], (int)i, vxx);
+        cpml_q<DIV>(f.psi[PVY_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], (int)i, vyx);
+        cpml_q<DIV>(f.psi[PVZ_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], (int)i, vzx);
     }
     if (gx > NX - NAB - F - 1) {
         i64 i = gx - NX + NAB + F + NAB, j = gy - F;
         int ind = 2 * NAB - 1 - (int)i;
         i64 q = (i * ny + j) * nz + k0;
-        cpml_q(f.psi[PVX_X], q, f.kinv[0][0], f.cx[CA], f.cx[CB], ind + 1, vxx);
-        cpml_q(f.psi[PVY_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, vyx);
-        cpml_q(f.psi[PVZ_X], q, f.kinv[0][1], f.cx[CAH], f.cx[CBH], ind, vzx);
+        cpml_q<DIV>(f.psi[PVX_X], q, ktab(f, 0, 0), f.cx[CA], f.cx[CB], ind + 1, vxx);
+        cpml_q<DIV>(f.psi[PVY_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ind, vyx);
+        cpml_q<DIV>(f.psi[PVZ_X], q, ktab(f, 0, 1), f.cx[CAH], f.cx[CBH], ind, vzx);
     }
 }
 
@@ -187,9 +190,10 @@ __device__ __forceinline__ void cpml_s3d_adj_q4(const Grid &g, const Fields &f, 
 // and memory variables, parameters, the M and mu gradient sums) and 3 CTAs
 // per SM, as k_adjv3d_q4.  The saved-boundary index of each cell of the quad
 // is found once and kept for the four phases.
-template <int F, int L, typename T, bool MB = false, bool PF = false>
+template <int R, int L, typename T, bool MB = false, bool PF = false>
 __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f, AdjFields a)
 {
+    constexpr int F = half_width(R);
     CELL3D_Q4
     if (MB) shot_adj(g, a, shot);
     const bool recon = !g.ckpt && !g.bp2;
@@ -222,7 +226,8 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
     Q4 vzxr = dfw_q<F>(a.wr[VZ], iv, sx, hc), vzyr = dfw_q<F>(a.wr[VZ], iv, sy, hc);
     Q4 vyxr = dfw_q<F>(a.wr[VY], iv, sx, hc), vyyr = dbw_q<F>(a.wr[VY], iv, sy, hc);
     Q4 vxxr = dbw_q<F>(a.wr[VX], iv, sx, hc), vxyr = dfw_q<F>(a.wr[VX], iv, sy, hc);
-    if (g.abs_type == 1) cpml_s3d_adj_q4(g, f, gz0, gy, gx, vxxr, vxyr, vxzr, vyxr, vyyr, vyzr, vzxr, vzyr, vzzr);
+    if (g.abs_type == 1)
+        cpml_s3d_adj_q4<!whole_rows(R)>(g, f, gz0, gy, gx, vxxr, vxyr, vxzr, vyxr, vyyr, vyzr, vzxr, vzyr, vzzr);
     Q4 rsh[3];   // adjoint shear sums vxy+vyx, vyz+vzy, vxz+vzx
 #pragma unroll
     for (int j = 0; j < 4; j++) {
@@ -501,38 +506,38 @@ __global__ void __launch_bounds__(128, PF ? 3 : 4) k_adjs3d_q4(Grid g, Fields f,
 }
 
 // ------------------------------------------------------------- launchers
-template <int F, int L, typename T>
+template <int R, int L, typename T>
 static void quad_adjs_l(const Grid &g, const Fields &f, const AdjFields &a, dim3 gr, dim3 b, cudaStream_t st)
 {
     // kernels 5 keeps the kernels without the prefetch
-    if (g.kernels == 0 && g.nb == 1) k_adjs3d_q4<F, L, T, false, true><<<gr, b, 0, st>>>(g, f, a);
-    else MB_DISPATCH(g, k_adjs3d_q4<F, L, T, MBV><<<gr, b, 0, st>>>(g, f, a))
+    if (g.kernels == 0 && g.nb == 1) k_adjs3d_q4<R, L, T, false, true><<<gr, b, 0, st>>>(g, f, a);
+    else MB_DISPATCH(g, k_adjs3d_q4<R, L, T, MBV><<<gr, b, 0, st>>>(g, f, a))
 }
 
-template <int F, typename T>
+template <int R, typename T>
 static void quad_adj_t(const Grid &g, const Fields &f, const AdjFields &a, bool stress, cudaStream_t st)
 {
     if (stress) {
         const dim3 b = q4_block(g, 16, 8, 1), gr = q4_grid(g, b);
         switch (g.L) {
-        case 0: quad_adjs_l<F, 0, T>(g, f, a, gr, b, st); break;
-        case 1: quad_adjs_l<F, 1, T>(g, f, a, gr, b, st); break;
-        case 2: quad_adjs_l<F, 2, T>(g, f, a, gr, b, st); break;
-        default: quad_adjs_l<F, 3, T>(g, f, a, gr, b, st); break;
+        case 0: quad_adjs_l<R, 0, T>(g, f, a, gr, b, st); break;
+        case 1: quad_adjs_l<R, 1, T>(g, f, a, gr, b, st); break;
+        case 2: quad_adjs_l<R, 2, T>(g, f, a, gr, b, st); break;
+        default: quad_adjs_l<R, 3, T>(g, f, a, gr, b, st); break;
         }
         return;
     }
     const dim3 b = q4_block(g, 8, 4, 4), gr = q4_grid(g, b);
-    if (g.kernels == 0 && g.nb == 1) k_adjv3d_q4<F, T, false, true><<<gr, b, 0, st>>>(g, f, a);
-    else MB_DISPATCH(g, k_adjv3d_q4<F, T, MBV><<<gr, b, 0, st>>>(g, f, a))
+    if (g.kernels == 0 && g.nb == 1) k_adjv3d_q4<R, T, false, true><<<gr, b, 0, st>>>(g, f, a);
+    else MB_DISPATCH(g, k_adjv3d_q4<R, T, MBV><<<gr, b, 0, st>>>(g, f, a))
 }
 
-template <int F>
+template <int R>
 void quad_update_adj(const Grid &g, const Fields &f, const AdjFields &a, bool stress, int prec, cudaStream_t st)
 {
-    if (prec == SFD_PREC_FP16) quad_adj_t<F, __half>(g, f, a, stress, st);
-    else if (prec == SFD_PREC_BF16) quad_adj_t<F, __nv_bfloat16>(g, f, a, stress, st);
-    else quad_adj_t<F, float>(g, f, a, stress, st);
+    if (prec == SFD_PREC_FP16) quad_adj_t<R, __half>(g, f, a, stress, st);
+    else if (prec == SFD_PREC_BF16) quad_adj_t<R, __nv_bfloat16>(g, f, a, stress, st);
+    else quad_adj_t<R, float>(g, f, a, stress, st);
 }
 
 }  // namespace sfd

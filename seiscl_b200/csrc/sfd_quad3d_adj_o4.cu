@@ -3,6 +3,6 @@
 
 namespace sfd {
 
-template void quad_update_adj<2>(const Grid &, const Fields &, const AdjFields &, bool, int, cudaStream_t);
+template void quad_update_adj<ROWS_O4>(const Grid &, const Fields &, const AdjFields &, bool, int, cudaStream_t);
 
 }  // namespace sfd

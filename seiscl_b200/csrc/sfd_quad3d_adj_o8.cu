@@ -1,8 +1,9 @@
-// sfd_quad3d_adj_o8.cu -- the 4-cell 3D adjoint kernels of order 8.
+// sfd_quad3d_adj_o8.cu -- the 4-cell 3D adjoint kernels of order 8 on rows
+// of whole quads.
 #include "sfd_quad3d_adj.cuh"
 
 namespace sfd {
 
-template void quad_update_adj<4>(const Grid &, const Fields &, const AdjFields &, bool, int, cudaStream_t);
+template void quad_update_adj<ROWS_WHOLE>(const Grid &, const Fields &, const AdjFields &, bool, int, cudaStream_t);
 
 }  // namespace sfd

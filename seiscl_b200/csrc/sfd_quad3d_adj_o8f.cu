@@ -1,0 +1,9 @@
+// sfd_quad3d_adj_o8f.cu -- the 4-cell 3D adjoint kernels of order 8 on rows
+// filled up with dummy cells.
+#include "sfd_quad3d_adj.cuh"
+
+namespace sfd {
+
+template void quad_update_adj<ROWS_FILLED>(const Grid &, const Fields &, const AdjFields &, bool, int, cudaStream_t);
+
+}  // namespace sfd

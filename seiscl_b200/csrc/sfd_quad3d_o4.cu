@@ -3,8 +3,8 @@
 
 namespace sfd {
 
-template void quad_update_v<2>(const Grid &, const Fields &, cudaStream_t);
-template bool quad_update_s<2>(const Grid &, const Fields &, cudaStream_t, bool);
-template void quad_update_s_bnd<2>(const Grid &, const Fields &, const BndSlot &, int, int64_t, bool, cudaStream_t);
+template void quad_update_v<ROWS_O4>(const Grid &, const Fields &, cudaStream_t);
+template bool quad_update_s<ROWS_O4>(const Grid &, const Fields &, cudaStream_t, Surf);
+template void quad_update_s_bnd<ROWS_O4>(const Grid &, const Fields &, const BndSlot &, int, int64_t, bool, cudaStream_t);
 
 }  // namespace sfd

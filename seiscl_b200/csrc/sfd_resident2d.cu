@@ -82,7 +82,8 @@ __device__ __forceinline__ int tile_field(int w)
 // CPML of one axis at one cell: 1/K, a, b at full and half nodes, and the
 // slab-local index (-1 outside the slabs)
 struct Slab {
-    float kf, af, bf, kh, ah, bh;
+    double kf, kh;
+    float af, bf, ah, bh;
     int at;
 };
 constexpr int R2_ROWS = 64, R2_COLS = 64;   // most rows and columns (16 warps x 4) of a tile
@@ -92,23 +93,24 @@ static_assert(sizeof(float) * R2_NF * field_floats(4, 4) + R2_POINTS * (sizeof(i
               "the largest tile and point list fit whatever the run");
 static_assert(sizeof(float) * 2 * R2_NF * field_floats(4, 2) + R2_POINTS * (sizeof(int4) + sizeof(float)) <= R2_SMEM,
               "and so do the adjoint's");
-__device__ __forceinline__ Slab slab_of(const Grid &g, const float *const *c, const float *const *ki, int i, int n, bool lo)
+__device__ __forceinline__ Slab slab_of(const Grid &g, const Fields &fl, int axis, int i, int n, bool lo)
 {
-    Slab s = {1.0f, 0.0f, 0.0f, 1.0f, 0.0f, 0.0f, -1};
+    Slab s = {1.0, 1.0, 0.0f, 0.0f, 0.0f, 0.0f, -1};
     if (g.abs_type != 1) return s;
     int f, h;   // profile indices of the full and half nodes
     if (i >= n) return s;   // a dummy row
     if (i >= n - g.nab) { s.at = i - n + 2 * g.nab; f = 2 * g.nab - s.at; h = f - 1; }
     else if (lo && i < g.nab) { s.at = f = h = i; }
     else return s;
-    s.kf = ki[0][f]; s.af = c[CA][f]; s.bf = c[CB][f];
-    s.kh = ki[1][h]; s.ah = c[CAH][h]; s.bh = c[CBH][h];
+    const float *const *c = axis == 0 ? fl.cx : fl.cz;
+    s.kf = fl.kq[axis][0][f]; s.af = c[CA][f]; s.bf = c[CB][f];
+    s.kh = fl.kq[axis][1][h]; s.ah = c[CAH][h]; s.bh = c[CBH][h];
     return s;
 }
-__device__ __forceinline__ void cpml_reg(float &psi, float k, float a, float b, float &d)
+__device__ __forceinline__ void cpml_reg(float &psi, double k, float a, float b, float &d)
 {
     psi = cpml_psi(psi, a, b, d);
-    d = __fmaf_rn(d, k, psi);
+    d = cpml_quot(d, k, psi);
 }
 
 template <typename T>
@@ -171,7 +173,7 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_resident2d(const __grid_const
     for (int i = tid; i < R2_NF * FS; i += R2_THREADS) w[i] = 0.0f;
     s_rec[tid] = s_src[tid] = -1;
     if (tid == 0) s_np = 0;
-    for (int x = tid; x < tx; x += R2_THREADS) s_sx[x] = slab_of(g, f.cx, f.kinv[0], x0 + x, g.nx, true);
+    for (int x = tid; x < tx; x += R2_THREADS) s_sx[x] = slab_of(g, f, 0, x0 + x, g.nx, true);
     __syncthreads();
 #pragma unroll
     for (int q = 0; q < R2_NF; q++) {
@@ -221,7 +223,7 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_resident2d(const __grid_const
         else mat[i] = s2d_visco(L, g.dt, f.p[PM][ip], f.p[PMU][ip], f.p[PMUIPKP][ip], f.p[PTAUP][ip], f.p[PTAUS][ip],
                                 f.p[PTAUSIPKP][ip]);
         sx_at[i] = s_sx[on[i] ? xb + i : 0].at;
-        if (i == 0) sz = slab_of(g, f.cz, f.kinv[2], zz - F, g.nz - g.zpad, !g.freesurf);
+        if (i == 0) sz = slab_of(g, f, 2, zz - F, g.nz - g.zpad, !g.freesurf);
         psi_sxx[i] = psi_sxzx[i] = psi_szz[i] = psi_sxzz[i] = psi_vxx[i] = psi_vzx[i] = psi_vzz[i] = psi_vxz[i] = 0.0f;
         if (sx_at[i] >= 0) {
             const i64 q = (i64)sx_at[i] * g.nz + (zz - F);
@@ -487,7 +489,7 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_resident2d(const __grid_const
                     if (z == 0) {
                         szz = 0.0f;
                         const Surf2d su = s_surf[xb + i];
-                        const float h = surf2d_h(su, vxx, vzz);
+                        const float h = surf2d_h<L == 0>(su, vxx, vzz);
                         if constexpr (L == 0) {
                             sxx = __fadd_rn(h, sxx);
                         } else {
@@ -501,7 +503,7 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_resident2d(const __grid_const
                             sump = 0;
 #pragma unroll
                             for (int l = 0; l < L; l++) {
-                                rr[i][0][l] = __fadd_rn(surf2d_hr(su, surf2d_b(g.eta[l]), vxx, vzz), rr[i][0][l]);
+                                rr[i][0][l] = __fadd_rn(__fmul_rn(surf2d_b(g.eta[l]), surf2d_hr(su, vxx, vzz)), rr[i][0][l]);
                                 sump += rr[i][0][l];
                             }
                             sxx = __fadd_rn(__fmul_rn(g.dt2, sump), sxx);
@@ -619,7 +621,7 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_resident2d_adj(const __grid_c
     for (int i = tid; i < 2 * R2_NF * FS; i += R2_THREADS) w[i] = 0.0f;
     s_rec[tid] = s_src[tid] = -1;
     if (tid == 0) s_np = 0;
-    for (int x = tid; x < tx; x += R2_THREADS) s_sx[x] = slab_of(g, f.cx, f.kinv[0], x0 + x, g.nx, true);
+    for (int x = tid; x < tx; x += R2_THREADS) s_sx[x] = slab_of(g, f, 0, x0 + x, g.nx, true);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < 2 * R2_NF; k++) {
@@ -670,7 +672,7 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_resident2d_adj(const __grid_c
         gmu[i] = q.grad[GMU][ip];
         gr[i] = q.grad[GRHO][ip];
         sx_at[i] = s_sx[on[i] ? xb + i : 0].at;
-        if (i == 0) sz = slab_of(g, f.cz, f.kinv[2], zz - F, g.nz - g.zpad, true);
+        if (i == 0) sz = slab_of(g, f, 2, zz - F, g.nz - g.zpad, true);
         psi_sxx[i] = psi_sxzx[i] = psi_szz[i] = psi_sxzz[i] = psi_vxx[i] = psi_vzx[i] = psi_vzz[i] = psi_vxz[i] = 0.0f;
         if (sx_at[i] >= 0) {
             const i64 k = (i64)sx_at[i] * g.nz + (zz - F);
@@ -918,7 +920,7 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_resident2d_adj(const __grid_c
                 }
                 const float lvx = __fmul_rn(__fadd_rn(xx, xzz), rip[i]), lvz = __fmul_rn(__fadd_rn(zz, xzx), rkp[i]);
                 float ux = __fadd_rn(w[(A + W_VX) * FS + c], lvx), uz = __fadd_rn(w[(A + W_VZ) * FS + c], lvz);
-                gr[i] += (double)__fmaf_rn(-vz, lvz, -__fmul_rn(vx, lvx));
+                gr[i] += (double)__fmaf_rn(-vx, lvx, -__fmul_rn(vz, lvz));
                 if (!on[i]) continue;
                 bad |= !isfinite(ux);
                 if (my_src >= 0) {

@@ -297,7 +297,7 @@ int alloc_model(sfd_plan *p)
     for (int k = 0; k < NPAR; k++) {
         p->f.p[k] = (const float *)dalloc(p, sizeof(float) * npar, &e);
         if (e) return fail(p, SFD_ERR_MEMORY, "parameter allocation failed");
-        if (g.zpad) CKC(cudaMemset((void *)p->f.p[k], 0, sizeof(float) * npar));   // dummy rows
+        if (g.zpad) CKC(cudaMemsetAsync((void *)p->f.p[k], 0, sizeof(float) * npar, p->stream));   // dummy rows
     }
     int nc = std::max(2 * g.nab, 1);
     double *kq = (double *)dalloc(p, const_bytes(nc), &e);
@@ -633,8 +633,9 @@ int alloc_ckpt(sfd_plan *p)
     return SFD_OK;
 }
 
-// FP16 wave-field storage: the unscaled parameters of the adjoint, uploaded
-// once per model
+// FP16 wave-field storage: the unscaled parameters of the adjoint, formed once
+// per model.  The scaling writes dummy rows too: nothing else touches the buffer,
+// and all of it happens on the plan's stream, which no other stream orders.
 int prepare_adjoint_params(sfd_plan *p)
 {
     for (int k = 0; k < NPAR; k++) p->padj[k] = p->f.p[k];
@@ -647,7 +648,6 @@ int prepare_adjoint_params(sfd_plan *p)
     if (!p->d_padj) {
         p->d_padj = (float *)dalloc(p, sizeof(float) * npar * nscaled, &e);
         if (!p->d_padj) return fail(p, SFD_ERR_MEMORY, "unscaled adjoint parameters do not fit in device memory");
-        if (g.zpad) CKC(cudaMemset(p->d_padj, 0, sizeof(float) * npar * nscaled));
     }
     int q = 0;
     for (int k = 0; k < NPAR; k++) {

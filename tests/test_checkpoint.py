@@ -172,3 +172,33 @@ def test_checkpoint_configuration_checks():
                 dict(checkpoint=5, batch=2), dict(checkpoint=5, field_precision="fp16", hout=1)):
         with pytest.raises(engine.SeisCLEngineError):
             engine.footprint(dataclasses.replace(ok, **bad), True, 1, 20)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fdorder,nz", [(8, 38), (4, 42)])
+def test_fp16_fields_adjoint_beside_a_busy_default_stream(fdorder, nz, cuda_device):
+    """FP16 wave fields on rows filled up with dummy cells: the adjoint's
+    unscaled parameters are formed on the plan's stream alone.  A first adjoint
+    while the process's default stream is busy, and a second one with the
+    parameters it left, give the gradient of a plan that had the device to
+    itself, bit for bit."""
+    import torch
+
+    from seiscl_b200.engine import Plan
+
+    cfg, model, acq = make_case(nd=3, freesurf=0, L=0, nz=nz, ny=28, nx=30, nt=60, nab=8, fdorder=fdorder)
+    outs, got = ["vx", "vy", "vz"], []
+    for busy in (False, True):
+        p = Plan(dataclasses.replace(engine_config(cfg), checkpoint=20, field_precision="fp16"))
+        p.set_model(model["vp"], model["vs"], model["rho"])
+        for turn in range(2):
+            d = p.forward(acq["src_pos"], acq["src"], acq["rec_pos"], outs, save_boundaries=True)
+            if busy and turn == 0:
+                torch.cuda._sleep(1000000000)   # about half a second on the default stream
+            p.zero_gradient()
+            p.adjoint(acq["src_pos"], acq["src"], acq["rec_pos"], d)
+            torch.cuda.synchronize()
+        got.append(p.gradient())
+        p.close()
+    for k in got[0]:
+        assert np.abs(got[0][k]).max() > 0 and np.array_equal(got[0][k], got[1][k]), k

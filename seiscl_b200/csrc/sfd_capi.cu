@@ -1244,6 +1244,10 @@ extern "C" void sfd_plan_destroy(sfd_plan *p)
 extern "C" const char *sfd_last_error(const sfd_plan *p) { return p ? p->err.c_str() : "null plan"; }
 
 namespace {
+// scratch of sample_model: up to 8192 sampled cells (index, two values) and nx
+// receivers' cells (index, three values)
+int64_t sample_bytes(const Grid &g) { return 8192 * 16 + (int64_t)g.nx * 24; }
+
 // A host copy of a transformed parameter [nx][(ny)][nz], unscaled
 int host_param(sfd_plan *p, int k, const float **out)
 {
@@ -1266,8 +1270,40 @@ int host_param(sfd_plan *p, int k, const float **out)
     return SFD_OK;
 }
 
-// log2 of the model's mean impedance sqrt(M / rip), from every step-th cell
-int impedance_shift(sfd_plan *p, char *scratch, int64_t bytes, int *shift)
+// M and then mu at the cells `at` of the device arrays, unscaled.  Several
+// threads may scale residuals of one plan.
+int gather_pressure(sfd_plan *p, const std::vector<int64_t> &at, std::vector<float> &v)
+{
+    const size_t n = at.size();
+    v.resize(2 * n);
+    if (!n) return SFD_OK;
+    std::lock_guard<std::mutex> lock(p->gather_m);
+    CKC(cudaSetDevice(p->device));
+    const size_t bytes = (sizeof(int64_t) + 2 * sizeof(float)) * n;
+    cudaError_t e;
+    int64_t *d_at = (int64_t *)dalloc_raw(p, bytes, &e);
+    if (!d_at) return fail(p, SFD_ERR_MEMORY, "residual scaling: gather buffers do not fit in device memory");
+    float *d_v = (float *)(d_at + n);
+    e = cudaMemcpyAsync(d_at, at.data(), sizeof(int64_t) * n, cudaMemcpyHostToDevice, p->stream);
+    launch_gather(p->f.p[PM], d_at, d_v, (int)n, p->stream);
+    launch_gather(p->f.p[PMU], d_at, d_v + n, (int)n, p->stream);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(v.data(), d_v, sizeof(float) * 2 * n, cudaMemcpyDeviceToHost, p->stream);
+    const cudaError_t es = cudaStreamSynchronize(p->stream);
+    dfree(p, d_at, bytes);
+    if (e == cudaSuccess) e = es;
+    if (e != cudaSuccess) return fail(p, SFD_ERR_CUDA, std::string("residual scaling: ") + cudaGetErrorString(e));
+    if (const int ex = p->g.fhalf ? param_exponent(PM, p->kshift) : 0)
+        for (float &q : v) q = std::ldexp(q, -ex);
+    return SFD_OK;
+}
+
+// The few values of a new model (before FP16 wave fields scale it) that the
+// host needs: log2 of its mean impedance sqrt(M / rip), from every step-th
+// cell, and the buoyancies at (x, x, x), which the residual scaling reads
+// (p->diag).  Copying those three arrays for the first residuals instead, 48
+// MB at 100 x 200 x 200, took 6 ms a model.
+int sample_model(sfd_plan *p, char *scratch, int64_t bytes, int *shift)
 {
     const Grid &g = p->g;
     const int nzu = g.nz - g.zpad;
@@ -1275,14 +1311,21 @@ int impedance_shift(sfd_plan *p, char *scratch, int64_t bytes, int *shift)
     std::vector<int64_t> at;
     for (int64_t i = 0; i < n; i += step) at.push_back(i / nzu * g.nz + i % nzu);
     const int cnt = (int)at.size();
-    if ((int64_t)cnt * (int64_t)(sizeof(int64_t) + 2 * sizeof(float)) > bytes) return fail(p, SFD_ERR_MEMORY, "scratch too small");
+    for (int64_t x = 0; x < g.nx; x++) {
+        const int64_t i = std::min(g.nd == 3 ? (x * g.ny + x) * nzu + x : x * nzu + x, n - 1);
+        at.push_back(i / nzu * g.nz + i % nzu);
+    }
+    const int nd = (int)at.size() - cnt;
+    if (sample_bytes(g) > bytes) return fail(p, SFD_ERR_MEMORY, "scratch too small");
     int64_t *d_at = (int64_t *)scratch;
-    float *d_v = (float *)(d_at + cnt);
-    std::vector<float> v(2 * cnt);
-    CKC(cudaMemcpyAsync(d_at, at.data(), sizeof(int64_t) * cnt, cudaMemcpyHostToDevice, p->stream));
+    float *d_v = (float *)(d_at + at.size());
+    std::vector<float> v(2 * cnt + 3 * nd);
+    CKC(cudaMemcpyAsync(d_at, at.data(), sizeof(int64_t) * at.size(), cudaMemcpyHostToDevice, p->stream));
     launch_gather(p->f.p[PM], d_at, d_v, cnt, p->stream);
     launch_gather(p->f.p[PRIP], d_at, d_v + cnt, cnt, p->stream);
-    CKC(cudaMemcpyAsync(v.data(), d_v, sizeof(float) * 2 * cnt, cudaMemcpyDeviceToHost, p->stream));
+    const int id[3] = {PRIP, PRJP, PRKP};
+    for (int k = 0; k < 3; k++) launch_gather(p->f.p[id[k]], d_at + cnt, d_v + 2 * cnt + k * nd, nd, p->stream);
+    CKC(cudaMemcpyAsync(v.data(), d_v, sizeof(float) * v.size(), cudaMemcpyDeviceToHost, p->stream));
     CKC(cudaStreamSynchronize(p->stream));
     double acc = 0.0;
     int64_t m = 0;
@@ -1291,6 +1334,7 @@ int impedance_shift(sfd_plan *p, char *scratch, int64_t bytes, int *shift)
         if (z > 0 && std::isfinite(z)) { acc += std::log2(z); m++; }
     }
     *shift = m ? (int)std::lround(acc / m) : 0;
+    for (int k = 0; k < 3; k++) p->diag[k].assign(v.begin() + 2 * cnt + k * nd, v.begin() + 2 * cnt + (k + 1) * nd);
     return SFD_OK;
 }
 
@@ -1367,7 +1411,7 @@ int store_model(sfd_plan *p, const float *const in[5], char *scratch, int planes
     p->surf_mu_zero = found.top_mu_zero != 0;
     // FP16 stores keep velocities as v * 2^b and stresses as s * 2^a with
     // b - a ~ log2 of the impedance, so both stay near the same magnitude
-    if ((rc = impedance_shift(p, scratch, bytes, &p->bshift))) return rc;
+    if ((rc = sample_model(p, scratch, bytes, &p->bshift))) return rc;
     if (g.fhalf) {
         // FP16 wave fields: the moduli carry 2^-kshift and the buoyancies
         // 2^kshift (exact power-of-two scalings of the FP32 parameters)
@@ -1400,7 +1444,7 @@ extern "C" int sfd_set_model(sfd_plan *p, const float *const *params)
     // planes), and returns to the pool
     const int64_t plane = (int64_t)(g.nz - g.zpad) * g.ny, narr = c.L > 0 ? 5 : 3;
     const int planes = (int)std::min<int64_t>(g.nx, std::max<int64_t>(2, (5 << 20) / plane));
-    const int64_t bytes = 256 + std::max<int64_t>(sizeof(float) * narr * plane * planes, 8192 * 16);
+    const int64_t bytes = 256 + std::max<int64_t>(sizeof(float) * narr * plane * planes, sample_bytes(g));
     cudaError_t e;
     char *scratch = (char *)dalloc_raw(p, bytes, &e);
     if (!scratch) return fail(p, SFD_ERR_MEMORY, "model staging does not fit in device memory");
@@ -1991,32 +2035,40 @@ extern "C" int sfd_residual_scale(sfd_plan *p, const sfd_shot *shot, const int *
     if (!p || !shot) return SFD_ERR_ARG;
     if (!p->model_set) return fail(p, SFD_ERR_STATE, "no model");
     const Grid &g = p->g;
-    const int NT = p->cfg.nt, tmax = p->cfg.tmax;
+    const int NT = p->cfg.nt, tmax = p->cfg.tmax, nrec = shot->nrec;
     const float dh = p->cfg.dh, dt = p->cfg.dt;
     const int nz = g.nz - g.zpad;
-    int64_t npar = user_cells(g);
+    const int64_t npar = user_cells(g);
+    // flat index of the cell a receiver's scaling reads, -1 outside the model
+    auto cell = [&](int r, bool pressure) {
+        const float *rp = shot->rec_pos + 8 * r;
+        const int x = (int)(rp[0] / dh), y = pressure ? (int)(rp[1] / dh) : x, z = pressure ? (int)(rp[2] / dh) : x;
+        const int64_t pos = g.nd == 3 ? ((int64_t)x * g.ny + y) * nz + z : (int64_t)x * nz + z;
+        return pos < 0 || pos >= npar ? (int64_t)-1 : pos;
+    };
     for (int o = 0; o < SFD_NOUT; o++) {
         if (!outsel || !outsel[o] || !res || !res[o]) continue;
-        if (o != SFD_OUT_VX && o != SFD_OUT_VY && o != SFD_OUT_VZ && o != SFD_OUT_P) continue;
-        const int id = o == SFD_OUT_P ? PM : o == SFD_OUT_VX ? PRIP : (o == SFD_OUT_VY ? PRJP : PRKP);
-        const float *par, *pmu = nullptr;
-        if (int rc_ = host_param(p, id, &par)) return rc_;
-        if (o == SFD_OUT_P)
-            if (int rc_ = host_param(p, PMU, &pmu)) return rc_;
-        for (int r = 0; r < shot->nrec; r++) {
-            const float *rp = shot->rec_pos + 8 * r;
-            int x, y, z;
-            if (o == SFD_OUT_P) { x = (int)(rp[0] / dh); y = (int)(rp[1] / dh); z = (int)(rp[2] / dh); }
-            else { x = (int)(rp[0] / dh); y = x; z = x; }
-            int64_t pos = g.nd == 3 ? ((int64_t)x * g.ny + y) * nz + z : (int64_t)x * nz + z;
-            if (pos < 0 || pos >= npar) return fail(p, SFD_ERR_ARG, "residual scaling index outside the model");
+        const bool pressure = o == SFD_OUT_P;
+        if (o != SFD_OUT_VX && o != SFD_OUT_VY && o != SFD_OUT_VZ && !pressure) continue;
+        for (int r = 0; r < nrec; r++)
+            if (cell(r, pressure) < 0) return fail(p, SFD_ERR_ARG, "residual scaling index outside the model");
+        std::vector<float> pm;   // M, then mu, per receiver
+        if (pressure) {
+            std::vector<int64_t> at(nrec);
+            for (int r = 0; r < nrec; r++) at[r] = cell(r, true) / nz * g.nz + cell(r, true) % nz;
+            if (int rc = gather_pressure(p, at, pm)) return rc;
+        }
+        for (int r = 0; r < nrec; r++) {
             float *row = res[o] + (int64_t)r * NT;
-            if (o == SFD_OUT_P) {
-                float parscal = -2.0 * (par[pos] - pmu[pos]) * dh / dt;
-                for (int t = 0; t < tmax; t++) row[t] *= parscal * dt;
+            if (pressure) {
+                float parscal = -2.0 * (pm[r] - pm[nrec + r]) * dh / dt;
+                const float f = parscal * dt;
+                for (int t = 0; t < tmax; t++) row[t] *= f;
             } else {
-                float parscal = 1.0 / par[pos] * dh / dt;
-                for (int t = 0; t < tmax; t++) row[t] *= 1.0 / parscal * dt;
+                const float par = p->diag[o == SFD_OUT_VX ? 0 : o == SFD_OUT_VY ? 1 : 2][(int)(shot->rec_pos[8 * r] / dh)];
+                float parscal = 1.0 / par * dh / dt;
+                const double f = 1.0 / parscal * dt;
+                for (int t = 0; t < tmax; t++) row[t] *= f;
             }
         }
     }

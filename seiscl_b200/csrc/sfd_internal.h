@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -147,9 +148,11 @@ struct sfd_plan {
     std::string err;
     double DH_lit;          // the reference's "%9.9f" dh literal
     double DT_lit;
-    // host copies of the transformed parameters, made when something asks
-    // (host_param); cleared with each new model
+    // host copies of the transformed parameters, made for the Hessian's
+    // transform (host_param); cleared with each new model
     std::vector<float> hp[sfd::NPAR];
+    std::vector<float> diag[3];   // PRIP, PRJP, PRKP of the model at (x, x, x), x < nx
+    std::mutex gather_m;    // pressure residuals scaled by several threads
     bool model_set;
     // device memory
     std::vector<std::pair<void *, size_t>> allocs;   // owned by the plan

@@ -369,7 +369,9 @@ int64_t sfd_debug_copy(sfd_plan *plan, int kind, int id, float *dst, int64_t cap
  * arrays -- which 0 velocity update, 1 stress update, 2 free surface
  * (forward), 3 free-surface adjoint on the adjoint fields (the reference's
  * surface_adj, src/surface2D_adj.cl:35-148, src/surface3D_adj.cl:29-116) --
- * returning after it finished.  No counterpart in the reference. */
+ * returning after it finished; 4 makes the next resident 2D launch count as
+ * refused by the driver, 5 runs one resident 2D step without its last tile and
+ * reports the waits that run out.  No counterpart in the reference. */
 int64_t sfd_debug_load(sfd_plan *plan, int kind, int id, const float *src, int64_t n);
 int sfd_debug_launch(sfd_plan *plan, int which);
 

@@ -316,6 +316,7 @@ int alloc_model(sfd_plan *p)
     p->d_words = nullptr;
     if (const int64_t wb = resident2d_bytes(g, p->batch)) {
         p->d_words = (unsigned long long *)dalloc(p, (size_t)wb, &e);
+        p->words_bytes = wb;
         if (e) return fail(p, SFD_ERR_MEMORY, "step exchange allocation failed");
     }
     // fused 3D step: ticket counter and per-unit flags (single-shot plans)
@@ -1092,6 +1093,39 @@ void init_grid(const sfd_config &c, Grid &g)
 }
 }  // namespace
 
+namespace {
+// SMs for the resident 2D steps: those of the device as this process sees it (a
+// partition has fewer), or SEISCL_B200_RESIDENT_SMS where that is less (0:
+// always the ordinary loop)
+int resident_sms(int device)
+{
+    int n = 0, coop = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop) {
+        cudaGetLastError();
+        return 0;
+    }
+    if (const char *e = std::getenv("SEISCL_B200_RESIDENT_SMS")) n = std::min(n, std::max(0, atoi(e)));
+    return n;
+}
+// a refused cooperative launch (fewer SMs free to this process than it
+// sees): nothing has run, the ordinary loop can take over
+bool launch_refused(sfd_plan *p, cudaError_t e)
+{
+    if (e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorLaunchOutOfResources && e != cudaErrorNotSupported)
+        return false;
+    cudaGetLastError();
+    p->sms = 0;
+    return true;
+}
+cudaError_t refuse_once(sfd_plan *p)
+{
+    const bool r = p->refuse_resident;
+    p->refuse_resident = false;
+    return r ? cudaErrorCooperativeLaunchTooLarge : cudaSuccess;
+}
+}  // namespace
+
 extern "C" int sfd_plan_create(const sfd_config *cfg, sfd_plan **out)
 {
     if (!cfg || !out) return SFD_ERR_ARG;
@@ -1117,6 +1151,9 @@ extern "C" int sfd_plan_create(const sfd_config *cfg, sfd_plan **out)
     p->d_ticket = nullptr;
     p->d_unstable = nullptr;
     p->d_words = nullptr;
+    p->words_bytes = 0;
+    p->refuse_resident = false;
+    p->sms = resident_sms(p->device);
     p->d_fsync = nullptr;
     p->dev_bytes = 0;
     p->batch = std::max(1, c.batch);
@@ -1618,8 +1655,8 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
     const bool bnd_shells = save_boundaries && !dft && !ckpt;
     // 2D P-SV runs whose wave fields fit on chip: the time loop in segments,
     // one cooperative launch each (sfd_resident2d.cu)
-    const Res2d rs = resident2d_plan(g, nshot, S.n + R.n);
-    const bool resident = rs.ctas > 0 && p->d_words && points.inside && !dft && !ckpt && !mv.n;
+    const Res2d rs = resident2d_plan(g, nshot, S.n + R.n, p->sms);
+    bool resident = rs.ctas > 0 && 8 * resident2d_words(rs, false) <= p->words_bytes && points.inside && !dft && !ckpt && !mv.n;
     LoopKey key;
     key.add(points.apart); key.add(mv.n); key.add(p->movout); key.add(p->d_mov); key.add(fuse2d); key.add(p->d_ticket); key.add(fuse3d);
     key.add(1); key.add(p->g); key.add(p->f); key.add_points(S); key.add_points(R); key.add(p->d_src);
@@ -1641,17 +1678,24 @@ extern "C" int sfd_forward_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
         if (tmax > 0) launch_sources(g, p->f, S, p->d_src, NT, 0, 1, st);
         Res2dRun a{R, S, p->d_src, p->d_seis, omask, NT, 0, 0, tmax, 0, bs, p->cfg.precision, p->d_words, p->d_unstable,
                    p->d_unstable + 1};
-        for (a.shot0 = 0; a.shot0 < nshot; a.shot0 += rs.shots) {
+        for (a.shot0 = 0; resident && a.shot0 < nshot; a.shot0 += rs.shots) {
             CKC(cudaMemsetAsync(p->d_words, 0, sizeof(*p->d_words) * (size_t)resident2d_words(rs, false), st));
             Res2d r = rs;
             r.ctas = r.ntz * r.ntx * std::min(rs.shots, nshot - a.shot0);
             for (a.t0 = 0; a.t0 < tmax; a.t0 = a.t1) {
                 a.t1 = std::min(a.t0 + RES2D_SEGMENT, tmax);
-                CKC(launch_resident2d(g, p->f, r, a, p->device, st));
+                cudaError_t e = refuse_once(p);
+                if (e == cudaSuccess) e = launch_resident2d(g, p->f, r, a, p->device, st);
+                if (a.shot0 == 0 && a.t0 == 0 && launch_refused(p, e)) {
+                    resident = false;   // the ordinary loop, from the start
+                    if ((rc = zero_forward_state(p, st))) return rc;
+                    break;
+                }
+                CKC(e);
             }
         }
-    } else
-    rcl = run_loop(p, p->gfwd, key.s, st, [&](cudaStream_t s) {
+    }
+    if (!resident) rcl = run_loop(p, p->gfwd, key.s, st, [&](cudaStream_t s) {
         if (fuse2d) {
             if (tmax > 0) launch_sources(g, p->f, S, p->d_src, NT, 0, 1, s);
             for (int t = 0; t < tmax; t++) {
@@ -1802,24 +1846,33 @@ extern "C" int sfd_adjoint_batch(sfd_plan *p, int nshot, const sfd_shot *shots, 
     CKC(cudaEventRecord(p->ev0, st));
     // shots whose forward and adjoint fields fit on chip: the loop in
     // segments, one cooperative launch each (sfd_resident2d.cu)
-    const Res2d rs = resident2d_adj_plan(g, nshot, S.n + R.n);
+    const Res2d rs = resident2d_adj_plan(g, nshot, S.n + R.n, p->sms);
     const int tmax = p->cfg.tmax, tmin = p->cfg.tmin;
     int rcl = SFD_OK;
-    if (rs.ctas > 0 && p->d_words && points.inside && !mv.n) {
+    bool resident = rs.ctas > 0 && 8 * resident2d_words(rs, true) <= p->words_bytes && points.inside && !mv.n;
+    if (resident) {
         for (int w = 0; w < NW; w++) a.bnd[w] = p->d_bnd[w];
         if (tmax - 1 > tmin) launch_residuals(g, p->f, a, R, p->d_res, NT, tmax - 1, omask, S, p->d_src, -1, st);
         Res2dAdj q{R, S, p->d_src, p->d_res, omask, NT, 0, 0, tmax, tmin, 0, p->d_words, p->d_unstable, p->d_unstable + 1};
-        for (q.shot0 = 0; q.shot0 < nshot; q.shot0 += rs.shots) {
+        for (q.shot0 = 0; resident && q.shot0 < nshot; q.shot0 += rs.shots) {
             CKC(cudaMemsetAsync(p->d_words, 0, sizeof(*p->d_words) * (size_t)resident2d_words(rs, true), st));
             Res2d r = rs;
             r.ctas = r.ntz * r.ntx * std::min(rs.shots, nshot - q.shot0);
             for (q.t0 = tmax - 1; q.t0 > tmin; q.t0 = q.t1) {
                 q.t1 = std::max(q.t0 - RES2D_SEGMENT, tmin);
-                CKC(launch_resident2d_adj(g, p->f, a, r, q, p->cfg.precision, p->device, st));
+                cudaError_t e = refuse_once(p);
+                if (e == cudaSuccess) e = launch_resident2d_adj(g, p->f, a, r, q, p->cfg.precision, p->device, st);
+                if (q.shot0 == 0 && q.t0 == tmax - 1 && launch_refused(p, e)) {
+                    resident = false;   // the ordinary loop, from the start
+                    for (int w = 0; w < NW; w++)
+                        if (p->a.wr[w]) CKC(cudaMemsetAsync(p->a.wr[w], 0, sizeof(float) * g.nvol * nshot, st));
+                    break;
+                }
+                CKC(e);
             }
         }
-    } else
-    rcl = run_loop(p, p->gadj, key.s, st, [&](cudaStream_t s) {
+    }
+    if (!resident) rcl = run_loop(p, p->gadj, key.s, st, [&](cudaStream_t s) {
         // the sources a step takes out of the reconstructed fields go with the
         // next step's residuals, unless a movie films the fields between
         int tsrc = -1;
@@ -2184,6 +2237,26 @@ extern "C" int sfd_debug_launch(sfd_plan *p, int which)
         if ((rc = alloc_adjoint(p))) return rc;
         launch_surface_adj(g, p->f, p->a, p->d_surf_q, st);
         break;
+    case 4: p->refuse_resident = true; break;
+    case 5: {
+        // one resident step of a grid of two tiles or more without its last
+        // tile: the others' waits run out after a millisecond
+        Res2d r = resident2d_plan(g, 1, 0, p->sms);
+        if (r.ctas < 2 || 8 * resident2d_words(r, false) > p->words_bytes)
+            return fail(p, SFD_ERR_STATE, "the plan's grid is not resident in two tiles or more");
+        Res2dRun a{};
+        a.t1 = a.tmax = a.nt_total = 1;
+        a.words = p->d_words;
+        a.first_bad = p->d_unstable;
+        a.status = p->d_unstable + 1;
+        a.wait_ns = 1000000;
+        CKC(cudaMemsetAsync(p->d_words, 0, sizeof(*p->d_words) * (size_t)resident2d_words(r, false), st));
+        if ((rc = arm_unstable(p, st))) return rc;
+        r.ctas--;
+        CKC(launch_resident2d(g, p->f, r, a, p->device, st));
+        CKC(cudaStreamSynchronize(st));
+        return take_unstable(p, st, "forward");
+    }
     default: return fail(p, SFD_ERR_ARG, "unknown kernel");
     }
     CKC(cudaGetLastError());

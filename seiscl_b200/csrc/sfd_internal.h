@@ -174,6 +174,9 @@ struct sfd_plan {
     int *d_unstable;        // first checked step with a non-finite wave field (0x7f7f7f7f: none), then
                             // the status of the resident 2D steps (0, or 1: a wait ran out)
     unsigned long long *d_words;   // exchange words of the resident 2D steps
+    int64_t words_bytes;
+    int sms;                // SMs the process has for them; 0 once a cooperative launch was refused
+    bool refuse_resident;   // tests: the next one counts as refused
     int *d_fsync;           // fused 3D step: ticket counter + one flag per work unit
     // checkpointed gradients (cfg.checkpoint = K > 0)
     char *d_snap;           // [nseg] snapshots: wave fields, memory variables (store type; FP16 wave-field

@@ -83,6 +83,7 @@ struct Res2d {              // tiles of a launch: ctas = ntz x ntx x shots, 0 wh
     int shots;              // shots of a launch
     size_t smem;
 };
+constexpr long long RES2D_WAIT_NS = 2000000000LL;
 struct Res2dRun {           // a segment of the time loop: steps t0 .. t1-1 of tmax
     PointSet rec, src;
     const float *stf;       // [nsrc][nt_total]
@@ -94,10 +95,13 @@ struct Res2dRun {           // a segment of the time loop: steps t0 .. t1-1 of t
     int prec;
     unsigned long long *words;   // exchange words, zeroed before the run's first segment
     int *first_bad, *status;
+    long long wait_ns = RES2D_WAIT_NS;   // bound of one wait
 };
 constexpr int RES2D_SEGMENT = 256;   // steps of one launch: bounds how long it holds the SMs
-Res2d resident2d_plan(const Grid &g, int nb, int npoints);   // launches for the nb shots of a run
-Res2d resident2d_adj_plan(const Grid &g, int nb, int npoints);
+constexpr int RES2D_SMS = 148;       // most CTAs of a launch, one per SM
+// launches for the nb shots of a run on the `sms` SMs a process has
+Res2d resident2d_plan(const Grid &g, int nb, int npoints, int sms);
+Res2d resident2d_adj_plan(const Grid &g, int nb, int npoints, int sms);
 int64_t resident2d_words(const Res2d &r, bool adjoint);
 int64_t resident2d_bytes(const Grid &g, int batch);   // exchange words of launches of up to `batch` shots
 struct Res2dAdj {           // a segment of the adjoint loop: steps t0, t0-1 .. t1+1 of tmax-1 .. tmin+1
@@ -107,6 +111,7 @@ struct Res2dAdj {           // a segment of the adjoint loop: steps t0, t0-1 .. 
     int nt_total, t0, t1, tmax, tmin, shot0;
     unsigned long long *words;
     int *first_bad, *status;
+    long long wait_ns = RES2D_WAIT_NS;
 };
 // q.bnd: the saved boundaries from step 0
 cudaError_t launch_resident2d_adj(const Grid &g, const Fields &f, const AdjFields &q, const Res2d &r, const Res2dAdj &a,

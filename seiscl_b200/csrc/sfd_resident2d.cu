@@ -46,11 +46,10 @@ namespace sfd {
 namespace {
 
 constexpr int R2_THREADS = 512;
-constexpr int R2_CTAS = 148;              // one CTA per SM
+constexpr int R2_CTAS = RES2D_SMS;        // one CTA per SM
 constexpr int R2_SMEM = 200 * 1024;       // dynamic shared memory a CTA may take
 constexpr int r2_words(int nc) { return nc == 4 ? 4 : 2; }   // most exchange words a thread receives in a half step
 constexpr int R2_POINTS = 4096;           // receivers and sources of a run
-constexpr long long R2_WAIT_NS = 2000000000LL;   // bound of one wait
 
 enum { W_VX, W_VZ, W_XX, W_ZZ, W_XZ, R2_NF };    // fields of a tile in shared memory
 
@@ -318,7 +317,7 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_resident2d(const __grid_const
             for (int spin = 1; (unsigned)(v[u] >> 32) != epoch && !failed; spin++) {
                 v[u] = ld_word(a.words + (from[u] + h));
                 if (spin % 1024) continue;   // now and then: has the wait run out?
-                if (!lim) lim = now_ns() + R2_WAIT_NS;
+                if (!lim) lim = now_ns() + a.wait_ns;
                 failed = now_ns() > lim;
             }
             const int c = cell_in[u];
@@ -748,7 +747,7 @@ __global__ void __launch_bounds__(R2_THREADS, 1) k_resident2d_adj(const __grid_c
             for (int spin = 1; (unsigned)(v[u] >> 32) != epoch && !failed; spin++) {
                 v[u] = ld_word(a.words + (from[u] + h));
                 if (spin % 1024) continue;
-                if (!lim) lim = now_ns() + R2_WAIT_NS;
+                if (!lim) lim = now_ns() + a.wait_ns;
                 failed = now_ns() > lim;
             }
             const int fld = (c >> 26) & 3, k = ((fld & 1) ? f1 : (c >> 28) & 1 ? fz : fx) + (fld >= 2 ? A : 0);
@@ -1002,7 +1001,7 @@ static double ordinary2d_step_us(const Grid &g, int nb)
 // 250,000 cells; larger grids fill the chip with ordinary launches.
 // adjoint: twice the fields and words, elastic without a free surface, at
 // most 2 cells a thread.
-static Res2d resident2d_shape(const Grid &g, int nb, int npoints, bool adjoint = false)
+static Res2d resident2d_shape(const Grid &g, int nb, int npoints, int sms, bool adjoint)
 {
     Res2d best;
     memset(&best, 0, sizeof best);
@@ -1013,7 +1012,7 @@ static Res2d resident2d_shape(const Grid &g, int nb, int npoints, bool adjoint =
     if (g.nz < F + 1 || g.nx < F + 1 || nb < 1 || npoints > R2_POINTS) return best;
     long bestc = 0;
     for (int nc = 1; nc <= (adjoint ? 2 : 4); nc *= 2) {
-        for (int ntz = 1; g.nz / ntz >= F + 1 && ntz * nb <= R2_CTAS; ntz++) {
+        for (int ntz = 1; g.nz / ntz >= F + 1 && ntz * nb <= sms; ntz++) {
             Res2d r;
             memset(&r, 0, sizeof r);
             r.F = F;
@@ -1028,7 +1027,7 @@ static Res2d resident2d_shape(const Grid &g, int nb, int npoints, bool adjoint =
             r.ctas = r.ntz * r.ntx * nb;
             r.side = std::max(r.tz, r.tx);
             const int words = (adjoint ? 8 : 4) * F * (r.tz + r.tx);
-            if (r.ctas > R2_CTAS || words > (adjoint ? 4 : r2_words(nc)) * R2_THREADS) continue;
+            if (r.ctas > sms || words > (adjoint ? 4 : r2_words(nc)) * R2_THREADS) continue;
             const size_t field = sizeof(float) * (size_t)field_floats(F, nc) * (adjoint ? 2 : 1) * R2_NF;
             r.smem = (field + 15) / 16 * 16 + (size_t)npoints * (sizeof(int4) + sizeof(float));
             // fewest cells a thread, then words a thread, then CTAs
@@ -1041,15 +1040,15 @@ static Res2d resident2d_shape(const Grid &g, int nb, int npoints, bool adjoint =
 }
 
 // Resident launches for the nb shots of a run: how many shots a launch takes
-// (r.shots; the launches follow one another), or ctas = 0 where the ordinary
-// launches take them all together in less time.
-Res2d resident2d_plan(const Grid &g, int nb, int npoints)
+// (r.shots; the launches follow one another) on `sms` SMs, or ctas = 0 where
+// the ordinary launches take them all together in less time.
+Res2d resident2d_plan(const Grid &g, int nb, int npoints, int sms)
 {
     Res2d best;
     memset(&best, 0, sizeof best);
     double best_us = 0.0;
     for (int n = nb; n >= 1; n--) {
-        Res2d r = resident2d_shape(g, n, npoints);
+        Res2d r = resident2d_shape(g, n, npoints, std::min(sms, R2_CTAS), false);
         if (!r.ctas) continue;
         r.shots = n;
         const double us = ((nb + n - 1) / n) * resident2d_step_us(r, g.L);
@@ -1064,13 +1063,13 @@ Res2d resident2d_plan(const Grid &g, int nb, int npoints)
 // 5.0 / 16.4, 300 x 400 order 8 7.5 / 16.6, 5 shots of 200 x 200 14.8 / 19.1
 // (two launches), 8 shots of 100 x 150 order 4 11.8 / 13.6; ordinary alone:
 // 4 shots of 240 x 480 25.8.
-Res2d resident2d_adj_plan(const Grid &g, int nb, int npoints)
+Res2d resident2d_adj_plan(const Grid &g, int nb, int npoints, int sms)
 {
     Res2d best;
     memset(&best, 0, sizeof best);
     double best_us = (g.F == 2 ? 12.0 : 15.5) + 2.3e-5 * nb * (double)g.nz * g.nx;
     for (int n = nb; n >= 1; n--) {
-        Res2d r = resident2d_shape(g, n, npoints, true);
+        Res2d r = resident2d_shape(g, n, npoints, std::min(sms, R2_CTAS), true);
         if (!r.ctas) continue;
         r.shots = n;
         const double step = g.F == 2 ? (r.nc == 1 ? 4.1 : 5.5) : r.nc == 1 ? 5.0 : 7.5;
@@ -1088,7 +1087,7 @@ int64_t resident2d_bytes(const Grid &g, int batch)
     int64_t b = 0;
     for (int nb = 1; nb <= batch; nb++)
         for (bool adjoint : {false, true})
-            b = std::max(b, (int64_t)sizeof(u64) * resident2d_words(resident2d_shape(g, nb, 0, adjoint), adjoint));
+            b = std::max(b, (int64_t)sizeof(u64) * resident2d_words(resident2d_shape(g, nb, 0, R2_CTAS, adjoint), adjoint));
     return b;
 }
 

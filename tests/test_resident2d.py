@@ -142,3 +142,76 @@ def test_resident_unstable_run_is_reported(cuda_device, monkeypatch):
     for p in _plans(cfg, model):
         with pytest.raises(SeisCLEngineError, match="unstable"):
             p.forward(acq["src_pos"], acq["src"], acq["rec_pos"], ["vx"])
+
+
+def _fwi(p, shots):
+    d = p.forward_batch(shots, ["vx", "vz"], save_boundaries=True)
+    p.zero_gradient()
+    p.adjoint_batch(shots, d)
+    return {**{"%s%d" % (k, i): v for i, s in enumerate(d) for k, v in s.items()}, **p.gradient(transform=False)}
+
+
+@pytest.mark.gpu
+def test_refused_launches_take_the_ordinary_loop(cuda_device):
+    """A cooperative launch that the driver refuses (an error code made on
+    the host): the call runs on the ordinary loop, and so do the plan's later
+    ones, with the same bits."""
+    cfg, model, acq = make_case(nd=2, nz=60, nx=71, nt=300, nab=8, freesurf=0)
+    shots = [(acq["src_pos"], acq["src"], acq["rec_pos"])] * 2
+    want, got = [], []
+    for refuse in ("none", "forward", "adjoint"):
+        p = _plans(cfg, model, batch=2)[0]
+        if refuse == "forward":
+            p.debug_launch(4)
+        d = p.forward_batch(shots, ["vx", "vz"], save_boundaries=True)
+        p.zero_gradient()
+        if refuse == "adjoint":
+            p.debug_launch(4)
+        p.adjoint_batch(shots, d)
+        got.append({**{k: v for k, v in d[1].items()}, **p.gradient(transform=False)})
+        want.append(_fwi(p, shots))
+    for g, w in zip(got[1:], want[1:]):
+        _same(g, got[0])
+        _same(w, want[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sms", [0, 5, 60, 1000])
+def test_fewer_sms(sms, cuda_device, monkeypatch):
+    """What a process with part of the device plans: fewer tiles, or none."""
+    cfg, model, acq = make_case(nd=2, nz=100, nx=150, nt=80, nab=16, fdorder=4, freesurf=0)
+    shots = [(acq["src_pos"], acq["src"] * (1 + b), acq["rec_pos"]) for b in range(2)]
+    want = _fwi(_plans(cfg, model, batch=2)[1], shots)
+    monkeypatch.setenv("SEISCL_B200_RESIDENT_SMS", str(sms))
+    _same(_fwi(_plans(cfg, model, batch=2)[0], shots), want)
+
+
+@pytest.mark.gpu
+def test_wait_that_runs_out(cuda_device):
+    """A tile whose neighbour never sends gives up after its bound, the host
+    reads it, and the plan goes on working."""
+    from seiscl_b200.engine import SeisCLEngineError
+
+    cfg, model, acq = make_case(nd=2, nz=100, nx=90, nt=60, nab=8)
+    p = _plans(cfg, model)[0]
+    want = p.forward(acq["src_pos"], acq["src"], acq["rec_pos"], ["vx"])
+    with pytest.raises(SeisCLEngineError, match="time bound"):
+        p.debug_launch(5)
+    _same(p.forward(acq["src_pos"], acq["src"], acq["rec_pos"], ["vx"]), want)
+
+
+@pytest.mark.gpu
+def test_plans_on_threads(cuda_device):
+    """Resident loops of several plans on threads of their own, forward and
+    adjoint, small grids and one of the whole chip: the bits of each alone."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    cases = [make_case(nd=2, nz=60, nx=71, nt=300, nab=8, freesurf=0, seed=1),
+             make_case(nd=2, nz=302, nx=391, nt=120, nab=20, freesurf=0, seed=2),
+             make_case(nd=2, nz=100, nx=150, nt=400, nab=16, fdorder=4, freesurf=0, seed=3)]
+    jobs = [(_plans(cfg, model)[0], [(acq["src_pos"], acq["src"], acq["rec_pos"])]) for cfg, model, acq in cases]
+    want = [_fwi(*j) for j in jobs]
+    with ThreadPoolExecutor(len(jobs)) as pool:
+        for _ in range(3):
+            for g, w in zip(pool.map(lambda j: _fwi(*j), jobs), want):
+                _same(g, w)

@@ -167,7 +167,10 @@ const char *sfd_last_error(const sfd_plan *plan);
  * gradient sums for back_prop_type 1; the transforms at nfreqs frequencies
  * for back_prop_type 2).  Computed from the configuration alone (no device
  * call), for admission control by a caller that shares one device among
- * many plans.  No counterpart in the reference. */
+ * many plans.  Not in it: staging that sfd_set_model and sfd_get_gradient give
+ * back before they return, up to 100 MB where there is room; on a full device a
+ * new model goes through the plan's own fields and a gradient through 200 kB.
+ * No counterpart in the reference. */
 int sfd_footprint(const sfd_config *cfg, int gradient, int nsrc, int64_t nrec_sel, int nfreqs, int64_t *bytes);
 /* Device bytes the plan holds now (every allocation it made and keeps). */
 int64_t sfd_plan_device_bytes(const sfd_plan *plan);
@@ -371,7 +374,8 @@ int64_t sfd_debug_copy(sfd_plan *plan, int kind, int id, float *dst, int64_t cap
  * surface_adj, src/surface2D_adj.cl:35-148, src/surface3D_adj.cl:29-116) --
  * returning after it finished; 4 makes the next resident 2D launch count as
  * refused by the driver, 5 runs one resident 2D step without its last tile and
- * reports the waits that run out.  No counterpart in the reference. */
+ * reports the waits that run out, 16 + n makes the next n attempts to allocate
+ * staging fail (before sfd_set_model too).  No counterpart in the reference. */
 int64_t sfd_debug_load(sfd_plan *plan, int kind, int id, const float *src, int64_t n);
 int sfd_debug_launch(sfd_plan *plan, int which);
 

@@ -1153,6 +1153,7 @@ extern "C" int sfd_plan_create(const sfd_config *cfg, sfd_plan **out)
     p->d_words = nullptr;
     p->words_bytes = 0;
     p->refuse_resident = false;
+    p->refuse_staging = 0;
     p->sms = resident_sms(p->device);
     p->d_fsync = nullptr;
     p->dev_bytes = 0;
@@ -1281,9 +1282,10 @@ extern "C" void sfd_plan_destroy(sfd_plan *p)
 extern "C" const char *sfd_last_error(const sfd_plan *p) { return p ? p->err.c_str() : "null plan"; }
 
 namespace {
-// scratch of sample_model: up to 8192 sampled cells (index, two values) and nx
-// receivers' cells (index, three values)
-int64_t sample_bytes(const Grid &g) { return 8192 * 16 + (int64_t)g.nx * 24; }
+// sample_model: its sampling step, and its scratch: the sampled cells (index, two
+// values) and nx receivers' cells (index, three values)
+int64_t sample_step(const Grid &g) { return std::max<int64_t>(1, user_cells(g) / 4096); }
+int64_t sample_bytes(const Grid &g) { return (user_cells(g) / sample_step(g) + 1) * 16 + (int64_t)g.nx * 24; }
 
 // A host copy of a transformed parameter [nx][(ny)][nz], unscaled
 int host_param(sfd_plan *p, int k, const float **out)
@@ -1344,7 +1346,7 @@ int sample_model(sfd_plan *p, char *scratch, int64_t bytes, int *shift)
 {
     const Grid &g = p->g;
     const int nzu = g.nz - g.zpad;
-    const int64_t n = user_cells(g), step = std::max<int64_t>(1, n / 4096);
+    const int64_t n = user_cells(g), step = sample_step(g);
     std::vector<int64_t> at;
     for (int64_t i = 0; i < n; i += step) at.push_back(i / nzu * g.nz + i % nzu);
     const int cnt = (int)at.size();
@@ -1375,9 +1377,51 @@ int sample_model(sfd_plan *p, char *scratch, int64_t bytes, int *shift)
     return SFD_OK;
 }
 
-// checks, transforms and stores the model through `scratch` (room for `planes`
-// x planes of every input and the check record)
-int store_model(sfd_plan *p, const float *const in[5], char *scratch, int planes, int64_t bytes)
+// Staging that a call gives back: what it would like where there is room, half
+// of that and so on down to `least` where the plan fills the device.  Not part
+// of the footprint for that reason.
+struct Staging {
+    sfd_plan *p;
+    char *base = nullptr;
+    int64_t bytes = 0;
+    bool borrowed = false;
+    bool take(int64_t want, int64_t least)
+    {
+        for (bytes = want;; bytes = std::max(bytes / 2, least)) {
+            cudaError_t e;
+            if (p->refuse_staging > 0) p->refuse_staging--;
+            else if ((base = (char *)dalloc_raw(p, bytes, &e))) return true;
+            if (bytes <= least) return false;
+        }
+    }
+    // the plan's first wave field, which the next run clears
+    bool borrow(int64_t least)
+    {
+        for (int w = 0; w < NW; w++) {
+            if (!p->f.w[w]) continue;
+            bytes = (int64_t)wave_elem(p->g) * p->g.nvol * p->batch - 256;
+            if (bytes < least) return false;
+            base = (char *)p->f.w[w];
+            base += (256 - (uintptr_t)base % 256) % 256;
+            return borrowed = true;
+        }
+        return false;
+    }
+    void give()
+    {
+        if (base && !borrowed) {
+            cudaStreamSynchronize(p->stream);
+            dfree(p, base, bytes);
+        }
+        base = nullptr;
+        borrowed = false;
+    }
+    ~Staging() { give(); }
+};
+
+// checks, transforms and stores the model through the staging: the check
+// record and as many x planes of every input as it holds
+int store_model(sfd_plan *p, const float *const in[5], Staging &stage, int64_t want, int64_t least)
 {
     const Grid &g = p->g;
     const sfd_config &c = p->cfg;
@@ -1395,8 +1439,15 @@ int store_model(sfd_plan *p, const float *const in[5], char *scratch, int planes
     m.dh = c.dh;
     m.sumu = phase_weights(c, m.wl);
     const int64_t plane = (int64_t)m.ny * m.nz;
-    ModelCheck *check = (ModelCheck *)scratch, found;
-    float *slab = (float *)(scratch + 256);
+    ModelCheck *check, found;
+    float *slab;
+    int planes;
+    auto staged = [&] {
+        check = (ModelCheck *)stage.base;
+        slab = (float *)(stage.base + 256);
+        planes = (int)std::min<int64_t>(g.nx, (stage.bytes - 256) / ((int64_t)sizeof(float) * (c.L > 0 ? 5 : 3) * plane));
+    };
+    staged();
     const float **dst[5] = {&m.a, &m.b, &m.rho, &m.taup, &m.taus};
     auto upload = [&](int x0) {
         m.x0 = x0;
@@ -1427,8 +1478,20 @@ int store_model(sfd_plan *p, const float *const in[5], char *scratch, int planes
     int rc;
     if ((rc = check_cfl(c, mb, mub, p->err))) return rc;
     // the model is accepted: from here on the old one is gone
+    bool uploaded = planes >= m.nx;
     if (!p->model_set) {
-        if ((rc = alloc_model(p))) return rc;
+        // a plan that fits only without the staging beside it has its arrays first
+        const size_t held = p->allocs.size();
+        if ((rc = alloc_model(p)) == SFD_ERR_MEMORY) {
+            for (; p->allocs.size() > held; p->allocs.pop_back()) dfree(p, p->allocs.back().first, p->allocs.back().second);
+            stage.give();
+            if ((rc = alloc_model(p))) return rc;
+            if (!stage.take(want, least) && !stage.borrow(least)) return fail(p, SFD_ERR_MEMORY, "model staging does not fit in device memory");
+            staged();
+            uploaded = false;
+            CKC(cudaMemsetAsync(check, 0, sizeof *check, st));
+        }
+        if (rc) return rc;
         if ((rc = upload_constants(p))) return rc;
     }
     for (int k = 0; k < NPAR; k++) p->hp[k].clear();
@@ -1437,7 +1500,7 @@ int store_model(sfd_plan *p, const float *const in[5], char *scratch, int planes
     ModelOut o;
     for (int k = 0; k < NPAR; k++) o.p[k] = (float *)p->f.p[k];
     for (int x0 = 0; x0 < m.nx; x0 += m.xs) {
-        if (planes < m.nx) CKC(upload(x0));
+        if (!uploaded) CKC(upload(x0));
         launch_model_params(m, o, check, st);
     }
     CKC(cudaMemcpyAsync(&found, check, sizeof found, cudaMemcpyDeviceToHost, st));
@@ -1448,7 +1511,7 @@ int store_model(sfd_plan *p, const float *const in[5], char *scratch, int planes
     p->surf_mu_zero = found.top_mu_zero != 0;
     // FP16 stores keep velocities as v * 2^b and stresses as s * 2^a with
     // b - a ~ log2 of the impedance, so both stay near the same magnitude
-    if ((rc = sample_model(p, scratch, bytes, &p->bshift))) return rc;
+    if ((rc = sample_model(p, stage.base, stage.bytes, &p->bshift))) return rc;
     if (g.fhalf) {
         // FP16 wave fields: the moduli carry 2^-kshift and the buoyancies
         // 2^kshift (exact power-of-two scalings of the FP32 parameters)
@@ -1477,17 +1540,19 @@ extern "C" int sfd_set_model(sfd_plan *p, const float *const *params)
     if (!(in[2][0] > 0)) return fail(p, SFD_ERR_ARG, "rho must be positive everywhere");
     if (c.param_type < 0 || c.param_type > 2) return fail(p, SFD_ERR_UNSUPPORTED, "param_type must be 0, 1 or 2");
     if (c.L > 0 && (!in[3] || !in[4])) return fail(p, SFD_ERR_ARG, "taup and taus are required when L > 0");
-    // a slab of x planes at a time: the scratch stays below 100 MB (or two
-    // planes), and returns to the pool
+    // a slab of x planes at a time: the staging stays below 100 MB (or two planes)
     const int64_t plane = (int64_t)(g.nz - g.zpad) * g.ny, narr = c.L > 0 ? 5 : 3;
-    const int planes = (int)std::min<int64_t>(g.nx, std::max<int64_t>(2, (5 << 20) / plane));
-    const int64_t bytes = 256 + std::max<int64_t>(sizeof(float) * narr * plane * planes, sample_bytes(g));
-    cudaError_t e;
-    char *scratch = (char *)dalloc_raw(p, bytes, &e);
-    if (!scratch) return fail(p, SFD_ERR_MEMORY, "model staging does not fit in device memory");
-    const int rc = store_model(p, in, scratch, planes, bytes);
+    auto bytes = [&](int64_t planes) {
+        return 256 + std::max<int64_t>(sizeof(float) * narr * plane * std::min<int64_t>(planes, g.nx), sample_bytes(g));
+    };
+    const int64_t want = bytes(std::max<int64_t>(2, (5 << 20) / plane)), least = bytes(2);
+    Staging stage{p};
+    if (!stage.take(want, least) && !(p->model_set && stage.borrow(least)))
+        return fail(p, SFD_ERR_MEMORY, "model staging does not fit in device memory");
+    const bool borrowed = stage.borrowed;
+    const int rc = store_model(p, in, stage, want, least);
+    if (borrowed) p->have_forward = false;   // a refused model, too, has been staged over the fields
     cudaStreamSynchronize(p->stream);
-    dfree(p, scratch, bytes);
     return rc;
 }
 
@@ -2059,14 +2124,16 @@ extern "C" int sfd_get_gradient(sfd_plan *p, int transform, float *g0, float *g1
     }
     // the result passes through a bounded staging area: a plan whose stores
     // fill the device still returns its gradient
-    const int64_t chunk = std::min<int64_t>(o.n, 8 << 20);
-    cudaError_t e;
-    float *stage = (float *)dalloc_raw(p, sizeof(float) * 3 * chunk, &e);
-    if (!stage) return fail(p, SFD_ERR_MEMORY, "gradient staging does not fit in device memory");
+    Staging stage{p};
+    const int64_t cell = 3 * sizeof(float);
+    if (!stage.take(cell * std::min<int64_t>(o.n, 8 << 20), cell * std::min<int64_t>(o.n, 1 << 14)))
+        return fail(p, SFD_ERR_MEMORY, "gradient staging does not fit in device memory");
+    const int64_t chunk = stage.bytes / cell;
+    cudaError_t e = cudaSuccess;
     float *const host[3] = {g0, g1, g2};
     for (o.first = 0; o.first < o.n && e == cudaSuccess; o.first += chunk) {
         o.count = std::min(chunk, o.n - o.first);
-        for (int k = 0; k < 3; k++) o.out[k] = stage + k * chunk;
+        for (int k = 0; k < 3; k++) o.out[k] = (float *)stage.base + k * chunk;
         launch_gradient_out(o, p->stream);
         e = cudaGetLastError();
         for (int k = 0; k < 3 && e == cudaSuccess; k++)
@@ -2074,7 +2141,6 @@ extern "C" int sfd_get_gradient(sfd_plan *p, int transform, float *g0, float *g1
                 e = cudaMemcpyAsync(host[k] + o.first, o.out[k], sizeof(float) * o.count, cudaMemcpyDeviceToHost,
                                     p->stream);
     }
-    dfree(p, stage, sizeof(float) * 3 * chunk);
     if (e == cudaSuccess) e = cudaStreamSynchronize(p->stream);
     if (e != cudaSuccess) return fail(p, SFD_ERR_CUDA, std::string("gradient: ") + cudaGetErrorString(e));
     return SFD_OK;
@@ -2219,6 +2285,7 @@ extern "C" int64_t sfd_debug_load(sfd_plan *p, int kind, int id, const float *sr
 extern "C" int sfd_debug_launch(sfd_plan *p, int which)
 {
     if (!p) return SFD_ERR_ARG;
+    if (which >= 16 && which < 80) { p->refuse_staging = which - 16; return SFD_OK; }
     if (!p->model_set) return fail(p, SFD_ERR_STATE, "sfd_set_model must be called first");
     cudaStream_t st = p->stream;
     p->g.nb = 1;

@@ -177,6 +177,7 @@ struct sfd_plan {
     int64_t words_bytes;
     int sms;                // SMs the process has for them; 0 once a cooperative launch was refused
     bool refuse_resident;   // tests: the next one counts as refused
+    int refuse_staging;     // tests: so many staging allocations count as failed
     int *d_fsync;           // fused 3D step: ticket counter + one flag per work unit
     // checkpointed gradients (cfg.checkpoint = K > 0)
     char *d_snap;           // [nseg] snapshots: wave fields, memory variables (store type; FP16 wave-field

@@ -430,7 +430,8 @@ class Plan:
     def debug_launch(self, which: int) -> None:
         """Run one kernel on the plan's arrays: 0 velocity update, 1 stress
         update, 2 free surface, 3 free-surface adjoint, 5 a resident 2D
-        step short of a tile; 4 refuses the next resident 2D launch (tests)."""
+        step short of a tile; 4 refuses the next resident 2D launch, 16 + n
+        the next n staging allocations (tests)."""
         self._check(self.lib.sfd_debug_launch(self.h, int(which)))
 
     def debug_array(self, kind: int, idx: int, n: int) -> np.ndarray:

@@ -764,7 +764,9 @@ def main():
     d2h = len(outs) * rp.shape[0] * w["nt"] * 4
     checks = (w["nt"] + 63) // 64   # finite checks of the instability detection
     if w["nd"] == 3:   # first sources; velocity and stress (or the fused step), [surface], receivers with the next sources
-        sep_surface = 1 if w["freesurf"] and fam != "vector" and not fused else 0
+        # the 4-cell kernels, whatever the rows, and the fused step carry the surface
+        folded = fused or args.kernels == "fast" or (args.kernels in ("vector", "async") and w["nz"] % 4 == 0)
+        sep_surface = 1 if w["freesurf"] and not folded else 0
         launches_per_shot = 1 + w["nt"] * ((1 if fused else 2) + sep_surface + 1) + checks
     elif args.kernels == "fast" and args.fields == "fp32" and cells <= 250000:   # first sources; segments of 256 resident steps
         launches_per_shot = 1 + (w["nt"] + 255) // 256

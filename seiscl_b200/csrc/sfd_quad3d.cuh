@@ -587,20 +587,6 @@ __device__ __forceinline__ void cpml_s3d_q4(const Grid &g, const Fields &f, int 
     }
 }
 
-// Stress and memory-variable update of four z cells (the arithmetic of
-// k_s3d_stream per cell).  The per-cell work runs in two phases -- normal
-// stresses (sxx, syy, szz with rxx, ryy, rzz) then shear stresses (sxy, syz,
-// sxz with rxy, ryz, rxz) -- each loading only its own memory variables and
-// parameters, so the live state fits in registers; the components are
-// independent, so the split changes no result.
-//
-// surf: the free surface of the same step follows the update in registers
-// (the fused step kernel; k_surf3d's arithmetic at z = F, forward direction):
-// the quad at gz0 = F zeroes szz and rzz there, corrects sxx, syy, rxx, ryy
-// with the velocity derivatives of the update (CPML-corrected as k_surf3d
-// forms them) and writes the images szz(F-m) = -szz(F+m) for m = 1..3 and
-// sxz(F-m) = -sxz(F+m-1), syz(F-m) = -syz(F+m-1) for m = 1..4; the quad at
-// gz0 = F+4 writes szz(F-4) = -szz(F+4).
 // the strains (vxx, vyy, vzz) the free surface takes at the top cell iv, as
 // k_surf3d forms them: derivatives times 1/K plus the memory of this step
 template <int F, class T>
@@ -665,6 +651,18 @@ __device__ __forceinline__ void bnd_save(const Grid &g, const BndQuad &q, int w,
         if (q.m[j] >= 0) ((TB *)q.b->p[w])[q.at + q.m[j]] = from_f<TB>(v.v[j] * g.bsc[w]);
 }
 
+// Stress and memory-variable update of four z cells (the arithmetic of
+// k_s3d_stream per cell).  The per-cell work runs in two phases -- normal
+// stresses (sxx, syy, szz with rxx, ryy, rzz) then shear stresses (sxy, syz,
+// sxz with rxy, ryz, rxz) -- each loading only its own memory variables and
+// parameters, so the live state fits in registers; the components are
+// independent, so the split changes no result.
+//
+// surf: the free surface of the same step follows the update in registers
+// (k_surf3d at z = F, forward direction): the quad at gz0 = F zeroes szz and
+// rzz there, corrects sxx, syy, rxx, ryy and writes the images
+// szz(F-m) = -szz(F+m), sxz(F-m) = -sxz(F+m-1) and syz(F-m) = -syz(F+m-1) that
+// its own cells give; at order 8 the quad at gz0 = F+4 writes szz(F-4).
 template <int R, int L, class T, class TR = T, class TB = void>
 __device__ __forceinline__ void s_normal_q4(const Grid &g, const Fields &f, int gz0, int gy, int gx, i64 iv, i64 ip,
                                             const Q4 &vxx, const Q4 &vyy, const Q4 &vzz, Surf surf = SURF_NONE,
@@ -1014,16 +1012,15 @@ static void quad_update_s_l(const Grid &g, const Fields &f, dim3 g4, dim3 b4, cu
     // the stream prefetch pays where memory variables add per-cell
     // streams: 256^3, L=2: 0.654 ms against 0.706; elastic (L=0):
     // 0.376 against 0.366 without it.  kernels 5 keeps k_s3d_q4.
-    const bool pf = g.nb == 1 && g.kernels == 0 && L > 0;
-    if (g.fhalf) {
-        if (pf) k_s3d_q4_pf<R, L, __half><<<g4, b4, 0, st>>>(g, f, surf);
-        else k_s3d_q4<R, L, __half><<<g4, b4, 0, st>>>(g, f, surf);
-        return;
-    }
     if constexpr (L > 0) {
-        if (pf && g.rhalf) { k_s3d_q4_pf<R, L, float, __half><<<g4, b4, 0, st>>>(g, f, surf); return; }
-        if (pf) { k_s3d_q4_pf<R, L, float><<<g4, b4, 0, st>>>(g, f, surf); return; }
+        if (g.nb == 1 && g.kernels == 0) {
+            if (g.fhalf) k_s3d_q4_pf<R, L, __half><<<g4, b4, 0, st>>>(g, f, surf);
+            else if (g.rhalf) k_s3d_q4_pf<R, L, float, __half><<<g4, b4, 0, st>>>(g, f, surf);
+            else k_s3d_q4_pf<R, L, float><<<g4, b4, 0, st>>>(g, f, surf);
+            return;
+        }
     }
+    if (g.fhalf) { k_s3d_q4<R, L, __half><<<g4, b4, 0, st>>>(g, f, surf); return; }
     MB_DISPATCH(g, k_s3d_q4<R, L, float, MBV><<<g4, b4, 0, st>>>(g, f, surf))
 }
 

@@ -16,6 +16,10 @@ CASES = [
     (dict(nd=3, nz=28, ny=25, nx=21), 2, dict(fdorder=4)),
     (dict(nd=2, nz=2306, nx=2411, L=1), 0, {}),       # two slabs
     (dict(nd=3, nz=1602, ny=1650, nx=3), 0, {}),      # slabs of two planes
+    (dict(nd=21, nz=38, nx=45), 0, {}),               # SH
+    (dict(nd=21, nz=40, nx=31), 2, {}),
+    (dict(nd=22, nz=42, nx=33), 1, {}),               # acoustic
+    (dict(nd=22, nz=42, nx=33, L=1), 0, {}),
 ]
 
 

@@ -104,19 +104,30 @@ def test_gradient(kw, how, cuda_device):
 @pytest.mark.gpu
 @pytest.mark.parametrize("kw", [CASES[0], CASES[2], CASES[3]], ids=[IDS[0], IDS[2], IDS[3]])
 def test_fp16_fields(kw, cuda_device):
-    """The same FP16 storage in both layouts: one rounding of 2^-11 a step on
-    fields that differ in the last FP32 bit, far below the storage's own error."""
+    """FP16 storage against FP32 storage on the same layout, by the criterion
+    of tests/test_gpu_parity.py, and against FP16 storage on rows without
+    dummy cells (kernels "general"): there both sides round the same FP32
+    values to FP16 in every step, but for the few whose last FP32 bit differs
+    and falls on a tie, each 2^-11 of its value, so well below the 2^-11 that
+    storage itself costs a trace (3e-3 measured against FP32)."""
     from seiscl_b200.engine import Plan
 
     cfg, model, acq = _case(dict(kw, nt=150))
-    got = []
-    for field in ("fp16", "fp32"):
-        p = Plan(dataclasses.replace(engine_config(cfg), field_precision=field))
+    got = {}
+    for field, kernels in (("fp16", "fast"), ("fp32", "fast"), ("fp16", "general")):
+        p = Plan(dataclasses.replace(engine_config(cfg), field_precision=field, kernels=kernels))
         p.set_model(model["vp"], model["vs"], model["rho"], model["taup"], model["taus"])
-        got.append(p.forward(acq["src_pos"], acq["src"], acq["rec_pos"], OUTS))
-    num = sum(float(((got[0][n].astype(np.float64) - got[1][n]) ** 2).sum()) for n in OUTS)
-    den = sum(float((got[1][n].astype(np.float64) ** 2).sum()) for n in OUTS)
-    assert 0 < den and num / den < 1e-3   # the criterion of tests/test_gpu_parity.py
+        got[field, kernels] = p.forward(acq["src_pos"], acq["src"], acq["rec_pos"], OUTS)
+
+    def off(a, b):
+        num = sum(float(((a[n].astype(np.float64) - b[n]) ** 2).sum()) for n in OUTS)
+        return num / sum(float((b[n].astype(np.float64) ** 2).sum()) for n in OUTS)
+
+    fp16, fp32, plain = got["fp16", "fast"], got["fp32", "fast"], got["fp16", "general"]
+    assert np.abs(fp32["vz"]).max() > 0
+    print("FP16 against FP32, against unpadded FP16 (squares):", off(fp16, fp32), off(fp16, plain))
+    assert off(fp16, fp32) < 1e-3
+    assert off(fp16, plain) <= 2.0 ** -22
 
 
 def test_footprint_counts_dummy_rows():

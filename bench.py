@@ -648,7 +648,7 @@ def main():
                          "fp16_mem: memory variables alone in FP16")
     ap.add_argument("--rate", type=float, default=20.0, help="serving: request arrival rate (1/s)")
     ap.add_argument("--workers", type=int, default=8,
-                    help="serving: worker threads (8: 18.8 shots/s against 18.0 with 4 on the 60-request mix)")
+                    help="serving: worker threads (8: 24.7 shots/s on the 60-request mix)")
     ap.add_argument("--no-plain", action="store_true", help="serving: skip the plain one-at-a-time arm")
     ap.add_argument("--batch", type=int, default=0, help="gradient workloads: shots per step (0: 8 in 2D, 1 in 3D)")
     ap.add_argument("--checkpoint", type=int, default=0,

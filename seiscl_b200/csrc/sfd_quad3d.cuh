@@ -458,8 +458,8 @@ __global__ void __launch_bounds__(128) k_v3d_q4(Grid g, Fields f)
 
 // The single-shot FP32 launch asks for NB resident CTAs per SM: 4, or 6 where
 // that (and not 4) holds the whole launch in one wave (72 x 64 x 80: 12.5 us
-// against 14.7).  4 (at most 128 registers, from 136, with a 24-byte spill):
-// 0.333 ms against 0.345 at 256^3 L=2 on a B200, 0.285 since.  5 CTAs (102
+// against 14.7).  4 (at most 128 registers, from 136, with a 36-byte spill):
+// 0.333 ms against 0.345 at 256^3 L=2 on a B200, 0.295 since.  5 CTAs (102
 // registers) is slower again, and a component-at-a-time update with 80
 // registers slower still (0.37 ms): the kernel is bound by the stencil loads
 // each thread keeps in flight.  CTAs of 256 or 512 threads: 0.323-0.343 ms.
@@ -945,8 +945,8 @@ __global__ void __launch_bounds__(128, 5) k_s3d_q4_bnd(Grid g, Fields f, BndSlot
 // with programmatic serialization itself, with the prefetch ahead of its
 // wait, it has to read the velocities with plain loads (a read-only-path load
 // counts as invariant, and the compiler may move it above the wait): 0.637 ms
-// against 0.622, and 919 us a step against 911; 122 x 131 x 117, L = 1 143.9
-// against 142.9.  256 and 384 threads a CTA: 0.686-0.721 ms.
+// against 0.622, and 919 us a step against 911 (0.625 and 919 with the general
+// kernels' roundings); 122 x 131 x 117, L = 1 143.9 against 142.9.  256 and 384 threads a CTA: 0.686-0.721 ms.
 // TR: storage type of the memory variables (FP16 under FP32 wave fields
 // with Grid::rhalf)
 template <int R, int L, class T, class TR = T>
